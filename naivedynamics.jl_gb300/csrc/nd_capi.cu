@@ -140,7 +140,7 @@ static nd_status spec_ok(const nd_bvh_spec* s) {
 // Upload host positions and build the tree on the context's scratch buffers.
 static nd_status tree_from_host(Ctx* c, const float* xyz, const nd_bvh_spec* s, int32_t order,
                                 int32_t boxes, int64_t nkeys, bool overwrite_root,
-                                TreeBuffers* t) {
+                                TreeBuffers* t, bool leaves_only = false) {
     const int32_t n = s->atom_count;
     nd_status st = ensure(c, c->xyz, 3 * sizeof(float) * (size_t)n);
     if (st) return st;
@@ -148,7 +148,13 @@ static nd_status tree_from_host(Ctx* c, const float* xyz, const nd_bvh_spec* s, 
                                     cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "position upload");
     return build_tree(c, (const float*)c->xyz.p, n, s->neighbor_distance, s->atomsperleaf, order,
-                      boxes, nkeys, overwrite_root, t);
+                      boxes, nkeys, overwrite_root, t, leaves_only);
+}
+
+// The unordered emission exists for leaves of four atoms; any other request is
+// served in order.
+static bool unordered_emission(const nd_bvh_spec* s, int32_t mode) {
+    return mode == ND_PAIRS_UNORDERED && s->atomsperleaf == 4;
 }
 
 static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec* s,
@@ -170,11 +176,12 @@ nd_status pairs_common(Ctx* c, const nd_bvh_spec* s, int32_t order, int32_t mode
     const int32_t boxes = (kind == 0) ? ND_BOX_LEAF : ND_BOX_ATOM;
     if (kind == 0 && n - 1 < 2 * nL - 1) return ND_ERR_SPEC;  // leafTreeData needs apl >= 2
     TreeBuffers t;
+    const bool leaves_only = kind == 0 && !unordered_emission(s, mode);
     if (host) {
-        st = tree_from_host(c, xyz, s, order, boxes, 2LL * nL - 1, false, &t);
+        st = tree_from_host(c, xyz, s, order, boxes, 2LL * nL - 1, false, &t, leaves_only);
     } else {
         st = build_tree(c, xyz, n, s->neighbor_distance, s->atomsperleaf, order, boxes,
-                        2LL * nL - 1, false, &t);
+                        2LL * nL - 1, false, &t, leaves_only);
     }
     if (st) return st;
     return pairs_from_tree(c, t, s, mode, kind, host, pi, pj, pd, capacity, count, criterion);
@@ -189,7 +196,7 @@ static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec
     const float r = s->neighbor_distance;
     const float r2 = pair_threshold(r, criterion);
     int64_t total = 0;
-    if (kind == 0 && mode == ND_PAIRS_UNORDERED && s->atomsperleaf == 4) {
+    if (kind == 0 && unordered_emission(s, mode)) {
         if (host) {
             int64_t devcap = (int64_t)(c->pairs_i.bytes / sizeof(int32_t));
             devcap = std::min(devcap, (int64_t)(c->pairs_d.bytes / sizeof(float)));
@@ -213,20 +220,33 @@ static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec
             return total > capacity ? ND_NEED_REALLOC : ND_OK;
         }
     } else {
-        if ((st = count_pairs(c, t, r2, kind, &total))) return st;
+        // count and write are enqueued together: the write pass reads the total
+        // on the device and writes nothing that does not fit
+        int64_t* total_dev = (int64_t*)(c->d_err + 4);
+        if ((st = count_pairs(c, t, r, r2, kind, total_dev))) return st;
+        int64_t devcap = capacity;
+        if (host) {
+            devcap = (int64_t)(std::min({c->pairs_i.bytes, c->pairs_j.bytes, c->pairs_d.bytes}) /
+                               sizeof(int32_t));
+            devcap = std::min(devcap, capacity);
+        }
+        if (devcap > 0 &&
+            (st = write_pairs(c, t, r, r2, kind, total_dev, devcap,
+                              host ? (int32_t*)c->pairs_i.p : pi, host ? (int32_t*)c->pairs_j.p : pj,
+                              host ? (float*)c->pairs_d.p : pd)))
+            return st;
+        if ((st = sync_and_check(c, "pair list"))) return st;
+        memcpy(&total, c->h_err + 4, sizeof(total));
         *count = total;
         if (total > capacity) return ND_NEED_REALLOC;
-        if (total == 0) return ND_OK;
-        if (host) {
+        if (!host) return ND_OK;
+        if (total > devcap) {
             if ((st = ensure(c, c->pairs_i, sizeof(int32_t) * (size_t)total))) return st;
             if ((st = ensure(c, c->pairs_j, sizeof(int32_t) * (size_t)total))) return st;
             if ((st = ensure(c, c->pairs_d, sizeof(float) * (size_t)total))) return st;
-            if ((st = write_pairs(c, t, r2, kind, (int32_t*)c->pairs_i.p, (int32_t*)c->pairs_j.p,
-                                  (float*)c->pairs_d.p)))
+            if ((st = write_pairs(c, t, r, r2, kind, total_dev, total, (int32_t*)c->pairs_i.p,
+                                  (int32_t*)c->pairs_j.p, (float*)c->pairs_d.p)))
                 return st;
-        } else {
-            if ((st = write_pairs(c, t, r2, kind, pi, pj, pd))) return st;
-            return sync_and_check(c, "pair write");
         }
     }
     // host copy-out

@@ -18,8 +18,10 @@ struct MDEngine;
 // ------------------------------------------------------------------ errors
 
 // Device error word layout: [0] first error status, [1] its info (an index),
-// [2] largest per-atom neighbour count seen (overflow diagnostics), [3] spare.
-constexpr int kErrWords = 4;
+// [2] largest per-atom neighbour count seen (overflow diagnostics), [3] spare,
+// [4, 5] the pair count of the call (int64), which so reaches the host with
+// the error word in one copy.
+constexpr int kErrWords = 6;
 
 __device__ __forceinline__ void set_error(int32_t* err, int32_t code, int32_t info) {
     if (atomicCAS(err, 0, code) == 0) atomicExch(err + 1, info);
@@ -178,10 +180,11 @@ nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32
                        int32_t* iota, const float* frame = nullptr);
 // Stable LSD radix sort of (codes, vals) on `bits` low bits; results in codes/vals.
 nd_status radix_sort_pairs(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int bits);
-// Full tree pipeline: codes -> sort -> gather -> leaf boxes -> Apetrei build.
+// Full tree pipeline: codes -> sort -> gather -> leaf boxes -> Apetrei build
+// (leaves_only: no internal nodes, all the ordered pair list needs).
 nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t apl,
                      int32_t order, int32_t boxes, int64_t nkeys, bool overwrite_root,
-                     TreeBuffers* out);
+                     TreeBuffers* out, bool leaves_only = false);
 // Tree of new positions in the order (1-based original indices idx1) and with
 // the sorted codes of an earlier build: same topology, new boxes (device
 // arrays); the leaf-box half-width is r/2 (leafTreeData).
@@ -245,7 +248,8 @@ const char* md_last_error(MDEngine* m);
 nd_status forces_pairs(Ctx* c, const nd_md_params* p, int32_t n, const double* x,
                        const double* q, const int32_t* pi, const int32_t* pj, int64_t np,
                        float* f, double* energy);
-// Two-phase ordered emission: count (computes per-query offsets, syncs) then write.
+// Two-phase ordered emission: count (per-query offsets, the total on the
+// device) then write.
 // Squared-distance threshold of a pair criterion (ND_CRIT_*).
 float pair_threshold(float r, int32_t criterion);
 // Bug-compatible force_lennardjones! (kind 0) / force_coulomb! (kind 1) over a
@@ -258,9 +262,10 @@ nd_status collect_objects(Ctx* c, const nd_collector* cl, uint64_t seed, float* 
 // simulate! as written over the all-pairs list (host arrays in and out).
 nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x, float* v,
                           float* force, const float* mass, const float* q, float* poslog);
-nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r2, int kind, int64_t* total);
-nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r2, int kind, int32_t* pi, int32_t* pj,
-                      float* pd);
+nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
+                      int64_t* total_dev);
+nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
+                      const int64_t* total_dev, int64_t cap, int32_t* pi, int32_t* pj, float* pd);
 nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_t* pi,
                          int32_t* pj, float* pd, int64_t capacity, int64_t* total);
 

@@ -101,7 +101,7 @@ extern "C" nd_status nd_leaf_pairs_noalloc_dev(const float* xyz, const nd_bvh_sp
     c.no_alloc = true;
     cudaGetDevice(&c.device);
     c.stream = (cudaStream_t)stream;
-    int32_t h_err[nd::kErrWords] = {0, 0, 0, 0};
+    int32_t h_err[nd::kErrWords] = {};
     c.h_err = h_err;
     unsigned char* cur = (unsigned char*)base;
     carve(c.codes, cur, kCodesB);
