@@ -26,11 +26,14 @@
 // sorted by i (stable, so each atom keeps its list order) and one thread per
 // atom adds its run.  Coulomb: every update reads the result of earlier ones
 // through force[i] and force[j]; for an arbitrary list the recurrence runs on
-// one thread in list order, for the all-pairs order of unique_pairs it splits
-// into levels of independent pairs (compat_simulate).
+// one thread in list order, for the all-pairs order of unique_pairs its columns
+// flow through bands of rows (compat_simulate).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "nd_internal.cuh"
 
@@ -127,85 +130,440 @@ __global__ void k_iota(int32_t* v, int64_t n) {
 // ------------------------------------------------ simulate! as written
 // The all-pairs list of unique_pairs (AllToAll.jl:65-80) holds (i, j) for
 // i < j, row by row (row i: j = i + 1 .. n - 1, 0-based).  Nothing of it is
-// stored in that order: the Lennard-Jones terms are stored by offset
-// k = j - i - 1 along the rows (entry (k, i) at koff(k) + i, so the threads
-// of consecutive atoms read consecutive entries), the Coulomb terms by level.
-
-__host__ __device__ inline int64_t koff(int32_t k, int32_t n) {
-    return (int64_t)k * (n - 1) - (int64_t)k * (k - 1) / 2;
-}
-
-// update_pairslist! (AllToAll.jl:7-62): d = sqrt(sum((a[i] .- a[j]).^2)),
-// the sum left to right, and the pair's force_lennardjones! term
-// (lennardjones_interior depends on d alone) with whether d < thr
-// (threshold_pairs, AllToAll.jl:83-88).  One block per row.
-__global__ void k_cs_pairs(const float* __restrict__ x, int32_t n, float thr,
-                           double* __restrict__ ljt, unsigned char* __restrict__ near) {
-    const int32_t i = blockIdx.x;
-    const float xi = x[3 * (int64_t)i], yi = x[3 * (int64_t)i + 1], zi = x[3 * (int64_t)i + 2];
-    for (int32_t j = i + 1 + threadIdx.x; j < n; j += blockDim.x) {
-        const float dx = __fsub_rn(xi, x[3 * (int64_t)j]);
-        const float dy = __fsub_rn(yi, x[3 * (int64_t)j + 1]);
-        const float dz = __fsub_rn(zi, x[3 * (int64_t)j + 2]);
-        const float dd = __fsqrt_rn(
-            __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-        const int64_t e = koff(j - i - 1, n) + i;
-        ljt[e] = lj_compat_term(dd);
-        near[e] = dd < thr;
-    }
-}
+// stored in that order: the Lennard-Jones terms are used as they are computed,
+// the Coulomb terms lie in the order the recurrence reads them.
 
 // force_lennardjones! over the whole list and over threshold_pairs(list,
-// thr): atom i's terms are its row, added in order to Float32 accumulators,
-// each addition rounded through Float64 as Julia's promotion does.  One thread
-// per atom, one warp per block so that the atoms' serial Float64 additions
-// spread over the SMs' Float64 pipes; the loads run 16 terms ahead.
-__global__ void k_cs_lj(const double* __restrict__ ljt, const unsigned char* __restrict__ near,
-                        int32_t n, float* __restrict__ ljthr, float* __restrict__ ljall) {
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int32_t L = n - 1 - i;
+// 0.01): atom i's terms are its row, added in order to Float32 accumulators,
+// each addition through Float64 as Julia's promotion does: fa <- Float32(
+// Float64(fa) + t).  The terms follow from the pair distances of
+// update_pairslist! (AllToAll.jl:7-62): d = sqrt(sum((a[i] .- a[j]).^2)), the
+// sum left to right.
+//
+// GB300 has few Float64 units (a term takes about 60 Float64 operations, an
+// addition three on a dependent chain: the term and sum kernels before took
+// 1,060 and 1,085 us at 4,096 atoms), so both run on Float32 pairs with a
+// bound on their error, and whatever the bound cannot decide is done again in
+// Float64 as written:
+//  * a term t = a c (4096 c - 1), c = (sigma / d)^6, a = Float32(24 eps / d)
+//    (the 12th power is 4096 c^2), as th + tl with a relative error below
+//    2^-41 against the Float64 value (the largest of 220,000 distances in each
+//    binade) for distances in [2^-10, 2^9]; outside, th = NaN;
+//  * an addition: s = fa + th and its error e (TwoSum); the sum lies within
+//    err = 2^-38 |th| + 2^-44 |s| + 1e-42 of s + (e + tl), which covers the
+//    term's error, the roundings here and the rounding to Float64.  Rounding
+//    to Float64 and then Float32 is monotonic, so when s + (r - err) and s +
+//    (r + err) round to the same Float32 that is the result; when not (about
+//    one addition in 10^5, and terms out of the range above) that addition is
+//    done in Float64.
+// A block serves 32 atoms: eight warps compute the terms of 64 columns at a
+// time into shared memory (a lane per atom, a column at a time), one warp adds
+// them up, a lane per atom; the chain of additions bounds it.
+constexpr int kLjCols = 64;  // columns per buffer: eight per producing warp
+
+__device__ __forceinline__ float compat_dist(const float3& a, const float* __restrict__ x,
+                                             int32_t j) {
+    const float dx = __fsub_rn(a.x, __ldg(&x[3 * (int64_t)j]));
+    const float dy = __fsub_rn(a.y, __ldg(&x[3 * (int64_t)j + 1]));
+    const float dz = __fsub_rn(a.z, __ldg(&x[3 * (int64_t)j + 2]));
+    return __fsqrt_rn(
+        __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+}
+
+// (h, l) <- (ah, al) (bh, bl) as Float32 pairs.
+__device__ __forceinline__ void pair_mul(float ah, float al, float bh, float bl, float& h,
+                                         float& l) {
+    h = __fmul_rn(ah, bh);
+    l = __fadd_rn(__fmaf_rn(ah, bh, -h), __fmaf_rn(ah, bl, __fmul_rn(al, bh)));
+}
+
+// lj_compat_term(d) as th + tl.
+__device__ __forceinline__ float2 lj_pair_term(float d) {
+    if (!(d >= 0x1p-10f && d <= 0x1p9f)) return make_float2(__int_as_float(0x7fffffff), 0.0f);
+    const double s6 = 0.0001 * 0.0001 * 0.0001 * 0.0001 * 0.0001 * 0.0001;
+    const float s6h = (float)s6, s6l = (float)(s6 - (double)s6h);
+    const float a = __fdiv_rn(__fmul_rn(24.0f, -1e10f), d);
+    const float ih = __frcp_rn(d);  // 1 / d = ih + il
+    const float il = __fmul_rn(ih, __fmaf_rn(-d, ih, 1.0f));
+    float zh, zl, wh, wl, vh, vl, ch, cl, uh, ul, ph, pl, th, tl;
+    pair_mul(ih, il, ih, il, zh, zl);
+    pair_mul(zh, zl, zh, zl, wh, wl);
+    pair_mul(wh, wl, zh, zl, vh, vl);    // d^-6
+    pair_mul(vh, vl, s6h, s6l, ch, cl);  // (sigma / d)^6
+    const float gh = __fmaf_rn(4096.0f, ch, -1.0f);
+    const float gl = __fmaf_rn(4096.0f, cl, __fmaf_rn(4096.0f, ch, -__fadd_rn(gh, 1.0f)));
+    pair_mul(a, 0.0f, s6h, s6l, uh, ul);
+    pair_mul(uh, ul, vh, vl, ph, pl);
+    pair_mul(ph, pl, gh, gl, th, tl);
+    return make_float2(th, tl);
+}
+
+__global__ void __launch_bounds__(288) k_cs_lj(const float* __restrict__ x, int32_t n, float thr,
+                                               float* __restrict__ ljthr,
+                                               float* __restrict__ ljall) {
+    __shared__ float2 st[2][kLjCols][32];
+    __shared__ unsigned char snear[2][32][8];  // bit m of [row][w]: column 8 w + m is near
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int32_t i0 = (int32_t)blockIdx.x * 32, i = i0 + lane;
+    float3 p = make_float3(0.f, 0.f, 0.f);
+    if (i < n)
+        p = make_float3(x[3 * (int64_t)i], x[3 * (int64_t)i + 1], x[3 * (int64_t)i + 2]);
+    const int32_t jb = i0 + 1;  // the first column of any row of the block
+    const int32_t nchunk = (n - jb + kLjCols - 1) / kLjCols;
     float fa = 0.0f, ft = 0.0f;
-    int64_t e = i;  // koff(0) + i
-    int32_t k = 0;
-    for (; k + 16 <= L; k += 16) {
-        double t[16];
-        unsigned char u[16];
-        int64_t ee = e;
+    auto produce = [&](int32_t c) {
+        const int32_t j0 = jb + c * kLjCols + 8 * w;
+        unsigned near = 0;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            t[r] = __ldg(&ljt[ee]);
-            u[r] = __ldg(&near[ee]);
-            ee += n - 1 - (k + r);
+        for (int m = 0; m < 8; ++m) {
+            const int32_t j = j0 + m;
+            if (j < n) {
+                const float d = compat_dist(p, x, j);
+                st[c & 1][8 * w + m][lane] = lj_pair_term(d);
+                if (d < thr && j > i) near |= 1u << m;
+            }
         }
+        snear[c & 1][lane][w] = (unsigned char)near;
+    };
+    // fa + t through Float64, decided in Float32: false when it cannot be
+    auto add = [](float& f, const float2& t) -> bool {
+        const float s = __fadd_rn(f, t.x);
+        const float b = __fsub_rn(s, f);
+        const float e = __fadd_rn(__fsub_rn(f, __fsub_rn(s, b)), __fsub_rn(t.x, b));
+        const float r = __fadd_rn(e, t.y);
+        const float err = __fmaf_rn(fabsf(t.x), 0x1p-38f, __fmaf_rn(fabsf(s), 0x1p-44f, 1e-42f));
+        const float up = __fadd_rn(s, __fadd_rn(r, err));
+        const bool sure = up == __fadd_rn(s, __fsub_rn(r, err));
+        f = up;
+        return sure;
+    };
+    auto consume = [&](int32_t c) {
+        if (i0 >= n) return;
+        for (int g = 0; g < 8; ++g) {
+            const int32_t j0 = jb + c * kLjCols + 8 * g;
+            if (j0 >= n) break;
+            const float f0 = fa;
+            bool good = j0 > i0 + 31 && j0 + 7 < n;  // every column belongs to every row
+            if (good) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            fa = __double2float_rn(__dadd_rn((double)fa, t[r]));
-            if (u[r]) ft = __double2float_rn(__dadd_rn((double)ft, t[r]));
+                for (int m = 0; m < 8; ++m) {
+                    const bool sure = add(fa, st[c & 1][8 * g + m][lane]);
+                    good = good && sure;
+                }
+            }
+            // a NaN stays one (and an infinity, whatever finite term is added)
+            if (!good && i < n && f0 == f0) {
+                fa = f0;
+                for (int m = 0; m < 8; ++m) {
+                    const int32_t j = j0 + m;
+                    if (j <= i || j >= n || fa != fa) continue;
+                    const float2 t = st[c & 1][8 * g + m][lane];
+                    float f = fa;
+                    if (add(f, t))
+                        fa = f;
+                    else if (!(isinf(fa) && isfinite(t.x)))
+                        fa = __double2float_rn(
+                            __dadd_rn((double)fa, lj_compat_term(compat_dist(p, x, j))));
+                }
+            }
+            unsigned near = snear[c & 1][lane][g];
+            while (near) {
+                const int32_t j = j0 + __ffs(near) - 1;
+                near &= near - 1;
+                ft = __double2float_rn(
+                    __dadd_rn((double)ft, lj_compat_term(compat_dist(p, x, j))));
+            }
         }
-        e = ee;
+    };
+    if (w < 8 && nchunk > 0) produce(0);
+    __syncthreads();
+    for (int32_t c = 0; c < nchunk; ++c) {
+        if (w == 8) consume(c);
+        else if (c + 1 < nchunk) produce(c + 1);
+        __syncthreads();
     }
-    for (; k < L; ++k) {
-        const double t = __ldg(&ljt[e]);
-        fa = __double2float_rn(__dadd_rn((double)fa, t));
-        if (__ldg(&near[e])) ft = __double2float_rn(__dadd_rn((double)ft, t));
-        e += n - 1 - k;
+    if (w == 8 && i < n) {
+        ljthr[i] = ft;
+        ljall[i] = fa;
     }
-    ljthr[i] = ft;
-    ljall[i] = fa;
 }
 
 // force_coulomb! over the all-pairs list.  Pair (i, j) depends on the pairs
 // before it that touch i or j: in this list order those are (i, j - 1) (or
-// (i - 1, i)) and (i - 1, j), so the pairs with i + j = s form one level
-// whose pairs touch distinct atoms, and level s follows level s - 1.  Running
-// the levels in order, each pair's two updates exactly as written, gives every
-// atom the same sequence of roundings as the sequential loop.
+// (i - 1, i)) and (i - 1, j).  Any schedule that keeps the two orders (along
+// a row, and down a column) and runs each pair's two updates as written gives
+// every atom the same sequence of roundings as the sequential loop.
+//
+// Bands (up to kBandMaxAtoms atoms): a warp owns 256 consecutive rows, eight a
+// lane, whose running forces stay in registers; the columns flow through its
+// lanes, four at a time.  At step t lane l takes the four columns 256 b + 4 (t -
+// l) .. + 3 from lane l - 1 by shuffles, adds the pair terms to its rows' forces
+// and subtracts those from the columns'; a row starts from its own column's
+// value when that arrives (j == i).  Columns pass from a band to the next
+// through an array in shared memory, each value with the number of bands it
+// has passed in the same 64-bit word (so no fence is needed); bands are spread
+// over a cluster of up to eight blocks, the last band of a block writing into
+// the next block's array.  The time is the dependence's: 95 steps a band, a step
+// of about 180 ns (64 dependent-in-pairs additions, shuffles, 4 KB of terms)
+// wherever the band lies.  4,096 atoms: 2,882 us a force evaluation with one
+// block running the anti-diagonals i + j behind a barrier each (the form
+// before), about 360 us so; one column and four rows a lane and step 460 us.
 //
 // The pair terms k q_i q_j / d^2 do not depend on the recurrence: they are
-// computed in parallel beforehand and stored level by level (level s at
-// s * stride for the shared-memory form, at level_off(s) when packed; its
-// pairs by increasing i), so each level is one contiguous, coalesced segment.
+// computed beforehand in the order the lanes read them, 4 KB a step.  Where a
+// lane has no pair the term is -0, which adds nothing to any value (signed
+// zeros included).
+constexpr int kBandRows = 256;         // rows of a band: eight a lane
+constexpr int kBandPad = 128;          // column words before the first (columns leaving a band early)
+constexpr int kBandMaxAtoms = 20480;   // the columns' array fits a block's shared memory
+
+constexpr int kBandCopy = 4;           // steps (of 4 KB) a copy brings
+// steps (tiles of four columns a lane) of band 0, padded to whole copies: band
+// b has band_steps(n) - 64 b
+__host__ __device__ inline int32_t band_steps(int32_t n) {
+    return ((n + 3) / 4 + 31 + kBandCopy - 1) / kBandCopy * kBandCopy;
+}
+__host__ __device__ inline int64_t band_off(int32_t b, int32_t P) {  // in steps
+    return (int64_t)b * P - 32LL * b * (b - 1);
+}
+// bytes of the columns' array (words written: 4 (band_steps(n) - 31) + kBandPad)
+__host__ __device__ inline int32_t band_col_bytes(int32_t n) {
+    return (8 * (4 * band_steps(n) + kBandPad) + 127) & ~127;
+}
+
+__device__ __forceinline__ float coulomb_term(float xi, float yi, float zi, float qi, float xj,
+                                              float yj, float zj, float qj) {
+    const float dx = __fsub_rn(xi, xj), dy = __fsub_rn(yi, yj), dz = __fsub_rn(zi, zj);
+    const float d = __fsqrt_rn(
+        __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+    // k * charge[i] * charge[j] ./ (d .^ 2), k = 1
+    return __fdiv_rn(__fmul_rn(qi, qj), __fmul_rn(d, d));
+}
+
+__global__ void __launch_bounds__(256)
+    k_cs_band_terms(const float* __restrict__ x, const float* __restrict__ q, int32_t n, int32_t P,
+                    float4* __restrict__ cterm) {
+    const int32_t b = blockIdx.y, lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+    const int32_t t = (int32_t)blockIdx.x;
+    if (t >= P - 64 * b) return;
+    const int32_t i = kBandRows * b + 8 * lane + r, j0 = kBandRows * b + 4 * (t - lane);
+    float c[4] = {-0.0f, -0.0f, -0.0f, -0.0f};
+    if (j0 + 3 > i && j0 < n) {
+        const float xi = __ldg(&x[3 * (int64_t)i]), yi = __ldg(&x[3 * (int64_t)i + 1]),
+                    zi = __ldg(&x[3 * (int64_t)i + 2]), qi = __ldg(&q[i]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int32_t j = j0 + k;
+            if (j > i && j < n)
+                c[k] = coulomb_term(xi, yi, zi, qi, __ldg(&x[3 * (int64_t)j]),
+                                    __ldg(&x[3 * (int64_t)j + 1]), __ldg(&x[3 * (int64_t)j + 2]),
+                                    __ldg(&q[j]));
+        }
+    }
+    cterm[(band_off(b, P) + t) * 256 + threadIdx.x] = make_float4(c[0], c[1], c[2], c[3]);
+}
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(unsigned long long* m) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(m)) : "memory");
+}
+// One bulk copy of `bytes` contiguous bytes (16-byte aligned on both sides),
+// completing on mbarrier m.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes,
+                                          unsigned long long* m) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(m)), "r"(bytes)
+                 : "memory");
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+            "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(m))
+        : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned long long* m, unsigned phase) {
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_addr(m)), "r"(phase)
+        : "memory");
+    return ok != 0;
+}
+
+// One cluster of blocks; warp w of block k runs band k * warps + w.  RING: the
+// terms come through a ring of 2^ldepth copies of kBandCopy steps a warp in
+// shared memory, filled by bulk copies that far ahead (registers cannot hold
+// enough loads to cover their latency); otherwise (more warps than rings fit
+// beside the columns) straight into registers, a step ahead.
+template <bool RING, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
+    k_cs_coulomb_bands(const float4* __restrict__ cterm, int32_t n, int32_t P, int32_t ldepth,
+                       float* __restrict__ F, int32_t* err) {
+    // columns (bands passed << 32 | value, column j at j + kBandPad), the
+    // rings, their barriers
+    extern __shared__ __align__(128) unsigned char sband[];
+    unsigned long long* scol = reinterpret_cast<unsigned long long*>(sband);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+    const int32_t b = (int32_t)rank * W + w;
+    const int32_t ncol = band_col_bytes(n) / 8, depth = 1 << ldepth;
+    constexpr int CP = kBandCopy;
+    float4* ring = reinterpret_cast<float4*>(sband + 8 * ncol) + (w << ldepth) * CP * 256;
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(
+                                  sband + 8 * ncol + ((int64_t)W << ldepth) * CP * 4096) +
+                              (w << ldepth);
+    for (int32_t k = threadIdx.x; k < ncol; k += blockDim.x) scol[k] = 0ull;
+    if (RING && lane == 0) {
+        for (int32_t k = 0; k < depth; ++k) mbar_init(bar + k);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cluster.sync();
+    const int32_t row0 = kBandRows * b;
+    if (row0 < n) {
+        constexpr int32_t kPolls = 1 << 22;  // a tenth of a second or more: never in a sound run
+        unsigned long long* out = scol;
+        if (w == W - 1 && rank + 1 < cluster.num_blocks())
+            out = cluster.map_shared_rank(scol, rank + 1);
+        const int32_t T = P - 64 * b, ncp = T / CP;  // P is a multiple of CP
+        const float4* __restrict__ C = cterm + band_off(b, P) * 256;
+        float a[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) a[r] = 0.0f;
+        bool lost = false;
+        float4 buf[2][8];
+        auto issue = [&](int32_t c) {
+            bulk_load(ring + (c & (depth - 1)) * CP * 256, C + (int64_t)c * CP * 256, CP * 4096,
+                      bar + (c & (depth - 1)));
+        };
+        if (RING && lane == 0)
+            for (int32_t c = 0; c < min(depth, ncp); ++c) issue(c);
+        const float4* src = ring + lane;
+        auto load = [&](float4 (&dst)[8], int32_t t) {
+            if (t >= T) return;
+            if constexpr (RING) {
+                if ((t & (CP - 1)) == 0) {
+                    const int32_t c = t / CP, slot = c & (depth - 1);
+                    for (int32_t polls = 0; !mbar_try(bar + slot, (unsigned)(c >> ldepth) & 1u); ++polls)
+                        if (polls > kPolls) {
+                            lost = true;
+                            if (lane == 0) set_error(err, ND_ERR_INTERNAL, b);
+                            break;
+                        }
+                    src = ring + slot * CP * 256 + lane;
+                    __syncwarp();
+                    // every lane has read the copy before: its slot takes a later one
+                    if (lane == 0 && c > 0 && c - 1 + depth < ncp) issue(c - 1 + depth);
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r) dst[r] = src[r * 32];
+                src += 256;
+            } else {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) dst[r] = __ldg(&C[(int64_t)t * 256 + r * 32 + lane]);
+            }
+        };
+        // columns row0 + 4 t .. + 3 and the bands they have passed (every lane
+        // reads the same words)
+        unsigned long long in[4] = {0, 0, 0, 0};
+        auto peek = [&](int32_t t) {
+            const unsigned at = smem_addr(scol + row0 + 4 * t + kBandPad);
+            asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];"
+                         : "=l"(in[0]), "=l"(in[1])
+                         : "r"(at)
+                         : "memory");
+            asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];"
+                         : "=l"(in[2]), "=l"(in[3])
+                         : "r"(at + 16)
+                         : "memory");
+        };
+        auto missing = [&]() {
+            const unsigned g = (unsigned)b;
+            return (((unsigned)(in[0] >> 32) ^ g) | ((unsigned)(in[1] >> 32) ^ g) |
+                    ((unsigned)(in[2] >> 32) ^ g) | ((unsigned)(in[3] >> 32) ^ g)) != 0u;
+        };
+        const int32_t tin = b > 0 ? T - 31 : 0;  // steps at which columns come in
+        if (tin > 0) peek(0);
+        float up[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // the columns from the lane below
+        unsigned long long* o = out + row0 - 4 * 31 + kBandPad;
+        const unsigned long long tag = (unsigned long long)(b + 1) << 32;
+        auto tile = [&](const float4 (&cc)[8], int32_t t) {
+            // this step's columns for lane 0 were looked at a step ago: a band
+            // that follows closely falls back by one step and then never waits
+            if (t < tin) {
+                for (int32_t polls = 0; missing() && !lost; ++polls) {
+                    peek(t);
+                    if (polls > kPolls) {
+                        lost = true;
+                        if (lane == 0) set_error(err, ND_ERR_INTERNAL, b);
+                    }
+                }
+                __syncwarp();
+            }
+            float f[4], t4[8][4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f[k] = lane == 0 ? __uint_as_float((unsigned)in[k]) : up[k];
+            if (t + 1 < tin) peek(t + 1);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                t4[r][0] = cc[r].x; t4[r][1] = cc[r].y; t4[r][2] = cc[r].z; t4[r][3] = cc[r].w;
+            }
+            // a row starts from its own column: row r of the lane at column
+            // r % 4 of its tile t - lane - 2 lane = r / 4
+            const bool s0 = t == 3 * lane, s1 = t == 3 * lane + 1;
+            // the tile by anti-diagonals, whose cells do not depend on one
+            // another: a cell adds its term to its row's force and subtracts
+            // that from its column's; a finished column leaves at once
+#pragma unroll
+            for (int s = 0; s < 11; ++s) {
+                float fi[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int r = s - k;
+                    if (r >= 0 && r < 8) fi[k] = __fadd_rn(a[r], t4[r][k]);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int r = s - k;
+                    if (r >= 0 && r < 8) {
+                        a[r] = (r & 3) == k && (r < 4 ? s0 : s1) ? f[k] : fi[k];
+                        f[k] = __fsub_rn(f[k], fi[k]);
+                        if (r == 7) up[k] = __shfl_up_sync(0xffffffffu, f[k], 1);
+                    }
+                }
+            }
+            // the columns that left lane 31 (also those no later band reads)
+            asm volatile(
+                "{\n.reg .pred p;\nsetp.eq.s32 p, %0, 31;\n"
+                "@p st.volatile.v2.u64 [%1], {%2, %3};\n"
+                "@p st.volatile.v2.u64 [%1+16], {%4, %5};\n}" ::"r"(lane),
+                "l"(o), "l"(tag | __float_as_uint(f[0])), "l"(tag | __float_as_uint(f[1])),
+                "l"(tag | __float_as_uint(f[2])), "l"(tag | __float_as_uint(f[3]))
+                : "memory");
+            o += 4;
+        };
+        load(buf[0], 0);
+        for (int32_t t = 0; t < T; t += 2) {  // T is even
+            load(buf[1], t + 1);
+            tile(buf[0], t);
+            load(buf[0], t + 2);
+            tile(buf[1], t + 1);
+        }
+        const int32_t i0 = row0 + 8 * lane;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            if (i0 + r < n) F[i0 + r] = a[r];
+    }
+    cluster.sync();  // the next block's array is written until here
+}
+
+// Beyond kBandMaxAtoms: the pairs with i + j = s form one level whose pairs
+// touch distinct atoms, and level s follows level s - 1; one block runs the
+// levels in order.  The pair terms are stored level by level (level s at
+// level_off(s); its pairs by increasing i).
 
 __host__ __device__ inline int32_t level_lo(int32_t s, int32_t n) { return max(0, s - (n - 1)); }
 __host__ __device__ inline int32_t level_count(int32_t s, int32_t n) {
@@ -222,107 +580,25 @@ __host__ __device__ inline int64_t level_off(int32_t s, int32_t n) {
 
 // The pair terms of one level per block, from the positions with the same
 // operations as update_pairslist! (so the same d).
-// stride > 0: level s at s * stride (16-byte aligned segments); else packed.
 __global__ void k_cs_cterms(const float* __restrict__ x, const float* __restrict__ q, int32_t n,
-                            int32_t stride, float* __restrict__ cterm) {
+                            float* __restrict__ cterm) {
     const int32_t s = blockIdx.x + 1;
     const int32_t ilo = level_lo(s, n), cnt = level_count(s, n);
-    float* out = cterm + (stride ? (int64_t)s * stride : level_off(s, n));
+    float* out = cterm + level_off(s, n);
     for (int32_t k = threadIdx.x; k < cnt; k += blockDim.x) {
         const int32_t i = ilo + k, j = s - i;
-        const float dx = __fsub_rn(x[3 * (int64_t)i], x[3 * (int64_t)j]);
-        const float dy = __fsub_rn(x[3 * (int64_t)i + 1], x[3 * (int64_t)j + 1]);
-        const float dz = __fsub_rn(x[3 * (int64_t)i + 2], x[3 * (int64_t)j + 2]);
-        const float d = __fsqrt_rn(
-            __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-        // k * charge[i] * charge[j] ./ (d .^ 2), k = 1
-        out[k] = __fdiv_rn(__fmul_rn(q[i], q[j]), __fmul_rn(d, d));
+        out[k] = coulomb_term(x[3 * (int64_t)i], x[3 * (int64_t)i + 1], x[3 * (int64_t)i + 2], q[i],
+                              x[3 * (int64_t)j], x[3 * (int64_t)j + 1], x[3 * (int64_t)j + 2], q[j]);
     }
 }
 
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
+constexpr int kLevelThreads = 128;  // fewest warps paying the per-level overhead (measured: 128 of 32-1024)
 
-__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(src) : "memory");
-}
-
-constexpr int kRingThreads = 128;  // fewest warps paying the per-level overhead (measured: 128 of 32-1024)
-constexpr int kLevelBatch = 8;  // pairs of a level per thread with their loads in flight
-
-// The recurrence, accumulators in shared memory, the pair terms of the next
-// RING - 1 levels copied ahead into a shared ring in 16-byte pieces (levels
-// at a fixed 16-byte-aligned stride).  One barrier per level: after a level's
-// updates each thread waits for its own copies of the next level, and the
-// barrier makes every thread's updates and copies visible to all.
-template <int RING>
-__global__ void __launch_bounds__(kRingThreads, 1) k_cs_coulomb_ring(const float* __restrict__ cterm,
-                                                                     int32_t n, int32_t stride,
-                                                                     float* __restrict__ F) {
-    extern __shared__ float4 sh4[];
-    float* ring = reinterpret_cast<float*>(sh4);  // RING x stride, 16-byte aligned
-    float* f = ring + (int64_t)RING * stride;
-    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) f[k] = 0.0f;
-    const int32_t smax = 2 * n - 3;
-    auto issue = [&](int32_t s) {
-        if (s <= smax) {
-            const int32_t pieces = (level_count(s, n) + 3) >> 2;
-            const float* src = cterm + (int64_t)s * stride;
-            float* dst = ring + (s % RING) * (int64_t)stride;
-            for (int32_t k = threadIdx.x; k < pieces; k += blockDim.x)
-                cp_async16(dst + 4 * k, src + 4 * k);
-        }
-        cp_async_commit();  // one group per level, empty or not
-    };
-    for (int32_t s = 1; s < RING; ++s) issue(s);
-    cp_async_wait<RING - 2>();  // level 1
-    __syncthreads();
-    for (int32_t s = 1; s <= smax; ++s) {
-        const float* cc = ring + (s % RING) * (int64_t)stride;
-        const int32_t ilo = level_lo(s, n), ihi = (s - 1) / 2;
-        // the pairs of a level touch distinct atoms: all of this thread's
-        // loads go first, then the updates (kLevelBatch pairs at a time)
-        for (int32_t i0 = ilo + (int32_t)threadIdx.x; i0 <= ihi;
-             i0 += kLevelBatch * (int32_t)blockDim.x) {
-            float a[kLevelBatch], b[kLevelBatch], t[kLevelBatch];
-#pragma unroll
-            for (int m = 0; m < kLevelBatch; ++m) {
-                const int32_t i = i0 + m * (int32_t)blockDim.x;
-                if (i <= ihi) {
-                    a[m] = f[i];
-                    b[m] = f[s - i];
-                    t[m] = cc[i - ilo];
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < kLevelBatch; ++m) {
-                const int32_t i = i0 + m * (int32_t)blockDim.x;
-                if (i <= ihi) {
-                    const float fi = __fadd_rn(a[m], t[m]);
-                    f[i] = fi;
-                    f[s - i] = __fsub_rn(b[m], fi);
-                }
-            }
-        }
-        issue(s + RING - 1);
-        cp_async_wait<RING - 2>();  // this thread's pieces of level s + 1
-        __syncthreads();
-    }
-    cp_async_wait<0>();
-    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) F[k] = f[k];
-}
-
-// The same recurrence with the accumulators in global memory (any n): the
+// The recurrence by levels, accumulators in global memory (any n): the
 // block's own writes are visible to it after each barrier.  The first item of
 // the next level is loaded ahead.
-__global__ void __launch_bounds__(kRingThreads, 1) k_cs_coulomb_global(const float* __restrict__ cterm,
-                                                               int32_t n, float* F) {
+__global__ void __launch_bounds__(kLevelThreads, 1)
+    k_cs_coulomb_global(const float* __restrict__ cterm, int32_t n, float* F) {
     for (int32_t k = threadIdx.x; k < n; k += blockDim.x) F[k] = 0.0f;
     __syncthreads();
     const int32_t smax = 2 * n - 3;
@@ -440,24 +716,16 @@ nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x
     const int64_t chunk =
         poslog ? std::max<int64_t>(1, std::min<int64_t>(spec->duration, chunk_frames)) : 0;
     nd_status st;
-    // Coulomb terms: levels at a 16-byte-aligned stride when the recurrence
-    // runs in shared memory (the widest level is level n - 1), else packed
-    const int32_t maxc = n > 1 ? level_count(n - 1, n) : 1;
-    const int32_t stride = (maxc + 3) & ~3;
-    auto shmem = [&](int r) { return sizeof(float) * ((size_t)r * stride + (size_t)n); };
-    int ring = 0;
-    for (int r : {8, 4, 3})
-        if (!ring && !force_global && shmem(r) <= 200 * 1024) ring = r;
+    // Coulomb terms: in band order, or by level for the global-memory form
+    const bool bands = !force_global && n <= kBandMaxAtoms;
+    const int32_t nband = (int32_t)cdiv(n, kBandRows), P4 = band_steps(n);
     const int32_t nlev = std::max(2 * n - 3, 0);
-    const size_t ncterm = ring ? (size_t)(nlev + 1) * stride : (size_t)std::max<int64_t>(P, 1);
+    const size_t ncterm =
+        bands ? 1024 * (size_t)band_off(nband, P4) : (size_t)std::max<int64_t>(P, 1);
     if ((st = ensure(c, c->leafpairs, sizeof(float) * ncterm))) return st;
-    if ((st = ensure(c, c->pairs_i, sizeof(double) * (size_t)std::max<int64_t>(P, 1)))) return st;
-    if ((st = ensure(c, c->pairs_j, (size_t)std::max<int64_t>(P, 1)))) return st;
     const size_t small = sizeof(float) * (4 * n3 + 6 * (size_t)n);
     if ((st = ensure(c, c->compat, small + (size_t)(chunk * frame_bytes)))) return st;
-    float* cterm = (float*)c->leafpairs.p;               // Coulomb pair terms, by level
-    double* ljt = (double*)c->pairs_i.p;                 // LJ pair terms, by row offset
-    unsigned char* near = (unsigned char*)c->pairs_j.p;  // d < 0.01, same layout
+    float* cterm = (float*)c->leafpairs.p;  // Coulomb pair terms
     float* dx = (float*)c->compat.p;
     float* dv = dx + n3;
     float* dF = dv + n3;
@@ -480,19 +748,27 @@ nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x
     if (e == cudaSuccess) e = cudaMemcpyAsync(dq, q, n * sizeof(float), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return cuda_fail(c, e, "compat simulate upload");
 
-    const size_t shb = ring ? shmem(ring) : 0;
-    if (ring) {
-        const void* fn = ring == 8   ? (const void*)k_cs_coulomb_ring<8>
-                         : ring == 4 ? (const void*)k_cs_coulomb_ring<4>
-                                     : (const void*)k_cs_coulomb_ring<3>;
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shb);
+    // bands over one cluster of up to eight blocks, the rings as deep as the
+    // shared memory beside the columns allows
+    const unsigned nblk = (unsigned)std::min(nband, 8), nwarp = (unsigned)cdiv(nband, nblk);
+    const void* band_fn = (const void*)k_cs_coulomb_bands<true, 160>;
+    size_t band_smem = (size_t)band_col_bytes(n);
+    int32_t ldepth = 3;
+    if (bands) {
+        int maxsm = 0;
+        cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+        auto ring = [&](int32_t l) { return ((size_t)nwarp * (kBandCopy * 4096 + 8)) << l; };
+        while (ldepth > 0 && (band_smem + ring(ldepth) > (size_t)maxsm || nwarp > 5)) --ldepth;
+        if (ldepth > 0) band_smem += ring(ldepth);
+        else band_fn = (const void*)k_cs_coulomb_bands<false, 320>;
+        // one limit whatever the size: the attribute belongs to the process
+        e = cudaFuncSetAttribute(band_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm);
         if (e != cudaSuccess) return cuda_fail(c, e, "compat simulate smem");
     }
     // Two chains per step, both from the list of the previous step's
     // positions: force_coulomb! (update_pairslist!'s Coulomb terms, then the
-    // levels on one SM) on the context's stream, and force_lennardjones!
-    // (the LJ terms of update_pairslist!, then the row sums) on a side stream
-    // over the other SMs.  The step kernel waits for both; the side chain of
+    // recurrence on up to eight SMs) on the context's stream, and
+    // force_lennardjones! on a side stream over the other SMs.  The step kernel waits for both; the side chain of
     // the next step waits for the step kernel.
     struct Side {
         cudaStream_t s2 = nullptr;
@@ -510,30 +786,46 @@ nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x
     if (e != cudaSuccess) return cuda_fail(c, e, "compat simulate streams");
     cudaStream_t s2 = side.s2;
     auto coulomb_terms = [&]() {
-        if (n > 1) {
-            k_cs_cterms<<<nlev, 256, 0, s>>>(dx, dq, n, ring ? stride : 0, cterm);
+        if (bands) {
+            k_cs_band_terms<<<dim3((unsigned)P4, (unsigned)nband), 256, 0, s>>>(
+                dx, dq, n, P4, (float4*)cterm);
+            c->launches++;
+        } else if (n > 1) {
+            k_cs_cterms<<<nlev, 256, 0, s>>>(dx, dq, n, cterm);
             c->launches++;
         }
     };
-    auto coulomb = [&]() {
-        if (ring == 8)
-            k_cs_coulomb_ring<8><<<1, kRingThreads, shb, s>>>(cterm, n, stride, cf);
-        else if (ring == 4)
-            k_cs_coulomb_ring<4><<<1, kRingThreads, shb, s>>>(cterm, n, stride, cf);
-        else if (ring == 3)
-            k_cs_coulomb_ring<3><<<1, kRingThreads, shb, s>>>(cterm, n, stride, cf);
-        else
-            k_cs_coulomb_global<<<1, kRingThreads, 0, s>>>(cterm, n, cf);
+    auto coulomb = [&]() -> cudaError_t {
         c->launches++;
+        if (!bands) {
+            k_cs_coulomb_global<<<1, kLevelThreads, 0, s>>>(cterm, n, cf);
+            return cudaSuccess;
+        }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(nblk);
+        cfg.blockDim = dim3(32 * nwarp);
+        cfg.dynamicSmemBytes = band_smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = nblk;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        const float4* ct = (const float4*)cterm;
+        int32_t nn = n, pp = P4, ld = ldepth;
+        float* ff = cf;
+        int32_t* ee = c->d_err;
+        void* args[] = {&ct, &nn, &pp, &ld, &ff, &ee};
+        return cudaLaunchKernelExC(&cfg, band_fn, args);
     };
-    // after the positions of stream `after` moved: the LJ terms and sums on s2
+    // after the positions of stream `after` moved: the LJ sums on s2
     auto lj_chain = [&](cudaStream_t after) -> cudaError_t {
         cudaError_t ee = cudaEventRecord(side.moved, after);
         if (ee == cudaSuccess) ee = cudaStreamWaitEvent(s2, side.moved, 0);
         if (ee != cudaSuccess) return ee;
-        if (n > 1) k_cs_pairs<<<n - 1, 256, 0, s2>>>(dx, n, 0.01f, ljt, near);
-        k_cs_lj<<<(unsigned)cdiv(n, 32), 32, 0, s2>>>(ljt, near, n, ljthr, ljall);
-        c->launches += n > 1 ? 2 : 1;
+        k_cs_lj<<<(unsigned)cdiv(n, 32), 288, 0, s2>>>(dx, n, 0.01f, ljthr, ljall);
+        c->launches++;
         return cudaEventRecord(side.lj, s2);
     };
     const float dt = (float)spec->stepwidth;
@@ -564,7 +856,7 @@ nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x
         // force_coulomb! runs twice per step on the same list and charges: one
         // evaluation gives both results; so does force_lennardjones!'s pass
         // over the whole list and its threshold_pairs part
-        coulomb();
+        if ((e = coulomb()) != cudaSuccess) return cuda_fail(c, e, "compat simulate (Coulomb)");
         float* frame = poslog ? dlog + pending * (int64_t)n3 : nullptr;
         e = cudaStreamWaitEvent(s, side.lj, 0);
         if (e != cudaSuccess) return cuda_fail(c, e, "compat simulate streams");
