@@ -267,7 +267,7 @@ nd_status nd_leaf_pairs_refresh(nd_ctx* ctx, const float* xyz, const nd_bvh_spec
  * positions (xyz, N x 3 Float32) and outputs (pi, pj, pd) are device pointers
  * on the current device; *count is a host pointer; work is enqueued on `stream`
  * (a cudaStream_t, NULL = default stream) and the call synchronises it to read
- * the pair count.  Scratch is one file-scope device array of ~5.3 MB reserved
+ * the pair count.  Scratch is one file-scope device array of ~5.4 MB reserved
  * on every GPU that loads the library until the process exits; nothing is
  * allocated.  Limits: atom_count <= 65536 and atomsperleaf >= 2 (in both
  * modes; an unordered request with another leaf width than 4 is served by the

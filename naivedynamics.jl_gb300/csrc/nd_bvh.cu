@@ -20,85 +20,30 @@ namespace nd {
 
 // =================================================================== Morton
 
-// mortoncodes! with K = Int32 (BVHTraverse.jl:259-284).
-__global__ void k_morton_reference(const float* __restrict__ xyz, int32_t n, float binwidth,
-                                   int32_t* __restrict__ codes, int32_t* __restrict__ iota,
-                                   int32_t* err) {
-    int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// mortoncodes! with K = Int32 (BVHTraverse.jl:259-284), one position.
+__device__ __forceinline__ int32_t code_reference(const float* __restrict__ xyz, int32_t i,
+                                                  float binwidth, int32_t* err) {
     const int32_t magic[3] = {153391689, 306783378, 613566756};
     int32_t code = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         float p = xyz[3 * (int64_t)i + d];
-        if (!isfinite(p)) { set_error(err, ND_ERR_NONFINITE, i); code = 0; break; }
+        if (!isfinite(p)) { set_error(err, ND_ERR_NONFINITE, i); return 0; }
         float q = floorf(__fdiv_rn(p, binwidth));
         // trunc(Int32, ::Float32) accepts -2^31 <= q < 2^31 (Julia Base float.jl)
-        if (!(q >= -2147483648.0f && q < 2147483648.0f)) { set_error(err, ND_ERR_RANGE, i); code = 0; break; }
+        if (!(q >= -2147483648.0f && q < 2147483648.0f)) { set_error(err, ND_ERR_RANGE, i); return 0; }
         int32_t qi = (int32_t)q;
         int32_t yin = qi & magic[d];
         int32_t yang = qi | ~magic[d];
         code |= (yin & yang);
     }
-    codes[i] = code;
-    if (iota) iota[i] = i;
-}
-
-// Bounding box of the positions (order-preserving uint atomics), used by the
-// spatial code.  bbox[0..2] = min keys, bbox[3..5] = max keys.
-__global__ void k_bbox(const float* __restrict__ xyz, int32_t n, uint32_t* bbox, int32_t* err) {
-    uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    uint32_t mx[3] = {0u, 0u, 0u};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            float p = xyz[3 * i + d];
-            if (!isfinite(p)) { set_error(err, ND_ERR_NONFINITE, (int32_t)i); continue; }
-            uint32_t o = f2o(p);
-            mn[d] = min(mn[d], o);
-            mx[d] = max(mx[d], o);
-        }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        for (int s = 16; s > 0; s >>= 1) {
-            mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], s));
-            mx[d] = max(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], s));
-        }
-    }
-    // block reduction first: one atomic per block and component
-    __shared__ uint32_t s_b[32][6];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int d = 0; d < 3; ++d) { s_b[warp][d] = mn[d]; s_b[warp][3 + d] = mx[d]; }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        const int k = threadIdx.x;
-        uint32_t v = s_b[0][k];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = k < 3 ? min(v, s_b[w][k]) : max(v, s_b[w][k]);
-        if (k < 3) atomicMin(&bbox[k], v);
-        else atomicMax(&bbox[k], v);
-    }
-}
-
-__global__ void k_bbox_init(uint32_t* bbox) {
-    if (threadIdx.x < 6) bbox[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
-}
-
-// A given frame in place of the bounding box.
-__global__ void k_bbox_set(uint32_t* bbox, float x0, float y0, float z0, float x1, float y1,
-                           float z1) {
-    const float v[6] = {x0, y0, z0, x1, y1, z1};
-    if (threadIdx.x < 6) bbox[threadIdx.x] = f2o(v[threadIdx.x]);
+    return code;
 }
 
 // Spatial code: 3-D Hilbert index over the bounding box, 1024 bins per axis.
-__global__ void k_morton_spatial(const float* __restrict__ xyz, int32_t n,
-                                 const uint32_t* __restrict__ bbox, int32_t* __restrict__ codes,
-                                 int32_t* __restrict__ iota) {
-    int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// bbox: order-preserving images (f2o) of min[3], max[3].
+__device__ __forceinline__ int32_t code_spatial(const float* __restrict__ xyz, int32_t i,
+                                                const uint32_t* bbox) {
     uint32_t q[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -109,20 +54,104 @@ __global__ void k_morton_spatial(const float* __restrict__ xyz, int32_t n,
         int32_t qi = (t < 0.0f) ? 0 : (t > 1023.0f ? 1023 : (int32_t)t);
         q[d] = (uint32_t)qi;
     }
-    codes[i] = (int32_t)hilbert3_10(q[0], q[1], q[2]);
-    if (iota) iota[i] = i;
+    return (int32_t)hilbert3_10(q[0], q[1], q[2]);
 }
 
-nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32_t* codes,
-                       int32_t* iota, const float* frame) {
-    if (n <= 0) return ND_OK;
+// Min and max images of the finite coordinates of position i.
+__device__ __forceinline__ void bbox_add(const float* __restrict__ xyz, int64_t i,
+                                         uint32_t (&mn)[3], uint32_t (&mx)[3], int32_t* err) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        float p = xyz[3 * i + d];
+        if (!isfinite(p)) { set_error(err, ND_ERR_NONFINITE, (int32_t)i); continue; }
+        uint32_t o = f2o(p);
+        mn[d] = min(mn[d], o);
+        mx[d] = max(mx[d], o);
+    }
+}
+
+// The warps' boxes in s_b[warp][6] (after this, a __syncthreads by the caller).
+__device__ __forceinline__ void bbox_warp(uint32_t (&mn)[3], uint32_t (&mx)[3],
+                                          uint32_t (*s_b)[6]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        mn[d] = __reduce_min_sync(0xffffffffu, mn[d]);
+        mx[d] = __reduce_max_sync(0xffffffffu, mx[d]);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) { s_b[warp][d] = mn[d]; s_b[warp][3 + d] = mx[d]; }
+}
+// Component k (0-2 min, 3-5 max) over the block's warps.
+__device__ __forceinline__ uint32_t bbox_block(const uint32_t (*s_b)[6], int k) {
+    uint32_t v = s_b[0][k];
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = k < 3 ? min(v, s_b[w][k]) : max(v, s_b[w][k]);
+    return v;
+}
+
+// Bounding box of the positions (order-preserving uint atomics), used by the
+// spatial code.  bbox[0..2] = min keys, bbox[3..5] = max keys.
+__global__ void k_bbox(const float* __restrict__ xyz, int32_t n, uint32_t* bbox, int32_t* err) {
+    uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
+    uint32_t mx[3] = {0u, 0u, 0u};
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        bbox_add(xyz, i, mn, mx, err);
+    // block reduction first: one atomic per block and component
+    __shared__ uint32_t s_b[32][6];
+    bbox_warp(mn, mx, s_b);
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int k = threadIdx.x;
+        const uint32_t v = bbox_block(s_b, k);
+        if (k < 3) atomicMin(&bbox[k], v);
+        else atomicMax(&bbox[k], v);
+    }
+}
+
+__global__ void k_bbox_init(uint32_t* bbox) {
+    if (threadIdx.x < 6) bbox[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+}
+
+// A given frame in place of the bounding box.
+struct CodeFrame {
+    float v[6];
+    int32_t given;
+};
+__global__ void k_bbox_set(uint32_t* bbox, CodeFrame fr) {
+    if (threadIdx.x < 6) bbox[threadIdx.x] = f2o(fr.v[threadIdx.x]);
+}
+
+constexpr int RS_BINS = 256;
+constexpr int RS_TILE = 2048;
+
+// Codes of all positions, the identity permutation, and (hist given) the
+// digit counts of the sort's first pass, per tile of RS_TILE positions.
+__global__ void k_morton(const float* __restrict__ xyz, int32_t n, int32_t order, float binwidth,
+                         const uint32_t* __restrict__ bbox, int32_t* __restrict__ codes,
+                         int32_t* __restrict__ iota, uint32_t* __restrict__ hist, int32_t* err) {
+    int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int32_t code = order == ND_ORDER_SPATIAL ? code_spatial(xyz, i, bbox)
+                                                   : code_reference(xyz, i, binwidth, err);
+    codes[i] = code;
+    if (iota) iota[i] = i;
+    if (hist) atomicAdd(&hist[(i / RS_TILE) * RS_BINS + (code & 0xff)], 1u);
+}
+
+constexpr float kBinWidth = (float)(1.0 / 1023.0);  // Float32(1/1023), BVHTraverse.jl:184
+
+static nd_status codes_kernels(Ctx* c, const float* xyz, int32_t n, int32_t order, int32_t* codes,
+                               int32_t* iota, const float* frame, uint32_t* hist) {
     const int T = 256;
     if (order == ND_ORDER_SPATIAL) {
         nd_status st = ensure(c, c->misc, 64);
         if (st) return st;
         if (frame) {
-            k_bbox_set<<<1, 32, 0, c->stream>>>((uint32_t*)c->misc.p, frame[0], frame[1], frame[2],
-                                                frame[3], frame[4], frame[5]);
+            CodeFrame fr{};
+            for (int k = 0; k < 6; ++k) fr.v[k] = frame[k];
+            k_bbox_set<<<1, 32, 0, c->stream>>>((uint32_t*)c->misc.p, fr);
             c->launches++;
         } else {
             k_bbox_init<<<1, 32, 0, c->stream>>>((uint32_t*)c->misc.p);
@@ -131,29 +160,259 @@ nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32
             k_bbox<<<blocks, T, 0, c->stream>>>(xyz, n, (uint32_t*)c->misc.p, c->d_err);
             c->launches++;
         }
-        k_morton_spatial<<<(int)cdiv(n, T), T, 0, c->stream>>>(xyz, n, (const uint32_t*)c->misc.p,
-                                                              codes, iota);
-        c->launches++;
-    } else {
-        const float binwidth = (float)(1.0 / 1023.0);  // Float32(1/1023), BVHTraverse.jl:184
-        k_morton_reference<<<(int)cdiv(n, T), T, 0, c->stream>>>(xyz, n, binwidth, codes, iota,
-                                                                c->d_err);
-        c->launches++;
     }
+    k_morton<<<(int)cdiv(n, T), T, 0, c->stream>>>(xyz, n, order, kBinWidth,
+                                                   (const uint32_t*)c->misc.p, codes, iota, hist,
+                                                   c->d_err);
+    c->launches++;
     return check_launch(c, "morton");
 }
 
-// ================================================================ radix sort
-// Stable LSD radix sort, 8-bit digits, reduce-then-scan (no inter-CTA waiting):
-//   upsweep: per-tile digit histograms, digit-major;
-//   scan:    per-digit exclusive scan over tiles + digit totals;
-//   scatter: stable in-tile ranks (warp match + per-warp prefix) -> global slot.
+nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32_t* codes,
+                       int32_t* iota, const float* frame) {
+    if (n <= 0) return ND_OK;
+    return codes_kernels(c, xyz, n, order, codes, iota, frame, nullptr);
+}
 
-constexpr int RS_BINS = 256;
+// ================================================================ radix sort
+// Stable LSD radix sort, 8-bit digits, no block waits for another.  Three
+// forms, by size:
+//  * up to kSmallSort keys: one block does everything (codes included), one
+//    launch; 512 positions took 15 launches, 50 us, before;
+//  * up to kDirectTiles tiles of 2,048 keys: one kernel per pass (k_rs_pass).
+//    A block adds up the digit counts of the tiles before its own by itself
+//    (coalesced rows, independent loads; at 256 tiles 256 KB from L2 a block)
+//    and counts, while it scatters, the next pass's digits at their
+//    destination tiles, so a pass needs no counting and no scanning kernel;
+//  * more: digit counts per tile (k_rs_upsweep), a scan per digit over the
+//    tiles (k_rs_scan), the scatter (k_rs_scatter): the rows would be read
+//    ntiles^2 times.
+
 constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 8;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+constexpr int RS_ITEMS = RS_TILE / RS_THREADS;
+constexpr int32_t kSmallSort = 4096;
+constexpr int32_t kDirectTiles = 256;
 static_assert(RS_THREADS == RS_BINS, "scatter maps one thread per digit");
+
+size_t sort_scratch_bytes(int32_t n) {
+    const size_t nt = (size_t)cdiv(n, RS_TILE);
+    const size_t rows = nt <= (size_t)kDirectTiles ? 4 * nt : nt;
+    return sizeof(uint32_t) * (RS_BINS * rows + RS_BINS);
+}
+
+// Ranks of a warp's ITEMS x 32 digits (held i-major: item i of lane l is the
+// (32 i + l)-th) among the equal digits before them in the warp; cnt[digit]
+// counts the warp's digits (zeroed by the caller).  Digit 256 is no item.
+template <int ITEMS, class C>
+__device__ __forceinline__ void warp_ranks(const uint32_t (&dg)[ITEMS], C* cnt,
+                                           uint32_t (&rank)[ITEMS]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const unsigned peers = __match_any_sync(0xffffffffu, dg[i]);
+        const int lead = __ffs(peers) - 1;
+        uint32_t old = 0;
+        if (lane == lead && dg[i] < 256u) {
+            old = cnt[dg[i]];
+            cnt[dg[i]] = (C)(old + __popc(peers));
+        }
+        old = __shfl_sync(0xffffffffu, old, lead);
+        rank[i] = old + __popc(peers & lt);
+        __syncwarp();
+    }
+}
+
+// Exclusive scan of one value per digit over the first 256 threads of the
+// block; every thread calls it.
+__device__ __forceinline__ uint32_t digits_scan(uint32_t v, uint32_t* s_warp) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        uint32_t y = __shfl_up_sync(0xffffffffu, x, s);
+        if (lane >= s) x += y;
+    }
+    if (warp < 8 && lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    uint32_t before = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) before += w < warp ? s_warp[w] : 0u;
+    return before + x - v;
+}
+
+// One block: codes (xyz given) or given keys and values, sorted into
+// keys/vals.  Each warp holds ITEMS x 32 consecutive items.
+template <int ITEMS>
+__global__ void __launch_bounds__(1024)
+    k_small_order(const float* __restrict__ xyz, int32_t n, int32_t order, float binwidth,
+                  CodeFrame frame, uint32_t* keys, int32_t* vals, int passes, int32_t* err) {
+    __shared__ uint16_t s_cnt[32][RS_BINS];
+    __shared__ uint32_t s_x[1024 * ITEMS];
+    __shared__ uint32_t s_part[4][RS_BINS];
+    __shared__ uint32_t s_warp[8];
+    __shared__ uint32_t s_b[32][6];
+    __shared__ uint32_t s_box[6];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    uint32_t key[ITEMS];
+    int32_t val[ITEMS];
+    const int32_t at0 = w * 32 * ITEMS + lane;
+    if (xyz) {
+        if (order == ND_ORDER_SPATIAL) {
+            uint32_t mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
+            uint32_t mx[3] = {0u, 0u, 0u};
+            if (!frame.given)
+                for (int32_t i = t; i < n; i += 1024) bbox_add(xyz, i, mn, mx, err);
+            bbox_warp(mn, mx, s_b);
+            __syncthreads();
+            if (t < 6) s_box[t] = frame.given ? f2o(frame.v[t]) : bbox_block(s_b, t);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const int32_t k = at0 + 32 * i;
+            val[i] = k;
+            key[i] = k >= n ? 0u
+                     : order == ND_ORDER_SPATIAL
+                         ? (uint32_t)code_spatial(xyz, k, s_box)
+                         : (uint32_t)code_reference(xyz, k, binwidth, err);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const int32_t k = at0 + 32 * i;
+            key[i] = k < n ? keys[k] : 0u;
+            val[i] = k < n ? vals[k] : 0;
+        }
+    }
+    for (int p = 0; p < passes; ++p) {
+        const int shift = 8 * p;
+        for (int k = t; k < 32 * RS_BINS / 2; k += 1024) reinterpret_cast<uint32_t*>(s_cnt)[k] = 0u;
+        __syncthreads();
+        uint32_t dg[ITEMS], rank[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) dg[i] = at0 + 32 * i < n ? (key[i] >> shift) & 0xffu : 256u;
+        warp_ranks<ITEMS>(dg, s_cnt[w], rank);
+        __syncthreads();
+        // digit-major prefix: four groups of eight warps' counts per digit
+        const int d = t & 255, g = t >> 8;
+        uint32_t sum = 0, c8[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { c8[k] = s_cnt[8 * g + k][d]; sum += c8[k]; }
+        s_part[g][d] = sum;
+        __syncthreads();
+        const uint32_t tot = s_part[0][d] + s_part[1][d] + s_part[2][d] + s_part[3][d];
+        const uint32_t ex = digits_scan(tot, s_warp);
+        if (g == 0) s_x[d] = ex;
+        __syncthreads();
+        uint32_t run = s_x[d];
+        for (int k = 0; k < g; ++k) run += s_part[k][d];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { s_cnt[8 * g + k][d] = (uint16_t)run; run += c8[k]; }
+        __syncthreads();
+        uint32_t pos[ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) pos[i] = dg[i] < 256u ? s_cnt[w][dg[i]] + rank[i] : 0u;
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            if (dg[i] < 256u) s_x[pos[i]] = key[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) key[i] = s_x[at0 + 32 * i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+            if (dg[i] < 256u) s_x[pos[i]] = (uint32_t)val[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) val[i] = (int32_t)s_x[at0 + 32 * i];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const int32_t k = at0 + 32 * i;
+        if (k < n) { keys[k] = key[i]; vals[k] = val[i]; }
+    }
+}
+
+static void small_order(Ctx* c, const float* xyz, int32_t n, int32_t order, const float* frame,
+                        uint32_t* keys, int32_t* vals, int passes) {
+    CodeFrame fr{};
+    if (frame) {
+        for (int k = 0; k < 6; ++k) fr.v[k] = frame[k];
+        fr.given = 1;
+    }
+#define ND_SMALL(I)                                                                             \
+    k_small_order<I><<<1, 1024, 0, c->stream>>>(xyz, n, order, kBinWidth, fr, keys, vals, passes, \
+                                                c->d_err)
+    if (n <= 1024) ND_SMALL(1);
+    else if (n <= 2048) ND_SMALL(2);
+    else ND_SMALL(4);
+#undef ND_SMALL
+    c->launches++;
+}
+
+// Digit counts per tile of keys that come from elsewhere.
+__global__ void k_rs_count(const uint32_t* __restrict__ keys, int32_t n, uint32_t* __restrict__ hist) {
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) atomicAdd(&hist[(i / RS_TILE) * RS_BINS + (keys[i] & 0xffu)], 1u);
+}
+
+// One pass over one tile: hist[tile][digit] are this pass's counts, hist_next
+// (null in the last pass) receives the next pass's.
+__global__ void __launch_bounds__(512)
+    k_rs_pass(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
+              uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int32_t n, int shift,
+              const uint32_t* __restrict__ hist, uint32_t* __restrict__ hist_next, int32_t ntiles) {
+    constexpr int W = 16, ITEMS = RS_TILE / 512;
+    __shared__ uint16_t s_cnt[W][RS_BINS];
+    __shared__ uint32_t s_pre[2][RS_BINS], s_tot[2][RS_BINS], s_base[RS_BINS], s_warp[8];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5, d = t & 255, g = t >> 8;
+    const int32_t tile = blockIdx.x;
+    const int64_t at0 = (int64_t)tile * RS_TILE + w * 32 * ITEMS + lane;
+    uint32_t key[ITEMS], dg[ITEMS], rank[ITEMS];
+    int32_t val[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const int64_t k = at0 + 32 * i;
+        key[i] = k < n ? kin[k] : 0u;
+        val[i] = k < n ? vin[k] : 0;
+        dg[i] = k < n ? (key[i] >> shift) & 0xffu : 256u;
+    }
+    for (int k = t; k < W * RS_BINS / 2; k += 512) reinterpret_cast<uint32_t*>(s_cnt)[k] = 0u;
+    uint32_t pre = 0, tot = 0;
+#pragma unroll 8
+    for (int32_t r = g; r < ntiles; r += 2) {
+        const uint32_t v = __ldg(&hist[r * RS_BINS + d]);
+        tot += v;
+        pre += r < tile ? v : 0u;
+    }
+    s_pre[g][d] = pre;
+    s_tot[g][d] = tot;
+    __syncthreads();
+    warp_ranks<ITEMS>(dg, s_cnt[w], rank);
+    const uint32_t ex = digits_scan(s_tot[0][d] + s_tot[1][d], s_warp);  // (a barrier inside)
+    if (g == 0) {
+        s_base[d] = ex + s_pre[0][d] + s_pre[1][d];
+        uint32_t run = 0;
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            const uint32_t cnt = s_cnt[k][d];
+            s_cnt[k][d] = (uint16_t)run;
+            run += cnt;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if (dg[i] < 256u) {
+            const uint32_t pos = s_base[dg[i]] + s_cnt[w][dg[i]] + rank[i];
+            kout[pos] = key[i];
+            vout[pos] = val[i];
+            if (hist_next)
+                atomicAdd(&hist_next[(pos / RS_TILE) * RS_BINS + ((key[i] >> (shift + 8)) & 0xffu)], 1u);
+        }
+}
 
 __global__ void __launch_bounds__(RS_THREADS)
     k_rs_upsweep(const uint32_t* __restrict__ keys, int32_t n, int shift,
@@ -268,21 +527,64 @@ __global__ void __launch_bounds__(RS_THREADS)
     }
 }
 
-nd_status radix_sort_pairs(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int bits) {
-    if (n <= 1) return ND_OK;
-    int32_t ntiles = (int32_t)cdiv(n, RS_TILE);
+// The passes of the direct form; hist[0] already counted.  Results end in
+// keys/vals.
+static nd_status direct_passes(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int passes) {
+    const int32_t ntiles = (int32_t)cdiv(n, RS_TILE);
+    uint32_t* hist = (uint32_t*)c->hist.p;
+    uint32_t *ka = keys, *kb = (uint32_t*)c->codes_alt.p;
+    int32_t *va = vals, *vb = (int32_t*)c->perm_alt.p;
+    const size_t row = (size_t)RS_BINS * ntiles;
+    for (int p = 0; p < passes; ++p) {
+        k_rs_pass<<<ntiles, 512, 0, c->stream>>>(ka, va, kb, vb, n, 8 * p, hist + p * row,
+                                                 p + 1 < passes ? hist + (p + 1) * row : nullptr,
+                                                 ntiles);
+        c->launches++;
+        std::swap(ka, kb);
+        std::swap(va, vb);
+    }
+    if (ka != keys) {
+        cudaMemcpyAsync(keys, ka, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, c->stream);
+        cudaMemcpyAsync(vals, va, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToDevice, c->stream);
+    }
+    return check_launch(c, "radix sort");
+}
+
+static nd_status sort_buffers(Ctx* c, int32_t n) {
     nd_status st;
     if ((st = ensure(c, c->codes_alt, sizeof(uint32_t) * (size_t)n))) return st;
     if ((st = ensure(c, c->perm_alt, sizeof(int32_t) * (size_t)n))) return st;
-    if ((st = ensure(c, c->hist, sizeof(uint32_t) * ((size_t)RS_BINS * ntiles + RS_BINS))))
-        return st;
+    return ensure(c, c->hist, sort_scratch_bytes(n));
+}
+
+static nd_status reset_counts(Ctx* c, int32_t n, int passes) {
+    cudaError_t e = cudaMemsetAsync(
+        c->hist.p, 0, sizeof(uint32_t) * RS_BINS * (size_t)cdiv(n, RS_TILE) * passes, c->stream);
+    return e == cudaSuccess ? ND_OK : cuda_fail(c, e, "digit counts reset");
+}
+
+nd_status radix_sort_pairs(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int bits) {
+    if (n <= 1) return ND_OK;
+    const int passes = (bits + 7) / 8;
+    if (n <= kSmallSort) {
+        small_order(c, nullptr, n, 0, nullptr, keys, vals, passes);
+        return check_launch(c, "radix sort");
+    }
+    nd_status st = sort_buffers(c, n);
+    if (st) return st;
+    int32_t ntiles = (int32_t)cdiv(n, RS_TILE);
+    if (ntiles <= kDirectTiles) {
+        if ((st = reset_counts(c, n, passes))) return st;
+        k_rs_count<<<(unsigned)cdiv(n, 256), 256, 0, c->stream>>>(keys, n, (uint32_t*)c->hist.p);
+        c->launches++;
+        return direct_passes(c, keys, vals, n, passes);
+    }
     uint32_t* hist = (uint32_t*)c->hist.p;
     uint32_t* totals = hist + (size_t)RS_BINS * ntiles;
     uint32_t* ka = keys;
     int32_t* va = vals;
     uint32_t* kb = (uint32_t*)c->codes_alt.p;
     int32_t* vb = (int32_t*)c->perm_alt.p;
-    int passes = (bits + 7) / 8;
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
         k_rs_upsweep<<<ntiles, RS_THREADS, 0, c->stream>>>(ka, n, shift, hist, ntiles);
@@ -298,6 +600,23 @@ nd_status radix_sort_pairs(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int
         cudaMemcpyAsync(vals, va, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToDevice, c->stream);
     }
     return check_launch(c, "radix sort");
+}
+
+nd_status order_positions(Ctx* c, const float* xyz, int32_t n, int32_t order, int32_t* codes,
+                          int32_t* perm, const float* frame) {
+    if (n <= 0) return ND_OK;
+    if (n <= kSmallSort) {
+        small_order(c, xyz, n, order, frame, (uint32_t*)codes, perm, 4);
+        return check_launch(c, "order");
+    }
+    nd_status st;
+    if (cdiv(n, RS_TILE) > kDirectTiles) {
+        if ((st = codes_kernels(c, xyz, n, order, codes, perm, frame, nullptr))) return st;
+        return radix_sort_pairs(c, (uint32_t*)codes, perm, n, 30);
+    }
+    if ((st = sort_buffers(c, n)) || (st = reset_counts(c, n, 4))) return st;
+    if ((st = codes_kernels(c, xyz, n, order, codes, perm, frame, (uint32_t*)c->hist.p))) return st;
+    return direct_passes(c, (uint32_t*)codes, perm, n, 4);
 }
 
 // ============================================================== leaf boxes
@@ -458,8 +777,7 @@ nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t a
     if ((st = ensure(c, c->store, sizeof(int32_t) * (size_t)std::max(nL - 1, 1)))) return st;
     int32_t* codes = (int32_t*)c->codes.p;
     int32_t* perm = (int32_t*)c->perm.p;
-    if ((st = morton_codes(c, xyz_dev, n, order, codes, perm))) return st;
-    if ((st = radix_sort_pairs(c, (uint32_t*)codes, perm, n, 30))) return st;
+    if ((st = order_positions(c, xyz_dev, n, order, codes, perm))) return st;
     float4* keys = (float4*)c->keys.p;
     if (!leaves_only) {
         cudaError_t e = cudaMemsetAsync(keys, 0, 32 * (size_t)nkeys, c->stream);

@@ -180,6 +180,11 @@ nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32
                        int32_t* iota, const float* frame = nullptr);
 // Stable LSD radix sort of (codes, vals) on `bits` low bits; results in codes/vals.
 nd_status radix_sort_pairs(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int bits);
+// Morton codes of n positions, sorted, and the sorting permutation: the two
+// together.  Scratch of the sort (c->hist): sort_scratch_bytes.
+nd_status order_positions(Ctx* c, const float* xyz, int32_t n, int32_t order, int32_t* codes,
+                          int32_t* perm, const float* frame = nullptr);
+size_t sort_scratch_bytes(int32_t n);
 // Full tree pipeline: codes -> sort -> gather -> leaf boxes -> Apetrei build
 // (leaves_only: no internal nodes, all the ordered pair list needs).
 nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t apl,

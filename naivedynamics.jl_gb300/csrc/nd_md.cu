@@ -1663,7 +1663,7 @@ static nd_status md_alloc(MDEngine* m) {
     if ((st = ensure(c, c->perm, sizeof(int32_t) * n))) return st;
     if ((st = ensure(c, c->codes_alt, sizeof(uint32_t) * n))) return st;
     if ((st = ensure(c, c->perm_alt, sizeof(int32_t) * n))) return st;
-    if ((st = ensure(c, c->hist, sizeof(uint32_t) * (256 * (size_t)cdiv(m->n, 2048) + 256)))) return st;
+    if ((st = ensure(c, c->hist, sort_scratch_bytes(m->n)))) return st;
     if ((st = ensure(c, c->misc, 64))) return st;
     return ND_OK;
 }
@@ -1904,10 +1904,9 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
         c->launches++;
         // a batched ensemble sorts on the fixed slot grid, so every system is
         // one contiguous run of the Hilbert order
-        if ((st = morton_codes(c, (const float*)m->xyz32.p, n, m->p.order, codes, perm,
-                               m->nsys > 0 ? m->tree_frame : nullptr)))
+        if ((st = order_positions(c, (const float*)m->xyz32.p, n, m->p.order, codes, perm,
+                                  m->nsys > 0 ? m->tree_frame : nullptr)))
             return st;
-        if ((st = radix_sort_pairs(c, (uint32_t*)codes, perm, n, 30))) return st;
         k_md_reorder<<<g, 256, 0, c->stream>>>(live, tmp, perm, (const float*)m->xyz32.p, n,
                                                m->fr, sys, (float4*)m->pos32.p,
                                                (int4*)m->rec_buf[0].p, (uint2*)m->recf_buf[0].p,

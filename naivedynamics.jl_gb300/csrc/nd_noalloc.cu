@@ -15,7 +15,7 @@
 //     unordered request with a leaf width other than 4 is served by the
 //     ordered emission); larger requests are rejected with ND_ERR_ARG before
 //     any work is enqueued;
-//   * the array (kNoAllocBytes, ~5.3 MB) is reserved on every GPU that loads
+//   * the array (kNoAllocBytes, ~5.4 MB) is reserved on every GPU that loads
 //     the library and stays there until the process exits;
 //   * all calls share the one array, so calls whose work overlaps on the GPU
 //     (different streams, or different host threads) race and corrupt each
@@ -42,7 +42,7 @@ constexpr size_t kPos4B = up256(16ull * kNoAllocMaxAtoms);               // sort
 constexpr size_t kIdxB = up256(4ull * kNoAllocMaxAtoms);                 // sorted index
 constexpr size_t kKeysB = up256(32ull * (2 * kMaxLeaves));               // GridKeys
 constexpr size_t kStoreB = up256(4ull * kMaxLeaves);                     // CAS slots
-constexpr size_t kHistB = up256(4ull * (256 * ((kNoAllocMaxAtoms + 2047) / 2048) + 256));
+constexpr size_t kHistB = up256(4ull * (4 * 256 * ((kNoAllocMaxAtoms + 2047) / 2048) + 256));
 constexpr size_t kCountsB = up256(8ull * (kMaxLeaves + 1));
 constexpr size_t kOffsetsB = up256(8ull * (kMaxLeaves + 2));
 constexpr size_t kPartialB = up256(8ull * (4 * ((kMaxLeaves + 4095) / 4096) + 64));
