@@ -401,11 +401,6 @@ __global__ void k_adj_gpar(const double* __restrict__ part, int32_t nb, double* 
 }
 
 
-// Marks an early refit taken after step t (runs inside the refit's conditional body).
-__global__ void k_adj_flag(uint8_t* flags, int32_t t) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) flags[t] = 1;
-}
-
 // ------------------------------------------------------------------ driver
 //
 // Schedule of one trajectory (t = 0 .. K-1, step t moves x_t to x_{t+1}):
@@ -415,8 +410,8 @@ __global__ void k_adj_flag(uint8_t* flags, int32_t t) {
 //   t % R == 0   otherwise: refit
 //   after step t, inside a window: an early refit when the step kernel finds
 //   an atom that could pass skin/2 in the next step -- decided on the device
-//   in the forward pass (a conditional graph node that also records the
-//   decision), replayed from the record in the backward pass.
+//   in the forward pass (the step's vote, a word of `flags`, gates the refit's
+//   kernels and is the record), replayed from the record in the backward pass.
 
 struct AdjEngine {
     Ctx* parent = nullptr;
@@ -506,14 +501,11 @@ static nd_status adj_copy(AdjEngine* A, void* dst, const void* src, size_t bytes
 }
 
 // One forward step of the engine (records ping-pong as in the plain engine).
-static void adj_step(AdjEngine* A, bool first, int use_cond = 0,
-                     cudaGraphConditionalHandle h = 0, int unchecked = 0) {
+static void adj_step(AdjEngine* A, bool first, unsigned* vote = nullptr, int unchecked = 0) {
     MDEngine* m = A->m;
     StepArgs a = md_step_args(m, m->rc);
-    a.use_cond = use_cond;
-    a.vote = use_cond;
+    a.vote = vote;
     a.unchecked = unchecked;
-    a.cond = h;
     md_launch_step(m, a, first);
     m->rc ^= 1;
 }
@@ -556,7 +548,7 @@ static nd_status adj_enqueue_forward(AdjEngine* A) {
     const size_t n = (size_t)A->n;
     char* ck = (char*)A->ckpt.p;
     cudaMemsetAsync(m->diag.p, 0, sizeof(unsigned long long), c->stream);
-    cudaMemsetAsync(A->flags.p, 0, (size_t)A->K, c->stream);
+    cudaMemsetAsync(A->flags.p, 0, sizeof(unsigned) * (size_t)A->K, c->stream);
     for (int32_t t = 0; t < A->K; ++t) {
         if (t % A->C == 0) {
             const int32_t sg = t / A->C;
@@ -566,22 +558,12 @@ static nd_status adj_enqueue_forward(AdjEngine* A) {
         }
         if ((st = adj_rebuild_before(A, t, true))) return st;
         const bool cond = adj_cond_after(A, t);
-        cudaGraphConditionalHandle h = 0;
-        if (cond && (st = md_cond_handle(m, &h))) return st;
+        unsigned* vote = cond ? (unsigned*)A->flags.p + t : nullptr;
         // the list is used unchecked after this step when no check follows
         // and no scheduled rebuild comes first (the loss at x_K included)
         const bool unchecked = !cond && ((t + 1) % A->R != 0 || t + 1 == A->K);
-        adj_step(A, t == 0, cond ? 1 : 0, h, unchecked ? 1 : 0);
-        if (cond &&
-            (st = md_add_cond_node(m, h, 1, [&](int) {
-                 nd_status s2 = md_rebuild(m, RB_REFIT, m->rc);
-                 if (s2 == ND_OK) {
-                     k_adj_flag<<<1, 32, 0, m->sub.stream>>>((uint8_t*)A->flags.p, t);
-                     m->sub.launches++;
-                 }
-                 return s2;
-             })))
-            return st;
+        adj_step(A, t == 0, vote, unchecked ? 1 : 0);
+        if (cond && (st = md_rebuild(m, RB_REFIT, m->rc, nullptr, false, vote))) return st;
     }
     if ((st = adj_copy(A, A->xK.p, live_set(A), 3 * sizeof(double) * n, "x_K")) ||
         (st = adj_copy(A, A->recK.p, m->rec_buf[m->rc].p, sizeof(int4) * n, "x_K records")))
@@ -792,7 +774,7 @@ nd_status adj_create(Ctx* parent, const nd_md_params* p, int32_t n, const double
         (st = ensure(c, A->cb, sizeof(float) * (size_t)sp.bins)) ||
         (st = ensure(c, A->scal, 4 * sizeof(double))) ||
         (st = ensure(c, A->outs, 12 * sizeof(double) * nn)) ||
-        (st = ensure(c, A->flags, (size_t)A->K))) {
+        (st = ensure(c, A->flags, sizeof(unsigned) * (size_t)A->K))) {
         parent->last_error = c->last_error;
         adj_destroy(A);
         return st;
@@ -849,13 +831,14 @@ nd_status adj_forward(AdjEngine* A, double* hist, double* loss) {
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint forward");
     double sc[4];
     std::vector<double> h((size_t)A->s.bins);
-    std::vector<uint8_t> sched((size_t)A->K);
+    std::vector<unsigned> sched((size_t)A->K);
     unsigned long long viol = 0;
     e = cudaMemcpyAsync(sc, A->scal.p, sizeof(sc), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h.data(), A->hist.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(sched.data(), A->flags.p, sched.size(), cudaMemcpyDeviceToHost, c->stream);
+        e = cudaMemcpyAsync(sched.data(), A->flags.p, sizeof(unsigned) * sched.size(),
+                            cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(&viol, m->diag.p, sizeof(viol), cudaMemcpyDeviceToHost, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint forward");
@@ -865,7 +848,7 @@ nd_status adj_forward(AdjEngine* A, double* hist, double* loss) {
                         "one step: raise skin or lower rebuild_every";
         return ND_ERR_OVERFLOW;
     }
-    A->sched = std::move(sched);
+    A->sched.assign(sched.begin(), sched.end());
     if (hist) std::copy(h.begin(), h.end(), hist);
     if (loss) *loss = sc[0];
     A->have_forward = true;

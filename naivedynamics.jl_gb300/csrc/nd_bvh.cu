@@ -678,11 +678,13 @@ __device__ __forceinline__ void load_box_cg(const float4* keys, int32_t node /*1
 // non-zero slot orders the sibling-box loads, which bypass L1 (ld.cg).  No
 // thread ever waits on another, so the kernel cannot hang; a climb longer than
 // nL levels flags ND_ERR_INTERNAL.  ranges (may be null): leaf range
-// [first, last] of internal node nL + q at ranges[q - 1].
+// [first, last] of internal node nL + q at ranges[q - 1].  gate (may be null):
+// nothing is done while *gate is 0.
 __global__ void k_bvh_build(float4* keys, int32_t* store, const int32_t* __restrict__ code,
-                            int32_t nL, int32_t apl, int2* ranges, int32_t* err) {
+                            int32_t nL, int32_t apl, int2* ranges, int32_t* err,
+                            const unsigned* __restrict__ gate) {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (i > nL) return;
+    if (i > nL || (gate && *gate == 0u)) return;
     int32_t rangel = i, ranger = i;
     int32_t dell = delta_ref(rangel - 1, code, nL, apl);
     int32_t delr = delta_ref(ranger, code, nL, apl);
@@ -755,11 +757,11 @@ __global__ void k_root_overwrite(float4* keys, int32_t nL) {
 }
 
 nd_status build_internal_nodes(Ctx* c, float4* keys, int32_t* store, const int32_t* codes,
-                               int32_t nL, int32_t apl, int2* ranges) {
+                               int32_t nL, int32_t apl, int2* ranges, const unsigned* gate) {
     cudaError_t e = cudaMemsetAsync(store, 0, sizeof(int32_t) * (size_t)(nL - 1), c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "store reset");
     k_bvh_build<<<(int)cdiv(nL, 256), 256, 0, c->stream>>>(keys, store, codes, nL, apl, ranges,
-                                                            c->d_err);
+                                                            c->d_err, gate);
     c->launches++;
     return check_launch(c, "bvh build");
 }

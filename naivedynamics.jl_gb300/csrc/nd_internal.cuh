@@ -211,7 +211,8 @@ nd_status pair_hash(Ctx* c, const int32_t* pi, const int32_t* pj, const float* p
 
 // Apetrei bottom-up build over already prepared leaf keys (used by the MD engine).
 nd_status build_internal_nodes(Ctx* c, float4* keys, int32_t* store, const int32_t* codes_sorted,
-                               int32_t nL, int32_t apl, int2* ranges = nullptr);
+                               int32_t nL, int32_t apl, int2* ranges = nullptr,
+                               const unsigned* gate = nullptr);
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -34,6 +34,7 @@ namespace nd {
 constexpr int kSmallTPA = 4;         // threads per atom of the step kernel for small systems
 constexpr int kSizingFcap = 8192;    // BFS frontier entries per buffer in the sizing build
 constexpr int kSizingUcap = 8192;    // union capacity of the sizing build
+constexpr int kDirectBlocks = 4096;  // blocks whose boxes the union search tests one by one
 constexpr double kMinTunedSkin = 0.1;  // smallest skin the autotuner tries
 
 // Scale of the wrap-around fixed-point grid: a listed pair is within
@@ -140,12 +141,32 @@ __global__ void k_md_init_scalars(const double* __restrict__ q_in, const double*
     if (sid) sid[i] = sid_in[i];
 }
 
+// Words of an engine's control array (ctl): kCtlEarly early refits done,
+// kCtlWindow windows begun, kCtlPressure a list near its capacity since the
+// last re-sort, kCtlDecision the last window's choice, kCtlResorts and
+// kCtlRefits rebuilds done at the start of windows; from kCtlVotes on one word
+// per step of a window: the step's vote for an early refit.
+constexpr int kCtlEarly = 2, kCtlWindow = 3, kCtlPressure = 4, kCtlDecision = 5, kCtlResorts = 6,
+              kCtlRefits = 7, kCtlVotes = 8;
+
+// Start of a window that re-sorts (by thread 0 and the first nvotes threads).
+__device__ __forceinline__ void window_opens(unsigned* ctl, int32_t nvotes, int32_t i, bool resort) {
+    for (int32_t k = i; k < nvotes; k += (int32_t)(gridDim.x * blockDim.x)) ctl[kCtlVotes + k] = 0u;
+    if (i != 0) return;
+    ctl[kCtlWindow] += 1u;
+    ctl[kCtlDecision] = resort ? 1u : 0u;
+    if (resort) ctl[kCtlPressure] = 0u;
+}
+
+// Float32 positions of the order.  ctl (engines that re-sort at every window):
+// the window's bookkeeping, which is otherwise k_md_window_begin's.
 __global__ void k_md_pos32(const double* __restrict__ x0, const double* __restrict__ x1,
                            const double* __restrict__ x2, const int32_t* __restrict__ sid,
                            const SysRow* __restrict__ sys, int32_t n, float* __restrict__ xyz,
-                           unsigned* counter) {
+                           unsigned* counter, unsigned* ctl, int32_t nvotes) {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (counter && i == 0) atomicAdd(counter, 1u);
+    if (ctl) window_opens(ctl, nvotes, i, true);
     if (i >= n) return;
     double o0 = 0.0, o1 = 0.0, o2 = 0.0;
     if (sid) {
@@ -157,92 +178,119 @@ __global__ void k_md_pos32(const double* __restrict__ x0, const double* __restri
     xyz[3 * (int64_t)i + 2] = (float)(x2[i] + o2);
 }
 
-
-// Gather every per-atom array into the new (sorted) order; write the pair
-// records and the Float32 positions of the tree.
-__global__ void k_md_reorder(SetPtrs src, SetPtrs dst, const int32_t* __restrict__ perm,
-                             const float* __restrict__ xyz32, int32_t n, Frame fr,
-                             const SysRow* __restrict__ sys, float4* __restrict__ pos32,
-                             int4* __restrict__ rec, uint2* __restrict__ recf,
-                             int4* __restrict__ recb, int32_t* err) {
+// Gather the state into the new (sorted) order, into the scratch set;
+// k_md_place copies it back, so the live set keeps its addresses and captured
+// graphs stay valid.
+__global__ void k_md_gather(SetPtrs src, SetPtrs dst, const int32_t* __restrict__ perm, int32_t n) {
     int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    int32_t o = perm[k];
-    const SysRow* r = nullptr;
-    if (src.sid) {
-        const int32_t sv = src.sid[o];
-        dst.sid[k] = sv;
-        r = sys + sv;
-    }
-    int32_t f[3];
-    uint32_t g[3];
+    const int32_t o = perm[k];
+    if (src.sid) dst.sid[k] = src.sid[o];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        double xv = src.x[d][o];
-        dst.x[d][k] = xv;
+        dst.x[d][k] = src.x[d][o];
         dst.w[d][k] = src.w[d][o];
-        f[d] = to_fixed(xv, r ? r->o[d] : fr.o[d], r ? r->s : fr.s, r ? r->lim : fr.lim, err, k,
-                        g[d]);
     }
-    recf[k] = pack_fine(g[0], g[1], g[2]);
-    double qv = src.q[o];
-    dst.q[k] = qv;
+    dst.q[k] = src.q[o];
     dst.im[k] = src.im[o];
     dst.orig[k] = src.orig[o];
-    pos32[k] = make_float4(xyz32[3 * (int64_t)o], xyz32[3 * (int64_t)o + 1],
-                           xyz32[3 * (int64_t)o + 2], __int_as_float(k));
-    rec[k] = make_int4(f[0], f[1], f[2], __float_as_int((float)qv));
-    recb[k] = rec[k];
-}
-
-// Copy a state set (after the gather into the scratch set, so the live set
-// keeps its addresses and captured graphs stay valid).
-__global__ void k_md_copy_set(SetPtrs src, SetPtrs dst, int32_t n) {
-    int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        dst.x[d][k] = src.x[d][k];
-        dst.w[d][k] = src.w[d][k];
-    }
-    dst.q[k] = src.q[k];
-    dst.im[k] = src.im[k];
-    dst.orig[k] = src.orig[k];
-    if (src.sid) dst.sid[k] = src.sid[k];
 }
 
 // Start of a rebuild window: re-sort on the schedule (every resort_every-th
 // window) or when some list has passed 90% of its capacity since the last
-// re-sort (the kept tree has loosened); refit otherwise.  ctl[3] counts
-// windows, ctl[4] holds the capacity-pressure flag, ctl[5] the decision.
-__global__ void k_md_window_begin(unsigned* ctl, int32_t resort_every,
+// re-sort (the kept tree has loosened); refit otherwise.
+__global__ void k_md_window_begin(unsigned* ctl, int32_t resort_every, int32_t nvotes,
                                   cudaGraphConditionalHandle h, int32_t use_cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const unsigned w = ctl[3];
-    const unsigned need = (w % (unsigned)resort_every == 0u || ctl[4] != 0u) ? 1u : 0u;
-    ctl[3] = w + 1u;
-    if (need) ctl[4] = 0u;
-    ctl[5] = need;
-    if (use_cond) cudaGraphSetConditional(h, need);
+    __shared__ unsigned s_need;
+    if (threadIdx.x == 0)
+        s_need = ctl[kCtlWindow] % (unsigned)resort_every == 0u || ctl[kCtlPressure] != 0u;
+    __syncthreads();
+    window_opens(ctl, nvotes, (int32_t)threadIdx.x, s_need != 0u);
+    if (threadIdx.x == 0 && use_cond) cudaGraphSetConditional(h, s_need);
 }
 
-// Leaf boxes (p -/+ h) of already sorted Float32 positions.
-__global__ void k_md_leaf_boxes(const float4* __restrict__ pos, int32_t nL, int32_t apl, float h,
-                                float4* __restrict__ keys) {
-    int32_t leaf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (leaf >= nL) return;
-    int64_t bird = (int64_t)leaf * apl;
-    float4 p0 = pos[bird];
-    float mn[3] = {__fsub_rn(p0.x, h), __fsub_rn(p0.y, h), __fsub_rn(p0.z, h)};
-    float mx[3] = {__fadd_rn(p0.x, h), __fadd_rn(p0.y, h), __fadd_rn(p0.z, h)};
-    for (int32_t a = 1; a < apl; ++a) {
-        float4 p = pos[bird + a];
-        mn[0] = jl_min(mn[0], __fsub_rn(p.x, h)); mx[0] = jl_max(mx[0], __fadd_rn(p.x, h));
-        mn[1] = jl_min(mn[1], __fsub_rn(p.y, h)); mx[1] = jl_max(mx[1], __fadd_rn(p.y, h));
-        mn[2] = jl_min(mn[2], __fsub_rn(p.z, h)); mx[2] = jl_max(mx[2], __fadd_rn(p.z, h));
+// Everything a rebuild derives from the positions in their (new or kept)
+// order, one block per kBlock atoms: Float32 positions, pair records and the
+// build records of the skin check, the leaf boxes (atoms -/+ h), the block's
+// box.  COPY (re-sort): the state comes from the gathered set src and is
+// written back to st.  gate (early refits): nothing is done while *gate is 0.
+// One kernel in place of a gather's record part, a copy, a leaf-box and a
+// block-box kernel: each was bound by its launch and one trip to memory.
+template <bool COPY>
+__global__ void __launch_bounds__(kBlock)
+    k_md_place(SetPtrs src, SetPtrs st, int32_t n, Frame fr, const SysRow* __restrict__ sys,
+               int32_t apl, float h, float4* __restrict__ pos32, int4* __restrict__ rec,
+               uint2* __restrict__ recf, int4* __restrict__ recb, float4* __restrict__ keys,
+               float4* __restrict__ bbox, int32_t* err, const unsigned* __restrict__ gate,
+               unsigned* counter) {
+    if (gate && *gate == 0u) return;
+    __shared__ float s_b[kBlock / 32][6];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int32_t k = (int32_t)blockIdx.x * kBlock + tid;
+    if (counter && k == 0) atomicAdd(counter, 1u);
+    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (k < n) {
+        const SetPtrs& from = COPY ? src : st;
+        const SysRow* r = nullptr;
+        if (from.sid) {
+            const int32_t sv = from.sid[k];
+            r = sys + sv;
+            if (COPY) st.sid[k] = sv;
+        }
+        int32_t f[3];
+        uint32_t g[3];
+        float xf[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double xv = from.x[d][k];
+            if (COPY) {
+                st.x[d][k] = xv;
+                st.w[d][k] = from.w[d][k];
+            }
+            xf[d] = (float)(r ? xv + r->off[d] : xv);
+            f[d] = to_fixed(xv, r ? r->o[d] : fr.o[d], r ? r->s : fr.s, r ? r->lim : fr.lim, err, k,
+                            g[d]);
+            mn[d] = __fsub_rn(xf[d], h);
+            mx[d] = __fadd_rn(xf[d], h);
+        }
+        const double qv = from.q[k];
+        if (COPY) {
+            st.q[k] = qv;
+            st.im[k] = from.im[k];
+            st.orig[k] = from.orig[k];
+        }
+        recf[k] = pack_fine(g[0], g[1], g[2]);
+        pos32[k] = make_float4(xf[0], xf[1], xf[2], __int_as_float(k));
+        const int4 rv = make_int4(f[0], f[1], f[2], __float_as_int((float)qv));
+        rec[k] = rv;
+        recb[k] = rv;
     }
-    keys[2 * (int64_t)leaf] = make_float4(mn[0], mn[1], mn[2], mx[0]);
-    keys[2 * (int64_t)leaf + 1] = make_float4(mx[1], mx[2], __int_as_float(0), __int_as_float(0));
+    // leaf boxes over the leaf's lanes, then the warp's and the block's box
+    auto widen = [&](int from, int to) {
+        for (int s = from; s < to; s <<= 1)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], s));
+                mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], s));
+            }
+    };
+    widen(1, apl);
+    if (k < n && (tid & (apl - 1)) == 0) {
+        const int64_t leaf = k / apl;
+        keys[2 * leaf] = make_float4(mn[0], mn[1], mn[2], mx[0]);
+        keys[2 * leaf + 1] = make_float4(mx[1], mx[2], __int_as_float(0), __int_as_float(0));
+    }
+    widen(apl, 32);
+    if (lane == 0)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) { s_b[warp][d] = mn[d]; s_b[warp][3 + d] = mx[d]; }
+    __syncthreads();
+    if (tid < 6) {
+        float v = s_b[0][tid];
+        for (int w = 1; w < kBlock / 32; ++w)
+            v = tid < 3 ? fminf(v, s_b[w][tid]) : fmaxf(v, s_b[w][tid]);
+        reinterpret_cast<float*>(bbox)[8 * (int64_t)blockIdx.x + tid] = v;
+    }
 }
 
 // ------------------------------------------------ block union (tree BFS)
@@ -256,56 +304,30 @@ __device__ __forceinline__ bool box_overlap(float qmnx, float qmny, float qmnz, 
            (qmxz > a.z);
 }
 
-// Boxes of the blocks of kBlock atoms (the union of their leaves' key boxes,
-// exact: min / max only) and of the super-blocks of 32 blocks, stored like
-// tree nodes (min xyz, max x), (max y, max z, 0, 0): blocks at [0, nblocks),
-// super-blocks after them.  One thread block of 32 warps per super-block,
-// one warp per block.
-__global__ void __launch_bounds__(1024)
-    k_md_block_boxes(const float4* __restrict__ keys, int32_t nL, int32_t nblocks, int32_t lpb,
-                     float4* __restrict__ bbox) {
-    __shared__ float s_b[32][6];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int32_t b = blockIdx.x * 32 + w;
-    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+// Boxes of the super-blocks of 32 blocks, after the blocks' own boxes (stored
+// like tree nodes: min xyz, max x), (max y, max z, 0, 0)): one warp each.
+__global__ void __launch_bounds__(256)
+    k_md_super_boxes(int32_t nblocks, float4* __restrict__ bbox, const unsigned* __restrict__ gate) {
+    if (gate && *gate == 0u) return;
+    const int lane = threadIdx.x & 31;
+    const int32_t sb = (int32_t)blockIdx.x * 8 + (int32_t)(threadIdx.x >> 5);
+    if (sb * 32 >= nblocks) return;
+    const int32_t b = sb * 32 + lane;
+    float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
     if (b < nblocks) {
-        const int32_t l1 = min((b + 1) * lpb, nL);
-        for (int32_t l = b * lpb + lane; l < l1; l += 32) {
-            const float4 a = __ldg(&keys[2 * (int64_t)l]), c = __ldg(&keys[2 * (int64_t)l + 1]);
-            mn[0] = fminf(mn[0], a.x); mn[1] = fminf(mn[1], a.y); mn[2] = fminf(mn[2], a.z);
-            mx[0] = fmaxf(mx[0], a.w); mx[1] = fmaxf(mx[1], c.x); mx[2] = fmaxf(mx[2], c.y);
-        }
+        const float4 p = __ldg(&bbox[2 * (int64_t)b]), q = __ldg(&bbox[2 * (int64_t)b + 1]);
+        v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w; v[4] = q.x; v[5] = q.y;
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d)
         for (int s = 16; s > 0; s >>= 1) {
-            mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], s));
-            mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], s));
+            v[d] = fminf(v[d], __shfl_xor_sync(0xffffffffu, v[d], s));
+            v[3 + d] = fmaxf(v[3 + d], __shfl_xor_sync(0xffffffffu, v[3 + d], s));
         }
     if (lane == 0) {
-        if (b < nblocks) {
-            bbox[2 * (int64_t)b] = make_float4(mn[0], mn[1], mn[2], mx[0]);
-            bbox[2 * (int64_t)b + 1] = make_float4(mx[1], mx[2], 0.f, 0.f);
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) { s_b[w][d] = mn[d]; s_b[w][3 + d] = mx[d]; }
-    }
-    __syncthreads();
-    if (w == 0) {
-        float v[6];
-#pragma unroll
-        for (int d = 0; d < 6; ++d) v[d] = s_b[lane][d];
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-            for (int s = 16; s > 0; s >>= 1) {
-                v[d] = fminf(v[d], __shfl_xor_sync(0xffffffffu, v[d], s));
-                v[3 + d] = fmaxf(v[3 + d], __shfl_xor_sync(0xffffffffu, v[3 + d], s));
-            }
-        if (lane == 0) {
-            const int64_t sb = nblocks + (int64_t)blockIdx.x;
-            bbox[2 * sb] = make_float4(v[0], v[1], v[2], v[3]);
-            bbox[2 * sb + 1] = make_float4(v[4], v[5], 0.f, 0.f);
-        }
+        const int64_t at = (int64_t)nblocks + sb;
+        bbox[2 * at] = make_float4(v[0], v[1], v[2], v[3]);
+        bbox[2 * at + 1] = make_float4(v[4], v[5], 0.f, 0.f);
     }
 }
 
@@ -337,11 +359,12 @@ __device__ __forceinline__ int32_t block_compact(bool keep, int32_t value, int32
 // eight warp boxes (their atoms -/+ hq) joins the block's union, sorted by
 // leaf index so list order, and hence force summation order, is
 // deterministic.  Two searches give the same union:
-//  - blocks (tree == 0): the super-block boxes, then the boxes of the blocks
-//    of overlapping super-blocks, are tested against the union of the warp
-//    boxes (a leaf overlapping a warp box lies in a block and a super-block
-//    whose boxes overlap that union); the leaves of the candidate blocks are
-//    tested against the warp boxes.  Enumerating in index order at every
+//  - blocks (tree == 0): the boxes of all blocks, or with more than
+//    kDirectBlocks of them the super-block boxes and then the boxes of the
+//    blocks of overlapping super-blocks, are tested against the union of the
+//    warp boxes (a leaf overlapping a warp box lies in a block and a
+//    super-block whose boxes overlap that union); the leaves of the candidate
+//    blocks are tested against the warp boxes.  Enumerating in index order at every
 //    level leaves the union sorted.
 //  - tree (tree == 1): the warp boxes are tested against the tree
 //    breadth-first -- all 256 threads expand the current level together, a
@@ -358,7 +381,8 @@ __global__ void __launch_bounds__(kBlock)
                      int32_t* __restrict__ ucount,
                      uint16_t* __restrict__ llist_leaf, int32_t* __restrict__ lcount_leaf,
                      int32_t lcap_leaf, int32_t* err, int32_t* diag, int32_t sizing,
-                     unsigned* pressure) {
+                     unsigned* pressure, const unsigned* __restrict__ gate) {
+    if (gate && *gate == 0u) return;
     extern __shared__ int32_t smem[];
     int32_t* fr[2] = {smem, smem + fcap};
     int32_t* su = smem + 2 * fcap;
@@ -413,7 +437,8 @@ __global__ void __launch_bounds__(kBlock)
                     u5 = s_ub[5];
         int32_t* csb = fr[0];
         int32_t* cb = fr[1];
-        const int32_t nsb = (nblocks + 31) >> 5;
+        const bool direct = nblocks <= kDirectBlocks;
+        const int32_t nsb = direct ? 0 : (nblocks + 31) >> 5;
         int32_t ncs = 0;
         for (int32_t base = 0; base < nsb; base += kBlock) {
             const int32_t s = base + tid;
@@ -423,10 +448,10 @@ __global__ void __launch_bounds__(kBlock)
             ncs += block_compact(keep, s, csb, ncs, fcap, s_w);
         }
         int32_t ncb = 0;
-        const int32_t ks = min(ncs, fcap) * 32;
+        const int32_t ks = direct ? nblocks : min(ncs, fcap) * 32;
         for (int32_t base = 0; base < ks; base += kBlock) {
             const int32_t k = base + tid;
-            const int32_t b = k < ks ? csb[k >> 5] * 32 + (k & 31) : nblocks;
+            const int32_t b = direct ? k : k < ks ? csb[k >> 5] * 32 + (k & 31) : nblocks;
             const bool keep = b < nblocks && box_overlap(u0, u1, u2, u3, u4, u5,
                                                          __ldg(&bbox[2 * (int64_t)b]),
                                                          __ldg(&bbox[2 * (int64_t)b + 1]));
@@ -674,7 +699,9 @@ __global__ void __launch_bounds__(kBlock)
                      const int32_t* __restrict__ ucount, const uint16_t* __restrict__ llist_leaf,
                      const int32_t* __restrict__ lcount_leaf, int32_t lcap_leaf, int32_t lcap,
                      uint16_t* __restrict__ llist, int32_t* __restrict__ ncount, int32_t* err,
-                     int32_t* diag, int32_t sizing, unsigned* pressure) {
+                     int32_t* diag, int32_t sizing, unsigned* pressure,
+                     const unsigned* __restrict__ gate) {
+    if (gate && *gate == 0u) return;
     extern __shared__ float4 spos[];
     const int tid = threadIdx.x;
     const int32_t* __restrict__ U = ulist + (int64_t)blockIdx.x * ucap;
@@ -765,34 +792,6 @@ __global__ void __launch_bounds__(kBlock)
     if (cnt > lcap && !sizing) set_error(err, ND_ERR_OVERFLOW, (int32_t)i);
     atomicMax(&diag[1], cnt);
     if (pressure && 10 * cnt > 9 * lcap) atomicOr(pressure, 1u);
-}
-
-// Refit: positions changed, order and tree topology kept.  Float32 positions
-// and pair records (and the build records of the skin check) from the FP64
-// state in its current order.
-__global__ void k_md_refit_pos(SetPtrs st, int32_t n, Frame fr, const SysRow* __restrict__ sys,
-                               float4* __restrict__ pos32, int4* __restrict__ rec,
-                               uint2* __restrict__ recf, int4* __restrict__ recb, int32_t* err,
-                               unsigned* counter) {
-    int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (counter && k == 0) atomicAdd(counter, 1u);
-    if (k >= n) return;
-    const SysRow* r = st.sid ? sys + st.sid[k] : nullptr;
-    int32_t f[3];
-    uint32_t g[3];
-    float xf[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        double xv = st.x[d][k];
-        xf[d] = (float)(r ? xv + r->off[d] : xv);
-        f[d] = to_fixed(xv, r ? r->o[d] : fr.o[d], r ? r->s : fr.s, r ? r->lim : fr.lim, err, k,
-                        g[d]);
-    }
-    recf[k] = pack_fine(g[0], g[1], g[2]);
-    pos32[k] = make_float4(xf[0], xf[1], xf[2], __int_as_float(k));
-    const int4 rv = make_int4(f[0], f[1], f[2], __float_as_int((float)st.q[k]));
-    rec[k] = rv;
-    recb[k] = rv;
 }
 
 // ------------------------------------------------------------- step kernel
@@ -1188,9 +1187,7 @@ __device__ __forceinline__ unsigned accum_pair2(const int4& ri, const int4& ra, 
 }
 
 // One block per 256 atoms.  MODE 0: step (force, pending half kick, kick,
-// drift, reflect, next record).  MODE 2: the same step inside a captured
-// window, whose last block also sets the early-refit condition of the graph
-// node after it.  MODE 1: measure (force, integer-step velocity and
+// drift, reflect, next record).  MODE 1: measure (force, integer-step velocity and
 // energies; state untouched).  MODE 3: measure without the potential energy
 // (forces and velocities for a read-back or a thermostat: the double-precision
 // pair energies are most of a measure pass's time).
@@ -1539,22 +1536,9 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             trig = sqrtf(e2) + a.trig_k * sqrtf(sx * sx + sy * sy + sz * sz) > 0.95f * hsu;
         }
         }
-        // Early refit request: the block votes, and the last block to finish
-        // (a ticket counter, no waiting) publishes the flag to the graph's
-        // conditional node that follows this step.
-        if (__syncthreads_or(trig) && threadIdx.x == 0) atomicOr(&a.ctl[0], 1u);
-        if constexpr (MODE == 2) {
-            if (threadIdx.x == 0) {
-                __threadfence();
-                const unsigned ticket = atomicAdd(&a.ctl[1], 1u);
-                if (ticket == gridDim.x - 1) {
-                    __threadfence();
-                    const unsigned f = atomicExch(&a.ctl[0], 0u);
-                    atomicExch(&a.ctl[1], 0u);
-                    cudaGraphSetConditional(a.cond, f ? 1u : 0u);
-                }
-            }
-        }
+        // Early refit request: the refit kernels that follow a voting step do
+        // nothing while its word is 0.
+        if (a.vote && __syncthreads_or(trig) && threadIdx.x == 0) atomicOr(a.vote, 1u);
     }
 }
 
@@ -1622,6 +1606,12 @@ __global__ void k_pair_forces(const double* __restrict__ x, const double* __rest
 // ------------------------------------------------------------- engine
 
 
+// Steps of a window that vote, and the bytes of the control array.
+static int32_t md_votes(const MDEngine* m) { return m->p.rebuild_every; }
+static size_t md_ctl_bytes(const MDEngine* m) {
+    return sizeof(unsigned) * (size_t)(kCtlVotes + md_votes(m));
+}
+
 static nd_status md_alloc(MDEngine* m) {
     Ctx* c = &m->sub;
     const size_t n = (size_t)m->n;
@@ -1653,8 +1643,8 @@ static nd_status md_alloc(MDEngine* m) {
     if ((st = ensure(c, m->acc, std::max<size_t>(64, 2 * sizeof(double) * (size_t)m->nsys)))) return st;
     if ((st = ensure(c, m->diag, 64))) return st;
     if (cudaMemsetAsync(m->diag.p, 0, 64, c->stream) != cudaSuccess) return ND_ERR_CUDA;
-    if ((st = ensure(c, m->ctl, 64))) return st;
-    if (cudaMemsetAsync(m->ctl.p, 0, 64, c->stream) != cudaSuccess) return ND_ERR_CUDA;
+    if ((st = ensure(c, m->ctl, md_ctl_bytes(m)))) return st;
+    if (cudaMemsetAsync(m->ctl.p, 0, md_ctl_bytes(m), c->stream) != cudaSuccess) return ND_ERR_CUDA;
     if ((st = ensure(c, m->obs, 64))) return st;
     if (cudaMemsetAsync(m->obs.p, 0, 64, c->stream) != cudaSuccess) return ND_ERR_CUDA;
     if ((st = ensure(c, m->obs_part, sizeof(double) * (size_t)cdiv(m->n, 256)))) return st;
@@ -1754,8 +1744,8 @@ static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t
         e = raise_smem_limit((const void*)k_md_step<C, MODE, false, kSmallTPA, 2>, maxsm);      \
     if (e == cudaSuccess)                                                                       \
         e = raise_smem_limit((const void*)k_md_step<C, MODE, false, kSmallTPA, 4>, maxsm);
-    ND_SMEM(true, 0) ND_SMEM(false, 0) ND_SMEM(true, 1) ND_SMEM(false, 1) ND_SMEM(true, 2)
-    ND_SMEM(false, 2) ND_SMEM(true, 3) ND_SMEM(false, 3)
+    ND_SMEM(true, 0) ND_SMEM(false, 0) ND_SMEM(true, 1) ND_SMEM(false, 1) ND_SMEM(true, 3)
+    ND_SMEM(false, 3)
 #undef ND_SMEM
     if (e != cudaSuccess) return cuda_fail(c, e, "shared memory opt-in");
     return ND_OK;
@@ -1802,10 +1792,7 @@ StepArgs md_step_args(MDEngine* m, int rec_in) {
     const float hs = (float)(std::max(0.0, 0.5 * p.skin - 4.0 * ulp) * S);
     a.half_skin2u = hs * hs;
     a.hsu = hs;
-    a.ctl = (unsigned*)m->ctl.p;
-    a.cond = 0;
-    a.use_cond = 0;
-    a.vote = 1;
+    a.vote = nullptr;
     a.trig_k = 2.0f * (float)std::max(m->check_every - 1, 1);
     a.unchecked = 0;
     for (int d = 0; d < 3; ++d) {
@@ -1830,7 +1817,7 @@ StepArgs md_step_args(MDEngine* m, int rec_in) {
 }
 
 template <int MODE>
-static void launch_step_impl(MDEngine* m, const StepArgs& a0, bool first) {
+static void launch_step(MDEngine* m, const StepArgs& a0, bool first) {
     Ctx* c = &m->sub;
     const unsigned grid = (unsigned)m->nblocks;
     const size_t sm = m->step_smem;
@@ -1854,19 +1841,8 @@ static void launch_step_impl(MDEngine* m, const StepArgs& a0, bool first) {
     c->launches++;
 }
 
-// MODE 0 steps inside a captured window publish their early-refit vote to the
-// conditional node after them (MODE 2); the others are plain kernels.
-template <int MODE>
-static void launch_step(MDEngine* m, const StepArgs& a, bool first) {
-    if (MODE == 0 && a.use_cond) launch_step_impl<2>(m, a, first);
-    else launch_step_impl<MODE>(m, a, first);
-}
-
 void md_launch_step(MDEngine* m, const StepArgs& a, bool first) { launch_step<0>(m, a, first); }
 
-// ctl words: [0] early-refit request, [1] finished-block tickets, [2] early
-// refits done, [3] window counter, [4] capacity pressure, [5] rebuild
-// decision, [6] re-sorts done, [7] scheduled refits done.
 static unsigned* ctl_word(MDEngine* m, int k) { return (unsigned*)m->ctl.p + k; }
 
 // Rebuild of the neighbour lists.
@@ -1878,8 +1854,11 @@ static unsigned* ctl_word(MDEngine* m, int k) { return (unsigned*)m->ctl.p + k; 
 // rec >= 0: a refit inside a window (early refit) whose records go to record
 // buffer `rec`, the one the next step reads; otherwise records go to buffer 0
 // and the step parity restarts.  counter: device count of this kind of
-// rebuild (nullptr: not counted).  sizing: capacity-sizing pass.
-nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool sizing) {
+// rebuild (nullptr: not counted).  sizing: capacity-sizing pass.  gate: device
+// word; the kernels (of a refit) do nothing while it is 0.  opens: a re-sort
+// that is its window's unconditional start and does its bookkeeping.
+nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool sizing,
+                     const unsigned* gate, bool opens) {
     NvtxRange nv(kind == RB_REFIT ? "nd md rebuild (refit)" : "nd md rebuild (re-sort)");
     Ctx* c = &m->sub;
     const int32_t n = m->n;
@@ -1889,55 +1868,54 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
     nd_status st;
     const SysRow* sys = (const SysRow*)m->sysrow.p;
     SetPtrs& live = m->set[0];
-    // a new list answers any pending early-refit request
-    if (cudaMemsetAsync(m->ctl.p, 0, 2 * sizeof(unsigned), c->stream) != cudaSuccess)
-        return cuda_fail(c, cudaGetLastError(), "md rebuild");
-    if (kind == RB_REFIT) {
-        k_md_refit_pos<<<g, 256, 0, c->stream>>>(
-            live, n, m->fr, sys, (float4*)m->pos32.p, (int4*)m->rec_buf[rec >= 0 ? rec : 0].p,
-            (uint2*)m->recf_buf[rec >= 0 ? rec : 0].p, (int4*)m->recb.p, c->d_err, counter);
+    SetPtrs& tmp = m->set[1];
+    float4* keys = (float4*)m->keys.p;
+    float4* bbox = (float4*)m->bbox.p;
+    const float rl = (float)(m->p.cutoff + m->p.skin);
+    const int rb = rec >= 0 ? rec : 0;
+    auto place = [&](auto copy) {
+        k_md_place<decltype(copy)::value><<<(unsigned)m->nblocks, kBlock, 0, c->stream>>>(
+            tmp, live, n, m->fr, sys, m->apl, rl / 2.0f, (float4*)m->pos32.p,
+            (int4*)m->rec_buf[rb].p, (uint2*)m->recf_buf[rb].p, (int4*)m->recb.p, keys, bbox,
+            c->d_err, gate, kind == RB_REFIT ? counter : nullptr);
         c->launches++;
+    };
+    if (kind == RB_REFIT) {
+        place(std::false_type{});
     } else {
-        SetPtrs& tmp = m->set[1];
         k_md_pos32<<<g, 256, 0, c->stream>>>(live.x[0], live.x[1], live.x[2], live.sid, sys, n,
-                                             (float*)m->xyz32.p, counter);
+                                             (float*)m->xyz32.p, counter,
+                                             opens ? (unsigned*)m->ctl.p : nullptr, md_votes(m));
         c->launches++;
         // a batched ensemble sorts on the fixed slot grid, so every system is
         // one contiguous run of the Hilbert order
         if ((st = order_positions(c, (const float*)m->xyz32.p, n, m->p.order, codes, perm,
                                   m->nsys > 0 ? m->tree_frame : nullptr)))
             return st;
-        k_md_reorder<<<g, 256, 0, c->stream>>>(live, tmp, perm, (const float*)m->xyz32.p, n,
-                                               m->fr, sys, (float4*)m->pos32.p,
-                                               (int4*)m->rec_buf[0].p, (uint2*)m->recf_buf[0].p,
-                                               (int4*)m->recb.p, c->d_err);
-        k_md_copy_set<<<g, 256, 0, c->stream>>>(tmp, live, n);
-        c->launches += 2;
+        k_md_gather<<<g, 256, 0, c->stream>>>(live, tmp, perm, n);
+        c->launches++;
+        place(std::true_type{});
     }
-    unsigned* pressure = sizing ? nullptr : ctl_word(m, 4);
-    float4* keys = (float4*)m->keys.p;
-    const float rl = (float)(m->p.cutoff + m->p.skin);
-    k_md_leaf_boxes<<<(unsigned)cdiv(m->nL, 128), 128, 0, c->stream>>>(
-        (const float4*)m->pos32.p, m->nL, m->apl, rl / 2.0f, keys);
-    c->launches++;
+    unsigned* pressure = sizing ? nullptr : ctl_word(m, kCtlPressure);
     const bool tree = m->p.union_search == ND_UNION_TREE;
     if (tree) {
-        if ((st = build_internal_nodes(c, keys, (int32_t*)m->store.p, codes, m->nL, m->apl)))
+        if ((st = build_internal_nodes(c, keys, (int32_t*)m->store.p, codes, m->nL, m->apl,
+                                       nullptr, gate)))
             return st;
-    } else {
-        k_md_block_boxes<<<(unsigned)cdiv(m->nblocks, 32), 1024, 0, c->stream>>>(
-            keys, m->nL, m->nblocks, kBlock / m->apl, (float4*)m->bbox.p);
+    } else if (m->nblocks > kDirectBlocks) {
+        k_md_super_boxes<<<(unsigned)cdiv(m->nblocks, 256), 256, 0, c->stream>>>(m->nblocks, bbox,
+                                                                                 gate);
         c->launches++;
     }
     // query boxes slightly above r_list/2 so the box tests never drop a pair;
     // the distance test alone decides membership
     const float hq = (rl / 2.0f) * 1.0001f + 1e-6f;
     k_md_block_union<<<(unsigned)m->nblocks, kBlock, m->union_smem, c->stream>>>(
-        keys, (const float4*)m->bbox.p, m->nblocks, tree ? 1 : 0, (const float4*)m->pos32.p,
+        keys, bbox, m->nblocks, tree ? 1 : 0, (const float4*)m->pos32.p,
         live.sid, n, m->nL, m->apl, hq, rl, m->fcap, m->ucap,
         m->upow2, (int32_t*)m->ulist.p, (int32_t*)m->ucount.p, (uint16_t*)m->llist_leaf.p,
         (int32_t*)m->lcount_leaf.p, m->lcap_leaf, c->d_err, (int32_t*)m->diag.p + 2,
-        sizing ? 1 : 0, pressure);
+        sizing ? 1 : 0, pressure, gate);
 #define ND_LISTS(A)                                                                             \
     k_md_block_lists<A><<<(unsigned)m->nblocks, kBlock, m->lists_smem, c->stream>>>(            \
         (const float4*)m->pos32.p, n, rl * rl,                                                  \
@@ -1946,7 +1924,7 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
         (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p,                                \
         (const uint16_t*)m->llist_leaf.p, (const int32_t*)m->lcount_leaf.p, m->lcap_leaf,       \
         m->lcap, (uint16_t*)m->llist.p, (int32_t*)m->ncount.p, c->d_err,                        \
-        (int32_t*)m->diag.p + 2, sizing ? 1 : 0, pressure)
+        (int32_t*)m->diag.p + 2, sizing ? 1 : 0, pressure, gate)
     switch (m->apl) {
         case 1: ND_LISTS(1); break;
         case 2: ND_LISTS(2); break;
@@ -1961,16 +1939,23 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
     return check_launch(c, "md rebuild");
 }
 
-// Rebuild at the start of a window, re-sort or refit as k_md_window_begin
-// decides on the device: inside a capture an IF/ELSE node, otherwise after
-// reading the decision back.
+// Rebuild at the start of a window.  An engine that re-sorts every time needs
+// no decision; otherwise re-sort or refit as k_md_window_begin decides on the
+// device: inside a capture an IF/ELSE node (about 11 us of GPU time), else
+// after reading the decision back.
 static nd_status md_window_begin(MDEngine* m, bool capture) {
     NvtxRange nv("nd md window begin");
     Ctx* c = &m->sub;
     nd_status st;
+    const int64_t l0 = c->launches;
+    if (m->resort_every == 1) {
+        st = md_rebuild(m, RB_RESORT, -1, ctl_word(m, kCtlResorts), false, nullptr, true);
+        m->resort_kernels = c->launches - l0;
+        return st;
+    }
     cudaGraphConditionalHandle h = 0;
     if (capture && (st = md_cond_handle(m, &h))) return st;
-    k_md_window_begin<<<1, 32, 0, c->stream>>>((unsigned*)m->ctl.p, m->resort_every, h,
+    k_md_window_begin<<<1, 32, 0, c->stream>>>((unsigned*)m->ctl.p, m->resort_every, md_votes(m), h,
                                                capture ? 1 : 0);
     c->launches++;
     if (capture) {
@@ -1978,22 +1963,22 @@ static nd_status md_window_begin(MDEngine* m, bool capture) {
         nd_status s2 = md_add_cond_node(
             m, h, 2,
             [&](int k) {
-                return k == 0 ? md_rebuild(m, RB_RESORT, -1, ctl_word(m, 6))
-                              : md_rebuild(m, RB_REFIT, -1, ctl_word(m, 7));
+                return k == 0 ? md_rebuild(m, RB_RESORT, -1, ctl_word(m, kCtlResorts))
+                              : md_rebuild(m, RB_REFIT, -1, ctl_word(m, kCtlRefits));
             },
             nk);
         if (s2 == ND_OK) { m->resort_kernels = nk[0]; m->refit_kernels = nk[1]; }
         return s2;
     }
     unsigned need = 0;
-    cudaError_t e = cudaMemcpyAsync(&need, ctl_word(m, 5), sizeof(need), cudaMemcpyDeviceToHost,
-                                    c->stream);
+    cudaError_t e = cudaMemcpyAsync(&need, ctl_word(m, kCtlDecision), sizeof(need),
+                                    cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "rebuild decision");
-    const int64_t l0 = c->launches;
-    st = need ? md_rebuild(m, RB_RESORT, -1, ctl_word(m, 6))
-              : md_rebuild(m, RB_REFIT, -1, ctl_word(m, 7));
-    m->eager_bodies += c->launches - l0;
+    const int64_t l1 = c->launches;
+    st = need ? md_rebuild(m, RB_RESORT, -1, ctl_word(m, kCtlResorts))
+              : md_rebuild(m, RB_REFIT, -1, ctl_word(m, kCtlRefits));
+    m->eager_bodies += c->launches - l1;
     return st;
 }
 
@@ -2008,8 +1993,8 @@ __global__ void k_md_due(const unsigned* __restrict__ ctl, int32_t R, int32_t p,
                          int32_t every_l, cudaGraphConditionalHandle ht,
                          cudaGraphConditionalHandle hl) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    // ctl[3] is the current window's number + 1
-    const long long g = (long long)(ctl[3] - 1u) * R + p + 1;
+    // the window counter is the current window's number + 1
+    const long long g = (long long)(ctl[kCtlWindow] - 1u) * R + p + 1;
     if (every_t > 0) cudaGraphSetConditional(ht, g % every_t == 0 ? 1u : 0u);
     if (every_l > 0) cudaGraphSetConditional(hl, g % every_l == 0 ? 1u : 0u);
 }
@@ -2158,10 +2143,11 @@ static nd_status md_observe(MDEngine* m, int32_t p, bool capture, int64_t g) {
 // Enqueue `k` steps of the current window, the first at window position pos0.
 // After the window's steps 0, M, 2M, ... (M = check_every) but not its last, a
 // refit runs if some atom could pass skin/2 from its list-build position
-// before the next check: inside a capture as a conditional node (one handle
-// per node, set by the step before it), otherwise eagerly after reading the
-// request flag.  ev (eager only): a pair
-// of events per step recorded around the step kernel.
+// before the next check: inside a capture its kernels follow every such step
+// and do nothing while the step's vote is 0 (three empty kernels, about 5 us,
+// where a conditional node took about 11 us whether it ran or not), otherwise
+// eagerly after reading the vote.  ev (eager only): a pair of events per step
+// recorded around the step kernel.
 static nd_status md_steps(MDEngine* m, int32_t k, int32_t pos0, bool capture = false,
                           cudaEvent_t* ev = nullptr) {
     NvtxRange nv(capture ? "nd md capture steps" : "nd md steps");
@@ -2172,33 +2158,28 @@ static nd_status md_steps(MDEngine* m, int32_t k, int32_t pos0, bool capture = f
         // a check follows the window's steps 0, M, 2M, ... but not its last
         const int32_t p = (pos0 + s) % R;
         const bool check = p != R - 1 && p % m->check_every == 0;
-        cudaGraphConditionalHandle h = 0;
-        if (capture && check && (st = md_cond_handle(m, &h))) return st;
         StepArgs a = md_step_args(m, m->rc);
-        a.use_cond = capture && check ? 1 : 0;
-        a.vote = check ? 1 : 0;
+        a.vote = check ? ctl_word(m, kCtlVotes + p) : nullptr;
         a.unchecked = !check && p != R - 1 ? 1 : 0;
-        a.cond = h;
         if (ev) cudaEventRecord(ev[2 * s], c->stream);
         launch_step<0>(m, a, m->first);
         if (ev) cudaEventRecord(ev[2 * s + 1], c->stream);
         m->first = false;
         m->rc ^= 1;
-        if (check && capture) {
-            if ((st = md_add_cond_node(
-                     m, h, 1, [&](int) { return md_rebuild(m, RB_REFIT, m->rc, ctl_word(m, 2)); },
-                     &m->refit_kernels)))
-                return st;
-        } else if (check) {
-            unsigned flag = 0;
-            cudaError_t e = cudaMemcpyAsync(&flag, m->ctl.p, sizeof(flag), cudaMemcpyDeviceToHost,
-                                            c->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-            if (e != cudaSuccess) return cuda_fail(c, e, "refit request");
+        if (check) {
+            unsigned flag = 1;
+            if (!capture) {
+                cudaError_t e = cudaMemcpyAsync(&flag, a.vote, sizeof(flag), cudaMemcpyDeviceToHost,
+                                                c->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+                if (e != cudaSuccess) return cuda_fail(c, e, "refit request");
+            }
             if (flag) {
                 const int64_t l0 = c->launches;
-                if ((st = md_rebuild(m, RB_REFIT, m->rc, ctl_word(m, 2)))) return st;
-                m->eager_bodies += c->launches - l0;
+                if ((st = md_rebuild(m, RB_REFIT, m->rc, ctl_word(m, kCtlEarly), false,
+                                     capture ? a.vote : nullptr)))
+                    return st;
+                m->refit_kernels = c->launches - l0;
             }
         }
         if ((st = md_observe(m, pos0 + s, capture, m->steps + s + 1))) return st;
@@ -2260,7 +2241,7 @@ static nd_status md_capture_main(MDEngine* m) {
 // Window counter after an opening build: that build was window 0.
 static nd_status md_opened(MDEngine* m) {
     const unsigned one = 1u;
-    cudaError_t e = cudaMemcpyAsync(ctl_word(m, 3), &one, sizeof(one), cudaMemcpyHostToDevice,
+    cudaError_t e = cudaMemcpyAsync(ctl_word(m, kCtlWindow), &one, sizeof(one), cudaMemcpyHostToDevice,
                                     m->sub.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->sub.stream);
     if (e != cudaSuccess) return cuda_fail(&m->sub, e, "window counter");
@@ -2350,7 +2331,7 @@ nd_status md_upload(MDEngine* m, const double* xd, const double* vd, const doubl
                                                 s.orig, s.sid);
     c->launches += 3;
     if (cudaMemsetAsync(m->diag.p, 0, 64, c->stream) != cudaSuccess) return ND_ERR_CUDA;
-    if (cudaMemsetAsync(m->ctl.p, 0, 64, c->stream) != cudaSuccess) return ND_ERR_CUDA;
+    if (cudaMemsetAsync(m->ctl.p, 0, md_ctl_bytes(m), c->stream) != cudaSuccess) return ND_ERR_CUDA;
     if (m->obs.p && cudaMemsetAsync(m->obs.p, 0, 64, c->stream) != cudaSuccess) return ND_ERR_CUDA;
     m->cur = 0;
     m->first = true;
@@ -2985,17 +2966,20 @@ nd_status md_diagnostics(MDEngine* m, nd_md_diag* out) {
     out->skin_violations = (int64_t)d[0];
     // diag int32 words 2 and 3 hold the largest union and list seen
     out->max_neighbors = (int32_t)(d[1] >> 32);
-    out->resorts = ctl[6];
-    out->refits = ctl[7];
-    out->early_refits = ctl[2];
+    out->resorts = ctl[kCtlResorts];
+    out->refits = ctl[kCtlRefits];
+    out->early_refits = ctl[kCtlEarly];
     out->resort_kernels = m->resort_kernels;
     out->refit_kernels = m->refit_kernels;
     // kernels run inside conditional bodies of graphs: all bodies run, less
-    // those the host ran (and counted) itself
-    out->body_kernels = (int64_t)ctl[6] * m->resort_kernels +
-                        ((int64_t)ctl[7] + ctl[2]) * m->refit_kernels +
-                        (int64_t)ob[1] * m->thermo_kernels + (int64_t)ob[0] * m->log_kernels -
+    // those the host ran (and counted) itself; early refits are kernels of
+    // the graph (or the host's), and so are the re-sorts of an engine that
+    // re-sorts at every window
+    out->body_kernels = (int64_t)ob[1] * m->thermo_kernels + (int64_t)ob[0] * m->log_kernels -
                         m->eager_bodies;
+    if (m->resort_every > 1)
+        out->body_kernels += (int64_t)ctl[kCtlResorts] * m->resort_kernels +
+                             (int64_t)ctl[kCtlRefits] * m->refit_kernels;
     return ND_OK;
 }
 

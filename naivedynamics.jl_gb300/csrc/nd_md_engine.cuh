@@ -134,15 +134,10 @@ struct StepArgs {
     const int32_t* __restrict__ sid;  // batched ensembles: system of each sorted atom
     const SysRow* __restrict__ sys;   // and the per-system constants
     int32_t nsys;
-    // early refit: ctl[0] request flag, ctl[1] finished-block tickets; inside a
-    // captured window the last block sets `cond` for the conditional refit node
     float hsu;  // skin/2 in fixed-point units (early-refit trigger)
-    unsigned* ctl;
-    cudaGraphConditionalHandle cond;
-    int32_t use_cond;
-    // this step votes for an early refit (a check follows it); the vote
-    // covers the next trig_k / 2 + 1 steps
-    int32_t vote;
+    // word this step's vote for an early refit goes to (nullptr: no check
+    // follows it); the vote covers the next trig_k / 2 + 1 steps
+    unsigned* vote;
     float trig_k;
     // the next step uses this step's list unchecked: an atom past skin/2 is a
     // skin violation
@@ -169,16 +164,16 @@ struct MDEngine {
     // level-log2(G) cells are the systems' slots
     int32_t nsys = 0;
     float tree_frame[6] = {0, 0, 0, 0, 0, 0};
-    // early refits: ctl = {request flag, block tickets, early refits done};
-    // the first window after an upload is captured too (graph_first), and the
-    // conditional refit bodies are captured on cap_stream
+    // ctl: control words, counters and the steps' votes (kCtl* in nd_md.cu);
+    // the first window after an upload is captured too (graph_first), and
+    // conditional bodies are captured on cap_stream
     DevBuf ctl;
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t graph_first = nullptr;
     int64_t graph_first_launches = 0, refit_kernels = 0;
     SetPtrs set[2];
-    // one captured window: a device-decided rebuild (re-sort or refit) and R
-    // steps with conditional early refits; the live state is always set 0
+    // one captured window: a rebuild (re-sort, or as the device decides) and R
+    // steps with gated early refits; the live state is always set 0
     cudaGraphExec_t graph_main = nullptr;
     int32_t resort_every = 1;  // re-sort (new order + topology) every k-th window, refit between
     int32_t check_every = 1;   // steps between early-refit checks
@@ -218,7 +213,7 @@ __device__ __forceinline__ int32_t list_slot(int32_t s, int32_t c, int32_t lcap)
 
 // Rebuild of the neighbour lists (re-sort or refit; see nd_md.cu).
 nd_status md_rebuild(MDEngine* m, int kind, int rec = -1, unsigned* counter = nullptr,
-                     bool sizing = false);
+                     bool sizing = false, const unsigned* gate = nullptr, bool opens = false);
 // Step-kernel arguments for the current state set, reading records `rec_in`.
 StepArgs md_step_args(MDEngine* m, int rec_in);
 // One velocity-Verlet step kernel (force, kick, drift, walls, next record).
