@@ -124,10 +124,18 @@ __global__ void k_bbox_set(uint32_t* bbox, CodeFrame fr) {
 }
 
 constexpr int RS_BINS = 256;
-constexpr int RS_TILE = 2048;
+constexpr int RS_TILE = 2048;  // keys per block of the counting and scattering kernels
+
+// Keys per block of the one-kernel pass: few keys go to small blocks (the time
+// of a pass is then a block's: 20,000 keys 7.6 us a pass with 2,048 keys a
+// block, 11.2 us with 4,096), many to large ones (the time is then in adding up
+// the tiles' counts: 262,144 keys 18.0 and 13.7 us).
+__host__ __device__ inline int32_t pass_tile(int32_t n) {
+    return n <= 32768 ? 1024 : n <= 131072 ? 2048 : 4096;
+}
 
 // Codes of all positions, the identity permutation, and (hist given) the
-// digit counts of the sort's first pass, per tile of RS_TILE positions.
+// digit counts of the sort's first pass, per tile of pass_tile(n) positions.
 __global__ void k_morton(const float* __restrict__ xyz, int32_t n, int32_t order, float binwidth,
                          const uint32_t* __restrict__ bbox, int32_t* __restrict__ codes,
                          int32_t* __restrict__ iota, uint32_t* __restrict__ hist, int32_t* err) {
@@ -137,7 +145,7 @@ __global__ void k_morton(const float* __restrict__ xyz, int32_t n, int32_t order
                                                    : code_reference(xyz, i, binwidth, err);
     codes[i] = code;
     if (iota) iota[i] = i;
-    if (hist) atomicAdd(&hist[(i / RS_TILE) * RS_BINS + (code & 0xff)], 1u);
+    if (hist) atomicAdd(&hist[(i / pass_tile(n)) * RS_BINS + (code & 0xff)], 1u);
 }
 
 constexpr float kBinWidth = (float)(1.0 / 1023.0);  // Float32(1/1023), BVHTraverse.jl:184
@@ -179,9 +187,9 @@ nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32
 // forms, by size:
 //  * up to kSmallSort keys: one block does everything (codes included), one
 //    launch; 512 positions took 15 launches, 50 us, before;
-//  * up to kDirectTiles tiles of 2,048 keys: one kernel per pass (k_rs_pass).
-//    A block adds up the digit counts of the tiles before its own by itself
-//    (coalesced rows, independent loads; at 256 tiles 256 KB from L2 a block)
+//  * up to kDirectKeys: one kernel per pass (k_rs_pass), at most 128 blocks.  A
+//    block adds up the digit counts of the tiles before its own by itself
+//    (coalesced rows, 16 or 32 loads in flight; at 128 tiles 128 KB from L2 a block)
 //    and counts, while it scatters, the next pass's digits at their
 //    destination tiles, so a pass needs no counting and no scanning kernel;
 //  * more: digit counts per tile (k_rs_upsweep), a scan per digit over the
@@ -191,13 +199,27 @@ nd_status morton_codes(Ctx* c, const float* xyz, int32_t n, int32_t order, int32
 constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = RS_TILE / RS_THREADS;
 constexpr int32_t kSmallSort = 4096;
-constexpr int32_t kDirectTiles = 256;
+constexpr int32_t kDirectKeys = 128 * 4096;
 static_assert(RS_THREADS == RS_BINS, "scatter maps one thread per digit");
 
 size_t sort_scratch_bytes(int32_t n) {
-    const size_t nt = (size_t)cdiv(n, RS_TILE);
-    const size_t rows = nt <= (size_t)kDirectTiles ? 4 * nt : nt;
+    const size_t rows = n <= kDirectKeys ? 4 * (size_t)cdiv(n, pass_tile(n)) : (size_t)cdiv(n, RS_TILE);
     return sizeof(uint32_t) * (RS_BINS * rows + RS_BINS);
+}
+
+// Lanes of the warp with this lane's digit (0 .. 255; 256 for no item): one
+// ballot per bit (a match instruction takes several times as long on 32
+// different values).
+__device__ __forceinline__ unsigned digit_peers(uint32_t dg) {
+    unsigned peers = __ballot_sync(0xffffffffu, dg < 256u);
+    if (dg >= 256u) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (dg >> b) & 1u;
+        const unsigned m = __ballot_sync(0xffffffffu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
 }
 
 // Ranks of a warp's ITEMS x 32 digits (held i-major: item i of lane l is the
@@ -210,7 +232,7 @@ __device__ __forceinline__ void warp_ranks(const uint32_t (&dg)[ITEMS], C* cnt,
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
-        const unsigned peers = __match_any_sync(0xffffffffu, dg[i]);
+        const unsigned peers = digit_peers(dg[i]);
         const int lead = __ffs(peers) - 1;
         uint32_t old = 0;
         if (lane == lead && dg[i] < 256u) {
@@ -355,21 +377,24 @@ static void small_order(Ctx* c, const float* xyz, int32_t n, int32_t order, cons
 // Digit counts per tile of keys that come from elsewhere.
 __global__ void k_rs_count(const uint32_t* __restrict__ keys, int32_t n, uint32_t* __restrict__ hist) {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) atomicAdd(&hist[(i / RS_TILE) * RS_BINS + (keys[i] & 0xffu)], 1u);
+    if (i < n) atomicAdd(&hist[(i / pass_tile(n)) * RS_BINS + (keys[i] & 0xffu)], 1u);
 }
 
-// One pass over one tile: hist[tile][digit] are this pass's counts, hist_next
-// (null in the last pass) receives the next pass's.
-__global__ void __launch_bounds__(512)
+// One pass over one tile of 1,024 keys per group of eight warps (GROUPS = 1,
+// 2, 4): hist[tile][digit] are this pass's counts, hist_next (null in the last
+// pass) receives the next pass's.
+template <int GROUPS>
+__global__ void __launch_bounds__(256 * GROUPS)
     k_rs_pass(const uint32_t* __restrict__ kin, const int32_t* __restrict__ vin,
               uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int32_t n, int shift,
               const uint32_t* __restrict__ hist, uint32_t* __restrict__ hist_next, int32_t ntiles) {
-    constexpr int W = 16, ITEMS = RS_TILE / 512;
+    constexpr int ITEMS = 4, THREADS = 256 * GROUPS, W = 8 * GROUPS, TILE = THREADS * ITEMS;
     __shared__ uint16_t s_cnt[W][RS_BINS];
-    __shared__ uint32_t s_pre[2][RS_BINS], s_tot[2][RS_BINS], s_base[RS_BINS], s_warp[8];
+    __shared__ uint32_t s_pre[GROUPS][RS_BINS], s_tot[GROUPS][RS_BINS], s_part[GROUPS][RS_BINS];
+    __shared__ uint32_t s_base[RS_BINS], s_warp[8];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5, d = t & 255, g = t >> 8;
     const int32_t tile = blockIdx.x;
-    const int64_t at0 = (int64_t)tile * RS_TILE + w * 32 * ITEMS + lane;
+    const int64_t at0 = (int64_t)tile * TILE + w * 32 * ITEMS + lane;
     uint32_t key[ITEMS], dg[ITEMS], rank[ITEMS];
     int32_t val[ITEMS];
 #pragma unroll
@@ -377,31 +402,45 @@ __global__ void __launch_bounds__(512)
         const int64_t k = at0 + 32 * i;
         key[i] = k < n ? kin[k] : 0u;
         val[i] = k < n ? vin[k] : 0;
-        dg[i] = k < n ? (key[i] >> shift) & 0xffu : 256u;
     }
-    for (int k = t; k < W * RS_BINS / 2; k += 512) reinterpret_cast<uint32_t*>(s_cnt)[k] = 0u;
+    for (int k = t; k < W * RS_BINS / 2; k += THREADS) reinterpret_cast<uint32_t*>(s_cnt)[k] = 0u;
     uint32_t pre = 0, tot = 0;
-#pragma unroll 8
-    for (int32_t r = g; r < ntiles; r += 2) {
-        const uint32_t v = __ldg(&hist[r * RS_BINS + d]);
-        tot += v;
-        pre += r < tile ? v : 0u;
+    constexpr int ROWS = GROUPS == 1 ? 32 : 16;  // in flight a thread
+    for (int32_t r0 = g; r0 < ntiles; r0 += ROWS * GROUPS) {
+        uint32_t v[ROWS];
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) {
+            const int32_t r = r0 + GROUPS * k;
+            v[k] = r < ntiles ? __ldg(&hist[r * RS_BINS + d]) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) {
+            tot += v[k];
+            pre += r0 + GROUPS * k < tile ? v[k] : 0u;
+        }
     }
     s_pre[g][d] = pre;
     s_tot[g][d] = tot;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) dg[i] = at0 + 32 * i < n ? (key[i] >> shift) & 0xffu : 256u;
     __syncthreads();
     warp_ranks<ITEMS>(dg, s_cnt[w], rank);
-    const uint32_t ex = digits_scan(s_tot[0][d] + s_tot[1][d], s_warp);  // (a barrier inside)
-    if (g == 0) {
-        s_base[d] = ex + s_pre[0][d] + s_pre[1][d];
-        uint32_t run = 0;
+    uint32_t all = 0, before = 0;
 #pragma unroll
-        for (int k = 0; k < W; ++k) {
-            const uint32_t cnt = s_cnt[k][d];
-            s_cnt[k][d] = (uint16_t)run;
-            run += cnt;
-        }
-    }
+    for (int k = 0; k < GROUPS; ++k) { all += s_tot[k][d]; before += s_pre[k][d]; }
+    const uint32_t ex = digits_scan(all, s_warp);  // (a barrier inside)
+    if (g == 0) s_base[d] = ex + before;
+    uint32_t sum = 0, c8[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { c8[k] = s_cnt[8 * g + k][d]; sum += c8[k]; }
+    s_part[g][d] = sum;
+    __syncthreads();
+    // positions of the warps' first items relative to the digit's first here
+    // (they fit 16 bits)
+    uint32_t run = 0;
+    for (int k = 0; k < g; ++k) run += s_part[k][d];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { s_cnt[8 * g + k][d] = (uint16_t)run; run += c8[k]; }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i)
@@ -410,7 +449,7 @@ __global__ void __launch_bounds__(512)
             kout[pos] = key[i];
             vout[pos] = val[i];
             if (hist_next)
-                atomicAdd(&hist_next[(pos / RS_TILE) * RS_BINS + ((key[i] >> (shift + 8)) & 0xffu)], 1u);
+                atomicAdd(&hist_next[(pos / TILE) * RS_BINS + ((key[i] >> (shift + 8)) & 0xffu)], 1u);
         }
 }
 
@@ -427,7 +466,7 @@ __global__ void __launch_bounds__(RS_THREADS)
         int64_t idx = base + k * RS_THREADS + threadIdx.x;
         bool valid = idx < n;
         uint32_t dg = valid ? ((keys[idx] >> shift) & 0xffu) : 0x100u;
-        unsigned peers = __match_any_sync(0xffffffffu, dg);
+        unsigned peers = digit_peers(dg);
         if (valid && lane == (unsigned)(__ffs(peers) - 1)) atomicAdd(&sh[dg], (uint32_t)__popc(peers));
     }
     __syncthreads();
@@ -503,7 +542,7 @@ __global__ void __launch_bounds__(RS_THREADS)
         uint32_t key = valid ? kin[idx] : 0u;
         int32_t val = valid ? vin[idx] : 0;
         uint32_t dg = valid ? ((key >> shift) & 0xffu) : 0x100u;
-        unsigned peers = __match_any_sync(0xffffffffu, dg);
+        unsigned peers = digit_peers(dg);
         int rank = __popc(peers & lt);
         if (valid && lane == __ffs(peers) - 1) s_wh[warp][dg] = (uint32_t)__popc(peers);
         __syncthreads();
@@ -530,15 +569,20 @@ __global__ void __launch_bounds__(RS_THREADS)
 // The passes of the direct form; hist[0] already counted.  Results end in
 // keys/vals.
 static nd_status direct_passes(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int passes) {
-    const int32_t ntiles = (int32_t)cdiv(n, RS_TILE);
+    const int32_t tile = pass_tile(n), ntiles = (int32_t)cdiv(n, tile);
     uint32_t* hist = (uint32_t*)c->hist.p;
     uint32_t *ka = keys, *kb = (uint32_t*)c->codes_alt.p;
     int32_t *va = vals, *vb = (int32_t*)c->perm_alt.p;
     const size_t row = (size_t)RS_BINS * ntiles;
     for (int p = 0; p < passes; ++p) {
-        k_rs_pass<<<ntiles, 512, 0, c->stream>>>(ka, va, kb, vb, n, 8 * p, hist + p * row,
-                                                 p + 1 < passes ? hist + (p + 1) * row : nullptr,
-                                                 ntiles);
+#define ND_PASS(G)                                                                               \
+    k_rs_pass<G><<<ntiles, 256 * G, 0, c->stream>>>(                                             \
+        ka, va, kb, vb, n, 8 * p, hist + p * row, p + 1 < passes ? hist + (p + 1) * row : nullptr, \
+        ntiles)
+        if (tile == 1024) ND_PASS(1);
+        else if (tile == 2048) ND_PASS(2);
+        else ND_PASS(4);
+#undef ND_PASS
         c->launches++;
         std::swap(ka, kb);
         std::swap(va, vb);
@@ -559,7 +603,7 @@ static nd_status sort_buffers(Ctx* c, int32_t n) {
 
 static nd_status reset_counts(Ctx* c, int32_t n, int passes) {
     cudaError_t e = cudaMemsetAsync(
-        c->hist.p, 0, sizeof(uint32_t) * RS_BINS * (size_t)cdiv(n, RS_TILE) * passes, c->stream);
+        c->hist.p, 0, sizeof(uint32_t) * RS_BINS * (size_t)cdiv(n, pass_tile(n)) * passes, c->stream);
     return e == cudaSuccess ? ND_OK : cuda_fail(c, e, "digit counts reset");
 }
 
@@ -572,13 +616,13 @@ nd_status radix_sort_pairs(Ctx* c, uint32_t* keys, int32_t* vals, int32_t n, int
     }
     nd_status st = sort_buffers(c, n);
     if (st) return st;
-    int32_t ntiles = (int32_t)cdiv(n, RS_TILE);
-    if (ntiles <= kDirectTiles) {
+    if (n <= kDirectKeys) {
         if ((st = reset_counts(c, n, passes))) return st;
         k_rs_count<<<(unsigned)cdiv(n, 256), 256, 0, c->stream>>>(keys, n, (uint32_t*)c->hist.p);
         c->launches++;
         return direct_passes(c, keys, vals, n, passes);
     }
+    const int32_t ntiles = (int32_t)cdiv(n, RS_TILE);
     uint32_t* hist = (uint32_t*)c->hist.p;
     uint32_t* totals = hist + (size_t)RS_BINS * ntiles;
     uint32_t* ka = keys;
@@ -610,7 +654,7 @@ nd_status order_positions(Ctx* c, const float* xyz, int32_t n, int32_t order, in
         return check_launch(c, "order");
     }
     nd_status st;
-    if (cdiv(n, RS_TILE) > kDirectTiles) {
+    if (n > kDirectKeys) {
         if ((st = codes_kernels(c, xyz, n, order, codes, perm, frame, nullptr))) return st;
         return radix_sort_pairs(c, (uint32_t*)codes, perm, n, 30);
     }

@@ -42,7 +42,8 @@ constexpr size_t kPos4B = up256(16ull * kNoAllocMaxAtoms);               // sort
 constexpr size_t kIdxB = up256(4ull * kNoAllocMaxAtoms);                 // sorted index
 constexpr size_t kKeysB = up256(32ull * (2 * kMaxLeaves));               // GridKeys
 constexpr size_t kStoreB = up256(4ull * kMaxLeaves);                     // CAS slots
-constexpr size_t kHistB = up256(4ull * (4 * 256 * ((kNoAllocMaxAtoms + 2047) / 2048) + 256));
+// (at most 32 tiles a pass up to 65,536 keys)
+constexpr size_t kHistB = up256(4ull * (4 * 256 * 32 + 256));
 constexpr size_t kCountsB = up256(8ull * (kMaxLeaves + 1));
 constexpr size_t kOffsetsB = up256(8ull * (kMaxLeaves + 2));
 constexpr size_t kPartialB = up256(8ull * (4 * ((kMaxLeaves + 4095) / 4096) + 64));

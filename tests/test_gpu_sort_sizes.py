@@ -9,7 +9,7 @@ from helpers import uniform
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [4, 1020, 1024, 1028, 2048, 2052, 4096, 4100, 6144, 6148, 20000,
+@pytest.mark.parametrize("n", [8, 1020, 1024, 1028, 2048, 2052, 4096, 4100, 20000, 32768, 32772, 131072, 131076,
                                524288, 524292])
 @pytest.mark.parametrize("same", [False, True])
 def test_tree_order_is_a_stable_sort(nd, oracle, n, same):
