@@ -189,13 +189,13 @@ __global__ void __launch_bounds__(kBlock * kAdjTPA) k_adj_reverse(AdjArgs a) {
     const float4 gi = a.g4_in[i];
     const int32_t cpk = valid ? __ldg(&a.ncount[i]) : 0;
     const int32_t cnt = list_total(cpk);
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * a.lcap * kBlock;
+    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
     float3 hv = make_float3(0.f, 0.f, 0.f);
     float eacc = 0.f, sacc = 0.f;
-    int32_t li = part < cnt ? L[llist_at(list_slot(part, cpk, a.lcap), al)] : 0;
+    int32_t li = part < cnt ? L[list_at(part, cpk, al, a.lcap)] : 0;
     for (int32_t s = part; s < cnt; s += kAdjTPA) {
         const int32_t sn = s + kAdjTPA;
-        const int32_t next = sn < cnt ? L[llist_at(list_slot(sn, cpk, a.lcap), al)] : 0;
+        const int32_t next = sn < cnt ? L[list_at(sn, cpk, al, a.lcap)] : 0;
         int4 rj;
         float4 gj;
         if (li < a.smrec) {
@@ -265,13 +265,13 @@ __global__ void __launch_bounds__(kBlock) k_adj_hist(AdjArgs a) {
     const int4 ri = __ldg(&a.recs[i]);
     const int32_t cpk = __ldg(&a.ncount[i]);
     const int32_t cnt = list_total(cpk);
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * a.lcap * kBlock;
+    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
     for (int32_t b0 = 0; b0 < a.bins; b0 += kHistChunk) {
         float acc[kHistChunk];
 #pragma unroll
         for (int k = 0; k < kHistChunk; ++k) acc[k] = 0.0f;
         for (int32_t s = 0; s < cnt; ++s) {
-            const int64_t j = adj_atom(U, L[llist_at(list_slot(s, cpk, a.lcap), tid)], a.apl);
+            const int64_t j = adj_atom(U, L[list_at(s, cpk, tid, a.lcap)], a.apl);
             if (j <= i) continue;
             const int4 rj = __ldg(&a.recs[j]);
             const float dx = (float)idiff(ri.x, rj.x) * a.invS;
@@ -337,10 +337,10 @@ __global__ void __launch_bounds__(kBlock) k_adj_terminal(AdjArgs a) {
     const int4 ri = __ldg(&a.recs[i]);
     const int32_t cpk = __ldg(&a.ncount[i]);
     const int32_t cnt = list_total(cpk);
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * a.lcap * kBlock;
+    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
     float gx = 0.f, gy = 0.f, gz = 0.f;
     for (int32_t s = 0; s < cnt; ++s) {
-        const int64_t j = adj_atom(U, L[llist_at(list_slot(s, cpk, a.lcap), tid)], a.apl);
+        const int64_t j = adj_atom(U, L[list_at(s, cpk, tid, a.lcap)], a.apl);
         const int4 rj = __ldg(&a.recs[j]);
         const float dx = (float)idiff(ri.x, rj.x) * a.invS;
         const float dy = (float)idiff(ri.y, rj.y) * a.invS;

@@ -14,8 +14,8 @@
 //   pos32[N]           float4 Float32 positions at the last rebuild (tree input)
 //   ulist[B][ucap]     per block of 256 atoms: the sorted leaves that hold any
 //                      neighbour of the block (the block's union), ucount[B]
-//   llist[B][lcap][256] uint16 per-atom neighbour lists as indices into the
-//                      block's union (slot-major inside the block), ncount[N]
+//   llist[B][words][256] per-atom neighbour lists: uint16 indices into the
+//                      block's union, four to an 8-byte word, ncount[N]
 // One MD step is ONE kernel: a block stages its union's records in shared
 // memory, each thread sums its atom's pair forces over its own exact list (no
 // atomics, deterministic), completes the pending half kick, kicks, drifts,
@@ -355,6 +355,33 @@ __device__ __forceinline__ int32_t block_compact(bool keep, int32_t value, int32
     return total;
 }
 
+// A leaf's box widened by a few ulps, so that no pair is lost to rounding: the
+// atom distance test decides.
+struct OwnBox {
+    float v[6];
+};
+__device__ __forceinline__ OwnBox own_box(const float4& a, const float4& b) {
+    OwnBox o;
+    o.v[0] = a.x - 1e-5f * fabsf(a.x) - 1e-6f;
+    o.v[1] = a.y - 1e-5f * fabsf(a.y) - 1e-6f;
+    o.v[2] = a.z - 1e-5f * fabsf(a.z) - 1e-6f;
+    o.v[3] = a.w + 1e-5f * fabsf(a.w) + 1e-6f;
+    o.v[4] = b.x + 1e-5f * fabsf(b.x) + 1e-6f;
+    o.v[5] = b.y + 1e-5f * fabsf(b.y) + 1e-6f;
+    return o;
+}
+
+// Euclidean gap test of key box (a, b) against box o: the per-axis gap of the
+// atom boxes is the key-box gap + r_list, and a Euclidean gap below r_list
+// implies overlapping key boxes.
+__device__ __forceinline__ bool gap_ok(const OwnBox& o, const float4& a, const float4& b, float rl,
+                                       float rl2g) {
+    const float gx = fmaxf(fmaxf(o.v[0] - a.w, a.x - o.v[3]) + rl, 0.0f);
+    const float gy = fmaxf(fmaxf(o.v[1] - b.x, a.y - o.v[4]) + rl, 0.0f);
+    const float gz = fmaxf(fmaxf(o.v[2] - b.y, a.z - o.v[5]) + rl, 0.0f);
+    return gx * gx + gy * gy + gz * gz < rl2g;
+}
+
 // One block per 256 atoms: every leaf whose box overlaps one of the block's
 // eight warp boxes (their atoms -/+ hq) joins the block's union, sorted by
 // leaf index so list order, and hence force summation order, is
@@ -372,7 +399,7 @@ __device__ __forceinline__ int32_t block_compact(bool keep, int32_t value, int32
 //    union is sorted (bitonic) afterwards.
 // Shared memory: two buffers of fcap entries (BFS frontiers, or candidate
 // super-blocks and blocks) and the union (upow2).
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 4)
     k_md_block_union(const float4* __restrict__ keys, const float4* __restrict__ bbox,
                      int32_t nblocks, int32_t tree, const float4* __restrict__ pos,
                      const int32_t* __restrict__ sid,
@@ -381,7 +408,7 @@ __global__ void __launch_bounds__(kBlock)
                      int32_t* __restrict__ ucount,
                      uint16_t* __restrict__ llist_leaf, int32_t* __restrict__ lcount_leaf,
                      int32_t lcap_leaf, int32_t* err, int32_t* diag, int32_t sizing,
-                     unsigned* pressure, const unsigned* __restrict__ gate) {
+                     unsigned* pressure, const unsigned* __restrict__ gate, int32_t candidates) {
     if (gate && *gate == 0u) return;
     extern __shared__ int32_t smem[];
     int32_t* fr[2] = {smem, smem + fcap};
@@ -466,18 +493,30 @@ __global__ void __launch_bounds__(kBlock)
         const int32_t lpb = kBlock / apl, lsh = __ffs(lpb) - 1;  // leaves per block (2^lsh)
         const int32_t kl = min(ncb, fcap) << lsh;
         nu = 0;
-        for (int32_t base = 0; base < kl; base += kBlock) {
-            const int32_t k = base + tid;
-            const int32_t leaf = k < kl ? (cb[k >> lsh] << lsh) + (k & (lpb - 1)) : nL;
-            bool hit = false;
-            if (leaf < nL) {
-                const float4 a = __ldg(&keys[2 * (int64_t)leaf]);
-                const float4 b = __ldg(&keys[2 * (int64_t)leaf + 1]);
-                for (int w = 0; w < nb && !hit; ++w)
-                    hit = box_overlap(s_wb[w][0], s_wb[w][1], s_wb[w][2], s_wb[w][3], s_wb[w][4],
-                                      s_wb[w][5], a, b);
+        // four leaves per thread in flight
+        for (int32_t base = 0; base < kl; base += 4 * kBlock) {
+            int32_t lf[4];
+            float4 ka[4], kb[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int32_t k = base + j * kBlock + tid;
+                lf[j] = k < kl ? (cb[k >> lsh] << lsh) + (k & (lpb - 1)) : nL;
+                if (lf[j] < nL) {
+                    ka[j] = __ldg(&keys[2 * (int64_t)lf[j]]);
+                    kb[j] = __ldg(&keys[2 * (int64_t)lf[j] + 1]);
+                }
             }
-            nu += block_compact(hit, leaf, su, nu, upow2, s_w);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (base + j * kBlock >= kl) break;  // block-uniform
+                bool hit = false;
+                if (lf[j] < nL && box_overlap(u0, u1, u2, u3, u4, u5, ka[j], kb[j])) {
+                    for (int w = 0; w < nb && !hit; ++w)
+                        hit = box_overlap(s_wb[w][0], s_wb[w][1], s_wb[w][2], s_wb[w][3],
+                                          s_wb[w][4], s_wb[w][5], ka[j], kb[j]);
+                }
+                nu += block_compact(hit, lf[j], su, nu, upow2, s_w);
+            }
         }
     } else {
         int cur = 0;
@@ -554,6 +593,7 @@ __global__ void __launch_bounds__(kBlock)
     int32_t* dst = ulist + (int64_t)blockIdx.x * ucap;
     for (int32_t k = tid; k < nu; k += kBlock) dst[k] = su[k];
     if (tid == 0) ucount[blockIdx.x] = nu;
+    if (!candidates) return;  // k_md_leaf_lists finds them itself
     // Per-leaf candidate lists: for each of its leaves a warp keeps the union
     // positions whose atoms can be within r_list of that leaf's atoms at all,
     // ballot-compacted in union order: leaf boxes are atom boxes -/+ r_list/2,
@@ -566,7 +606,7 @@ __global__ void __launch_bounds__(kBlock)
     // that pass are queued (per warp, in union order) and tested 32 at a time
     // against each of those own leaves.  The own boxes are widened by a few
     // ulps so no pair is lost to rounding; the atom distance test decides.
-    __shared__ float s_own[kBlock / 32][8][6];
+    __shared__ OwnBox s_own[kBlock / 32][8];
     __shared__ int32_t s_qu[kBlock / 32][64];    // per-warp queue: union index
     __shared__ float s_qb[kBlock / 32][6][64];   // and its key box
     const unsigned below = (1u << lane) - 1u;
@@ -579,36 +619,22 @@ __global__ void __launch_bounds__(kBlock)
             const int64_t own = first_own + k0 + lane;
             float4 oa = make_float4(1.f, 1.f, 1.f, -1.f), ob = make_float4(-1.f, -1.f, 0.f, 0.f);
             if (own < nL) { oa = __ldg(&keys[2 * own]); ob = __ldg(&keys[2 * own + 1]); }
-            s_own[warp][lane][0] = oa.x - 1e-5f * fabsf(oa.x) - 1e-6f;
-            s_own[warp][lane][1] = oa.y - 1e-5f * fabsf(oa.y) - 1e-6f;
-            s_own[warp][lane][2] = oa.z - 1e-5f * fabsf(oa.z) - 1e-6f;
-            s_own[warp][lane][3] = oa.w + 1e-5f * fabsf(oa.w) + 1e-6f;
-            s_own[warp][lane][4] = ob.x + 1e-5f * fabsf(ob.x) + 1e-6f;
-            s_own[warp][lane][5] = ob.y + 1e-5f * fabsf(ob.y) + 1e-6f;
+            s_own[warp][lane] = own_box(oa, ob);
         }
         __syncwarp();
         // the group box: the union of these own boxes; a union leaf whose
         // atoms cannot come within r_list of it is dropped for all of them
-        float gb[6];
+        OwnBox gb;
 #pragma unroll
         for (int d = 0; d < 6; ++d) {
-            float v = lane < nown ? s_own[warp][lane][d] : (d < 3 ? INFINITY : -INFINITY);
+            float v = lane < nown ? s_own[warp][lane].v[d] : (d < 3 ? INFINITY : -INFINITY);
 #pragma unroll
             for (int sh = 16; sh > 0; sh >>= 1) {
                 const float w = __shfl_xor_sync(0xffffffffu, v, sh);
                 v = d < 3 ? fminf(v, w) : fmaxf(v, w);
             }
-            gb[d] = v;
+            gb.v[d] = v;
         }
-        // Euclidean gap test of key box (a, b) against box o (6 floats): the
-        // per-axis gap of the atom boxes is the key-box gap + r_list, and a
-        // Euclidean gap below r_list implies overlapping key boxes
-        auto near_box = [&](const float* o, const float4& a, const float4& b) {
-            const float gx = fmaxf(fmaxf(o[0] - a.w, a.x - o[3]) + rl, 0.0f);
-            const float gy = fmaxf(fmaxf(o[1] - b.x, a.y - o[4]) + rl, 0.0f);
-            const float gz = fmaxf(fmaxf(o[2] - b.y, a.z - o[5]) + rl, 0.0f);
-            return gx * gx + gy * gy + gz * gz < rl2g;
-        };
         int32_t lc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         // the passing union leaves go through a per-warp queue (in union
         // order), tested against the own leaves 32 at a time
@@ -621,7 +647,7 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
             for (int kl = 0; kl < 8; ++kl) {
                 if (kl >= nown) break;
-                const bool hit = live && near_box(s_own[warp][kl], a, b);
+                const bool hit = live && gap_ok(s_own[warp][kl], a, b, rl, rl2g);
                 const unsigned m = __ballot_sync(0xffffffffu, hit);
                 const int32_t pos = lc[kl] + __popc(m & below);
                 if (hit && pos < lcap_leaf)
@@ -630,15 +656,24 @@ __global__ void __launch_bounds__(kBlock)
             }
         };
         int32_t qn = 0;
+        // the next 32 boxes are loaded while the current ones are tested
+        const float4 none_a = make_float4(1.f, 1.f, 1.f, -1.f),
+                     none_b = make_float4(-1.f, -1.f, 0.f, 0.f);
+        float4 na = none_a, nb4 = none_b;
+        if (lane < nu) {
+            const int32_t leaf = su[lane];
+            na = __ldg(&keys[2 * (int64_t)leaf]);
+            nb4 = __ldg(&keys[2 * (int64_t)leaf + 1]);
+        }
         for (int32_t base = 0; base < nu; base += 32) {
             const int32_t u = base + lane;
-            float4 a = make_float4(1.f, 1.f, 1.f, -1.f), b = make_float4(-1.f, -1.f, 0.f, 0.f);
-            if (u < nu) {
-                const int32_t leaf = su[u];
-                a = __ldg(&keys[2 * (int64_t)leaf]);
-                b = __ldg(&keys[2 * (int64_t)leaf + 1]);
+            const float4 a = na, b = nb4;
+            if (u + 32 < nu) {
+                const int32_t leaf = su[u + 32];
+                na = __ldg(&keys[2 * (int64_t)leaf]);
+                nb4 = __ldg(&keys[2 * (int64_t)leaf + 1]);
             }
-            const bool pass = u < nu && near_box(gb, a, b);
+            const bool pass = u < nu && gap_ok(gb, a, b, rl, rl2g);
             const unsigned m = __ballot_sync(0xffffffffu, pass);
             if (pass) {
                 const int32_t at = qn + __popc(m & below);  // < 64: qn < 32 here
@@ -662,6 +697,10 @@ __global__ void __launch_bounds__(kBlock)
             }
         }
         if (qn > 0) test_queue(qn);
+        int32_t most = 0;
+#pragma unroll
+        for (int kl = 0; kl < 8; ++kl) most = max(most, lc[kl]);
+        if (lane == 0) atomicMax(&diag[2], most);
         if (lane < nown) {
             int32_t mine = 0;
 #pragma unroll
@@ -670,7 +709,6 @@ __global__ void __launch_bounds__(kBlock)
             const int64_t own = first_own + k0 + lane;
             if (own < nL) {
                 lcount_leaf[own] = min(mine, lcap_leaf);
-                atomicMax(&diag[2], mine);
                 if (pressure && 10 * mine > 9 * lcap_leaf) atomicOr(pressure, 1u);
                 if (mine > lcap_leaf && !sizing) set_error(err, ND_ERR_OVERFLOW, (int32_t)own);
             }
@@ -681,15 +719,18 @@ __global__ void __launch_bounds__(kBlock)
 
 // Exact per-atom lists inside the block's union: the union's Float32
 // positions are staged in shared memory (up to smpos entries; the rest are read
-// from L2), then the APL lanes of a leaf walk that leaf's candidate list
-// together, each testing its own atom against the candidate leaf's atoms with
-// the reference distance (Float32, d^2 < r_list^2) and storing union indices
-// as uint16: entries closer than the near bound (rnb2, or the atom's system's)
-// from slot 0 upwards, the others from slot lcap - 1 downwards.  pos.w holds
-// the atom's sorted index (excludes the atom itself).  (Two atoms per packed
-// f32x2 instruction measured slower here, and its sums are not always the
-// scalar operations' bits: one pair of the 512-system ensemble came out 1 ulp
-// above r_list^2.)
+// from L2), then the atoms of a leaf walk that leaf's candidate list, testing
+// the candidate leaf's atoms with the reference distance (Float32, d^2 <
+// r_list^2) and storing union indices as uint16: entries closer than the near
+// bound (rnb2, or the atom's system's) in the near segment, the others in the
+// other.  pos.w holds the atom's sorted index (excludes the atom itself).
+// A thread per atom, the APL threads of a leaf together; the last entries of
+// each segment wait in a register pair and are stored four at a time, as a
+// word: stored one by one the 85 entries an atom touched as many 32-byte
+// sectors (262,144 atoms: 182 us, now 145).
+// (Two atoms per packed f32x2 instruction measured slower here, and its sums
+// are not always the scalar operations' bits: one pair of the 512-system
+// ensemble came out 1 ulp above r_list^2.)
 template <int APL>
 __global__ void __launch_bounds__(kBlock)
     k_md_block_lists(const float4* __restrict__ pos, int32_t n, float rl2, float rnb2,
@@ -703,14 +744,14 @@ __global__ void __launch_bounds__(kBlock)
                      const unsigned* __restrict__ gate) {
     if (gate && *gate == 0u) return;
     extern __shared__ float4 spos[];
-    const int tid = threadIdx.x;
-    const int32_t* __restrict__ U = ulist + (int64_t)blockIdx.x * ucap;
+    const int32_t blk = (int32_t)blockIdx.x;
+    const int32_t* __restrict__ U = ulist + (int64_t)blk * ucap;
+    const int32_t nu = min(__ldg(&ucount[blk]), ucap);
     {
         // four positions per thread in flight: their leaf indices, then the
         // positions
-        const int32_t nu = min(__ldg(&ucount[blockIdx.x]), ucap);
         const int32_t m = min(nu * APL, smpos);
-        for (int32_t k = tid; k < m; k += 4 * kBlock) {
+        for (int32_t k = threadIdx.x; k < m; k += 4 * kBlock) {
             int32_t lf[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -731,20 +772,29 @@ __global__ void __launch_bounds__(kBlock)
         }
     }
     __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * kBlock + tid;
+    const int tid = (int)threadIdx.x;
+    const int64_t i = (int64_t)blk * kBlock + tid;
     const bool valid = i < n;
-    const int64_t own = (valid ? i : (int64_t)blockIdx.x * kBlock) / APL;
-    const float4 p = __ldg(&pos[valid ? i : (int64_t)blockIdx.x * kBlock]);
+    const int64_t ii = valid ? i : (int64_t)blk * kBlock;
+    const int64_t own = ii / APL;
+    const float4 p = __ldg(&pos[ii]);
     const int32_t nc = valid ? min(__ldg(&lcount_leaf[own]), lcap_leaf) : 0;
     // candidate entries eight at a time (a leaf's list starts on a 16-byte
     // boundary: lcap_leaf is a multiple of 8), the next eight loaded while the
     // current ones are tested
     const uint4* __restrict__ C = reinterpret_cast<const uint4*>(llist_leaf + own * lcap_leaf);
-    uint16_t* __restrict__ L = llist + (int64_t)blockIdx.x * lcap * kBlock + tid;
+    uint16_t* __restrict__ L = llist + (int64_t)blk * list_block(lcap);
     const int32_t self = (int32_t)i;
-    const float nb2 = sid ? __ldg(&sys[__ldg(&sid[valid ? i : (int64_t)blockIdx.x * kBlock])].nk.rnb2)
-                          : rnb2;
+    const float nb2 = sid ? __ldg(&sys[__ldg(&sid[ii])].nk.rnb2) : rnb2;
     int32_t cnt = 0, nn = 0, nf = 0;  // all hits; near and other entries stored
+    // the near and the other entries not yet stored, the latest in the top 16 bits
+    uint2 nw = make_uint2(0u, 0u), fw = make_uint2(0u, 0u);
+    uint2* __restrict__ nearp = reinterpret_cast<uint2*>(L) + tid;
+    uint2* __restrict__ farp = nearp + (int64_t)(list_words(lcap) - 1) * kBlock;
+    auto push = [](uint2& w, uint32_t li) {
+        w.x = __byte_perm(w.x, w.y, 0x5432);
+        w.y = __byte_perm(w.y, li, 0x5432);
+    };
     // compiled twice: for a block whose whole union is staged (block-uniform)
     // the positions come from shared memory with no test
     auto walk = [&](auto staged) {
@@ -769,29 +819,175 @@ __global__ void __launch_bounds__(kBlock)
                 }
 #pragma unroll
                 for (int e = 0; e < APL; ++e) {
-                    // branch-free: a predicated store to the near or the far end
+                    // branch-free: every step predicated
                     const float d2 = dist2_ref(p.x, p.y, p.z, q[e].x, q[e].y, q[e].z);
                     const bool hit = d2 < rl2 && __float_as_int(q[e].w) != self;
                     const bool put = hit && cnt < lcap;
-                    const bool near = d2 < nb2;
-                    const int32_t slot = near ? nn : lcap - 1 - nf;
-                    if (put) L[slot * kBlock] = (uint16_t)(u * APL + e);
-                    nn += (put && near) ? 1 : 0;
-                    nf += (put && !near) ? 1 : 0;
+                    const bool near = put && d2 < nb2, far = put && !(d2 < nb2);
+                    const uint32_t li = (uint32_t)(u * APL + e);
+                    if (far) {
+                        push(fw, li);
+                        if ((++nf & 3) == 0) { *farp = fw; farp -= kBlock; }
+                    }
+                    if (near) {
+                        push(nw, li);
+                        if ((++nn & 3) == 0) { *nearp = nw; nearp += kBlock; }
+                    }
                     cnt += hit ? 1 : 0;
                 }
             }
         }
     };
-    if (min(__ldg(&ucount[blockIdx.x]), ucap) * APL <= smpos)
+    if (nu * APL <= smpos)
         walk(std::true_type{});
     else
         walk(std::false_type{});
+    const unsigned most = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
+    if ((threadIdx.x & 31) == 0) atomicMax(&diag[1], (int32_t)most);
     if (!valid) return;
+    // the last words, their entries moved down to the first place
+    auto rest = [](uint2 w, int32_t k) {
+        for (; k < 4; ++k) {
+            w.x = __byte_perm(w.x, w.y, 0x5432);
+            w.y >>= 16;
+        }
+        return w;
+    };
+    if (nf & 3) *farp = rest(fw, nf & 3);
+    if (nn & 3) *nearp = rest(nw, nn & 3);
     ncount[i] = nn | (nf << 16);
     if (cnt > lcap && !sizing) set_error(err, ND_ERR_OVERFLOW, (int32_t)i);
-    atomicMax(&diag[1], cnt);
     if (pressure && 10 * cnt > 9 * lcap) atomicOr(pressure, 1u);
+}
+
+// The same lists for few blocks, where the threads of an atom each, walking
+// about 480 tests one after the other, would leave the SMs idle (4,096 atoms:
+// 27 us for 16 blocks of threads): a warp per leaf.  It tests the boxes of the
+// block's union against its leaf 32 at a time (the candidate lists of
+// k_md_block_union's second half, with the same tests, kept in shared memory),
+// then the candidates' atoms 32 at a time, one a lane, against each of its own
+// atoms; an entry's place in the list comes from the ballots.  cand: 8 *
+// lcap_leaf pairs of shared memory.
+template <int APL>
+__global__ void __launch_bounds__(kBlock)
+    k_md_leaf_lists(const float4* __restrict__ keys, const float4* __restrict__ pos, int32_t nL,
+                    float rl, float rl2, float rnb2, const int32_t* __restrict__ sid,
+                    const SysRow* __restrict__ sys, int32_t ucap,
+                    const int32_t* __restrict__ ulist, const int32_t* __restrict__ ucount,
+                    int32_t lcap_leaf, int32_t lcap, uint16_t* __restrict__ llist,
+                    int32_t* __restrict__ ncount, int32_t* err, int32_t* diag, int32_t sizing,
+                    unsigned* pressure, const unsigned* __restrict__ gate) {
+    if (gate && *gate == 0u) return;
+    extern __shared__ uint2 cand_all[];
+    constexpr int LPB = kBlock / APL, CPB = LPB / 8;  // leaves, thread blocks per block of atoms
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t blk = (int32_t)blockIdx.x / CPB;
+    const int32_t first = ((int32_t)blockIdx.x % CPB) * 8 + warp;  // the leaf in the block
+    const int32_t own = blk * LPB + first;
+    if (own >= nL) return;  // whole warp
+    const unsigned below = (1u << lane) - 1u;
+    uint2* cand = cand_all + warp * lcap_leaf;  // (union index, leaf)
+    const int32_t* __restrict__ U = ulist + (int64_t)blk * ucap;
+    const int32_t nu = min(__ldg(&ucount[blk]), ucap);
+    float4 p[APL];
+#pragma unroll
+    for (int a = 0; a < APL; ++a) p[a] = __ldg(&pos[(int64_t)own * APL + a]);
+    const float nb2 = sid ? __ldg(&sys[__ldg(&sid[(int64_t)own * APL])].nk.rnb2) : rnb2;
+    int32_t nc = 0;
+    {
+        const OwnBox o = own_box(__ldg(&keys[2 * (int64_t)own]), __ldg(&keys[2 * (int64_t)own + 1]));
+        const float rl2g = rl * rl * 1.0002f;
+        // the next 64 boxes are loaded while the current ones are tested
+        int32_t lf[2];
+        float4 ka[2], kb[2];
+        auto load = [&](int32_t base) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int32_t u = base + 32 * j + lane;
+                lf[j] = u < nu ? __ldg(&U[u]) : -1;
+                if (u < nu) {
+                    ka[j] = __ldg(&keys[2 * (int64_t)lf[j]]);
+                    kb[j] = __ldg(&keys[2 * (int64_t)lf[j] + 1]);
+                }
+            }
+        };
+        load(0);
+        for (int32_t base = 0; base < nu; base += 64) {
+            const int32_t l0[2] = {lf[0], lf[1]};
+            const float4 a0[2] = {ka[0], ka[1]}, b0[2] = {kb[0], kb[1]};
+            load(base + 64);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const bool hit = l0[j] >= 0 && gap_ok(o, a0[j], b0[j], rl, rl2g);
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                const int32_t at = nc + __popc(m & below);
+                if (hit && at < lcap_leaf)
+                    cand[at] = make_uint2((unsigned)(base + 32 * j + lane), (unsigned)l0[j]);
+                nc += __popc(m);
+            }
+        }
+        if (lane == 0) {
+            atomicMax(&diag[2], nc);
+            if (pressure && 10 * nc > 9 * lcap_leaf) atomicOr(pressure, 1u);
+            if (nc > lcap_leaf && !sizing) set_error(err, ND_ERR_OVERFLOW, own);
+        }
+        nc = min(nc, lcap_leaf);
+    }
+    __syncwarp();
+    uint16_t* __restrict__ L = llist + (int64_t)blk * list_block(lcap);
+    const int32_t total = nc * APL;
+    int32_t nn[APL], nf[APL];
+#pragma unroll
+    for (int a = 0; a < APL; ++a) nn[a] = nf[a] = 0;
+    constexpr int B = APL <= 8 ? 4 : 1;  // batches of 32 candidate atoms in flight
+    for (int32_t c0 = 0; c0 < total; c0 += 32 * B) {
+        float4 q[B];
+        int32_t li[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int32_t c = c0 + 32 * k + lane;
+            li[k] = -1;
+            if (c < total) {
+                const uint2 e = cand[c / APL];
+                li[k] = (int32_t)e.x * APL + c % APL;
+                q[k] = __ldg(&pos[(int64_t)e.y * APL + c % APL]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            if (c0 + 32 * k >= total) break;  // warp-uniform
+#pragma unroll
+            for (int a = 0; a < APL; ++a) {
+                const float d2 = dist2_ref(p[a].x, p[a].y, p[a].z, q[k].x, q[k].y, q[k].z);
+                const bool hit =
+                    li[k] >= 0 && d2 < rl2 && __float_as_int(q[k].w) != own * APL + a;
+                const unsigned hm = __ballot_sync(0xffffffffu, hit);
+                const unsigned nm = __ballot_sync(0xffffffffu, hit && d2 < nb2);
+                const unsigned fm = hm & ~nm;
+                if (hit && nn[a] + nf[a] + __popc(hm & below) < lcap) {
+                    const int32_t t = first * APL + a;
+                    const int32_t at = d2 < nb2 ? near_at(nn[a] + __popc(nm & below), t)
+                                                : far_at(nf[a] + __popc(fm & below), t, lcap);
+                    L[at] = (uint16_t)li[k];
+                }
+                nn[a] += __popc(nm);
+                nf[a] += __popc(fm);
+            }
+        }
+    }
+    int32_t most = 0;
+#pragma unroll
+    for (int a = 0; a < APL; ++a) {
+        const int32_t cnt = nn[a] + nf[a];
+        most = max(most, cnt);
+        // (an overflowing list reports its error: its count is kept in range)
+        if (lane == a) ncount[(int64_t)own * APL + a] = cnt > lcap ? 0 : nn[a] | (nf[a] << 16);
+        if (lane == 0 && cnt > lcap && !sizing) set_error(err, ND_ERR_OVERFLOW, own * APL + a);
+    }
+    if (lane == 0) {
+        atomicMax(&diag[1], most);
+        if (pressure && 10 * most > 9 * lcap) atomicOr(pressure, 1u);
+    }
 }
 
 // ------------------------------------------------------------- step kernel
@@ -1210,6 +1406,13 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
     int64_t i = (int64_t)blk * kBlock + tid;
     const bool valid = i < a.n;
     const bool own = part == 0;  // the thread that updates the atom
+    // idle lanes (last block) run with an empty list and store nothing; they
+    // join the warp reductions (measure) and the block vote (step)
+    if (!valid) i = a.n - 1;
+    // the atom's own loads go first, beside the staging's
+    const int4 ri = __ldg(&a.rec_in[i]);
+    const uint2 fi = __ldg(&a.recf_in[i]);
+    const int32_t cpk = valid ? __ldg(&a.ncount[i]) : 0;
     const int32_t* __restrict__ U = a.ulist + (int64_t)blk * a.ucap;
     // stage the block's union: record of atom (leaf * apl + e) at u * apl + e,
     // up to the shared-memory capacity; larger unions read the rest from L2
@@ -1241,10 +1444,6 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
         }
     }
     __syncthreads();
-    // idle lanes (last block) run with an empty list and store nothing; they
-    // join the warp reductions (measure) and the block vote (step)
-    if (!valid) i = a.n - 1;
-    const int4 ri = __ldg(&a.rec_in[i]);
     PairK pk{a.rc2u, a.sig2u, a.eps24u, a.eps4, a.kcu, a.kceu,
              a.nk.rn2u, a.nk.sig2lo, a.nk.e24lo, a.nk.kclo, a.nk.rc2lo, a.nk.hmask};
     int32_t sv = 0;
@@ -1270,13 +1469,13 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
         hs2u = __ldg(&row->hs2u);
         hsu = __ldg(&row->hsu);
     }
-    // near entries (slots 0, 1, ...) and the others (slots lcap - 1, lcap - 2, ...)
-    const int32_t cpk = valid ? __ldg(&a.ncount[i]) : 0;
+    // near entries (words 0, 1, ...) and the others (from the last word down)
     const int32_t nn = list_near(cpk), nf = cpk >> 16;
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blk * a.lcap * kBlock + tid;
-    const uint16_t* __restrict__ LF = L + (int64_t)(a.lcap - 1) * kBlock;
+    const uint16_t* __restrict__ L = a.llist + (int64_t)blk * list_block(a.lcap);
+    const uint2* __restrict__ LW = reinterpret_cast<const uint2*>(L) + tid;
+    auto near_entry = [&](int32_t s) -> int32_t { return L[near_at(s, tid)]; };
+    auto far_entry = [&](int32_t s) -> int32_t { return L[far_at(s, tid, a.lcap)]; };
     const int32_t lsh = __ffs(a.apl) - 1, emask = a.apl - 1;
-    const uint2 fi = __ldg(&a.recf_in[i]);
     // near terms in two-float sums, the others in single precision
     DF3 nacc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float fx = 0.f, fy = 0.f, fz = 0.f;
@@ -1300,54 +1499,69 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             // (the measure pass, and ensembles, whose per-system constants leave
             // no registers for the packed form)
             int32_t s = part;
-            int32_t li = s < nn ? L[(int64_t)s * kBlock] : 0;
+            int32_t li = s < nn ? near_entry(s) : 0;
             for (; s < nn; s += TPA) {
                 const int32_t sn = s + TPA;
-                const int32_t next = sn < nn ? L[(int64_t)sn * kBlock] : 0;
+                const int32_t next = sn < nn ? near_entry(sn) : 0;
                 accum_near<COUL, MODE == 1>(ri, fetch(li), fi, fine(li), pk, nacc, ue);
                 li = next;
+            }
+        } else if constexpr (TPA == 1) {
+            // near entries two at a time (packed), half a word each, the next
+            // word loaded ahead; an odd last one alone
+            int32_t s = 0, w = 0;
+            uint2 cur = nn > 0 ? __ldg(&LW[0]) : make_uint2(0u, 0u), nxt = cur;
+            for (; s + 1 < nn; s += 2) {
+                if ((s & 2) == 0 && s + 4 < nn) nxt = __ldg(&LW[++w * kBlock]);
+                const int32_t la = cur.x & 0xffffu, lb = cur.x >> 16;
+                const int4 ra = fetch(la), rb = fetch(lb);
+                const uint2 fa = fine(la), fb = fine(lb);
+                if (s & 2) cur = nxt;
+                else cur.x = cur.y;
+                accum_near2<COUL>(ri, ra, rb, fi, fa, fb, pk, nacc);
+            }
+            if (s < nn) {
+                const int32_t li = cur.x & 0xffffu;
+                accum_near<COUL, false>(ri, fetch(li), fi, fine(li), pk, nacc, ue);
             }
         } else {
             // near entries of this thread's slice two at a time (packed), the
             // next two indices loaded ahead; an odd last one alone
             int32_t s = part;
-            int32_t la = s < nn ? L[(int64_t)s * kBlock] : 0;
-            int32_t lb = s + TPA < nn ? L[(int64_t)(s + TPA) * kBlock] : 0;
+            int32_t la = s < nn ? near_entry(s) : 0;
+            int32_t lb = s + TPA < nn ? near_entry(s + TPA) : 0;
             for (; s + TPA < nn; s += 2 * TPA) {
                 const int32_t s2 = s + 2 * TPA;
                 const int4 ra = fetch(la), rb = fetch(lb);
                 const uint2 fa = fine(la), fb = fine(lb);
-                la = s2 < nn ? L[(int64_t)s2 * kBlock] : 0;
-                lb = s2 + TPA < nn ? L[(int64_t)(s2 + TPA) * kBlock] : 0;
+                la = s2 < nn ? near_entry(s2) : 0;
+                lb = s2 + TPA < nn ? near_entry(s2 + TPA) : 0;
                 accum_near2<COUL>(ri, ra, rb, fi, fa, fb, pk, nacc);
             }
             if (s < nn) accum_near<COUL, false>(ri, fetch(la), fi, fine(la), pk, nacc, ue);
         }
         // an entry of the other segment that came closer than 1.3 sigma
         auto far_near = [&](int32_t s) {
-            const int32_t li = LF[-(int64_t)s * kBlock];
+            const int32_t li = far_entry(s);
             accum_near<COUL, MODE == 1>(ri, fetch(li), fi, fine(li), pk, nacc, ue);
         };
         if constexpr (TPA == 1) {
-            // groups of four neighbours; the next group's indices are loaded
-            // while the current group is computed
+            // groups of four neighbours, one word of the list each; the next
+            // word is loaded while the current group is computed
             const PairK2 pk2c(pk);
             [[maybe_unused]] uint64_t fx2 = 0, fy2 = 0, fz2 = 0;  // packed (0.0f, 0.0f)
             [[maybe_unused]] float gx = 0.f, gy = 0.f, gz = 0.f;  // measure pass: odd entries
             int32_t s = 0;
-            int32_t li[4];
-            if (nf >= 4) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) li[k] = LF[-(int64_t)k * kBlock];
-            }
+            const uint2* __restrict__ lw = LW + (list_words(a.lcap) - 1) * kBlock;
+            uint2 cur = nf > 0 ? __ldg(lw) : make_uint2(0u, 0u);
             for (; s + 4 <= nf; s += 4) {
                 int4 rj[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) rj[k] = fetch(li[k]);
-                if (s + 8 <= nf) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) li[k] = LF[-(int64_t)(s + 4 + k) * kBlock];
-                }
+                rj[0] = fetch((int32_t)(cur.x & 0xffffu));
+                rj[1] = fetch((int32_t)(cur.x >> 16));
+                rj[2] = fetch((int32_t)(cur.y & 0xffffu));
+                rj[3] = fetch((int32_t)(cur.y >> 16));
+                lw -= kBlock;
+                if (s + 4 < nf) cur = __ldg(lw);
                 if constexpr (MEASURE) {
                     // even entries into (fx, fy, fz), odd ones into (gx, gy, gz),
                     // as the two halves of the packed form
@@ -1380,10 +1594,12 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
                 fy += gy;
                 fz += gz;
             }
-            for (; s < nf; ++s)
-                if (accum_pair<COUL, MODE == 1>(ri, fetch(LF[-(int64_t)s * kBlock]), pk, fx, fy,
-                                                fz, ue))
-                    far_near(s);
+            for (; s < nf; ++s) {
+                const int32_t li = (int32_t)(cur.x & 0xffffu);
+                cur.x = __funnelshift_r(cur.x, cur.y, 16);
+                cur.y >>= 16;
+                if (accum_pair<COUL, MODE == 1>(ri, fetch(li), pk, fx, fy, fz, ue)) far_near(s);
+            }
             // the force: two-float near sums with the single-precision sums added
             // to their low parts, rounded once
             fx = __fadd_rn(nacc.xh, __fadd_rn(nacc.xl, fx));
@@ -1397,7 +1613,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int32_t sk = s0 + k * TPA;
-                    li[k] = sk < nf ? LF[-(int64_t)sk * kBlock] : 0;
+                    li[k] = sk < nf ? far_entry(sk) : 0;
                 }
             };
             int32_t s = part;
@@ -1450,11 +1666,11 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
         pairs(std::true_type{});
     else
         pairs(std::false_type{});
-    if (valid && own) a.f_out[i] = make_float4(fx, fy, fz, 0.f);
     const bool MASS = a.has_mass != 0, FIRST = a.first != 0;
-    const double imv = MASS ? a.im[i] : 1.0;
     const float fv[3] = {fx, fy, fz};
     if constexpr (MEASURE) {
+        const double imv = MASS ? a.im[i] : 1.0;
+        if (valid && own) a.f_out[i] = make_float4(fx, fy, fz, 0.f);
         double ke = 0.0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -1492,10 +1708,21 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
         uint32_t xf[3];
         bool trig = false;
         if (valid && own) {
+        // all loads before the first store (the state is updated in place, so
+        // the compiler keeps their order: one trip to memory instead of four)
+        double wv[3], xv[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            double v = a.w[d][i] + (double)(kdt * fv[d]) * imv;
-            double x = fma(a.dt, v, a.x[d][i]);
+            wv[d] = a.w[d][i];
+            xv[d] = a.x[d][i];
+        }
+        const int4 rb = __ldg(&a.rec_build[i]);
+        const double imv = MASS ? a.im[i] : 1.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double kick = (double)(kdt * fv[d]);
+            double v = MASS ? fma(kick, imv, wv[d]) : wv[d] + kick;
+            double x = fma(a.dt, v, xv[d]);
             const double os = BATCH ? __ldg(&row->os[d]) : a.os[d];
             long long q = __double2ll_rn(fma(x, S * kFine, -os));
             // integer pre-check (before the wrap); the exact FP64 test of
@@ -1520,7 +1747,6 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
         // A list built at r_c + skin stays valid while no atom moved more than
         // skin/2 since the build; count the atom-steps that broke that bound
         // where the next step keeps the list without a check.
-        const int4 rb = __ldg(&a.rec_build[i]);
         const float ex = (float)idiff(xi[0], rb.x), ey = (float)idiff(xi[1], rb.y),
                     ez = (float)idiff(xi[2], rb.z);
         const float e2 = ex * ex + ey * ey + ez * ez;
@@ -1666,6 +1892,13 @@ static cudaError_t raise_smem_limit(const void* fn, int maxsm) {
                                 maxsm - (int)fa.sharedSizeBytes);
 }
 
+// Whether the lists are built by a warp per leaf: while there is at most one
+// block of kBlock atoms per SM, whose threads (one an atom) would walk their
+// candidates on a part of the chip, and the candidates fit shared memory.
+static bool md_leaf_warps(const MDEngine* m) {
+    return m->nblocks <= m->nsm && 8 * sizeof(uint2) * (size_t)m->lcap_leaf <= 200 * 1024;
+}
+
 // Union and list buffers for capacities (ucap, lcap), and the shared-memory
 // opt-ins of the kernels that stage them.
 static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t lcap_leaf,
@@ -1682,11 +1915,12 @@ static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t
     m->upow2 = p2;
     int maxsm = 0;
     cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+    cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, c->device);
     // staged records must fit the block's shared memory
     m->ucap_sm = std::max(0, std::min(m->ucap_sm, (maxsm - 1024) / (16 * m->apl)));
     if ((st = ensure(c, m->ulist, sizeof(int32_t) * (size_t)ucap * m->nblocks))) return st;
     if (lcap > 0 &&
-        (st = ensure(c, m->llist, sizeof(uint16_t) * (size_t)lcap * kBlock * m->nblocks)))
+        (st = ensure(c, m->llist, sizeof(uint16_t) * (size_t)list_block(lcap) * m->nblocks)))
         return st;
     if (lcap_leaf > 0 &&
         (st = ensure(c, m->llist_leaf, sizeof(uint16_t) * (size_t)lcap_leaf * m->nL)))
@@ -1699,8 +1933,7 @@ static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t
     // waves of one block per SM, when the slice partials fit beside the
     // staged union
     {
-        int nsm = 0;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+        const int nsm = m->nsm;
         auto fits = [&](int t) {
             const size_t part_sm = sizeof(float) * 8 * kBlock * (size_t)(t - 1);
             return (int)(m->step_smem + part_sm) + 1024 <= maxsm;
@@ -1729,11 +1962,17 @@ static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t
     // memory) rather than set per engine.
     cudaError_t e = raise_smem_limit((const void*)k_md_block_union, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<1>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<1>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<2>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<2>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<4>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<4>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<8>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<8>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<16>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<16>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<32>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<32>, maxsm);
 #define ND_SMEM(C, MODE)                                                                        \
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_step<C, MODE, false>, maxsm);   \
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_step<C, MODE, true>, maxsm);    \
@@ -1915,16 +2154,26 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
         live.sid, n, m->nL, m->apl, hq, rl, m->fcap, m->ucap,
         m->upow2, (int32_t*)m->ulist.p, (int32_t*)m->ucount.p, (uint16_t*)m->llist_leaf.p,
         (int32_t*)m->lcount_leaf.p, m->lcap_leaf, c->d_err, (int32_t*)m->diag.p + 2,
-        sizing ? 1 : 0, pressure, gate);
-#define ND_LISTS(A)                                                                             \
-    k_md_block_lists<A><<<(unsigned)m->nblocks, kBlock, m->lists_smem, c->stream>>>(            \
-        (const float4*)m->pos32.p, n, rl * rl,                                                  \
-        md_near(m->p.sigma, m->p.epsilon, m->p.coulomb_k, m->p.cutoff, m->fr.s).rnb2,           \
-        m->nsys > 0 ? live.sid : nullptr, sys, m->ucap, m->lists_smpos,                         \
-        (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p,                                \
-        (const uint16_t*)m->llist_leaf.p, (const int32_t*)m->lcount_leaf.p, m->lcap_leaf,       \
-        m->lcap, (uint16_t*)m->llist.p, (int32_t*)m->ncount.p, c->d_err,                        \
-        (int32_t*)m->diag.p + 2, sizing ? 1 : 0, pressure, gate)
+        sizing ? 1 : 0, pressure, gate, md_leaf_warps(m) ? 0 : 1);
+    const float rnb2 = md_near(m->p.sigma, m->p.epsilon, m->p.coulomb_k, m->p.cutoff, m->fr.s).rnb2;
+    const int32_t* sid = m->nsys > 0 ? live.sid : nullptr;
+#define ND_LISTS(A)                                                                              \
+    do {                                                                                         \
+        if (md_leaf_warps(m))                                                                    \
+            k_md_leaf_lists<A><<<(unsigned)m->nblocks * (kBlock / A / 8), kBlock,                \
+                                 8 * sizeof(uint2) * (size_t)m->lcap_leaf, c->stream>>>(         \
+                keys, (const float4*)m->pos32.p, m->nL, rl, rl * rl, rnb2, sid, sys, m->ucap,    \
+                (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p, m->lcap_leaf, m->lcap,  \
+                (uint16_t*)m->llist.p, (int32_t*)m->ncount.p, c->d_err,                          \
+                (int32_t*)m->diag.p + 2, sizing ? 1 : 0, pressure, gate);                        \
+        else                                                                                     \
+            k_md_block_lists<A><<<(unsigned)m->nblocks, kBlock, m->lists_smem, c->stream>>>(     \
+                (const float4*)m->pos32.p, n, rl * rl, rnb2, sid, sys, m->ucap, m->lists_smpos,  \
+                (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p,                         \
+                (const uint16_t*)m->llist_leaf.p, (const int32_t*)m->lcount_leaf.p,              \
+                m->lcap_leaf, m->lcap, (uint16_t*)m->llist.p, (int32_t*)m->ncount.p, c->d_err,   \
+                (int32_t*)m->diag.p + 2, sizing ? 1 : 0, pressure, gate);                        \
+    } while (0)
     switch (m->apl) {
         case 1: ND_LISTS(1); break;
         case 2: ND_LISTS(2); break;
@@ -2899,11 +3148,11 @@ __global__ void k_md_list_pairs(const int32_t* __restrict__ ncount,
     if (i >= n) return;
     const int32_t b = i / kBlock, t = i - b * kBlock;
     const int32_t c = ncount[i];
-    const uint16_t* L = llist + (int64_t)b * lcap * kBlock;
+    const uint16_t* L = llist + (int64_t)b * list_block(lcap);
     const int32_t* U = ulist + (int64_t)b * ucap;
     const int32_t tot = list_total(c), nn = list_near(c);
     for (int32_t s = 0; s < tot; ++s) {
-        const int32_t li = L[llist_at(list_slot(s, c, lcap), t)];
+        const int32_t li = L[list_at(s, c, t, lcap)];
         const int32_t j = U[li / apl] * apl + li % apl;
         const unsigned long long k = atomicAdd(cursor, 1ull);
         if ((int64_t)k < cap) {

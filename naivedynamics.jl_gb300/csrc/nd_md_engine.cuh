@@ -181,6 +181,7 @@ struct MDEngine {
     int64_t resort_kernels = 0;       // kernels of one re-sort rebuild
     int64_t eager_bodies = 0;         // kernels of rebuild bodies run eagerly (counted by the host)
     size_t step_smem = 0, union_smem = 0, lists_smem = 0;
+    int nsm = 0;              // SMs of the device
     int32_t lists_smpos = 0;  // positions the list kernel stages in shared memory
     int32_t split = 1;  // thread blocks of the step kernel per block of kBlock atoms
     int32_t tpa = 1;  // threads per atom of the step kernel
@@ -195,20 +196,31 @@ struct MDEngine {
 enum { RB_RESORT = 0, RB_REFIT = 1 };
 
 // Per-atom neighbour lists (uint16 indices into the block's union), per block
-// of kBlock atoms, slot-major: slot s of the block's thread t is element
-// s * kBlock + t, so a warp reading its atoms' s-th entries reads 64
-// contiguous bytes.  Each list has two segments: the near entries from slot
-// 0 upwards and the others from slot lcap - 1 downwards; ncount packs the
-// two counts (near in the low 16 bits).
-__device__ __forceinline__ int64_t llist_at(int32_t s, int32_t t) {
-    return (int64_t)s * kBlock + t;
-}
+// of kBlock atoms, in 8-byte words of four consecutive entries: word w of the
+// block's thread t is word w * kBlock + t, so a warp reading its atoms' w-th
+// words reads 256 contiguous bytes and a list is written and read four entries
+// at a time.  Each list has two segments: the near entries from word 0
+// upwards and the others from word list_words(lcap) - 1 downwards; ncount
+// packs the two counts (near in the low 16 bits).  A list of lcap entries (a
+// multiple of 4) fits whatever its split: one word more than lcap / 4.
+__host__ __device__ inline int32_t list_words(int32_t lcap) { return lcap / 4 + 1; }
 __device__ __forceinline__ int32_t list_near(int32_t c) { return c & 0xffff; }
 __device__ __forceinline__ int32_t list_total(int32_t c) { return (c & 0xffff) + (c >> 16); }
-// slot of logical entry s (near entries first, then the others in build order)
-__device__ __forceinline__ int32_t list_slot(int32_t s, int32_t c, int32_t lcap) {
+// element (uint16) of near entry s, of other entry s, of thread t
+__device__ __forceinline__ int32_t near_at(int32_t s, int32_t t) {
+    return ((s >> 2) * kBlock + t) * 4 + (s & 3);
+}
+__device__ __forceinline__ int32_t far_at(int32_t s, int32_t t, int32_t lcap) {
+    return ((list_words(lcap) - 1 - (s >> 2)) * kBlock + t) * 4 + (s & 3);
+}
+// element of logical entry s (near entries first, then the others in build order)
+__device__ __forceinline__ int32_t list_at(int32_t s, int32_t c, int32_t t, int32_t lcap) {
     const int32_t nn = c & 0xffff;
-    return s < nn ? s : lcap - 1 - (s - nn);
+    return s < nn ? near_at(s, t) : far_at(s - nn, t, lcap);
+}
+// elements of a block's lists
+__host__ __device__ inline int64_t list_block(int32_t lcap) {
+    return (int64_t)list_words(lcap) * 4 * kBlock;
 }
 
 // Rebuild of the neighbour lists (re-sort or refit; see nd_md.cu).
