@@ -495,6 +495,7 @@ static size_t adj_statics_bytes(const AdjEngine* A) {
 }
 
 static nd_status adj_copy(AdjEngine* A, void* dst, const void* src, size_t bytes, const char* what) {
+    A->m->gated = false;
     cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, A->m->sub.stream);
     if (e != cudaSuccess) return cuda_fail(&A->m->sub, e, what);
     return ND_OK;
@@ -676,7 +677,9 @@ static nd_status adj_capture(AdjEngine* A, cudaGraphExec_t* out, F&& body) {
     const int64_t l0 = c->launches;
     cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(c, e, "begin capture");
+    A->m->gated = false;
     nd_status st = body();
+    A->m->gated = false;
     e = cudaStreamEndCapture(c->stream, &g);
     c->launches = l0;
     if (st) { if (g) cudaGraphDestroy(g); return st; }
@@ -702,8 +705,11 @@ nd_status adj_destroy(AdjEngine* A) {
     DevBuf* bufs[] = {&A->ckpt, &A->perms, &A->codes, &A->statics, &A->traj, &A->trajrec, &A->recK, &A->lam, &A->lam_tmp, &A->g4[0],
                       &A->g4[1], &A->gpart, &A->xK, &A->hatom, &A->hist, &A->target, &A->cb,
                       &A->scal, &A->outs, &A->flags};
-    for (DevBuf* b : bufs)
-        if (b->p) cudaFree(b->p);
+    for (DevBuf* b : bufs) {
+        if (!b->p) continue;
+        if (A->m && A->m->sub.pool) A->m->sub.pool->put(*b);
+        else cudaFree(b->p);
+    }
     if (A->m) md_destroy(A->m);
     delete A;
     return ND_OK;

@@ -20,6 +20,7 @@ struct nd_md;
 struct nd_adj;
 
 struct nd_ctx {
+    nd::BufPool pool;
     nd::Ctx c;
     std::set<nd_md*> engines;
     std::set<nd_adj*> adjoints;
@@ -57,6 +58,44 @@ nd_status check_launch(Ctx* c, const char* what) {
     return ND_OK;
 }
 
+bool BufPool::take(DevBuf& b, size_t bytes) {
+    std::lock_guard<std::mutex> lock(mu);
+    size_t best = idle.size();
+    for (size_t k = 0; k < idle.size(); ++k)
+        // the smallest that fits, not much larger than asked for
+        if (idle[k].bytes >= bytes && idle[k].bytes <= 2 * bytes + 65536 &&
+            (best == idle.size() || idle[k].bytes < idle[best].bytes))
+            best = k;
+    if (best == idle.size()) return false;
+    b = idle[best];
+    held -= b.bytes;
+    idle[best] = idle.back();
+    idle.pop_back();
+    return true;
+}
+
+void BufPool::put(DevBuf& b) {
+    if (!b.p) return;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (idle.size() < kMost && held + b.bytes <= kBytes) {
+            idle.push_back(b);
+            held += b.bytes;
+            b = DevBuf{};
+            return;
+        }
+    }
+    cudaFree(b.p);
+    b = DevBuf{};
+}
+
+void BufPool::clear() {
+    std::lock_guard<std::mutex> lock(mu);
+    for (DevBuf& b : idle) cudaFree(b.p);
+    idle.clear();
+    held = 0;
+}
+
 nd_status ensure(Ctx* c, DevBuf& b, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (b.p && b.bytes >= bytes) return ND_OK;
@@ -69,7 +108,13 @@ nd_status ensure(Ctx* c, DevBuf& b, size_t bytes) {
         b.p = nullptr;
         b.bytes = 0;
     }
+    if (c->pool && c->pool->take(b, bytes)) return ND_OK;
     cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e != cudaSuccess && c->pool) {
+        cudaGetLastError();
+        c->pool->clear();
+        e = cudaMalloc(&b.p, bytes);
+    }
     if (e != cudaSuccess) {
         b.p = nullptr;
         cudaGetLastError();
@@ -304,6 +349,7 @@ nd_status nd_ctx_create(nd_ctx** out, int32_t device) {
     if (!h) return ND_ERR_NOMEM;
     Ctx* c = &h->c;
     c->device = device;
+    c->pool = &h->pool;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_err, sizeof(int32_t) * nd::kErrWords);
@@ -342,6 +388,7 @@ nd_status nd_ctx_destroy(nd_ctx* h) {
                           &c->partial, &c->pairs_i, &c->pairs_j, &c->pairs_d, &c->misc, &c->hash,
                           &c->leafpairs, &c->ranges, &c->tasks, &c->compat};
     for (nd::DevBuf* b : bufs) nd::free_buf(*b);
+    h->pool.clear();
     if (c->d_err) cudaFree(c->d_err);
     if (c->h_err) cudaFreeHost(c->h_err);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -626,18 +673,7 @@ nd_status nd_forces(nd_ctx* h, const nd_md_params* p, int32_t n, const double* x
     nd_md_params pp = *p;
     if (pp.rebuild_every <= 0) pp.rebuild_every = 1;
     if (!(pp.dt > 0)) pp.dt = 1.0;
-    std::vector<double> v0(3 * (size_t)n, 0.0);
-    nd::MDEngine* m = nullptr;
-    if ((st = nd::md_create(c, &pp, n, x, v0.data(), q, nullptr, true, false, &m))) return st;
-    st = nd::md_get(m, nullptr, nullptr, force, true);
-    if (st == ND_OK && energy) {
-        double pot = 0.0;
-        st = nd::md_energy(m, &pot, nullptr);
-        *energy = pot;
-    }
-    if (st) c->last_error = nd::md_last_error(m);
-    nd::md_destroy(m);
-    return st;
+    return nd::md_forces(c, &pp, n, x, q, force, energy);
 }
 
 nd_status nd_md_create(nd_ctx* h, const nd_md_params* p, int32_t n, const double* x,

@@ -6,7 +6,9 @@
 #include <stdint.h>
 
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/naivegpu.h"
 #include <nvtx3/nvToolsExt.h>
@@ -138,6 +140,27 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// Device buffers of destroyed engines, kept by their context for the next
+// engine: an engine holds about 35 of them, and a call that makes one for
+// itself (forces(), simulate_ with a log) spent a third of its time in
+// cudaMalloc and cudaFree.  At most kMost blocks and kBytes bytes wait; they
+// are freed with the context, or when an allocation fails.  A buffer comes
+// here only after its stream was synchronised, and one context's engines share
+// one stream.
+class BufPool {
+public:
+    bool take(DevBuf& b, size_t bytes);
+    void put(DevBuf& b);
+    void clear();
+    ~BufPool() { clear(); }
+
+private:
+    static constexpr size_t kMost = 128, kBytes = size_t(512) << 20;
+    std::mutex mu;
+    std::vector<DevBuf> idle;
+    size_t held = 0;
+};
+
 // Context shared by all entry points (defined in nd_capi.cu).
 struct Ctx {
     int device = 0;
@@ -151,7 +174,39 @@ struct Ctx {
         partial, pairs_i, pairs_j, pairs_d, misc, hash, leafpairs, ranges, tasks, compat;
     struct MDEngine* sim_cache = nullptr;  // engine re-used by nd_simulate
     bool no_alloc = false;                 // buffers are fixed slices: never grow them
+    BufPool* pool = nullptr;               // idle buffers of the context (may be null)
 };
+
+// Programmatic dependent launch, for kernels that mostly find nothing to do
+// (gated refits) and the step behind them.  A kernel launched with chained =
+// true starts with chain_wait(): its blocks may be resident before the kernel
+// in front of it has ended, and the wait holds until that kernel is complete
+// and its writes are visible.  Every such kernel waits on every path, so
+// completion passes along the chain.  (4,096 atoms, a check after every step:
+// 16.3 -> 15.5 us a step; chaining the steps to each other or a rebuild's own
+// kernels gained nothing, steps lost 0.8 us.)
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch_chained(Ctx* c, bool chained, void (*k)(P...), unsigned grid, unsigned block,
+                           size_t smem, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    if (chained) {
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+    }
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
+    c->launches++;
+}
 
 // Grow `b` to at least `bytes` (contents are not preserved).
 nd_status ensure(Ctx* c, DevBuf& b, size_t bytes);
@@ -224,6 +279,9 @@ struct MDEngine;
 nd_status md_create(Ctx* parent, const nd_md_params* p, int32_t n, const double* x,
                     const double* v, const double* q, const double* mass, bool host,
                     bool capture, MDEngine** out);
+// Forces (host, N x 3) and potential energy (may be null) of a configuration.
+nd_status md_forces(Ctx* parent, const nd_md_params* p, int32_t n, const double* x,
+                    const double* q, float* force, double* energy);
 nd_status md_destroy(MDEngine* m);
 nd_status md_create_batch(Ctx* parent, const nd_md_params* p, int32_t nsys, const nd_system* sys,
                           const double* x, const double* v, const double* q, const double* mass,

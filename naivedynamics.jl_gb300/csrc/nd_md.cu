@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(kBlock)
                uint2* __restrict__ recf, int4* __restrict__ recb, float4* __restrict__ keys,
                float4* __restrict__ bbox, int32_t* err, const unsigned* __restrict__ gate,
                unsigned* counter) {
+    chain_wait();
     if (gate && *gate == 0u) return;
     __shared__ float s_b[kBlock / 32][6];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -308,6 +309,7 @@ __device__ __forceinline__ bool box_overlap(float qmnx, float qmny, float qmnz, 
 // like tree nodes: min xyz, max x), (max y, max z, 0, 0)): one warp each.
 __global__ void __launch_bounds__(256)
     k_md_super_boxes(int32_t nblocks, float4* __restrict__ bbox, const unsigned* __restrict__ gate) {
+    chain_wait();
     if (gate && *gate == 0u) return;
     const int lane = threadIdx.x & 31;
     const int32_t sb = (int32_t)blockIdx.x * 8 + (int32_t)(threadIdx.x >> 5);
@@ -409,6 +411,7 @@ __global__ void __launch_bounds__(kBlock, 4)
                      uint16_t* __restrict__ llist_leaf, int32_t* __restrict__ lcount_leaf,
                      int32_t lcap_leaf, int32_t* err, int32_t* diag, int32_t sizing,
                      unsigned* pressure, const unsigned* __restrict__ gate, int32_t candidates) {
+    chain_wait();
     if (gate && *gate == 0u) return;
     extern __shared__ int32_t smem[];
     int32_t* fr[2] = {smem, smem + fcap};
@@ -742,6 +745,7 @@ __global__ void __launch_bounds__(kBlock)
                      uint16_t* __restrict__ llist, int32_t* __restrict__ ncount, int32_t* err,
                      int32_t* diag, int32_t sizing, unsigned* pressure,
                      const unsigned* __restrict__ gate) {
+    chain_wait();
     if (gate && *gate == 0u) return;
     extern __shared__ float4 spos[];
     const int32_t blk = (int32_t)blockIdx.x;
@@ -877,6 +881,7 @@ __global__ void __launch_bounds__(kBlock)
                     int32_t lcap_leaf, int32_t lcap, uint16_t* __restrict__ llist,
                     int32_t* __restrict__ ncount, int32_t* err, int32_t* diag, int32_t sizing,
                     unsigned* pressure, const unsigned* __restrict__ gate) {
+    chain_wait();
     if (gate && *gate == 0u) return;
     extern __shared__ uint2 cand_all[];
     constexpr int LPB = kBlock / APL, CPB = LPB / 8;  // leaves, thread blocks per block of atoms
@@ -1403,6 +1408,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
     const int32_t blk = (int32_t)(blockIdx.x / SPLIT);
     const int tid = (int)(blockIdx.x % SPLIT) * APB + (int)(threadIdx.x & (APB - 1));  // the atom
     const int part = threadIdx.x / APB;  // its list slice
+    if constexpr (MODE == 0) chain_wait();
     int64_t i = (int64_t)blk * kBlock + tid;
     const bool valid = i < a.n;
     const bool own = part == 0;  // the thread that updates the atom
@@ -1943,13 +1949,15 @@ static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t
         else if (req > 0) m->tpa = fits(req) ? req : 1;
         else m->tpa = (m->nblocks < 2 * nsm && fits(kSmallTPA)) ? kSmallTPA : 1;
         // thread blocks per block of atoms with 4 threads per atom: the given
-        // number, or (0) the most that keep the grid within one block per SM
-        // (32,768 atoms: 128 blocks of 1,024 threads ran faster than 256 of 512)
+        // number, or (0) four of 256 threads while an SM gets at most two of
+        // them, else one of 1,024 threads.  us a step with 1 / 2 / 4: 16 blocks
+        // of atoms 12.3 / 8.4 / 7.5, 40 14.7 / 10.0 / 8.9, 76 15.2 / 10.7 / 10.8,
+        // 94 15.3 / 17.6 / 16.7, 128 15.2 / 17.7 / 18.0 (eight of 128 threads: no
+        // faster anywhere, each stages the whole union).
         m->split = 1;
         if (m->tpa == kSmallTPA) {
             if (m->p.cta_split > 0) m->split = m->p.cta_split;
-            else if (4 * m->nblocks <= nsm) m->split = 4;
-            else if (2 * m->nblocks <= nsm) m->split = 2;
+            else if (4 * m->nblocks <= 2 * nsm) m->split = 4;
         }
     }
     if ((int)m->union_smem + 1024 > maxsm || (lcap > 0 && (int)m->step_smem + 1024 > maxsm)) {
@@ -2064,11 +2072,14 @@ static void launch_step(MDEngine* m, const StepArgs& a0, bool first) {
     StepArgs a = a0;
     a.first = first ? 1 : 0;
     a.has_mass = m->has_m ? 1 : 0;
+    // in a captured window a step that follows a gated refit is its dependent
+    const bool chained = MODE == 0 && m->gated;
+    m->gated = false;
 #define ND_STEP(BATCH, TPA, SPLIT)                                                              \
     do {                                                                                        \
         const unsigned gs = grid * SPLIT, bs = kBlock * TPA / SPLIT;                            \
-        if (coul) k_md_step<true, MODE, BATCH, TPA, SPLIT><<<gs, bs, sm, c->stream>>>(a);       \
-        else k_md_step<false, MODE, BATCH, TPA, SPLIT><<<gs, bs, sm, c->stream>>>(a);           \
+        if (coul) launch_chained(c, chained, k_md_step<true, MODE, BATCH, TPA, SPLIT>, gs, bs, sm, a);   \
+        else launch_chained(c, chained, k_md_step<false, MODE, BATCH, TPA, SPLIT>, gs, bs, sm, a);       \
     } while (0)
     if (m->nsys > 0) ND_STEP(true, 1, 1);
     else if (m->tpa == kSmallTPA && m->split == 4) ND_STEP(false, kSmallTPA, 4);
@@ -2077,7 +2088,6 @@ static void launch_step(MDEngine* m, const StepArgs& a0, bool first) {
     else if (m->tpa == 2) ND_STEP(false, 2, 1);
     else ND_STEP(false, 1, 1);
 #undef ND_STEP
-    c->launches++;
 }
 
 void md_launch_step(MDEngine* m, const StepArgs& a, bool first) { launch_step<0>(m, a, first); }
@@ -2113,11 +2123,10 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
     const float rl = (float)(m->p.cutoff + m->p.skin);
     const int rb = rec >= 0 ? rec : 0;
     auto place = [&](auto copy) {
-        k_md_place<decltype(copy)::value><<<(unsigned)m->nblocks, kBlock, 0, c->stream>>>(
-            tmp, live, n, m->fr, sys, m->apl, rl / 2.0f, (float4*)m->pos32.p,
-            (int4*)m->rec_buf[rb].p, (uint2*)m->recf_buf[rb].p, (int4*)m->recb.p, keys, bbox,
-            c->d_err, gate, kind == RB_REFIT ? counter : nullptr);
-        c->launches++;
+        launch_chained(c, gate != nullptr, k_md_place<decltype(copy)::value>, (unsigned)m->nblocks,
+                       kBlock, 0, tmp, live, n, m->fr, sys, m->apl, rl / 2.0f, (float4*)m->pos32.p,
+                       (int4*)m->rec_buf[rb].p, (uint2*)m->recf_buf[rb].p, (int4*)m->recb.p, keys,
+                       bbox, c->d_err, gate, kind == RB_REFIT ? counter : nullptr);
     };
     if (kind == RB_REFIT) {
         place(std::false_type{});
@@ -2142,15 +2151,14 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
                                        nullptr, gate)))
             return st;
     } else if (m->nblocks > kDirectBlocks) {
-        k_md_super_boxes<<<(unsigned)cdiv(m->nblocks, 256), 256, 0, c->stream>>>(m->nblocks, bbox,
-                                                                                 gate);
-        c->launches++;
+        launch_chained(c, gate != nullptr, k_md_super_boxes, (unsigned)cdiv(m->nblocks, 256), 256, 0, m->nblocks, bbox,
+                       gate);
     }
     // query boxes slightly above r_list/2 so the box tests never drop a pair;
     // the distance test alone decides membership
     const float hq = (rl / 2.0f) * 1.0001f + 1e-6f;
-    k_md_block_union<<<(unsigned)m->nblocks, kBlock, m->union_smem, c->stream>>>(
-        keys, bbox, m->nblocks, tree ? 1 : 0, (const float4*)m->pos32.p,
+    launch_chained(
+        c, gate && !tree, k_md_block_union, (unsigned)m->nblocks, kBlock, m->union_smem, keys, bbox, m->nblocks, tree ? 1 : 0, (const float4*)m->pos32.p,
         live.sid, n, m->nL, m->apl, hq, rl, m->fcap, m->ucap,
         m->upow2, (int32_t*)m->ulist.p, (int32_t*)m->ucount.p, (uint16_t*)m->llist_leaf.p,
         (int32_t*)m->lcount_leaf.p, m->lcap_leaf, c->d_err, (int32_t*)m->diag.p + 2,
@@ -2160,14 +2168,17 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
 #define ND_LISTS(A)                                                                              \
     do {                                                                                         \
         if (md_leaf_warps(m))                                                                    \
-            k_md_leaf_lists<A><<<(unsigned)m->nblocks * (kBlock / A / 8), kBlock,                \
-                                 8 * sizeof(uint2) * (size_t)m->lcap_leaf, c->stream>>>(         \
-                keys, (const float4*)m->pos32.p, m->nL, rl, rl * rl, rnb2, sid, sys, m->ucap,    \
+            launch_chained(                                                                      \
+                c, gate != nullptr, k_md_leaf_lists<A>,                                          \
+                (unsigned)m->nblocks * (kBlock / A / 8), kBlock,                                 \
+                8 * sizeof(uint2) * (size_t)m->lcap_leaf, keys, (const float4*)m->pos32.p, m->nL, rl, rl * rl, rnb2, sid, sys, m->ucap,    \
                 (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p, m->lcap_leaf, m->lcap,  \
                 (uint16_t*)m->llist.p, (int32_t*)m->ncount.p, c->d_err,                          \
                 (int32_t*)m->diag.p + 2, sizing ? 1 : 0, pressure, gate);                        \
         else                                                                                     \
-            k_md_block_lists<A><<<(unsigned)m->nblocks, kBlock, m->lists_smem, c->stream>>>(     \
+            launch_chained(                                                                      \
+                c, gate != nullptr, k_md_block_lists<A>, (unsigned)m->nblocks, kBlock,           \
+                m->lists_smem,                                                                   \
                 (const float4*)m->pos32.p, n, rl * rl, rnb2, sid, sys, m->ucap, m->lists_smpos,  \
                 (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p,                         \
                 (const uint16_t*)m->llist_leaf.p, (const int32_t*)m->lcount_leaf.p,              \
@@ -2183,7 +2194,7 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
         default: ND_LISTS(32); break;
     }
 #undef ND_LISTS
-    c->launches += 2;
+    m->gated = gate != nullptr;
     if (rec < 0) m->rc = 0;
     return check_launch(c, "md rebuild");
 }
@@ -2377,6 +2388,7 @@ static nd_status md_observe(MDEngine* m, int32_t p, bool capture, int64_t g) {
     cudaGraphConditionalHandle ht = 0, hl = 0;
     if (pt && (st = md_cond_handle(m, &ht))) return st;
     if (pl && (st = md_cond_handle(m, &hl))) return st;
+    m->gated = false;
     k_md_due<<<1, 32, 0, c->stream>>>((const unsigned*)m->ctl.p, R, p, pt ? m->thermo_every : 0,
                                       pl ? m->log_every : 0, ht, hl);
     c->launches++;
@@ -2448,7 +2460,9 @@ static nd_status md_capture_first(MDEngine* m) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(c, e, "begin capture");
+    m->gated = false;
     nd_status st = md_steps(m, m->p.rebuild_every, 0, true);
+    m->gated = false;
     e = cudaStreamEndCapture(c->stream, &g);
     if (st) { if (g) cudaGraphDestroy(g); return st; }
     if (e != cudaSuccess) return cuda_fail(c, e, "end capture");
@@ -2472,8 +2486,10 @@ static nd_status md_capture_main(MDEngine* m) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(c, e, "begin capture");
+    m->gated = false;
     nd_status st = md_window_begin(m, true);
     if (st == ND_OK) st = md_steps(m, m->p.rebuild_every, 0, true);
+    m->gated = false;
     e = cudaStreamEndCapture(c->stream, &g);
     if (st) { if (g) cudaGraphDestroy(g); return st; }
     if (e != cudaSuccess) return cuda_fail(c, e, "end capture");
@@ -2567,7 +2583,9 @@ nd_status md_upload(MDEngine* m, const double* xd, const double* vd, const doubl
     double* am = aq + (size_t)n;
     cudaMemcpyKind kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     cudaError_t e = cudaMemcpyAsync(ax, xd, bytes, kind, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(av, vd, bytes, kind, c->stream);
+    if (e == cudaSuccess)  // no velocities (forces of a configuration): at rest
+        e = vd ? cudaMemcpyAsync(av, vd, bytes, kind, c->stream)
+               : cudaMemsetAsync(av, 0, bytes, c->stream);
     if (e == cudaSuccess && qd) e = cudaMemcpyAsync(aq, qd, sizeof(double) * n, kind, c->stream);
     if (e == cudaSuccess && md_) e = cudaMemcpyAsync(am, md_, sizeof(double) * n, kind, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "md upload");
@@ -2700,8 +2718,9 @@ static nd_status md_frame_batch(MDEngine* m, const nd_system* sys) {
 static nd_status md_create_common(Ctx* parent, const nd_md_params* p, int32_t n,
                                   const double* xd, const double* vd, const double* qd,
                                   const double* md_, bool host, bool capture, MDEngine** out,
-                                  int32_t nsys = 0, const nd_system* sys = nullptr) {
-    if (!parent || !p || !out || !xd || !vd || n <= 0) return ND_ERR_ARG;
+                                  int32_t nsys = 0, const nd_system* sys = nullptr,
+                                  bool at_rest = false) {
+    if (!parent || !p || !out || !xd || (!vd && !at_rest) || n <= 0) return ND_ERR_ARG;
     if (p->atomsperleaf <= 0 || n % p->atomsperleaf || n / p->atomsperleaf < 2) return ND_ERR_SPEC;
     if (32 % p->atomsperleaf != 0) return ND_ERR_SPEC;  // a warp holds whole leaves
     if (p->rebuild_every <= 0 || !(p->cutoff > 0) || !(p->skin >= 0) || !(p->dt > 0) ||
@@ -2731,6 +2750,7 @@ static nd_status md_create_common(Ctx* parent, const nd_md_params* p, int32_t n,
     m->sub.stream = parent->stream;
     m->sub.d_err = parent->d_err;
     m->sub.h_err = parent->h_err;
+    m->sub.pool = parent->pool;
     m->p = *p;
     m->n = n;
     m->apl = p->atomsperleaf;
@@ -2937,8 +2957,11 @@ nd_status md_destroy(MDEngine* m) {
                       &m->sub.codes_alt, &m->sub.perm, &m->sub.perm_alt, &m->sub.hist,
                       &m->sub.misc};
     if (m->sub.stream) cudaStreamSynchronize(m->sub.stream);
-    for (DevBuf* b : bufs)
-        if (b->p) cudaFree(b->p);
+    for (DevBuf* b : bufs) {
+        if (!b->p) continue;
+        if (m->sub.pool) m->sub.pool->put(*b);
+        else cudaFree(b->p);
+    }
     if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
     delete m;
     return ND_OK;
@@ -3074,6 +3097,37 @@ nd_status md_get(MDEngine* m, double* x, double* v, float* f, bool host) {
     m->parent->launches += c->launches;
     c->launches = 0;
     return sync_and_check(c, "md get");
+}
+
+nd_status md_forces(Ctx* parent, const nd_md_params* p, int32_t n, const double* x,
+                    const double* q, float* force, double* energy) {
+    MDEngine* m = nullptr;
+    nd_status st = md_create_common(parent, p, n, x, nullptr, q, nullptr, true, false, &m, 0, nullptr,
+                                    true);
+    if (st) return st;
+    Ctx* c = &m->sub;
+    // one pass for both: the forces, and the energy when it is asked for
+    double pot = 0.0;
+    st = md_measure(m, energy != nullptr);
+    float* df = (float*)m->vtmp.p;  // (the velocities of the pass are not wanted)
+    if (st == ND_OK) {
+        k_md_unsort<<<(unsigned)cdiv(n, 256), 256, 0, c->stream>>>(
+            m->set[m->cur].orig, n, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+            (const float4*)m->f.p, nullptr, nullptr, force ? df : nullptr);
+        c->launches++;
+        cudaError_t e = cudaSuccess;
+        if (force)
+            e = cudaMemcpyAsync(force, df, 3 * sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost,
+                                c->stream);
+        if (e == cudaSuccess && energy)
+            e = cudaMemcpyAsync(&pot, m->acc.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+        st = e == cudaSuccess ? sync_and_check(c, "forces") : cuda_fail(c, e, "forces");
+    }
+    if (st == ND_OK && energy) *energy = pot;
+    if (st) parent->last_error = c->last_error;
+    parent->launches += c->launches;
+    md_destroy(m);
+    return st;
 }
 
 nd_status md_energy(MDEngine* m, double* pot, double* kin) {
