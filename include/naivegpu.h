@@ -255,6 +255,32 @@ nd_status nd_leaf_pairs_refresh(nd_ctx* ctx, const float* xyz, const nd_bvh_spec
                                 nd_gridkey* keys, int64_t nkeys, float* position, int32_t* pi,
                                 int32_t* pj, float* pd, int64_t capacity, int64_t* count);
 
+/* One entry of a pair list: Tuple{Int32,Int32,Float32} (1-based indices). */
+typedef struct {
+    int32_t i, j;
+    float d;
+} nd_pair;
+
+/* Receives a list's length and returns host memory for that many entries (NULL:
+ * give up, ND_ERR_NOMEM).  Called once, on the calling thread, inside the call. */
+typedef nd_pair* (*nd_pair_alloc)(int64_t count, void* user);
+
+/*
+ * gpubvh_neighborlist (ext/NaiveKA.jl:470-558) in one call: the leaf tree and
+ * the ordered pair list over it, built once; the list's memory is asked for
+ * when its length is known, so no call has to be repeated with a larger buffer.
+ * criterion: ND_CRIT_SQUARED (leafbuild_traverse_bvh) or ND_CRIT_SQRT
+ * (simdbuild_traverse_bvh).  kept_index and kept_code (both or neither): the
+ * kept order and codes of gpubvh_neighborlist!, as in nd_leaf_pairs_refresh,
+ * in place of `order`.  keys (nkeys entries), index, morton_code, position and
+ * perm: the outputs of nd_tree (leafTreeData), each may be NULL.
+ */
+nd_status nd_leaf_pair_list(nd_ctx* ctx, const float* xyz, const nd_bvh_spec* spec, int32_t order,
+                            int32_t criterion, const int32_t* kept_index, const int32_t* kept_code,
+                            nd_gridkey* keys, int64_t nkeys, int32_t* index, int32_t* morton_code,
+                            float* position, int32_t* perm, nd_pair_alloc alloc, void* user,
+                            int64_t* count);
+
 /*
  * The leaf pair-list pipeline of nd_leaf_pairs_dev for callers that cannot
  * allocate device memory (the same kernels: in ND_PAIRS_ORDERED mode the same

@@ -196,6 +196,40 @@ static nd_status tree_from_host(Ctx* c, const float* xyz, const nd_bvh_spec* s, 
                       boxes, nkeys, overwrite_root, t, leaves_only);
 }
 
+// A kept order must be a permutation of 1..n and its codes ascending.
+static bool kept_order_ok(const int32_t* index, const int32_t* code, int32_t n) {
+    std::vector<uint8_t> seen((size_t)n, 0);
+    for (int32_t k = 0; k < n; ++k) {
+        const int32_t v = index[k];
+        if (v < 1 || v > n || seen[v - 1]) return false;
+        seen[v - 1] = 1;
+        if (code[k] < 0 || (k > 0 && code[k] < code[k - 1])) return false;
+    }
+    return true;
+}
+
+// Upload positions and a kept order and build that order's tree over them.
+static nd_status tree_kept_from_host(Ctx* c, const float* xyz, const nd_bvh_spec* s,
+                                     const int32_t* index, const int32_t* code, int64_t nkeys,
+                                     TreeBuffers* t) {
+    const size_t n = (size_t)s->atom_count;
+    nd_status st;
+    if ((st = ensure(c, c->xyz, 3 * sizeof(float) * n))) return st;
+    if ((st = ensure(c, c->perm_alt, sizeof(int32_t) * n))) return st;
+    if ((st = ensure(c, c->codes, sizeof(int32_t) * n))) return st;
+    cudaError_t e = cudaMemcpyAsync(c->xyz.p, xyz, 3 * sizeof(float) * n, cudaMemcpyHostToDevice,
+                                    c->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(c->perm_alt.p, index, sizeof(int32_t) * n, cudaMemcpyHostToDevice,
+                            c->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(c->codes.p, code, sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream);
+    if (e != cudaSuccess) return cuda_fail(c, e, "kept order upload");
+    return build_tree_kept(c, (const float*)c->xyz.p, (int32_t)n, s->neighbor_distance,
+                           s->atomsperleaf, (const int32_t*)c->perm_alt.p, (const int32_t*)c->codes.p,
+                           nkeys, t);
+}
+
 // The unordered emission exists for leaves of four atoms; any other request is
 // served in order.
 static bool unordered_emission(const nd_bvh_spec* s, int32_t mode) {
@@ -535,36 +569,12 @@ nd_status nd_leaf_pairs_refresh(nd_ctx* h, const float* xyz, const nd_bvh_spec* 
     const int32_t n = s->atom_count, nL = s->leaves_count;
     if (n - 1 < 2 * nL - 1) return ND_ERR_SPEC;  // leafTreeData needs atomsperleaf >= 2
     if (mode != ND_PAIRS_ORDERED && mode != ND_PAIRS_UNORDERED) return ND_ERR_ARG;
-    // the kept order must be a permutation and its codes ascending
-    {
-        std::vector<uint8_t> seen((size_t)n, 0);
-        for (int32_t k = 0; k < n; ++k) {
-            const int32_t v = index[k];
-            if (v < 1 || v > n || seen[v - 1]) return ND_ERR_ARG;
-            seen[v - 1] = 1;
-            if (morton_code[k] < 0 || (k > 0 && morton_code[k] < morton_code[k - 1]))
-                return ND_ERR_ARG;
-        }
-    }
+    if (!nd::kept_order_ok(index, morton_code, n)) return ND_ERR_ARG;
     if ((st = nd::set_device(c))) return st;
-    if ((st = nd::ensure(c, c->xyz, 3 * sizeof(float) * (size_t)n))) return st;
-    if ((st = nd::ensure(c, c->perm_alt, sizeof(int32_t) * (size_t)n))) return st;
-    if ((st = nd::ensure(c, c->codes, sizeof(int32_t) * (size_t)n))) return st;
-    cudaError_t e = cudaMemcpyAsync(c->xyz.p, xyz, 3 * sizeof(float) * (size_t)n,
-                                    cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->perm_alt.p, index, sizeof(int32_t) * (size_t)n,
-                            cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->codes.p, morton_code, sizeof(int32_t) * (size_t)n,
-                            cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return nd::cuda_fail(c, e, "refresh upload");
     const int64_t need = std::max<int64_t>(2LL * nL - 1, n - 1);
     nd::TreeBuffers t;
-    if ((st = nd::build_tree_kept(c, (const float*)c->xyz.p, n, s->neighbor_distance,
-                                  s->atomsperleaf, (const int32_t*)c->perm_alt.p,
-                                  (const int32_t*)c->codes.p, need, &t)))
-        return st;
+    if ((st = nd::tree_kept_from_host(c, xyz, s, index, morton_code, need, &t))) return st;
+    cudaError_t e = cudaSuccess;
     const nd_status pst = pairs_from_tree(c, t, s, mode, 0, true, pi, pj, pd, capacity, count,
                                           ND_CRIT_SQUARED);
     if (pst != ND_OK && pst != ND_NEED_REALLOC) return pst;
@@ -591,6 +601,78 @@ nd_status nd_leaf_pairs_refresh(nd_ctx* h, const float* xyz, const nd_bvh_spec* 
             position[3 * (size_t)i + 2] = pos4[i].z;
         }
     return pst;
+}
+
+nd_status nd_leaf_pair_list(nd_ctx* h, const float* xyz, const nd_bvh_spec* s, int32_t order,
+                            int32_t criterion, const int32_t* kept_index, const int32_t* kept_code,
+                            nd_gridkey* keys, int64_t nkeys, int32_t* index, int32_t* morton_code,
+                            float* position, int32_t* perm, nd_pair_alloc alloc, void* user,
+                            int64_t* count) {
+    if (!h || !xyz || !alloc || !count) return ND_ERR_ARG;
+    nd::NvtxRange nv("nd leaf pair list");
+    Ctx* c = &h->c;
+    nd_status st = nd::spec_ok(s);
+    if (st) return st;
+    if (order != ND_ORDER_REFERENCE && order != ND_ORDER_SPATIAL) return ND_ERR_ARG;
+    if (criterion != ND_CRIT_SQUARED && criterion != ND_CRIT_SQRT) return ND_ERR_ARG;
+    if ((kept_index != nullptr) != (kept_code != nullptr)) return ND_ERR_ARG;
+    if (keys && nkeys < 0) return ND_ERR_ARG;
+    const int32_t n = s->atom_count, nL = s->leaves_count;
+    if (n - 1 < 2 * nL - 1) return ND_ERR_SPEC;  // leafTreeData needs atomsperleaf >= 2
+    if (kept_index && !nd::kept_order_ok(kept_index, kept_code, n)) return ND_ERR_ARG;
+    if ((st = nd::set_device(c))) return st;
+    const int64_t nodes = 2LL * nL - 1;
+    nd::TreeBuffers t;
+    // the internal nodes are built only for a caller that takes the keys
+    st = kept_index ? nd::tree_kept_from_host(c, xyz, s, kept_index, kept_code, nodes, &t)
+                    : nd::tree_from_host(c, xyz, s, order, ND_BOX_LEAF, nodes, false, &t, !keys);
+    if (st) return st;
+    const float r = s->neighbor_distance, r2 = nd::pair_threshold(r, criterion);
+    int64_t* total_dev = (int64_t*)(c->d_err + 4);
+    if ((st = nd::count_pairs(c, t, r, r2, 0, total_dev))) return st;
+    // the list is written to what memory there is before its length is known here
+    const int64_t have = (int64_t)(c->pairs_i.bytes / sizeof(nd_pair));
+    if (have > 0 &&
+        (st = nd::write_pair_triples(c, t, r, r2, total_dev, have, (int32_t*)c->pairs_i.p)))
+        return st;
+    cudaError_t e = cudaSuccess;
+    if (keys && nkeys > 0) {
+        nd::root_overwrite(c, t.keys, nL);
+        const int64_t k = std::min(nkeys, nodes);
+        e = cudaMemcpyAsync(keys, t.keys, 32 * (size_t)k, cudaMemcpyDeviceToHost, c->stream);
+        if (nkeys > k) memset(keys + k, 0, 32 * (size_t)(nkeys - k));
+    }
+    const size_t nb = sizeof(int32_t) * (size_t)n;
+    if (e == cudaSuccess && index)
+        e = cudaMemcpyAsync(index, t.idx, nb, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && perm)  // the 1-based sortperm is the index of each sorted slot
+        e = cudaMemcpyAsync(perm, t.idx, nb, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && morton_code)
+        e = cudaMemcpyAsync(morton_code, t.codes, nb, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && position) {
+        nd::unpack_positions(c, t.pos4, n, (float*)c->xyz.p);  // (the upload is used up)
+        e = cudaMemcpyAsync(position, c->xyz.p, 3 * nb, cudaMemcpyDeviceToHost, c->stream);
+    }
+    if (e != cudaSuccess) return nd::cuda_fail(c, e, "pair list download");
+    if ((st = nd::sync_and_check(c, "pair list"))) return st;
+    int64_t total = 0;
+    memcpy(&total, c->h_err + 4, sizeof(total));
+    nd_pair* out = alloc(total, user);
+    if (!out && total > 0) {
+        c->last_error = "no memory for the pair list";
+        return ND_ERR_NOMEM;
+    }
+    *count = total;
+    if (total == 0) return ND_OK;
+    if (total > have) {
+        if ((st = nd::ensure(c, c->pairs_i, sizeof(nd_pair) * (size_t)total))) return st;
+        if ((st = nd::write_pair_triples(c, t, r, r2, total_dev, total, (int32_t*)c->pairs_i.p)))
+            return st;
+    }
+    e = cudaMemcpyAsync(out, c->pairs_i.p, sizeof(nd_pair) * (size_t)total, cudaMemcpyDeviceToHost,
+                        c->stream);
+    if (e != cudaSuccess) return nd::cuda_fail(c, e, "pair list download");
+    return nd::sync_and_check(c, "pair list");
 }
 
 nd_status nd_simd_leaf_pairs(nd_ctx* h, const float* xyz, const nd_bvh_spec* s, int32_t order,

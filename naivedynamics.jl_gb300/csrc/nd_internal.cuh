@@ -330,6 +330,11 @@ nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
                       int64_t* total_dev);
 nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
                       const int64_t* total_dev, int64_t cap, int32_t* pi, int32_t* pj, float* pd);
+// The leaf path's pairs as (i, j, d) triples of words.
+nd_status write_pair_triples(Ctx* c, const TreeBuffers& t, float r, float r2,
+                             const int64_t* total_dev, int64_t cap, int32_t* out);
+// Sorted positions (w dropped) into out (3 n floats).
+void unpack_positions(Ctx* c, const float4* pos4, int32_t n, float* out);
 nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_t* pi,
                          int32_t* pj, float* pd, int64_t capacity, int64_t* total);
 

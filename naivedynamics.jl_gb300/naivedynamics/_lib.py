@@ -125,6 +125,9 @@ _f = ctypes.c_float
 _d = ctypes.c_double
 _pp = ctypes.POINTER(ctypes.c_void_p)
 
+# nd_pair_alloc: length -> address of that many PAIR_DTYPE entries
+PAIR_ALLOC = ctypes.CFUNCTYPE(_vp, _i64, _vp)
+
 # name -> (restype, argtypes); every symbol declared in include/naivegpu.h
 SIGNATURES = {
     "nd_ctx_create": (_i32, [_pp, _i32]),
@@ -142,6 +145,8 @@ SIGNATURES = {
                        _vp]),
     "nd_leaf_pairs": (_i32, [_vp, _vp, ctypes.POINTER(BVHSpec), _i32, _i32, _vp, _vp, _vp, _i64,
                              ctypes.POINTER(_i64)]),
+    "nd_leaf_pair_list": (_i32, [_vp, _vp, ctypes.POINTER(BVHSpec), _i32, _i32, _vp, _vp, _vp, _i64,
+                                 _vp, _vp, _vp, _vp, PAIR_ALLOC, _vp, ctypes.POINTER(_i64)]),
     "nd_leaf_pairs_refresh": (_i32, [_vp, _vp, ctypes.POINTER(BVHSpec), _vp, _vp, _i32, _vp, _i64,
                                      _vp, _vp, _vp, _vp, _i64, ctypes.POINTER(_i64)]),
     "nd_leaf_pairs_dev": (_i32, [_vp, _vp, ctypes.POINTER(BVHSpec), _i32, _i32, _vp, _vp, _vp,

@@ -19,7 +19,7 @@ from typing import NamedTuple
 import numpy as np
 
 from . import _lib
-from ._lib import (GRIDKEY_DTYPE, ND_BOX_ATOM, ND_BOX_LEAF, ND_NEED_REALLOC, ND_OK,
+from ._lib import (GRIDKEY_DTYPE, ND_BOX_ATOM, ND_BOX_LEAF, ND_CRIT_SQRT, ND_CRIT_SQUARED, ND_NEED_REALLOC, ND_OK,
                    ND_ORDER_REFERENCE, ND_ORDER_SPATIAL, ND_PAIRS_ORDERED, ND_PAIRS_UNORDERED,
                    PAIR_DTYPE, SpecError, default_context, ptr)
 
@@ -134,6 +134,42 @@ def _pairs(fn, ctx, *args, capacity_hint=None):
         return out
 
 
+def _pair_list(ctx, x, spec, order, criterion=ND_CRIT_SQUARED, kept=None, tree=None, into=None):
+    """nd_leaf_pair_list: the ordered list in one call, its memory taken when
+    the length is known (`into`: a PAIR_DTYPE array resized in place).  kept:
+    (index, code) of a kept order; tree: (keys, index, code, position, perm)
+    arrays to fill, each may be None."""
+    got = []
+
+    def alloc(count, _user):
+        try:
+            if into is None:
+                out = np.empty(count, PAIR_DTYPE)
+            else:
+                into.resize(count, refcheck=False)
+                if not into.flags.writeable:
+                    raise ValueError("neighborlist is read-only")
+                out = into
+        except (MemoryError, ValueError) as e:
+            got.append(e)
+            return None
+        got.append(out)
+        return out.ctypes.data
+
+    keys, idx, code, pos, perm = tree or (None,) * 5
+    cs = spec.c_spec()
+    count = ctypes.c_int64()
+    st = _lib.lib().nd_leaf_pair_list(
+        ctx.handle, ptr(x), ctypes.byref(cs), order, criterion,
+        *((ptr(kept[0]), ptr(kept[1])) if kept else (None, None)), ptr(keys),
+        0 if keys is None else int(keys.shape[0]), ptr(idx), ptr(code), ptr(pos), ptr(perm),
+        _lib.PAIR_ALLOC(alloc), None, ctypes.byref(count))
+    if got and isinstance(got[0], Exception):
+        raise got[0]
+    ctx.check(st, "pair list")
+    return got[0]
+
+
 def leafbuild_traverse_bvh(position, spec: SpheresBVHSpecs, order: int = ND_ORDER_REFERENCE,
                            mode: int = ND_PAIRS_ORDERED, ctx=None, capacity_hint=None):
     """leafbuild_traverse_bvh (BVHTraverse.jl:1423-1428): the half pair list.
@@ -144,6 +180,8 @@ def leafbuild_traverse_bvh(position, spec: SpheresBVHSpecs, order: int = ND_ORDE
     """
     ctx = ctx or default_context()
     x = _positions(position)
+    if mode == ND_PAIRS_ORDERED:
+        return _pair_list(ctx, x, spec, order)
     cs = spec.c_spec()
     fn = lambda h, *a: _lib.lib().nd_leaf_pairs(h, ptr(x), ctypes.byref(cs), order, mode, *a)
     return _pairs(fn, ctx, capacity_hint=capacity_hint)
@@ -159,6 +197,8 @@ def simdbuild_traverse_bvh(position, spec: SpheresBVHSpecs, order: int = ND_ORDE
     """
     ctx = ctx or default_context()
     x = _positions(position)
+    if mode == ND_PAIRS_ORDERED and spec.atomsperleaf == 4:
+        return _pair_list(ctx, x, spec, order, ND_CRIT_SQRT)
     cs = spec.c_spec()
     fn = lambda h, *a: _lib.lib().nd_simd_leaf_pairs(h, ptr(x), ctypes.byref(cs), order, mode, *a)
     return _pairs(fn, ctx, capacity_hint=capacity_hint)
@@ -189,9 +229,15 @@ def gpubvh_neighborlist(backend, position, spec: SpheresBVHSpecs, order: int = N
         ctx = default_context(backend or 0)
     else:
         ctx = backend
-    keys, pos, perm, store = leafTreeData(position, spec, order=order, ctx=ctx)
-    pairs = leafbuild_traverse_bvh(position, spec, order=order, ctx=ctx)
-    return GPUNeighborList(pairs, (keys, pos, perm, store))
+    x = _positions(position)
+    n = spec.atom_count
+    if x.shape[0] != n:
+        raise ValueError("position length differs from spec.atom_count")
+    tree = (np.empty(n - 1, GRIDKEY_DTYPE), np.empty(n, np.int32), np.empty(n, np.int32),
+            np.empty((n, 3), np.float32), np.empty(n, np.int32))
+    pairs = _pair_list(ctx, x, spec, order, tree=tree)
+    keys, idx, code, pos, perm = tree
+    return GPUNeighborList(pairs, (keys, APointPrimitive(idx, code, pos), perm, None))
 
 
 def gpubvh_neighborlist_(neighborlist, treedata, spec: SpheresBVHSpecs, backend, position=None,
@@ -225,8 +271,16 @@ def gpubvh_neighborlist_(neighborlist, treedata, spec: SpheresBVHSpecs, backend,
         x = _positions(position)
     if x.shape[0] != n or index.shape[0] != n:
         raise ValueError("position length differs from spec.atom_count")
-    cs = spec.c_spec()
     newpos = np.empty((n, 3), np.float32)
+    if mode == ND_PAIRS_ORDERED:
+        out = neighborlist
+        if out is None or out.dtype != PAIR_DTYPE:
+            out = None
+        out = _pair_list(ctx, x, spec, ND_ORDER_REFERENCE, kept=(index, code),
+                         tree=(keys, None, None, newpos, None), into=out)
+        mpos.position[...] = newpos
+        return GPUNeighborList(out, (keys, mpos, perm, store))
+    cs = spec.c_spec()
     count = ctypes.c_int64()
     cap = 0
     while True:
