@@ -721,11 +721,10 @@ __device__ __forceinline__ void load_box_cg(const float4* keys, int32_t node /*1
 // publishes this thread's node writes; the fence after a successful read of a
 // non-zero slot orders the sibling-box loads, which bypass L1 (ld.cg).  No
 // thread ever waits on another, so the kernel cannot hang; a climb longer than
-// nL levels flags ND_ERR_INTERNAL.  ranges (may be null): leaf range
-// [first, last] of internal node nL + q at ranges[q - 1].  gate (may be null):
-// nothing is done while *gate is 0.
+// nL levels flags ND_ERR_INTERNAL.  gate (may be null): nothing is done while
+// *gate is 0.
 __global__ void k_bvh_build(float4* keys, int32_t* store, const int32_t* __restrict__ code,
-                            int32_t nL, int32_t apl, int2* ranges, int32_t* err,
+                            int32_t nL, int32_t apl, int32_t* err,
                             const unsigned* __restrict__ gate) {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (i > nL || (gate && *gate == 0u)) return;
@@ -776,7 +775,6 @@ __global__ void k_bvh_build(float4* keys, int32_t* store, const int32_t* __restr
         }
         int32_t q = (delr < dell) ? ranger : rangel;
         int32_t parent = nL + q;
-        if (ranges) ranges[q - 1] = make_int2(rangel, ranger);
         int32_t skip;
         if (ranger == nL) {
             skip = 0;
@@ -801,11 +799,10 @@ __global__ void k_root_overwrite(float4* keys, int32_t nL) {
 }
 
 nd_status build_internal_nodes(Ctx* c, float4* keys, int32_t* store, const int32_t* codes,
-                               int32_t nL, int32_t apl, int2* ranges, const unsigned* gate) {
+                               int32_t nL, int32_t apl, const unsigned* gate) {
     cudaError_t e = cudaMemsetAsync(store, 0, sizeof(int32_t) * (size_t)(nL - 1), c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "store reset");
-    k_bvh_build<<<(int)cdiv(nL, 256), 256, 0, c->stream>>>(keys, store, codes, nL, apl, ranges,
-                                                            c->d_err, gate);
+    k_bvh_build<<<(int)cdiv(nL, 256), 256, 0, c->stream>>>(keys, store, codes, nL, apl, c->d_err, gate);
     c->launches++;
     return check_launch(c, "bvh build");
 }
@@ -835,17 +832,9 @@ nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t a
                                                            (int32_t*)c->idx.p, keys);
     c->launches++;
     if ((st = check_launch(c, "leaf boxes"))) return st;
-    // leaf ranges of the internal nodes, for the split walks of the two-phase
-    // emission (not kept by the allocation-free entry point)
-    int2* ranges = nullptr;
-    if (!leaves_only) {
-        if (!c->no_alloc) {
-            if ((st = ensure(c, c->ranges, sizeof(int2) * (size_t)std::max(nL - 1, 1)))) return st;
-            ranges = (int2*)c->ranges.p;
-        }
-        if ((st = build_internal_nodes(c, keys, (int32_t*)c->store.p, codes, nL, apl, ranges)))
-            return st;
-    }
+    if (!leaves_only &&
+        (st = build_internal_nodes(c, keys, (int32_t*)c->store.p, codes, nL, apl)))
+        return st;
     if (overwrite_root) {
         k_root_overwrite<<<1, 1, 0, c->stream>>>(keys, nL);
         c->launches++;
@@ -858,7 +847,6 @@ nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t a
     out->pos4 = (const float4*)c->pos4.p;
     out->idx = (const int32_t*)c->idx.p;
     out->keys = keys;
-    out->ranges = ranges;
     out->nkeys = nkeys;
     return check_launch(c, "tree");
 }
@@ -886,7 +874,6 @@ nd_status build_tree_kept(Ctx* c, const float* xyz_dev, int32_t n, float r, int3
     if ((st = ensure(c, c->idx, sizeof(int32_t) * (size_t)n))) return st;
     if ((st = ensure(c, c->keys, 32 * (size_t)nkeys))) return st;
     if ((st = ensure(c, c->store, sizeof(int32_t) * (size_t)std::max(nL - 1, 1)))) return st;
-    if ((st = ensure(c, c->ranges, sizeof(int2) * (size_t)std::max(nL - 1, 1)))) return st;
     int32_t* perm = (int32_t*)c->perm.p;
     k_kept_perm<<<(unsigned)cdiv(n, 256), 256, 0, c->stream>>>(idx1, n, perm);
     c->launches++;
@@ -898,8 +885,7 @@ nd_status build_tree_kept(Ctx* c, const float* xyz_dev, int32_t n, float r, int3
                                                            (int32_t*)c->idx.p, keys);
     c->launches++;
     if ((st = check_launch(c, "kept leaf boxes"))) return st;
-    int2* ranges = (int2*)c->ranges.p;
-    if ((st = build_internal_nodes(c, keys, (int32_t*)c->store.p, codes_sorted, nL, apl, ranges)))
+    if ((st = build_internal_nodes(c, keys, (int32_t*)c->store.p, codes_sorted, nL, apl)))
         return st;
     out->n = n;
     out->nL = nL;
@@ -909,7 +895,6 @@ nd_status build_tree_kept(Ctx* c, const float* xyz_dev, int32_t n, float r, int3
     out->pos4 = (const float4*)c->pos4.p;
     out->idx = (const int32_t*)c->idx.p;
     out->keys = keys;
-    out->ranges = ranges;
     out->nkeys = nkeys;
     return check_launch(c, "kept tree");
 }
@@ -1565,230 +1550,253 @@ __global__ void __launch_bounds__(128)
     atom_query(qi, keys, pos, apl, r2, 2 * (n / apl) - 1, err, s);
 }
 
-// Two-phase form of the one-pass emission, for callers that allow scratch
-// memory.  Broad phase: the candidate leaf pairs (q, t) -- t > q with
-// overlapping boxes, and (q, q) for the pairs inside q -- are recorded through
-// per-warp shared buffers; the work per visited leaf is one box test.  Narrow
-// phase: one thread per candidate leaf pair runs the 4 x 4 distance tests and
-// emits through the warp buffers of k_leaf_warp4.  The distance tests, most of
-// the work, are then spread evenly over the GPU however dense the points are.
-//
-// The broad phase itself is split in two so that no walk is long: the union
-// walk of a warp's 32 query leaves (as in k_leaf_warp4) stops at subtrees of
-// at most kTaskLeaves leaves and records each overlapping one as a task
-// (group, subtree root); a flat pool of warps then walks the tasks' subtrees.
-// In a dense cluster one warp's union overlaps thousands of leaves; its walk
-// becomes a few hundred steps plus many short walks on other warps.
-constexpr int kLeafBuf = 256;    // candidate leaf pairs buffered per warp
-constexpr int kTaskLeaves = 64;  // largest subtree recorded as one task
+// Unordered emission for callers that allow scratch memory.  First the pairs
+// (g, h >= g) of groups of 32 leaves whose boxes overlap are listed: one warp
+// per group searches the group boxes 32 at a time, super-groups first.  Then
+// warps stride over these tasks.  A task tests the leaves of each group
+// against the other group's box (one a lane), then takes the survivors of the
+// shorter side one at a time against the other side's 32 lanes; leaf pairs
+// that overlap and whose atoms can be within r go through a queue in shared
+// memory, 32 at a time, one a lane, to the 4 x 4 distance tests, and the hits
+// through a buffer in shared memory to the list.  A dense cluster only means
+// more tasks, all of one size at most.
+// The second kernel is bound by instruction issue and by the list's writes
+// (12 bytes a pair).  In the form before, rope walks recorded subtrees, a
+// second kernel scanned them leaf by leaf with every query leaf and recorded
+// candidate leaf pairs, a third tested those: the walks' tail and the
+// candidates' way through memory and the host are gone.  64 clusters in us,
+// before and now: 131,072 points 336, 211; 1,048,576 points 1593, 1350;
+// 4,194,304 points (2.97e9 pairs, 35.6 GB) 13707, 11490.  A buffer of 256 hits
+// a warp (one reservation for 190 instead of 450) takes 14300; writing from a
+// ring while its reservation is under way 13900 (more instructions).
+constexpr int kTaskBuf = 128;  // tasks buffered per warp
 
-__device__ __forceinline__ void lp_flush(int2* buf, int& nb, unsigned long long* cursor, int64_t cap,
-                                         int2* __restrict__ out) {
+__global__ void __launch_bounds__(128)
+    k_group_tasks(const float4* __restrict__ gbox, int32_t nL, unsigned long long* tcursor,
+                  int64_t tcap, int2* __restrict__ tasks) {
+    __shared__ int32_t sbuf[4][kTaskBuf];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int32_t ng = (nL + 31) >> 5, ns = (ng + 31) >> 5;
+    const int32_t g = (int32_t)blockIdx.x * 4 + w;
+    if (g >= ng) return;  // whole warp
+    int32_t* buf = sbuf[w];
+    const Node un = load_node(gbox, g + 1);
+    if (lane == 0) buf[0] = g;  // the pairs inside the group, whatever its box
+    int nb = 1;
+    auto flush = [&]() {
+        __syncwarp();
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(tcursor, (unsigned long long)nb);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int k = lane; k < nb; k += 32)
+            if ((int64_t)(base + k) < tcap) tasks[base + k] = make_int2(g, buf[k]);
+        __syncwarp();
+        nb = 0;
+    };
+    for (int32_t sb = g >> 10; sb < ns; sb += 32) {
+        const int32_t s = sb + lane;
+        unsigned sm = __ballot_sync(
+            0xffffffffu, s < ns && overlap(un, load_node(gbox, ng + min(s, ns - 1) + 1)));
+        while (sm) {
+            const int32_t h = (sb + __ffs(sm) - 1) * 32 + lane;
+            sm &= sm - 1;
+            const bool in = h > g && h < ng && overlap(un, load_node(gbox, min(h, ng - 1) + 1));
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) buf[nb + __popc(m & ((1u << lane) - 1u))] = h;
+            nb += __popc(m);
+            if (nb > kTaskBuf - 32) flush();
+        }
+    }
+    if (nb) flush();
+}
+
+constexpr int kPairBuf = 512;  // hits buffered per warp
+
+// A warp's hits on their way to the list.  Squared distances are kept; the
+// flush takes their roots with every lane busy.
+struct PairBuf {
+    int32_t i[kPairBuf], j[kPairBuf];
+    float d2[kPairBuf];
+};
+
+__device__ __forceinline__ void pair_buf_flush(PairBuf& b, int& nb, unsigned long long* cursor,
+                                               int64_t cap, int32_t* pi, int32_t* pj, float* pd) {
     const int lane = threadIdx.x & 31;
+    __syncwarp();
     unsigned long long base = 0;
     if (lane == 0 && nb) base = atomicAdd(cursor, (unsigned long long)nb);
     base = __shfl_sync(0xffffffffu, base, 0);
-    for (int k = lane; k < nb; k += 32) {
-        const unsigned long long w = base + (unsigned long long)k;
-        if ((int64_t)w < cap) out[w] = buf[k];
+    // entries of the run that fit (32-bit offsets from its first slot)
+    const int64_t room = cap - (int64_t)base;
+    const int n = room >= nb ? nb : room > 0 ? (int)room : 0;
+    int32_t* __restrict__ qi = pi + base;
+    int32_t* __restrict__ qj = pj + base;
+    float* __restrict__ qd = pd + base;
+    int k = lane;
+    for (; k + 96 < n; k += 128) {
+#pragma unroll
+        for (int u = 0; u < 128; u += 32) {
+            qi[k + u] = b.i[k + u];
+            qj[k + u] = b.j[k + u];
+            qd[k + u] = __fsqrt_rn(b.d2[k + u]);
+        }
+    }
+    for (; k < n; k += 32) {
+        qi[k] = b.i[k];
+        qj[k] = b.j[k];
+        qd[k] = __fsqrt_rn(b.d2[k]);
     }
     __syncwarp();
     nb = 0;
 }
 
-__device__ __forceinline__ void lp_append(bool want, int32_t q, int32_t t, int2* buf, int& nb,
-                                          unsigned long long* cursor, int64_t cap,
-                                          int2* __restrict__ out) {
-    const unsigned bal = __ballot_sync(0xffffffffu, want);
-    if (!bal) return;
-    const int total = __popc(bal);
-    if (nb + total > kLeafBuf) lp_flush(buf, nb, cursor, cap, out);
-    if (want) buf[nb + __popc(bal & ((1u << (threadIdx.x & 31)) - 1u))] = make_int2(q, t);
-    __syncwarp();
-    nb += total;
-}
-
-// The query group of a warp: leaves q0 .. q0 + 31 (lane's own leaf, empty box
-// past nL) and the union of their boxes.
-__device__ __forceinline__ void group_boxes(const float4* __restrict__ keys, int32_t nL,
-                                            int32_t q, Node& ql, Node& un) {
-    if (q <= nL) {
-        ql = load_node(keys, q);
-    } else {
-        ql.mnx = ql.mny = ql.mnz = INFINITY;
-        ql.mxx = ql.mxy = ql.mxz = -INFINITY;
-        ql.left = ql.skip = 0;
-    }
-    un = ql;
-    for (int sh = 16; sh > 0; sh >>= 1) {
-        un.mnx = fminf(un.mnx, __shfl_xor_sync(0xffffffffu, un.mnx, sh));
-        un.mny = fminf(un.mny, __shfl_xor_sync(0xffffffffu, un.mny, sh));
-        un.mnz = fminf(un.mnz, __shfl_xor_sync(0xffffffffu, un.mnz, sh));
-        un.mxx = fmaxf(un.mxx, __shfl_xor_sync(0xffffffffu, un.mxx, sh));
-        un.mxy = fmaxf(un.mxy, __shfl_xor_sync(0xffffffffu, un.mxy, sh));
-        un.mxz = fmaxf(un.mxz, __shfl_xor_sync(0xffffffffu, un.mxz, sh));
-    }
-}
-
-// Broad phase, first half: one warp per group of 32 query leaves.  The pairs
-// inside each leaf go to the candidate list; the union walk from the skip rope
-// of the group's first leaf records (group, node) for every overlapping node
-// of at most kTaskLeaves leaves instead of descending into it.  Tasks are
-// warp-uniform: lane k holds the k-th pending one, 32 are written at a time.
-__global__ void __launch_bounds__(128)
-    k_leaf_tasks4(const float4* __restrict__ keys, const int2* __restrict__ ranges, int32_t nL,
-                  unsigned long long* cursor, int64_t cap, int2* __restrict__ out,
-                  unsigned long long* tcursor, int64_t tcap, int2* __restrict__ tasks,
-                  int32_t* err) {
-    __shared__ int2 sbuf[4][kLeafBuf];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int32_t g = (int32_t)(blockIdx.x * 4 + w);
-    const int32_t q0 = g * 32 + 1;
-    if (q0 > nL) return;  // whole warp
-    int2* buf = sbuf[w];
-    const int32_t q = q0 + lane;
-    Node ql, un;
-    group_boxes(keys, nL, q, ql, un);
-    int nb = 0;
-    lp_append(q <= nL, q, q, buf, nb, cursor, cap, out);  // pairs inside the leaf
-    lp_flush(buf, nb, cursor, cap, out);
-    int2 mine = make_int2(0, 0);
-    int npend = 0;
-    auto flush_tasks = [&]() {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(tcursor, (unsigned long long)npend);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (lane < npend && (int64_t)(base + lane) < tcap) tasks[base + lane] = mine;
-        npend = 0;
-    };
-    int32_t t = __shfl_sync(0xffffffffu, ql.skip, 0);
-    int32_t visits = 0;
-    const int32_t nnodes = 2 * nL - 1;
-    while (t != 0) {
-        if (t < 1 || t > nnodes || ++visits > nnodes) {
-            if (lane == 0) set_error(err, ND_ERR_INTERNAL, q0);
-            break;
-        }
-        const Node nd_ = load_node(keys, t);
-        int32_t size = 1;
-        if (t > nL) {
-            const int2 rg = __ldg(&ranges[t - nL - 1]);
-            size = rg.y - rg.x + 1;
-        }
-        if (overlap(un, nd_)) {
-            if (size <= kTaskLeaves) {
-                if (lane == npend) mine = make_int2(g, t);
-                if (++npend == 32) flush_tasks();
-                t = nd_.skip;
-            } else {
-                t = nd_.left;
-            }
-        } else {
-            t = nd_.skip;
-        }
-    }
-    if (npend) flush_tasks();
-}
-
-// Broad phase, second half: warps stride over the tasks.  A task's subtree
-// holds the leaves of one contiguous range (at most kTaskLeaves); the warp
-// scans them in order, four node loads in flight at a time, and records
-// (q, t) for the lanes whose own leaf q < t overlaps t (a leaf overlapping q
-// overlaps every ancestor, so these are the candidates a walk pruning with
-// the group's union box would find) and whose atoms can be within r at all
-// (leaf_gap_ok: about 40 % of the overlapping leaves in dense clusters are
-// not).
-__global__ void __launch_bounds__(128)
-    k_leaf_subwalk4(const float4* __restrict__ keys, const int2* __restrict__ ranges, int32_t nL,
-                    float r, const unsigned long long* __restrict__ tcount, int64_t tcap,
-                    const int2* __restrict__ tasks, unsigned long long* cursor, int64_t cap,
-                    int2* __restrict__ out, int32_t* err) {
+__global__ void __launch_bounds__(128, 6)
+    k_group_pairs(const float4* __restrict__ keys, const float4* __restrict__ gbox,
+                  const float4* __restrict__ pos, int32_t nL, float r, float r2,
+                  const unsigned long long* __restrict__ tcount, int64_t tcap,
+                  const int2* __restrict__ tasks, unsigned long long* ticket,
+                  unsigned long long* cursor, int64_t cap, int32_t* __restrict__ pi,
+                  int32_t* __restrict__ pj, float* __restrict__ pd) {
+    __shared__ PairBuf sbuf[4];
+    __shared__ float4 sbox[4][2][64];  // leaf boxes of the task's groups, their slack beside
+    __shared__ int2 squeue[4][64];
     const float r2g = r * r * 1.0001f;  // the gap test is a filter: the distance test decides
-    __shared__ int2 sbuf[4][kLeafBuf];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int2* buf = sbuf[w];
-    int nb = 0;
-    const int64_t ntask = min((int64_t)*tcount, tcap);
-    const int32_t nnodes = 2 * nL - 1;
-    for (int64_t k = (int64_t)blockIdx.x * 4 + w; k < ntask; k += (int64_t)gridDim.x * 4) {
-        const int2 tk = __ldg(&tasks[k]);
-        const int32_t q0 = tk.x * 32 + 1;
-        const int32_t q = q0 + lane;
-        const bool valid = q <= nL;
-        Node ql, un;
-        group_boxes(keys, nL, q, ql, un);
-        const int32_t root = tk.y;
-        if (root < 1 || root > nnodes) {
-            if (lane == 0) set_error(err, ND_ERR_INTERNAL, tk.x);
-            continue;
+    const unsigned below = (1u << lane) - 1u;
+    const int64_t ntask = (int64_t)*tcount;
+    if (ntask > tcap) return;  // the list of tasks has to grow first
+    PairBuf& buf = sbuf[w];
+    int2* queue = squeue[w];
+    int nb = 0, qn = 0;
+    auto put = [&](bool hit, float4 a, float4 b, float d2) {
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
+            const int at = nb + __popc(m & below);
+            buf.i[at] = __float_as_int(a.w);
+            buf.j[at] = __float_as_int(b.w);
+            buf.d2[at] = d2;
         }
-        int32_t la = root, lb = root;  // leaf range of the subtree
-        if (root > nL) {
-            const int2 rg = __ldg(&ranges[root - nL - 1]);
-            la = rg.x;
-            lb = rg.y;
-        }
-        if (la < 1 || lb > nL || lb - la + 1 > kTaskLeaves) {
-            if (lane == 0) set_error(err, ND_ERR_INTERNAL, tk.x);
-            continue;
-        }
-        const float slack = valid ? leaf_slack(ql) : 0.0f;
-        // leaves after the group's first only (t > q for some lane)
-        for (int32_t t0 = max(la, q0 + 1); t0 <= lb; t0 += 4) {
-            Node nd4[4];
+        nb += __popc(m);
+    };
+    auto room = [&]() {  // for 128 more
+        if (nb > kPairBuf - 128) pair_buf_flush(buf, nb, cursor, cap, pi, pj, pd);
+    };
+    // the 4 x 4 tests of the first nc candidates, one a lane
+    auto test = [&](int nc) {
+        const int2 e = queue[lane < nc ? lane : 0];
+        const float thr = lane < nc ? r2 : -1.0f;  // no squared distance is below -1
+        float4 qa[4], tb[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (t0 + u <= lb) nd4[u] = load_node(keys, t0 + u);
+        for (int i = 0; i < 4; ++i) qa[i] = __ldg(&pos[(int64_t)e.x * 4 + i]);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int32_t t = t0 + u;
-                if (t > lb) break;  // warp-uniform
-                const Node& b = nd4[u];
-                const bool want =
-                    valid && t > q && overlap(ql, b) && leaf_gap_ok(ql, b, r, r2g, slack);
-                lp_append(want, q, t, buf, nb, cursor, cap, out);
+        for (int j = 0; j < 4; ++j) tb[j] = __ldg(&pos[(int64_t)e.y * 4 + j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            room();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float d2 = dist2_ref(qa[i].x, qa[i].y, qa[i].z, tb[j].x, tb[j].y, tb[j].z);
+                put(d2 < thr, qa[i], tb[j], d2);
+            }
+        }
+    };
+    // this lane's leaf of group g (an empty box past the end) into side s
+    auto load_side = [&](int s, int32_t g, Node& b, float& slack) {
+        const int32_t l = g * 32 + lane;
+        if (l < nL) {
+            b = load_node(keys, l + 1);
+            slack = leaf_slack(b);
+        } else {
+            b.mnx = b.mny = b.mnz = INFINITY;
+            b.mxx = b.mxy = b.mxz = -INFINITY;
+            slack = 0.0f;
+        }
+        __syncwarp();
+        sbox[w][s][2 * lane] = make_float4(b.mnx, b.mny, b.mnz, b.mxx);
+        sbox[w][s][2 * lane + 1] = make_float4(b.mxy, b.mxz, slack, 0.0f);
+        __syncwarp();
+    };
+    int32_t g = -1;
+    Node un, ql;
+    float qslack = 0.0f;
+    // Tasks are drawn a few in a row (they mostly share their first group) from
+    // a counter, the next draw in flight: the tasks of a dense cluster hold a
+    // hundred times those at its rim, and with a fixed share for each warp
+    // half of the SM time went by idle.
+    const int64_t chunk = min(max(ntask / ((int64_t)gridDim.x * 64), (int64_t)1), (int64_t)4);
+    unsigned long long next = 0;
+    if (lane == 0) next = atomicAdd(ticket, (unsigned long long)chunk);
+    for (;;) {
+        const int64_t k0 = (int64_t)__shfl_sync(0xffffffffu, next, 0);
+        if (k0 >= ntask) break;
+        if (lane == 0) next = atomicAdd(ticket, (unsigned long long)chunk);
+        for (int64_t k = k0; k < min(k0 + chunk, ntask); ++k) {
+            const int2 tk = __ldg(&tasks[k]);
+            const int32_t h = tk.y;
+            if (tk.x != g) {
+                g = tk.x;
+                un = load_node(gbox, g + 1);
+                load_side(0, g, ql, qslack);
+            }
+            const Node uh = load_node(gbox, h + 1);
+            Node tl;
+            float tslack;
+            load_side(1, h, tl, tslack);
+            if (h == g) {  // the six pairs inside each leaf
+                const bool valid = g * 32 + lane < nL;
+                const int64_t A = (int64_t)(valid ? g * 32 + lane : 0) * 4;
+                const float thr = valid ? r2 : -1.0f;
+                float4 qa[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) qa[i] = __ldg(&pos[A + i]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    room();
+#pragma unroll
+                    for (int j = i + 1; j < 4; ++j) {
+                        const float d2 =
+                            dist2_ref(qa[i].x, qa[i].y, qa[i].z, qa[j].x, qa[j].y, qa[j].z);
+                        put(d2 < thr, qa[i], qa[j], d2);
+                    }
+                }
+            }
+            const unsigned mq = __ballot_sync(0xffffffffu, overlap(ql, uh));
+            const unsigned mt = __ballot_sync(0xffffffffu, overlap(un, tl));
+            // the shorter side goes one by one, the other one stays in the lanes
+            const bool by_t = __popc(mt) <= __popc(mq);
+            const Node own = by_t ? ql : tl;
+            const float slack = by_t ? qslack : tslack;
+            const bool in = ((by_t ? mq : mt) >> lane) & 1u;
+            const float4* other = sbox[w][by_t ? 1 : 0];
+            for (unsigned m = by_t ? mt : mq; m; m &= m - 1) {
+                const int b = __ffs(m) - 1;
+                const float4 b0 = other[2 * b], b1 = other[2 * b + 1];
+                Node o;
+                o.mnx = b0.x; o.mny = b0.y; o.mnz = b0.z;
+                o.mxx = b0.w; o.mxy = b1.x; o.mxz = b1.y;
+                const bool after = h > g || (by_t ? b > lane : lane > b);  // t > q
+                const bool want = in && after && overlap(own, o) &&
+                                  leaf_gap_ok(own, o, r, r2g, fmaxf(slack, b1.z));
+                const unsigned c = __ballot_sync(0xffffffffu, want);
+                if (!c) continue;
+                if (want)
+                    queue[qn + __popc(c & below)] =
+                        make_int2(g * 32 + (by_t ? lane : b), h * 32 + (by_t ? b : lane));
+                qn += __popc(c);
+                __syncwarp();
+                if (qn >= 32) {
+                    test(32);
+                    const int2 rest = queue[32 + (lane < qn - 32 ? lane : 0)];
+                    __syncwarp();
+                    if (lane < qn - 32) queue[lane] = rest;
+                    qn -= 32;
+                    __syncwarp();
+                }
             }
         }
     }
-    lp_flush(buf, nb, cursor, cap, out);
-}
-
-__global__ void __launch_bounds__(256)
-    k_leaf_narrow4(const int2* __restrict__ lp, int64_t nlp, const float4* __restrict__ pos,
-                   float r2, unsigned long long* cursor, int64_t cap, int32_t* pi, int32_t* pj,
-                   float* pd) {
-    constexpr int APL = 4;
-    __shared__ int2 sbij[8][kWarpBuf];
-    __shared__ float sbd[8][kWarpBuf];
-    const int w = threadIdx.x >> 5;
-    int2* bij = sbij[w];
-    float* bd = sbd[w];
-    int nb = 0;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    // warp-uniform trip count: lanes past the end test nothing but join the ballots
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-         __any_sync(0xffffffffu, k < nlp); k += stride) {
-        unsigned mask = 0;
-        float d2[16];
-        int32_t ia[APL] = {0, 0, 0, 0}, ib[APL] = {0, 0, 0, 0};
-        if (k < nlp) {
-            const int2 e = __ldg(&lp[k]);
-            const int64_t A = (int64_t)(e.x - 1) * APL, B = (int64_t)(e.y - 1) * APL;
-            float4 qa[APL], tb[APL];
-#pragma unroll
-            for (int i = 0; i < APL; ++i) qa[i] = __ldg(&pos[A + i]);
-#pragma unroll
-            for (int j = 0; j < APL; ++j) tb[j] = __ldg(&pos[B + j]);
-            mask = leaf_tests16(qa, tb, e.x == e.y, r2, d2);
-#pragma unroll
-            for (int i = 0; i < APL; ++i) {
-                ia[i] = __float_as_int(qa[i].w);
-                ib[i] = __float_as_int(tb[i].w);
-            }
-        }
-        warp_emit16(mask, d2, ia, ib, bij, bd, nb, cursor, cap, pi, pj, pd);
-    }
-    warp_buf_flush(bij, bd, nb, cursor, cap, pi, pj, pd);
+    if (qn) test(qn);
+    pair_buf_flush(buf, nb, cursor, cap, pi, pj, pd);
 }
 
 // The pair criterion as a threshold on the Float32 squared distance d2:
@@ -1811,7 +1819,6 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
     nd_status st;
     if ((st = ensure(c, c->misc, 64))) return st;
     unsigned long long* cursor = (unsigned long long*)c->misc.p;
-    unsigned long long tot = 0;
     cudaError_t e;
     if (c->no_alloc) {
         // no scratch for candidate pairs: the one-pass walk
@@ -1819,69 +1826,48 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
         k_leaf_warp4<<<(unsigned)cdiv(t.nL, 128), 128, 0, c->stream>>>(
             t.keys, t.pos4, t.nL, r, r2, cursor, capacity, pi, pj, pd, c->d_err);
         c->launches++;
-    } else {
-        // broad phase: tasks, then the tasks' subtree walks; re-run with
-        // larger buffers while either list overflowed
-        if (!t.ranges) return ND_ERR_INTERNAL;
-        unsigned long long* tcursor = cursor + 1;
-        unsigned long long nlp = 0, ntask = 0;
-        int nsm = 0, occ = 0;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_leaf_subwalk4, 128, 0);
-        const int64_t ngroups = cdiv(t.nL, 32);
-        for (int attempt = 0;; ++attempt) {
-            int64_t lcap = (int64_t)(c->leafpairs.bytes / sizeof(int2));
-            if (lcap < 16 * (int64_t)t.nL) {
-                if ((st = ensure(c, c->leafpairs, sizeof(int2) * 16 * (size_t)t.nL))) return st;
-                lcap = 16 * (int64_t)t.nL;
-            }
-            int64_t tcap = (int64_t)(c->tasks.bytes / sizeof(int2));
-            if (tcap < 16 * ngroups) {
-                if ((st = ensure(c, c->tasks, sizeof(int2) * 16 * (size_t)ngroups))) return st;
-                tcap = 16 * ngroups;
-            }
-            cudaMemsetAsync(cursor, 0, 2 * sizeof(unsigned long long), c->stream);
-            k_leaf_tasks4<<<(unsigned)cdiv(t.nL, 128), 128, 0, c->stream>>>(
-                t.keys, t.ranges, t.nL, cursor, lcap, (int2*)c->leafpairs.p, tcursor, tcap,
-                (int2*)c->tasks.p, c->d_err);
-            k_leaf_subwalk4<<<(unsigned)(nsm * std::max(occ, 1)), 128, 0, c->stream>>>(
-                t.keys, t.ranges, t.nL, r, tcursor, tcap, (const int2*)c->tasks.p, cursor, lcap,
-                (int2*)c->leafpairs.p, c->d_err);
-            c->launches += 2;
-            if ((st = check_launch(c, "leaf pairs (broad phase)"))) return st;
-            unsigned long long h[2] = {0, 0};
-            e = cudaMemcpyAsync(h, cursor, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-            if (e != cudaSuccess) return cuda_fail(c, e, "candidate leaf pairs");
-            nlp = h[0];
-            ntask = h[1];
-            if ((int64_t)nlp <= lcap && (int64_t)ntask <= tcap) break;
-            if (attempt == 2) {
-                c->last_error = "candidate leaf pairs: buffers kept overflowing";
-                return ND_ERR_INTERNAL;
-            }
-            if ((int64_t)ntask > tcap &&
-                (st = ensure(c, c->tasks, sizeof(int2) * (size_t)(ntask + ntask / 4))))
-                return st;
-            if ((int64_t)nlp > lcap &&
-                (st = ensure(c, c->leafpairs, sizeof(int2) * (size_t)(nlp + nlp / 4))))
-                return st;
-        }
-        cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), c->stream);
-        const int64_t blocks = std::min<int64_t>(cdiv((int64_t)nlp, 256), (int64_t)nsm * 32);
-        if (nlp > 0) {
-            k_leaf_narrow4<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, c->stream>>>(
-                (const int2*)c->leafpairs.p, (int64_t)nlp, t.pos4, r2, cursor, capacity, pi, pj,
-                pd);
-            c->launches++;
-        }
+        if ((st = check_launch(c, "leaf pairs (unordered)"))) return st;
+        unsigned long long tot = 0;
+        e = cudaMemcpyAsync(&tot, cursor, sizeof(tot), cudaMemcpyDeviceToHost, c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "pair count");
+        if ((st = sync_and_check(c, "leaf pairs (unordered)"))) return st;
+        *total = (int64_t)tot;
+        return ND_OK;
     }
-    if ((st = check_launch(c, "leaf pairs (unordered)"))) return st;
-    e = cudaMemcpyAsync(&tot, cursor, sizeof(tot), cudaMemcpyDeviceToHost, c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "pair count");
-    if ((st = sync_and_check(c, "leaf pairs (unordered)"))) return st;
-    *total = (int64_t)tot;
-    return ND_OK;
+    // run again with a longer task list while it overflowed
+    unsigned long long* tcursor = cursor + 1;
+    unsigned long long* ticket = cursor + 2;
+    int nsm = 0, occ = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_group_pairs, 128, 0);
+    const int64_t ng = cdiv(t.nL, 32), ns = cdiv(ng, 32);
+    if ((st = ensure(c, c->store, 32 * (size_t)(ng + ns)))) return st;
+    if ((st = ensure(c, c->tasks, sizeof(int2) * 128 * (size_t)ng))) return st;
+    float4* gbox = (float4*)c->store.p;
+    k_group_boxes<<<(unsigned)ns, 1024, 0, c->stream>>>(t.keys, t.nL, gbox);
+    c->launches++;
+    for (int attempt = 0;; ++attempt) {
+        const int64_t tcap = (int64_t)(c->tasks.bytes / sizeof(int2));
+        cudaMemsetAsync(cursor, 0, 3 * sizeof(unsigned long long), c->stream);
+        k_group_tasks<<<(unsigned)cdiv(ng, 4), 128, 0, c->stream>>>(gbox, t.nL, tcursor, tcap,
+                                                                    (int2*)c->tasks.p);
+        k_group_pairs<<<(unsigned)(nsm * std::max(occ, 1)), 128, 0, c->stream>>>(
+            t.keys, gbox, t.pos4, t.nL, r, r2, tcursor, tcap, (const int2*)c->tasks.p, ticket,
+            cursor, capacity, pi, pj, pd);
+        c->launches += 2;
+        if ((st = check_launch(c, "leaf pairs (unordered)"))) return st;
+        unsigned long long h[2] = {0, 0};
+        e = cudaMemcpyAsync(h, cursor, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "pair count");
+        if ((st = sync_and_check(c, "leaf pairs (unordered)"))) return st;
+        *total = (int64_t)h[0];
+        if ((int64_t)h[1] <= tcap) return ND_OK;
+        if (attempt == 2) {
+            c->last_error = "overlapping leaf groups: buffer kept overflowing";
+            return ND_ERR_INTERNAL;
+        }
+        if ((st = ensure(c, c->tasks, sizeof(int2) * (size_t)h[1]))) return st;
+    }
 }
 
 // Ordered emission: per-query counts, their scan, then the pairs at their

@@ -255,7 +255,8 @@ nd_status pairs_common(Ctx* c, const nd_bvh_spec* s, int32_t order, int32_t mode
     const int32_t boxes = (kind == 0) ? ND_BOX_LEAF : ND_BOX_ATOM;
     if (kind == 0 && n - 1 < 2 * nL - 1) return ND_ERR_SPEC;  // leafTreeData needs apl >= 2
     TreeBuffers t;
-    const bool leaves_only = kind == 0 && !unordered_emission(s, mode);
+    // only the allocation-free unordered walk follows the tree's ropes
+    const bool leaves_only = kind == 0 && !(c->no_alloc && unordered_emission(s, mode));
     if (host) {
         st = tree_from_host(c, xyz, s, order, boxes, 2LL * nL - 1, false, &t, leaves_only);
     } else {
@@ -420,7 +421,7 @@ nd_status nd_ctx_destroy(nd_ctx* h) {
     nd::DevBuf* bufs[] = {&c->xyz, &c->codes, &c->codes_alt, &c->perm, &c->perm_alt, &c->pos4,
                           &c->idx, &c->keys, &c->store, &c->hist, &c->counts, &c->offsets,
                           &c->partial, &c->pairs_i, &c->pairs_j, &c->pairs_d, &c->misc, &c->hash,
-                          &c->leafpairs, &c->ranges, &c->tasks, &c->compat};
+                          &c->leafpairs, &c->tasks, &c->compat};
     for (nd::DevBuf* b : bufs) nd::free_buf(*b);
     h->pool.clear();
     if (c->d_err) cudaFree(c->d_err);

@@ -171,7 +171,7 @@ struct Ctx {
     std::string last_error;
     // scratch buffers of the neighbour-search pipeline, grown on demand
     DevBuf xyz, codes, codes_alt, perm, perm_alt, pos4, idx, keys, store, hist, counts, offsets,
-        partial, pairs_i, pairs_j, pairs_d, misc, hash, leafpairs, ranges, tasks, compat;
+        partial, pairs_i, pairs_j, pairs_d, misc, hash, leafpairs, tasks, compat;
     struct MDEngine* sim_cache = nullptr;  // engine re-used by nd_simulate
     bool no_alloc = false;                 // buffers are fixed slices: never grow them
     BufPool* pool = nullptr;               // idle buffers of the context (may be null)
@@ -224,7 +224,6 @@ struct TreeBuffers {
     const float4* pos4 = nullptr;    // sorted positions, w = bits of 1-based index (n)
     const int32_t* idx = nullptr;    // sorted 1-based original index (n)
     float4* keys = nullptr;          // 2 float4 per node, nd_gridkey layout (nkeys)
-    const int2* ranges = nullptr;    // leaf range of internal node nL + q at q - 1 (or null)
     int64_t nkeys = 0;
 };
 
@@ -241,7 +240,7 @@ nd_status order_positions(Ctx* c, const float* xyz, int32_t n, int32_t order, in
                           int32_t* perm, const float* frame = nullptr);
 size_t sort_scratch_bytes(int32_t n);
 // Full tree pipeline: codes -> sort -> gather -> leaf boxes -> Apetrei build
-// (leaves_only: no internal nodes, all the ordered pair list needs).
+// (leaves_only: no internal nodes, all the leaf pair lists need).
 nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t apl,
                      int32_t order, int32_t boxes, int64_t nkeys, bool overwrite_root,
                      TreeBuffers* out, bool leaves_only = false);
@@ -266,8 +265,7 @@ nd_status pair_hash(Ctx* c, const int32_t* pi, const int32_t* pj, const float* p
 
 // Apetrei bottom-up build over already prepared leaf keys (used by the MD engine).
 nd_status build_internal_nodes(Ctx* c, float4* keys, int32_t* store, const int32_t* codes_sorted,
-                               int32_t nL, int32_t apl, int2* ranges = nullptr,
-                               const unsigned* gate = nullptr);
+                               int32_t nL, int32_t apl, const unsigned* gate = nullptr);
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -2148,7 +2148,7 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
     const bool tree = m->p.union_search == ND_UNION_TREE;
     if (tree) {
         if ((st = build_internal_nodes(c, keys, (int32_t*)m->store.p, codes, m->nL, m->apl,
-                                       nullptr, gate)))
+                                       gate)))
             return st;
     } else if (m->nblocks > kDirectBlocks) {
         launch_chained(c, gate != nullptr, k_md_super_boxes, (unsigned)cdiv(m->nblocks, 256), 256, 0, m->nblocks, bbox,
