@@ -42,6 +42,8 @@ namespace nd {
 
 constexpr int kHistChunk = 16;  // histogram bins a thread accumulates per pass
 constexpr int kAdjTPA = 4;      // threads per atom in the reverse step
+constexpr int kAdjAhead = 4;    // list entries in flight per thread of the reverse step
+constexpr int kTermTPA = 8;     // threads per atom in the terminal adjoint
 
 struct AdjArgs {
     int32_t n, apl, ucap, smrec;
@@ -116,18 +118,21 @@ __device__ __forceinline__ void hvp_pair(const AdjArgs& a, const int4& ri, const
     hv.z += g * ez + rd * dz;
 }
 
-// Fixed-order block sum of two values over NT threads; thread 0 adds them to
+// Fixed-order block sum of two values over the first NT threads (the whole
+// block calls it); thread 0 adds them to
 // this block's partials (one writer per block and launches in stream order:
 // deterministic).
 template <int NT>
 __device__ __forceinline__ void block_add2(double v0, double v1, double* part) {
     __shared__ double s[2][NT / 32];
-    for (int sh = 16; sh > 0; sh >>= 1) {
-        v0 += __shfl_xor_sync(0xffffffffu, v0, sh);
-        v1 += __shfl_xor_sync(0xffffffffu, v1, sh);
-    }
     const int warp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { s[0][warp] = v0; s[1][warp] = v1; }
+    if (warp < NT / 32) {
+        for (int sh = 16; sh > 0; sh >>= 1) {
+            v0 += __shfl_xor_sync(0xffffffffu, v0, sh);
+            v1 += __shfl_xor_sync(0xffffffffu, v1, sh);
+        }
+        if ((threadIdx.x & 31) == 0) { s[0][warp] = v0; s[1][warp] = v1; }
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         double t0 = 0.0, t1 = 0.0;
@@ -140,13 +145,13 @@ __device__ __forceinline__ void block_add2(double v0, double v1, double* part) {
 // Prepare the adjoints of the previous step from the adjoints (lx, lu) of this
 // step's positions and velocities: a = (1 - M) lx, g = (1 - 2M) lu + dt a,
 // M from x_t at the walls.
-__device__ __forceinline__ void adj_prepare(const AdjArgs& a, int64_t i, const double lx[3],
-                                            const double lu[3]) {
+__device__ __forceinline__ void adj_prepare(const AdjArgs& a, int64_t i, const double xt[3],
+                                            const double lx[3], const double lu[3]) {
     float4 g4;
     float* gf = &g4.x;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const double xv = a.xt[d][i];
+        const double xv = xt[d];
         const bool M = (xv == a.lo[d]) || (xv == a.hi[d]);
         const double ab = M ? 0.0 : lx[d];
         const double g = (M ? -lu[d] : lu[d]) + a.dt * ab;
@@ -174,6 +179,20 @@ __global__ void __launch_bounds__(kBlock * kAdjTPA) k_adj_reverse(AdjArgs a) {
     int64_t i = (int64_t)blockIdx.x * kBlock + al;
     const bool valid = i < a.n;
     const int32_t* __restrict__ U = a.ulist + (int64_t)blockIdx.x * a.ucap;
+    if (!valid) i = a.n - 1;
+    const int4 ri = __ldg(&a.recs[i]);
+    const float4 gi = a.g4_in[i];
+    const int32_t cpk = valid ? __ldg(&a.ncount[i]) : 0;
+    const int32_t cnt = list_total(cpk);
+    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
+    // the first list entries and the atom's state are on their way while the
+    // union is staged
+    int32_t ahead[kAdjAhead];
+#pragma unroll
+    for (int u = 0; u < kAdjAhead; ++u) {
+        const int32_t s = part + u * kAdjTPA;
+        ahead[u] = s < cnt ? L[list_at(s, cpk, al, a.lcap)] : 0;
+    }
     {
         const int32_t nu = min(__ldg(&a.ucount[blockIdx.x]), a.ucap);
         const int32_t m = min(nu * a.apl, a.smrec);
@@ -184,30 +203,27 @@ __global__ void __launch_bounds__(kBlock * kAdjTPA) k_adj_reverse(AdjArgs a) {
         }
     }
     __syncthreads();
-    if (!valid) i = a.n - 1;
-    const int4 ri = __ldg(&a.recs[i]);
-    const float4 gi = a.g4_in[i];
-    const int32_t cpk = valid ? __ldg(&a.ncount[i]) : 0;
-    const int32_t cnt = list_total(cpk);
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
     float3 hv = make_float3(0.f, 0.f, 0.f);
     float eacc = 0.f, sacc = 0.f;
-    int32_t li = part < cnt ? L[list_at(part, cpk, al, a.lcap)] : 0;
-    for (int32_t s = part; s < cnt; s += kAdjTPA) {
-        const int32_t sn = s + kAdjTPA;
-        const int32_t next = sn < cnt ? L[list_at(sn, cpk, al, a.lcap)] : 0;
-        int4 rj;
-        float4 gj;
-        if (li < a.smrec) {
-            rj = srec[li];
-            gj = sg[li];
-        } else {
-            const int64_t at = adj_atom(U, li, a.apl);
-            rj = __ldg(&a.recs[at]);
-            gj = a.g4_in[at];
+    for (int32_t s0 = part; s0 < cnt; s0 += kAdjAhead * kAdjTPA) {
+#pragma unroll
+        for (int u = 0; u < kAdjAhead; ++u) {
+            const int32_t s = s0 + u * kAdjTPA;
+            if (s >= cnt) break;
+            const int32_t li = ahead[u], sn = s + kAdjAhead * kAdjTPA;
+            if (sn < cnt) ahead[u] = L[list_at(sn, cpk, al, a.lcap)];
+            int4 rj;
+            float4 gj;
+            if (li < a.smrec) {
+                rj = srec[li];
+                gj = sg[li];
+            } else {
+                const int64_t at = adj_atom(U, li, a.apl);
+                rj = __ldg(&a.recs[at]);
+                gj = a.g4_in[at];
+            }
+            hvp_pair<COUL>(a, ri, gi, rj, gj, hv, eacc, sacc);
         }
-        hvp_pair<COUL>(a, ri, gi, rj, gj, hv, eacc, sacc);
-        li = next;
     }
     if (part > 0) {
         spart[part - 1][0][al] = hv.x;
@@ -237,10 +253,11 @@ __global__ void __launch_bounds__(kBlock * kAdjTPA) k_adj_reverse(AdjArgs a) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) { a.lx0[d][i] = lx[d]; a.lv0[d][i] = lu[d]; }
         } else {
-            adj_prepare(a, i, lx, lu);
+            const double xt[3] = {a.xt[0][i], a.xt[1][i], a.xt[2][i]};
+            adj_prepare(a, i, xt, lx, lu);
         }
     }
-    block_add2<kBlock * kAdjTPA>(ts, te, a.gpart);
+    block_add2<kBlock>(ts, te, a.gpart);  // (the other slices hold nothing)
 }
 
 // Smooth pair weight of the histogram: 1 below r_switch, C2 switch to 0 at r_max.
@@ -256,7 +273,9 @@ __device__ __forceinline__ void hist_switch(const AdjArgs& a, float r, float& sw
 }
 
 // Per-atom histogram rows of x_t (each unordered pair once: partners later in
-// sorted order), kHistChunk bins per pass over the list.
+// sorted order), kHistChunk bins per pass over the list and one pass a block
+// (one block for all passes left most of the chip idle: 228 us for 32,768
+// atoms and 64 bins, 122 now).
 __global__ void __launch_bounds__(kBlock) k_adj_hist(AdjArgs a) {
     const int tid = threadIdx.x;
     const int64_t i = (int64_t)blockIdx.x * kBlock + tid;
@@ -266,7 +285,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_hist(AdjArgs a) {
     const int32_t cpk = __ldg(&a.ncount[i]);
     const int32_t cnt = list_total(cpk);
     const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
-    for (int32_t b0 = 0; b0 < a.bins; b0 += kHistChunk) {
+    {
+        const int32_t b0 = (int32_t)blockIdx.y * kHistChunk;
         float acc[kHistChunk];
 #pragma unroll
         for (int k = 0; k < kHistChunk; ++k) acc[k] = 0.0f;
@@ -311,59 +331,93 @@ __global__ void __launch_bounds__(256) k_adj_hist_reduce(const float* __restrict
 }
 
 // Loss L = sum_b (h_b - target_b)^2 and the terminal coefficients 2 (h_b - t_b) / N.
-__global__ void k_adj_loss(const double* __restrict__ h, const double* __restrict__ target,
-                           int32_t bins, int32_t n, double* __restrict__ loss,
-                           float* __restrict__ cb) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One block; the differences and coefficients side by side, the sum in bin
+// order (by one thread alone 37 us for 64 bins, most of it divisions).
+__global__ void __launch_bounds__(256) k_adj_loss(const double* __restrict__ h,
+                                                  const double* __restrict__ target, int32_t bins,
+                                                  int32_t n, double* __restrict__ loss,
+                                                  float* __restrict__ cb) {
+    __shared__ double se[256];
     double L = 0.0;
-    for (int32_t b = 0; b < bins; ++b) {
-        const double e = h[b] - target[b];
-        L += e * e;
-        cb[b] = (float)(2.0 * e / (double)n);
+    for (int32_t b0 = 0; b0 < bins; b0 += 256) {
+        const int32_t b = b0 + (int32_t)threadIdx.x;
+        if (b < bins) {
+            const double e = h[b] - target[b];
+            se[threadIdx.x] = e;
+            cb[b] = (float)(2.0 * e / (double)n);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int32_t k = 0; k < min(256, bins - b0); ++k) L += se[k] * se[k];
+        __syncthreads();
     }
-    *loss = L;
+    if (threadIdx.x == 0) *loss = L;
 }
 
 // dL/dx_K from the histogram (per atom over its whole list) and the adjoints
-// of the last step.
-__global__ void __launch_bounds__(kBlock) k_adj_terminal(AdjArgs a) {
+// of the last step.  kTermTPA lanes an atom: each takes the bins of one list
+// entry, and the entries are added in list order (a thread an atom: 217 us for
+// 32,768 atoms and 64 bins, the exponentials of about 25 entries in a chain;
+// 121 now).
+__global__ void __launch_bounds__(256) k_adj_terminal(AdjArgs a) {
     extern __shared__ float scb[];
-    const int tid = threadIdx.x;
-    for (int32_t b = tid; b < a.bins; b += kBlock) scb[b] = a.cb[b];
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int32_t b = tid; b < a.bins; b += 256) scb[b] = a.cb[b];
     __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * kBlock + tid;
-    if (i >= a.n) return;
-    const int32_t* __restrict__ U = a.ulist + (int64_t)blockIdx.x * a.ucap;
-    const int4 ri = __ldg(&a.recs[i]);
-    const int32_t cpk = __ldg(&a.ncount[i]);
+    const int64_t i = (int64_t)blockIdx.x * (256 / kTermTPA) + tid / kTermTPA;
+    const int sub = tid % kTermTPA, lane0 = lane - sub;
+    const bool valid = i < a.n;
+    const int64_t il = valid ? i : 0;
+    const int32_t block = (int32_t)(il / kBlock), al = (int32_t)(il % kBlock);
+    const int32_t* __restrict__ U = a.ulist + (int64_t)block * a.ucap;
+    const int4 ri = __ldg(&a.recs[il]);
+    const int32_t cpk = valid ? __ldg(&a.ncount[il]) : 0;
     const int32_t cnt = list_total(cpk);
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blockIdx.x * list_block(a.lcap);
+    const uint16_t* __restrict__ L = a.llist + (int64_t)block * list_block(a.lcap);
     float gx = 0.f, gy = 0.f, gz = 0.f;
-    for (int32_t s = 0; s < cnt; ++s) {
-        const int64_t j = adj_atom(U, L[list_at(s, cpk, tid, a.lcap)], a.apl);
-        const int4 rj = __ldg(&a.recs[j]);
-        const float dx = (float)idiff(ri.x, rj.x) * a.invS;
-        const float dy = (float)idiff(ri.y, rj.y) * a.invS;
-        const float dz = (float)idiff(ri.z, rj.z) * a.invS;
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (!(r2 < a.rmax2)) continue;
-        const float r = sqrtf(r2);
-        float sw, dsw;
-        hist_switch(a, r, sw, dsw);
-        float c = 0.0f;
-        for (int32_t b = 0; b < a.bins; ++b) {
-            const float u = r - ((float)b + 0.5f) * a.bw;
-            const float e = expf(-u * u * a.inv2w2);
-            c += scb[b] * e * (dsw - sw * u * a.invw2);
+    for (int32_t s0 = 0; __any_sync(0xffffffffu, s0 < cnt); s0 += kTermTPA) {
+        const int32_t s = s0 + sub;
+        float dx = 0.f, dy = 0.f, dz = 0.f, c = 0.f;
+        bool in = false;
+        if (s < cnt) {
+            const int64_t j = adj_atom(U, L[list_at(s, cpk, al, a.lcap)], a.apl);
+            const int4 rj = __ldg(&a.recs[j]);
+            dx = (float)idiff(ri.x, rj.x) * a.invS;
+            dy = (float)idiff(ri.y, rj.y) * a.invS;
+            dz = (float)idiff(ri.z, rj.z) * a.invS;
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            in = r2 < a.rmax2;
+            if (in) {
+                const float r = sqrtf(r2);
+                float sw, dsw;
+                hist_switch(a, r, sw, dsw);
+                for (int32_t b = 0; b < a.bins; ++b) {
+                    const float u = r - ((float)b + 0.5f) * a.bw;
+                    const float e = expf(-u * u * a.inv2w2);
+                    c += scb[b] * e * (dsw - sw * u * a.invw2);
+                }
+                c /= r;
+            }
         }
-        c /= r;
-        gx += c * dx;
-        gy += c * dy;
-        gz += c * dz;
+        const unsigned m = (__ballot_sync(0xffffffffu, in) >> lane0) & ((1u << kTermTPA) - 1u);
+#pragma unroll
+        for (int k = 0; k < kTermTPA; ++k) {
+            const float ck = __shfl_sync(0xffffffffu, c, lane0 + k);
+            const float xk = __shfl_sync(0xffffffffu, dx, lane0 + k);
+            const float yk = __shfl_sync(0xffffffffu, dy, lane0 + k);
+            const float zk = __shfl_sync(0xffffffffu, dz, lane0 + k);
+            if ((m >> k) & 1u) {
+                gx += ck * xk;
+                gy += ck * yk;
+                gz += ck * zk;
+            }
+        }
     }
+    if (!valid || sub != 0) return;
+    const double xt[3] = {a.xt[0][i], a.xt[1][i], a.xt[2][i]};
     const double lx[3] = {(double)gx, (double)gy, (double)gz};
     const double lu[3] = {0.0, 0.0, 0.0};
-    adj_prepare(a, i, lx, lu);
+    adj_prepare(a, i, xt, lx, lu);
 }
 
 // Undo a re-sort on the adjoints: old[perm[k]] = new[k].
@@ -392,12 +446,20 @@ __global__ void k_adj_unsort(const int32_t* __restrict__ orig, int32_t n,
     }
 }
 
-__global__ void k_adj_gpar(const double* __restrict__ part, int32_t nb, double* __restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0, e = 0.0;
-    for (int32_t b = 0; b < nb; ++b) { s += part[2 * b]; e += part[2 * b + 1]; }
-    out[0] = s;
-    out[1] = e;
+// Sums of the blocks' partials in block order, the loads side by side.
+__global__ void __launch_bounds__(256) k_adj_gpar(const double* __restrict__ part, int32_t nb,
+                                                  double* __restrict__ out) {
+    __shared__ double sp[2 * 256];
+    double t = 0.0;  // thread 0: dL/dsigma, thread 1: dL/deps
+    for (int32_t b0 = 0; b0 < nb; b0 += 256) {
+        const int32_t m = min(256, nb - b0);
+        for (int32_t k = threadIdx.x; k < 2 * m; k += 256) sp[k] = part[2 * (int64_t)b0 + k];
+        __syncthreads();
+        if (threadIdx.x < 2)
+            for (int32_t k = 0; k < m; ++k) t += sp[2 * k + threadIdx.x];
+        __syncthreads();
+    }
+    if (threadIdx.x < 2) out[threadIdx.x] = t;
 }
 
 
@@ -571,10 +633,10 @@ static nd_status adj_enqueue_forward(AdjEngine* A) {
         return st;
     AdjArgs a = adj_args(A, (const double*)A->xK.p, (const int4*)A->recK.p);
     const unsigned nb = (unsigned)m->nblocks;
-    k_adj_hist<<<nb, kBlock, 0, c->stream>>>(a);
+    k_adj_hist<<<dim3(nb, (unsigned)cdiv(A->s.bins, kHistChunk)), kBlock, 0, c->stream>>>(a);
     k_adj_hist_reduce<<<(unsigned)A->s.bins, 256, 0, c->stream>>>((const float*)A->hatom.p, A->n,
                                                                    (double*)A->hist.p);
-    k_adj_loss<<<1, 32, 0, c->stream>>>((const double*)A->hist.p, (const double*)A->target.p,
+    k_adj_loss<<<1, 256, 0, c->stream>>>((const double*)A->hist.p, (const double*)A->target.p,
                                         A->s.bins, A->n, (double*)A->scal.p, (float*)A->cb.p);
     c->launches += 3;
     return check_launch(c, "adjoint forward");
@@ -599,7 +661,8 @@ static nd_status adj_enqueue_backward(AdjEngine* A) {
     {
         AdjArgs a = adj_args(A, (const double*)A->xK.p, (const int4*)A->recK.p);
         a.g4_out = (float4*)A->g4[gc].p;
-        k_adj_terminal<<<nb, kBlock, sizeof(float) * (size_t)A->s.bins, c->stream>>>(a);
+        k_adj_terminal<<<(unsigned)cdiv(A->n, 256 / kTermTPA), 256, sizeof(float) * (size_t)A->s.bins,
+                         c->stream>>>(a);
         c->launches++;
     }
     for (int32_t sg = A->nseg - 1; sg >= 0; --sg) {
@@ -628,10 +691,13 @@ static nd_status adj_enqueue_backward(AdjEngine* A) {
             for (int32_t s = e - 1; s >= a0; --s) {
                 const bool start = s == a0 || s % A->R == 0 || sched[s - 1];
                 if (!start) continue;
-                if ((st = adj_copy(A, live_set(A), traj + (s - t0) * 3 * n, 3 * sizeof(double) * n,
-                                   "epoch")))
-                    return st;
-                if ((st = md_rebuild(m, RB_REFIT))) return st;
+                // (the last epoch's lists are there: the recomputation ended on them)
+                if (e < t0 + A->C) {
+                    if ((st = adj_copy(A, live_set(A), traj + (s - t0) * 3 * n,
+                                       3 * sizeof(double) * n, "epoch")))
+                        return st;
+                    if ((st = md_rebuild(m, RB_REFIT))) return st;
+                }
                 for (int32_t t = e - 1; t >= s; --t) {
                     AdjArgs a = adj_args(A, traj + (t - t0) * 3 * n, trec + (t - t0) * n);
                     a.g4_in = (const float4*)A->g4[gc].p;
@@ -663,7 +729,7 @@ static nd_status adj_enqueue_backward(AdjEngine* A) {
     k_adj_unsort<<<g256, 256, 0, c->stream>>>(m->set[0].orig, A->n, outs, outs + 3 * n,
                                               (double*)A->outs.p + 6 * n,
                                               (double*)A->outs.p + 9 * n);
-    k_adj_gpar<<<1, 32, 0, c->stream>>>((const double*)A->gpart.p, (int32_t)nb,
+    k_adj_gpar<<<1, 256, 0, c->stream>>>((const double*)A->gpart.p, (int32_t)nb,
                                         (double*)A->scal.p + 1);
     c->launches += 2;
     return check_launch(c, "adjoint backward");
