@@ -167,6 +167,10 @@ __device__ __forceinline__ void adj_prepare(const AdjArgs& a, int64_t i, const d
 // the forward step's union is staged (the step's fixed-point position records
 // and the Float32 velocity adjoints), thread p of an atom gathers over list
 // slots p, p + kAdjTPA, ..., and the slices are added in a fixed order.
+// 128 blocks for 32,768 atoms are less than a wave, so the time is one block's
+// chain of loads and gathers: list entries kAdjAhead deep, the first of them
+// under way during the staging, and block sums over the one slice that has any
+// (30.6 us a step before, 25.3 now).
 template <bool COUL>
 __global__ void __launch_bounds__(kBlock * kAdjTPA) k_adj_reverse(AdjArgs a) {
     extern __shared__ int4 adj_smem[];

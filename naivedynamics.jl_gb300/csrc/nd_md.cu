@@ -1898,11 +1898,14 @@ static cudaError_t raise_smem_limit(const void* fn, int maxsm) {
                                 maxsm - (int)fa.sharedSizeBytes);
 }
 
-// Whether the lists are built by a warp per leaf: while there is at most one
-// block of kBlock atoms per SM, whose threads (one an atom) would walk their
-// candidates on a part of the chip, and the candidates fit shared memory.
+// Whether the lists are built by a warp per leaf: while there are at most two
+// blocks of kBlock atoms per SM, whose threads (one an atom) would walk their
+// candidates on a part of the chip, and the candidates fit shared memory.  A
+// rebuild with a thread an atom and with a warp a leaf, us: 40,960 atoms 228
+// and 175, 65,536 atoms 251 and 220; but 98,304 atoms 250 and 266, 262,144
+// atoms 536 and 706.
 static bool md_leaf_warps(const MDEngine* m) {
-    return m->nblocks <= m->nsm && 8 * sizeof(uint2) * (size_t)m->lcap_leaf <= 200 * 1024;
+    return m->nblocks <= 2 * m->nsm && 8 * sizeof(uint2) * (size_t)m->lcap_leaf <= 200 * 1024;
 }
 
 // Union and list buffers for capacities (ucap, lcap), and the shared-memory

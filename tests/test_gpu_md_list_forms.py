@@ -1,4 +1,4 @@
-"""The two list builds (a warp per leaf up to one block of 256 atoms per SM, a
+"""The two list builds (a warp per leaf up to two blocks of 256 atoms per SM, a
 thread per atom beyond) at every leaf width and ragged block ends: the engine's
 lists are exactly the pairs within r_c + skin of the positions they were built
 from."""
@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,apl", [(64, 1), (254, 2), (256, 4), (260, 4), (1288, 8), (1040, 16),
-                                   (2080, 32), (38912, 4), (39168, 4), (39176, 8), (39200, 32)])
+                                   (2080, 32), (38912, 4), (39168, 4), (39176, 8), (39200, 32),
+                                   (77824, 4), (77832, 8)])
 def test_lists_are_the_pairs_within_the_list_radius(nd, oracle, n, apl):
     side = (n / 0.83) ** (1.0 / 3.0)
     x, v, _ = nd.synth.lj_system(n, n, side, 0.8)
