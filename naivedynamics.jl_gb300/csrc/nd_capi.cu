@@ -60,17 +60,16 @@ nd_status check_launch(Ctx* c, const char* what) {
 
 bool BufPool::take(DevBuf& b, size_t bytes) {
     std::lock_guard<std::mutex> lock(mu);
-    size_t best = idle.size();
-    for (size_t k = 0; k < idle.size(); ++k)
+    size_t best = count;
+    for (size_t k = 0; k < count; ++k)
         // the smallest that fits, not much larger than asked for
         if (idle[k].bytes >= bytes && idle[k].bytes <= 2 * bytes + 65536 &&
-            (best == idle.size() || idle[k].bytes < idle[best].bytes))
+            (best == count || idle[k].bytes < idle[best].bytes))
             best = k;
-    if (best == idle.size()) return false;
+    if (best == count) return false;
     b = idle[best];
     held -= b.bytes;
-    idle[best] = idle.back();
-    idle.pop_back();
+    idle[best] = idle[--count];
     return true;
 }
 
@@ -78,8 +77,8 @@ void BufPool::put(DevBuf& b) {
     if (!b.p) return;
     {
         std::lock_guard<std::mutex> lock(mu);
-        if (idle.size() < kMost && held + b.bytes <= kBytes) {
-            idle.push_back(b);
+        if (count < kMost && held + b.bytes <= kBytes) {
+            idle[count++] = b;
             held += b.bytes;
             b = DevBuf{};
             return;
@@ -91,9 +90,8 @@ void BufPool::put(DevBuf& b) {
 
 void BufPool::clear() {
     std::lock_guard<std::mutex> lock(mu);
-    for (DevBuf& b : idle) cudaFree(b.p);
-    idle.clear();
-    held = 0;
+    for (size_t k = 0; k < count; ++k) cudaFree(idle[k].p);
+    count = held = 0;
 }
 
 nd_status ensure(Ctx* c, DevBuf& b, size_t bytes) {

@@ -157,8 +157,8 @@ public:
 private:
     static constexpr size_t kMost = 128, kBytes = size_t(512) << 20;
     std::mutex mu;
-    std::vector<DevBuf> idle;
-    size_t held = 0;
+    DevBuf idle[kMost];  // (no growing array: nothing here throws)
+    size_t count = 0, held = 0;
 };
 
 // Context shared by all entry points (defined in nd_capi.cu).

@@ -20,7 +20,7 @@ def test_unordered_matches_ordered(nd, leaves, shape):
     x = uniform(77 + leaves, n)
     r = np.float32(0.9 * n ** (-1.0 / 3.0))
     if shape == "clusters":
-        x[: n // 2] = 0.5 + 0.02 * (x[: n // 2] - 0.5)
+        x[: n // 2] = 0.5 + 0.2 * (x[: n // 2] - 0.5)
     elif shape == "point":  # boxes of one size, some distances exactly zero
         if n > 256:
             pytest.skip("every pair is a hit")
