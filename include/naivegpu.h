@@ -192,7 +192,7 @@ nd_status nd_tree(nd_ctx* ctx, const float* xyz, const nd_bvh_spec* spec, int32_
  * and ND_NEED_REALLOC is returned (call again with capacity >= *count, or with
  * capacity 0 to only count).  mode: ND_PAIRS_ORDERED (the order the reference
  * emits on one thread) or ND_PAIRS_UNORDERED (the same pairs in the order the
- * GPU produces them: the two-phase warp-cooperative emission, which needs
+ * GPU produces them: the warp-cooperative emission, which needs
  * atomsperleaf == 4; with any other leaf width an unordered request is served
  * by the ordered emission).
  */
