@@ -1008,6 +1008,22 @@ struct PairK {
     __device__ __forceinline__ float band() const { return rc2u * 1.9073486328125e-06f; }
 };
 
+// The potential energy of an atom in the measure pass, in double precision:
+// sums of s^12 - s^6 and of q_j / r, their constants applied at the end.  The
+// pass is bound by GB300's FP64 pipe (2 operations a clock and SM), so what
+// counts is operations a pair: 37 with each term complete and two Newton steps
+// for 1/r and for 1/r^2 each, 21 so (30,004 atoms with charges: 190 us before,
+// 125 now).
+struct EnergySum {
+    double sig2 = 0.0;  // sigma^2 in grid units
+    double lj = 0.0, coul = 0.0;
+    __device__ __forceinline__ void add_lj(double s6) { lj = fma(s6, s6 - 1.0, lj); }
+    __device__ __forceinline__ void add_coul(float qj, double ir) { coul = fma((double)qj, ir, coul); }
+    __device__ __forceinline__ double total(const PairK& a, float qi) const {
+        return (double)a.eps4 * lj + (double)a.kceu * (double)qi * coul;
+    }
+};
+
 // Low part of a separation split: the value in [0, 2^23) as a float, exact,
 // by placing it in the mantissa of 2^23.
 __device__ __forceinline__ float lo_part(int32_t v) {
@@ -1052,7 +1068,7 @@ __device__ __forceinline__ float fine_diff(uint32_t a, uint32_t b, int sh) {
 // a product whose residual is taken separately.
 template <bool COUL, bool ENERGY>
 __device__ __forceinline__ void accum_near(const int4& ri, const int4& rj, const uint2& fi,
-                                           const uint2& fj, const PairK& a, DF3& acc, double& ue) {
+                                           const uint2& fj, const PairK& a, DF3& acc, EnergySum& ue) {
     const int32_t ix = idiff(ri.x, rj.x), iy = idiff(ri.y, rj.y), iz = idiff(ri.z, rj.z);
     const float hx = __int2float_rn(ix & a.hmask), lx = lo_part(ix & ~a.hmask);
     const float hy = __int2float_rn(iy & a.hmask), ly = lo_part(iy & ~a.hmask);
@@ -1099,11 +1115,7 @@ __device__ __forceinline__ void accum_near(const int4& ri, const int4& rj, const
     float fh = __fmul_rn(a.eps24u, p2);
     float fl = __fmaf_rn(a.e24lo, p2, __fmaf_rn(a.eps24u, p2l, __fmaf_rn(a.eps24u, p2, -fh)));
     // energy (measure pass only): from the two-float s6 in double precision
-    double uu = 0.0;
-    if (ENERGY) {
-        const double s6d = (double)s6 + (double)s6l;
-        uu = (double)a.eps4 * s6d * (s6d - 1.0);
-    }
+    if (ENERGY) ue.add_lj((double)s6 + (double)s6l);
     if (COUL) {
         const float qi = __int_as_float(ri.w), qj = __int_as_float(rj.w);
         const float qh = __fmul_rn(qi, qj), ql = __fmaf_rn(qi, qj, -qh);
@@ -1121,7 +1133,7 @@ __device__ __forceinline__ void accum_near(const int4& ri, const int4& rj, const
         const float se = __fadd_rn(__fsub_rn(fh, __fsub_rn(sh, sb)), __fsub_rn(ch, sb));
         fh = sh;
         fl = __fadd_rn(fl, __fadd_rn(cl2, se));
-        if (ENERGY) uu += (double)a.kceu * ((double)qi * (double)qj) * ((double)ir + (double)irl);
+        if (ENERGY) ue.add_coul(qj, (double)ir + (double)irl);
     }
     // components fmag * d, into the two-float sums
     {
@@ -1132,7 +1144,6 @@ __device__ __forceinline__ void accum_near(const int4& ri, const int4& rj, const
         const float tz = __fmul_rn(fh, dzh);
         df_acc(acc.zh, acc.zl, tz, __fmaf_rn(fl, dzh, __fmaf_rn(fh, dzl, __fmaf_rn(fh, dzh, -tz))));
     }
-    if (ENERGY) ue += uu;
 }
 
 // Pair (i, j) from fixed-point records: the integer difference is exact, its
@@ -1144,7 +1155,7 @@ __device__ __forceinline__ void accum_near(const int4& ri, const int4& rj, const
 // cannot decide it): the caller evaluates it with accum_near.
 template <bool COUL, bool ENERGY>
 __device__ __forceinline__ bool accum_pair(const int4& ri, const int4& rj, const PairK& a,
-                                          float& fx, float& fy, float& fz, double& ue) {
+                                          float& fx, float& fy, float& fz, EnergySum& ue) {
     const float dx = (float)idiff(ri.x, rj.x);
     const float dy = (float)idiff(ri.y, rj.y);
     const float dz = (float)idiff(ri.z, rj.z);
@@ -1176,26 +1187,24 @@ __device__ __forceinline__ bool accum_pair(const int4& ri, const int4& rj, const
             // bias of a fraction of an ulp, which ten million pairs add up)
             const double xd = (double)idiff(ri.x, rj.x), yd = (double)idiff(ri.y, rj.y),
                          zd = (double)idiff(ri.z, rj.z);
-            // 1/r^2 and 1/r by two Newton-Raphson steps each in double
-            // precision (y <- y (2 - r^2 y), y <- y (3 - r^2 y^2) / 2) from the
-            // single-precision reciprocal and reciprocal square root: a double
-            // division or square root costs several times more on GB300's FP64
-            // pipe, and these terms run for every pair of the pass
+            // One step of third order from the single-precision 1/r or 1/r^2
+            // (relative error e / 2 or e, about 2e-7; e^3 is below 1e-19):
+            // with e = 1 - r^2 y^2, y (1 + e/2 + 3 e^2/8); with e = 1 - r^2 y,
+            // y (1 + e + e^2).
             const double r2d = xd * xd + yd * yd + zd * zd;
-            double ir2d = (double)__frcp_rn((float)r2d);
-            ir2d = ir2d * (2.0 - r2d * ir2d);
-            ir2d = ir2d * (2.0 - r2d * ir2d);
-            const double s2d = ((double)a.sig2u + (double)a.sig2lo) * ir2d;
-            const double s6d = s2d * s2d * s2d;
-            double ud = (double)a.eps4 * s6d * (s6d - 1.0);
+            double ir2d;
             if (COUL) {
-                double ird = (double)rsqrtf((float)r2d);
-                ird = ird * (1.5 - 0.5 * r2d * ird * ird);
-                ird = ird * (1.5 - 0.5 * r2d * ird * ird);
-                ud += (double)a.kceu * ((double)__int_as_float(ri.w) * (double)__int_as_float(rj.w)) *
-                      ird;
+                double y = (double)inv_r;
+                const double e = fma(-r2d * y, y, 1.0);
+                y = fma(y * e, fma(0.375, e, 0.5), y);
+                ir2d = y * y;
+                ue.add_coul(__int_as_float(rj.w), y);
+            } else {
+                const double y = (double)inv_r2, e = fma(-r2d, y, 1.0);
+                ir2d = fma(y, fma(e, e, e), y);
             }
-            ue += ud;
+            const double s2d = ue.sig2 * ir2d;
+            ue.add_lj(s2d * s2d * s2d);
         }
     }
     return false;
@@ -1350,7 +1359,7 @@ __device__ __forceinline__ unsigned accum_pair2(const int4& ri, const int4& ra, 
     const float band = k1.band();
     if ((r2a < k1.rn2u) | (r2b < k1.rn2u) | (fabsf(r2a - k1.rc2u) <= band) |
         (fabsf(r2b - k1.rc2u) <= band)) {
-        double ue = 0.0;
+        EnergySum ue;
         unsigned m = accum_pair<COUL, false>(ri, ra, k1, sx, sy, sz, ue) ? 1u : 0u;
         m |= accum_pair<COUL, false>(ri, rb, k1, sx, sy, sz, ue) ? 2u : 0u;
         return m;
@@ -1486,6 +1495,8 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
     DF3 nacc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float fx = 0.f, fy = 0.f, fz = 0.f;
     double ue = 0.0;  // potential energy (measure pass only)
+    EnergySum en;
+    if constexpr (MODE == 1) en.sig2 = (double)pk.sig2u + (double)pk.sig2lo;
     __shared__ float spart[TPA > 1 ? TPA - 1 : 1][8][kBlock];
     // The pair loops, compiled twice: for a block whose whole union is staged
     // (the usual case; a block-uniform choice) a record is read from shared
@@ -1509,7 +1520,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             for (; s < nn; s += TPA) {
                 const int32_t sn = s + TPA;
                 const int32_t next = sn < nn ? near_entry(sn) : 0;
-                accum_near<COUL, MODE == 1>(ri, fetch(li), fi, fine(li), pk, nacc, ue);
+                accum_near<COUL, MODE == 1>(ri, fetch(li), fi, fine(li), pk, nacc, en);
                 li = next;
             }
         } else if constexpr (TPA == 1) {
@@ -1528,7 +1539,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             }
             if (s < nn) {
                 const int32_t li = cur.x & 0xffffu;
-                accum_near<COUL, false>(ri, fetch(li), fi, fine(li), pk, nacc, ue);
+                accum_near<COUL, false>(ri, fetch(li), fi, fine(li), pk, nacc, en);
             }
         } else {
             // near entries of this thread's slice two at a time (packed), the
@@ -1544,12 +1555,12 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
                 lb = s2 + TPA < nn ? near_entry(s2 + TPA) : 0;
                 accum_near2<COUL>(ri, ra, rb, fi, fa, fb, pk, nacc);
             }
-            if (s < nn) accum_near<COUL, false>(ri, fetch(la), fi, fine(la), pk, nacc, ue);
+            if (s < nn) accum_near<COUL, false>(ri, fetch(la), fi, fine(la), pk, nacc, en);
         }
         // an entry of the other segment that came closer than 1.3 sigma
         auto far_near = [&](int32_t s) {
             const int32_t li = far_entry(s);
-            accum_near<COUL, MODE == 1>(ri, fetch(li), fi, fine(li), pk, nacc, ue);
+            accum_near<COUL, MODE == 1>(ri, fetch(li), fi, fine(li), pk, nacc, en);
         };
         if constexpr (TPA == 1) {
             // groups of four neighbours, one word of the list each; the next
@@ -1573,8 +1584,8 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
                     // as the two halves of the packed form
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const bool nr = (k & 1) ? accum_pair<COUL, MODE == 1>(ri, rj[k], pk, gx, gy, gz, ue)
-                                                : accum_pair<COUL, MODE == 1>(ri, rj[k], pk, fx, fy, fz, ue);
+                        const bool nr = (k & 1) ? accum_pair<COUL, MODE == 1>(ri, rj[k], pk, gx, gy, gz, en)
+                                                : accum_pair<COUL, MODE == 1>(ri, rj[k], pk, fx, fy, fz, en);
                         if (nr) far_near(s + k);
                     }
                 } else {
@@ -1604,8 +1615,9 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
                 const int32_t li = (int32_t)(cur.x & 0xffffu);
                 cur.x = __funnelshift_r(cur.x, cur.y, 16);
                 cur.y >>= 16;
-                if (accum_pair<COUL, MODE == 1>(ri, fetch(li), pk, fx, fy, fz, ue)) far_near(s);
+                if (accum_pair<COUL, MODE == 1>(ri, fetch(li), pk, fx, fy, fz, en)) far_near(s);
             }
+            if constexpr (MODE == 1) ue = en.total(pk, __int_as_float(ri.w));
             // the force: two-float near sums with the single-precision sums added
             // to their low parts, rounded once
             fx = __fadd_rn(nacc.xh, __fadd_rn(nacc.xl, fx));
@@ -1631,12 +1643,13 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
                 load4(s + 4 * TPA);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (accum_pair<COUL, MODE == 1>(ri, rj[k], pk, fx, fy, fz, ue))
+                    if (accum_pair<COUL, MODE == 1>(ri, rj[k], pk, fx, fy, fz, en))
                         far_near(s + k * TPA);
             }
             // at most three entries left, their indices already loaded
             for (int k = 0; s < nf && k < 4; s += TPA, ++k)
-                if (accum_pair<COUL, MODE == 1>(ri, fetch(li[k]), pk, fx, fy, fz, ue)) far_near(s);
+                if (accum_pair<COUL, MODE == 1>(ri, fetch(li[k]), pk, fx, fy, fz, en)) far_near(s);
+            if constexpr (MODE == 1) ue = en.total(pk, __int_as_float(ri.w));
             // each slice as a two-float value (its single-precision sum in the low
             // part); the slices added in a fixed order
             nacc.xl = __fadd_rn(nacc.xl, fx);
@@ -2519,10 +2532,10 @@ static nd_status md_opened(MDEngine* m) {
 // Sizing build pass: diag int32 words 2..6 collect the largest union, the
 // largest per-atom list, the largest per-leaf candidate list, the sum of
 // union sizes and the largest BFS frontier.
-static nd_status md_sizing_pass(MDEngine* m, int32_t h[5]) {
+static nd_status md_sizing_pass(MDEngine* m, int kind, int32_t h[5]) {
     Ctx* c = &m->sub;
     cudaMemsetAsync((int32_t*)m->diag.p + 2, 0, 5 * sizeof(int32_t), c->stream);
-    nd_status st = md_rebuild(m, RB_RESORT, -1, nullptr, true);
+    nd_status st = md_rebuild(m, kind, -1, nullptr, true);
     if (st) return st;
     cudaError_t e = cudaMemcpyAsync(h, (int32_t*)m->diag.p + 2, 5 * sizeof(int32_t),
                                     cudaMemcpyDeviceToHost, c->stream);
@@ -2541,7 +2554,7 @@ static nd_status md_size_lists(MDEngine* m) {
     nd_status st;
     int32_t h[5];
     if ((st = md_alloc_lists(m, kSizingFcap, kSizingUcap, 0, 0, 0))) return st;
-    if ((st = md_sizing_pass(m, h))) return st;
+    if ((st = md_sizing_pass(m, RB_RESORT, h))) return st;
     const int32_t max_u = h[0], max_c = h[2], max_f = h[4];
     const double mean_u = (double)h[3] / m->nblocks;
     if (max_u > kSizingUcap || max_f > kSizingFcap) {
@@ -2556,7 +2569,7 @@ static nd_status md_size_lists(MDEngine* m) {
     // a block whose union is larger reads its remaining records from L2.
     const int32_t ucap_sm = m->p.stage_policy == 1 ? ucap : round_up(mean_u * 1.2 + 16, 16);
     if ((st = md_alloc_lists(m, fcap, ucap, lcap_leaf, 0, ucap_sm))) return st;
-    if ((st = md_sizing_pass(m, h))) return st;
+    if ((st = md_sizing_pass(m, RB_RESORT, h))) return st;
     const int32_t max_n = h[1];
     int32_t lcap = m->p.max_neighbors > 0 ? round_up(m->p.max_neighbors, 8)
                                           : round_up(max_n * 1.35 + 16, 8);
