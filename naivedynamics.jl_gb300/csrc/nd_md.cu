@@ -2569,7 +2569,7 @@ static nd_status md_size_lists(MDEngine* m) {
     // a block whose union is larger reads its remaining records from L2.
     const int32_t ucap_sm = m->p.stage_policy == 1 ? ucap : round_up(mean_u * 1.2 + 16, 16);
     if ((st = md_alloc_lists(m, fcap, ucap, lcap_leaf, 0, ucap_sm))) return st;
-    if ((st = md_sizing_pass(m, RB_RESORT, h))) return st;
+    if ((st = md_sizing_pass(m, RB_REFIT, h))) return st;  // (the order stands)
     const int32_t max_n = h[1];
     int32_t lcap = m->p.max_neighbors > 0 ? round_up(m->p.max_neighbors, 8)
                                           : round_up(max_n * 1.35 + 16, 8);
