@@ -2547,8 +2547,9 @@ static int32_t round_up(double v, int32_t q) { return (((int32_t)std::ceil(v)) +
 
 // First builds: (1) generous union and frontier, lists not stored -> union,
 // frontier and per-leaf capacities; (2) per-leaf lists stored, per-atom lists
-// counted -> list capacity; (3) the real build.  Capacities carry head-room
-// for the drift until later rebuilds.
+// counted -> list capacity; (3) the real build.  Only the first sorts: the
+// positions are the same in all three.  Capacities carry head-room for the
+// drift until later rebuilds.
 static nd_status md_size_lists(MDEngine* m) {
     Ctx* c = &m->sub;
     nd_status st;
@@ -2569,12 +2570,12 @@ static nd_status md_size_lists(MDEngine* m) {
     // a block whose union is larger reads its remaining records from L2.
     const int32_t ucap_sm = m->p.stage_policy == 1 ? ucap : round_up(mean_u * 1.2 + 16, 16);
     if ((st = md_alloc_lists(m, fcap, ucap, lcap_leaf, 0, ucap_sm))) return st;
-    if ((st = md_sizing_pass(m, RB_REFIT, h))) return st;  // (the order stands)
+    if ((st = md_sizing_pass(m, RB_REFIT, h))) return st;
     const int32_t max_n = h[1];
     int32_t lcap = m->p.max_neighbors > 0 ? round_up(m->p.max_neighbors, 8)
                                           : round_up(max_n * 1.35 + 16, 8);
     if ((st = md_alloc_lists(m, fcap, ucap, lcap_leaf, lcap, ucap_sm))) return st;
-    if ((st = md_rebuild(m, RB_RESORT))) return st;
+    if ((st = md_rebuild(m, RB_REFIT))) return st;
     if ((st = md_opened(m))) return st;
     m->in_window = 0;
     m->rebuild_due = false;
