@@ -265,6 +265,14 @@ nd_status pairs_common(Ctx* c, const nd_bvh_spec* s, int32_t order, int32_t mode
     return pairs_from_tree(c, t, s, mode, kind, host, pi, pj, pd, capacity, count, criterion);
 }
 
+// Entries all three host-list arrays hold.  Each of them may be larger than the
+// others: pairs_i alone also takes whole entries (nd_leaf_pair_list), and idle
+// blocks come larger than asked for.
+static int64_t list_capacity(const Ctx* c) {
+    return (int64_t)(std::min({c->pairs_i.bytes, c->pairs_j.bytes, c->pairs_d.bytes}) /
+                     sizeof(int32_t));
+}
+
 // Pair emission over a built tree (the second half of pairs_common).
 static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec* s,
                                  int32_t mode, int kind, bool host, int32_t* pi, int32_t* pj,
@@ -276,8 +284,7 @@ static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec
     int64_t total = 0;
     if (kind == 0 && unordered_emission(s, mode)) {
         if (host) {
-            int64_t devcap = (int64_t)(c->pairs_i.bytes / sizeof(int32_t));
-            devcap = std::min(devcap, (int64_t)(c->pairs_d.bytes / sizeof(float)));
+            const int64_t devcap = list_capacity(c);
             if ((st = emit_unordered(c, t, r, r2, (int32_t*)c->pairs_i.p, (int32_t*)c->pairs_j.p,
                                      (float*)c->pairs_d.p, devcap, &total)))
                 return st;
@@ -303,11 +310,7 @@ static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec
         int64_t* total_dev = (int64_t*)(c->d_err + 4);
         if ((st = count_pairs(c, t, r, r2, kind, total_dev))) return st;
         int64_t devcap = capacity;
-        if (host) {
-            devcap = (int64_t)(std::min({c->pairs_i.bytes, c->pairs_j.bytes, c->pairs_d.bytes}) /
-                               sizeof(int32_t));
-            devcap = std::min(devcap, capacity);
-        }
+        if (host) devcap = std::min(list_capacity(c), capacity);
         if (devcap > 0 &&
             (st = write_pairs(c, t, r, r2, kind, total_dev, devcap,
                               host ? (int32_t*)c->pairs_i.p : pi, host ? (int32_t*)c->pairs_j.p : pj,
