@@ -35,6 +35,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "nd_bands.cuh"
 #include "nd_internal.cuh"
 
 namespace nd {
@@ -313,24 +314,6 @@ __global__ void __launch_bounds__(288) k_cs_lj(const float* __restrict__ x, int3
 // computed beforehand in the order the lanes read them, 4 KB a step.  Where a
 // lane has no pair the term is -0, which adds nothing to any value (signed
 // zeros included).
-constexpr int kBandRows = 256;         // rows of a band: eight a lane
-constexpr int kBandPad = 128;          // column words before the first (columns leaving a band early)
-constexpr int kBandMaxAtoms = 20480;   // the columns' array fits a block's shared memory
-
-constexpr int kBandCopy = 4;           // steps (of 4 KB) a copy brings
-// steps (tiles of four columns a lane) of band 0, padded to whole copies: band
-// b has band_steps(n) - 64 b
-__host__ __device__ inline int32_t band_steps(int32_t n) {
-    return ((n + 3) / 4 + 31 + kBandCopy - 1) / kBandCopy * kBandCopy;
-}
-__host__ __device__ inline int64_t band_off(int32_t b, int32_t P) {  // in steps
-    return (int64_t)b * P - 32LL * b * (b - 1);
-}
-// bytes of the columns' array (words written: 4 (band_steps(n) - 31) + kBandPad)
-__host__ __device__ inline int32_t band_col_bytes(int32_t n) {
-    return (8 * (4 * band_steps(n) + kBandPad) + 127) & ~127;
-}
-
 __device__ __forceinline__ float coulomb_term(float xi, float yi, float zi, float qi, float xj,
                                               float yj, float zj, float qj) {
     const float dx = __fsub_rn(xi, xj), dy = __fsub_rn(yi, yj), dz = __fsub_rn(zi, zj);
@@ -346,9 +329,9 @@ __global__ void __launch_bounds__(256)
     const int32_t b = blockIdx.y, lane = threadIdx.x & 31, r = threadIdx.x >> 5;
     const int32_t t = (int32_t)blockIdx.x;
     if (t >= P - 64 * b) return;
-    const int32_t i = kBandRows * b + 8 * lane + r, j0 = kBandRows * b + 4 * (t - lane);
+    const int32_t i = band_row(b, lane, r), j0 = band_col(b, lane, t);
     float c[4] = {-0.0f, -0.0f, -0.0f, -0.0f};
-    if (j0 + 3 > i && j0 < n) {
+    if (band_tile_has_pair(i, j0, n)) {
         const float xi = __ldg(&x[3 * (int64_t)i]), yi = __ldg(&x[3 * (int64_t)i + 1]),
                     zi = __ldg(&x[3 * (int64_t)i + 2]), qi = __ldg(&q[i]);
 #pragma unroll
