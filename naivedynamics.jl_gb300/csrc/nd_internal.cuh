@@ -182,7 +182,10 @@ struct Ctx {
 // true starts with chain_wait(): its blocks may be resident before the kernel
 // in front of it has ended, and the wait holds until that kernel is complete
 // and its writes are visible.  Every such kernel waits on every path, so
-// completion passes along the chain.  (4,096 atoms, a check after every step:
+// completion passes along the chain.  What the chain's kernels write (records,
+// boxes, unions, lists, counts, the gate) is read with plain loads: __ldg, and
+// const __restrict__ parameters, promise data that nobody writes while the
+// kernel is resident.  (4,096 atoms, a check after every step:
 // 16.3 -> 15.5 us a step; chaining the steps to each other or a rebuild's own
 // kernels gained nothing, steps lost 0.8 us.)
 __device__ __forceinline__ void chain_wait() {

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kBlock)
     k_md_place(SetPtrs src, SetPtrs st, int32_t n, Frame fr, const SysRow* __restrict__ sys,
                int32_t apl, float h, float4* __restrict__ pos32, int4* __restrict__ rec,
                uint2* __restrict__ recf, int4* __restrict__ recb, float4* __restrict__ keys,
-               float4* __restrict__ bbox, int32_t* err, const unsigned* __restrict__ gate,
+               float4* __restrict__ bbox, int32_t* err, const unsigned* gate,
                unsigned* counter) {
     chain_wait();
     if (gate && *gate == 0u) return;
@@ -308,7 +308,7 @@ __device__ __forceinline__ bool box_overlap(float qmnx, float qmny, float qmnz, 
 // Boxes of the super-blocks of 32 blocks, after the blocks' own boxes (stored
 // like tree nodes: min xyz, max x), (max y, max z, 0, 0)): one warp each.
 __global__ void __launch_bounds__(256)
-    k_md_super_boxes(int32_t nblocks, float4* __restrict__ bbox, const unsigned* __restrict__ gate) {
+    k_md_super_boxes(int32_t nblocks, float4* bbox, const unsigned* gate) {
     chain_wait();
     if (gate && *gate == 0u) return;
     const int lane = threadIdx.x & 31;
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256)
     const int32_t b = sb * 32 + lane;
     float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
     if (b < nblocks) {
-        const float4 p = __ldg(&bbox[2 * (int64_t)b]), q = __ldg(&bbox[2 * (int64_t)b + 1]);
+        const float4 p = bbox[2 * (int64_t)b], q = bbox[2 * (int64_t)b + 1];
         v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w; v[4] = q.x; v[5] = q.y;
     }
 #pragma unroll
@@ -402,15 +402,15 @@ __device__ __forceinline__ bool gap_ok(const OwnBox& o, const float4& a, const f
 // Shared memory: two buffers of fcap entries (BFS frontiers, or candidate
 // super-blocks and blocks) and the union (upow2).
 __global__ void __launch_bounds__(kBlock, 4)
-    k_md_block_union(const float4* __restrict__ keys, const float4* __restrict__ bbox,
-                     int32_t nblocks, int32_t tree, const float4* __restrict__ pos,
+    k_md_block_union(const float4* keys, const float4* bbox,
+                     int32_t nblocks, int32_t tree, const float4* pos,
                      const int32_t* __restrict__ sid,
                      int32_t n, int32_t nL, int32_t apl, float hq, float rl, int32_t fcap,
                      int32_t ucap, int32_t upow2, int32_t* __restrict__ ulist,
                      int32_t* __restrict__ ucount,
                      uint16_t* __restrict__ llist_leaf, int32_t* __restrict__ lcount_leaf,
                      int32_t lcap_leaf, int32_t* err, int32_t* diag, int32_t sizing,
-                     unsigned* pressure, const unsigned* __restrict__ gate, int32_t candidates) {
+                     unsigned* pressure, const unsigned* gate, int32_t candidates) {
     chain_wait();
     if (gate && *gate == 0u) return;
     extern __shared__ int32_t smem[];
@@ -473,8 +473,8 @@ __global__ void __launch_bounds__(kBlock, 4)
         for (int32_t base = 0; base < nsb; base += kBlock) {
             const int32_t s = base + tid;
             const bool keep = s < nsb && box_overlap(u0, u1, u2, u3, u4, u5,
-                                                     __ldg(&bbox[2 * ((int64_t)nblocks + s)]),
-                                                     __ldg(&bbox[2 * ((int64_t)nblocks + s) + 1]));
+                                                     bbox[2 * ((int64_t)nblocks + s)],
+                                                     bbox[2 * ((int64_t)nblocks + s) + 1]);
             ncs += block_compact(keep, s, csb, ncs, fcap, s_w);
         }
         int32_t ncb = 0;
@@ -483,8 +483,8 @@ __global__ void __launch_bounds__(kBlock, 4)
             const int32_t k = base + tid;
             const int32_t b = direct ? k : k < ks ? csb[k >> 5] * 32 + (k & 31) : nblocks;
             const bool keep = b < nblocks && box_overlap(u0, u1, u2, u3, u4, u5,
-                                                         __ldg(&bbox[2 * (int64_t)b]),
-                                                         __ldg(&bbox[2 * (int64_t)b + 1]));
+                                                         bbox[2 * (int64_t)b],
+                                                         bbox[2 * (int64_t)b + 1]);
             ncb += block_compact(keep, b, cb, ncb, fcap, s_w);
         }
         if (tid == 0) {
@@ -505,8 +505,8 @@ __global__ void __launch_bounds__(kBlock, 4)
                 const int32_t k = base + j * kBlock + tid;
                 lf[j] = k < kl ? (cb[k >> lsh] << lsh) + (k & (lpb - 1)) : nL;
                 if (lf[j] < nL) {
-                    ka[j] = __ldg(&keys[2 * (int64_t)lf[j]]);
-                    kb[j] = __ldg(&keys[2 * (int64_t)lf[j] + 1]);
+                    ka[j] = keys[2 * (int64_t)lf[j]];
+                    kb[j] = keys[2 * (int64_t)lf[j] + 1];
                 }
             }
 #pragma unroll
@@ -530,8 +530,8 @@ __global__ void __launch_bounds__(kBlock, 4)
                 const int32_t e = fr[cur][k];
                 const int32_t t = e >> 1;
                 if (t < 1 || t > 2 * nL - 1) { set_error(err, ND_ERR_INTERNAL, (int32_t)blockIdx.x); continue; }
-                const float4 a = __ldg(&keys[2 * (int64_t)(t - 1)]);
-                const float4 b = __ldg(&keys[2 * (int64_t)(t - 1) + 1]);
+                const float4 a = keys[2 * (int64_t)(t - 1)];
+                const float4 b = keys[2 * (int64_t)(t - 1) + 1];
                 const int32_t left = __float_as_int(b.z), skip = __float_as_int(b.w);
                 if (e & 1) {  // a left child: its skip rope is its right sibling
                     int32_t slot = atomicAdd(&s_cnt[cur ^ 1], 1);
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(kBlock, 4)
         if (lane < nown) {
             const int64_t own = first_own + k0 + lane;
             float4 oa = make_float4(1.f, 1.f, 1.f, -1.f), ob = make_float4(-1.f, -1.f, 0.f, 0.f);
-            if (own < nL) { oa = __ldg(&keys[2 * own]); ob = __ldg(&keys[2 * own + 1]); }
+            if (own < nL) { oa = keys[2 * own]; ob = keys[2 * own + 1]; }
             s_own[warp][lane] = own_box(oa, ob);
         }
         __syncwarp();
@@ -665,16 +665,16 @@ __global__ void __launch_bounds__(kBlock, 4)
         float4 na = none_a, nb4 = none_b;
         if (lane < nu) {
             const int32_t leaf = su[lane];
-            na = __ldg(&keys[2 * (int64_t)leaf]);
-            nb4 = __ldg(&keys[2 * (int64_t)leaf + 1]);
+            na = keys[2 * (int64_t)leaf];
+            nb4 = keys[2 * (int64_t)leaf + 1];
         }
         for (int32_t base = 0; base < nu; base += 32) {
             const int32_t u = base + lane;
             const float4 a = na, b = nb4;
             if (u + 32 < nu) {
                 const int32_t leaf = su[u + 32];
-                na = __ldg(&keys[2 * (int64_t)leaf]);
-                nb4 = __ldg(&keys[2 * (int64_t)leaf + 1]);
+                na = keys[2 * (int64_t)leaf];
+                nb4 = keys[2 * (int64_t)leaf + 1];
             }
             const bool pass = u < nu && gap_ok(gb, a, b, rl, rl2g);
             const unsigned m = __ballot_sync(0xffffffffu, pass);
@@ -736,21 +736,21 @@ __global__ void __launch_bounds__(kBlock, 4)
 // ensemble came out 1 ulp above r_list^2.)
 template <int APL>
 __global__ void __launch_bounds__(kBlock)
-    k_md_block_lists(const float4* __restrict__ pos, int32_t n, float rl2, float rnb2,
+    k_md_block_lists(const float4* pos, int32_t n, float rl2, float rnb2,
                      const int32_t* __restrict__ sid, const SysRow* __restrict__ sys,
                      int32_t ucap,
-                     int32_t smpos, const int32_t* __restrict__ ulist,
-                     const int32_t* __restrict__ ucount, const uint16_t* __restrict__ llist_leaf,
-                     const int32_t* __restrict__ lcount_leaf, int32_t lcap_leaf, int32_t lcap,
+                     int32_t smpos, const int32_t* ulist,
+                     const int32_t* ucount, const uint16_t* llist_leaf,
+                     const int32_t* lcount_leaf, int32_t lcap_leaf, int32_t lcap,
                      uint16_t* __restrict__ llist, int32_t* __restrict__ ncount, int32_t* err,
                      int32_t* diag, int32_t sizing, unsigned* pressure,
-                     const unsigned* __restrict__ gate) {
+                     const unsigned* gate) {
     chain_wait();
     if (gate && *gate == 0u) return;
     extern __shared__ float4 spos[];
     const int32_t blk = (int32_t)blockIdx.x;
-    const int32_t* __restrict__ U = ulist + (int64_t)blk * ucap;
-    const int32_t nu = min(__ldg(&ucount[blk]), ucap);
+    const int32_t* U = ulist + (int64_t)blk * ucap;
+    const int32_t nu = min(ucount[blk], ucap);
     {
         // four positions per thread in flight: their leaf indices, then the
         // positions
@@ -760,13 +760,13 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int32_t kk = k + j * kBlock;
-                lf[j] = kk < m ? __ldg(&U[kk / APL]) : 0;
+                lf[j] = kk < m ? U[kk / APL] : 0;
             }
             float4 r[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int32_t kk = k + j * kBlock;
-                if (kk < m) r[j] = __ldg(&pos[(int64_t)lf[j] * APL + (kk % APL)]);
+                if (kk < m) r[j] = pos[(int64_t)lf[j] * APL + (kk % APL)];
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -781,12 +781,12 @@ __global__ void __launch_bounds__(kBlock)
     const bool valid = i < n;
     const int64_t ii = valid ? i : (int64_t)blk * kBlock;
     const int64_t own = ii / APL;
-    const float4 p = __ldg(&pos[ii]);
-    const int32_t nc = valid ? min(__ldg(&lcount_leaf[own]), lcap_leaf) : 0;
+    const float4 p = pos[ii];
+    const int32_t nc = valid ? min(lcount_leaf[own], lcap_leaf) : 0;
     // candidate entries eight at a time (a leaf's list starts on a 16-byte
     // boundary: lcap_leaf is a multiple of 8), the next eight loaded while the
     // current ones are tested
-    const uint4* __restrict__ C = reinterpret_cast<const uint4*>(llist_leaf + own * lcap_leaf);
+    const uint4* C = reinterpret_cast<const uint4*>(llist_leaf + own * lcap_leaf);
     uint16_t* __restrict__ L = llist + (int64_t)blk * list_block(lcap);
     const int32_t self = (int32_t)i;
     const float nb2 = sid ? __ldg(&sys[__ldg(&sid[ii])].nk.rnb2) : rnb2;
@@ -803,10 +803,10 @@ __global__ void __launch_bounds__(kBlock)
     // the positions come from shared memory with no test
     auto walk = [&](auto staged) {
         constexpr bool ALL = decltype(staged)::value;
-        uint4 nxt = nc > 0 ? __ldg(&C[0]) : make_uint4(0u, 0u, 0u, 0u);
+        uint4 nxt = nc > 0 ? C[0] : make_uint4(0u, 0u, 0u, 0u);
         for (int32_t k0 = 0; k0 < nc; k0 += 8) {
             const uint4 cur = nxt;
-            if (k0 + 8 < nc) nxt = __ldg(&C[(k0 >> 3) + 1]);
+            if (k0 + 8 < nc) nxt = C[(k0 >> 3) + 1];
             const uint32_t cw[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
@@ -817,9 +817,9 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
                     for (int e = 0; e < APL; ++e) q[e] = spos[u * APL + e];
                 } else {
-                    const int64_t base = (int64_t)__ldg(&U[u]) * APL;
+                    const int64_t base = (int64_t)U[u] * APL;
 #pragma unroll
-                    for (int e = 0; e < APL; ++e) q[e] = __ldg(&pos[base + e]);
+                    for (int e = 0; e < APL; ++e) q[e] = pos[base + e];
                 }
 #pragma unroll
                 for (int e = 0; e < APL; ++e) {
@@ -874,13 +874,13 @@ __global__ void __launch_bounds__(kBlock)
 // lcap_leaf pairs of shared memory.
 template <int APL>
 __global__ void __launch_bounds__(kBlock)
-    k_md_leaf_lists(const float4* __restrict__ keys, const float4* __restrict__ pos, int32_t nL,
+    k_md_leaf_lists(const float4* keys, const float4* pos, int32_t nL,
                     float rl, float rl2, float rnb2, const int32_t* __restrict__ sid,
                     const SysRow* __restrict__ sys, int32_t ucap,
-                    const int32_t* __restrict__ ulist, const int32_t* __restrict__ ucount,
+                    const int32_t* ulist, const int32_t* ucount,
                     int32_t lcap_leaf, int32_t lcap, uint16_t* __restrict__ llist,
                     int32_t* __restrict__ ncount, int32_t* err, int32_t* diag, int32_t sizing,
-                    unsigned* pressure, const unsigned* __restrict__ gate) {
+                    unsigned* pressure, const unsigned* gate) {
     chain_wait();
     if (gate && *gate == 0u) return;
     extern __shared__ uint2 cand_all[];
@@ -892,15 +892,15 @@ __global__ void __launch_bounds__(kBlock)
     if (own >= nL) return;  // whole warp
     const unsigned below = (1u << lane) - 1u;
     uint2* cand = cand_all + warp * lcap_leaf;  // (union index, leaf)
-    const int32_t* __restrict__ U = ulist + (int64_t)blk * ucap;
-    const int32_t nu = min(__ldg(&ucount[blk]), ucap);
+    const int32_t* U = ulist + (int64_t)blk * ucap;
+    const int32_t nu = min(ucount[blk], ucap);
     float4 p[APL];
 #pragma unroll
-    for (int a = 0; a < APL; ++a) p[a] = __ldg(&pos[(int64_t)own * APL + a]);
+    for (int a = 0; a < APL; ++a) p[a] = pos[(int64_t)own * APL + a];
     const float nb2 = sid ? __ldg(&sys[__ldg(&sid[(int64_t)own * APL])].nk.rnb2) : rnb2;
     int32_t nc = 0;
     {
-        const OwnBox o = own_box(__ldg(&keys[2 * (int64_t)own]), __ldg(&keys[2 * (int64_t)own + 1]));
+        const OwnBox o = own_box(keys[2 * (int64_t)own], keys[2 * (int64_t)own + 1]);
         const float rl2g = rl * rl * 1.0002f;
         // the next 64 boxes are loaded while the current ones are tested
         int32_t lf[2];
@@ -909,10 +909,10 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int32_t u = base + 32 * j + lane;
-                lf[j] = u < nu ? __ldg(&U[u]) : -1;
+                lf[j] = u < nu ? U[u] : -1;
                 if (u < nu) {
-                    ka[j] = __ldg(&keys[2 * (int64_t)lf[j]]);
-                    kb[j] = __ldg(&keys[2 * (int64_t)lf[j] + 1]);
+                    ka[j] = keys[2 * (int64_t)lf[j]];
+                    kb[j] = keys[2 * (int64_t)lf[j] + 1];
                 }
             }
         };
@@ -955,7 +955,7 @@ __global__ void __launch_bounds__(kBlock)
             if (c < total) {
                 const uint2 e = cand[c / APL];
                 li[k] = (int32_t)e.x * APL + c % APL;
-                q[k] = __ldg(&pos[(int64_t)e.y * APL + c % APL]);
+                q[k] = pos[(int64_t)e.y * APL + c % APL];
             }
         }
 #pragma unroll
@@ -1425,16 +1425,16 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
     // join the warp reductions (measure) and the block vote (step)
     if (!valid) i = a.n - 1;
     // the atom's own loads go first, beside the staging's
-    const int4 ri = __ldg(&a.rec_in[i]);
-    const uint2 fi = __ldg(&a.recf_in[i]);
-    const int32_t cpk = valid ? __ldg(&a.ncount[i]) : 0;
-    const int32_t* __restrict__ U = a.ulist + (int64_t)blk * a.ucap;
+    const int4 ri = a.rec_in[i];
+    const uint2 fi = a.recf_in[i];
+    const int32_t cpk = valid ? a.ncount[i] : 0;
+    const int32_t* U = a.ulist + (int64_t)blk * a.ucap;
     // stage the block's union: record of atom (leaf * apl + e) at u * apl + e,
     // up to the shared-memory capacity; larger unions read the rest from L2
     {
         // four records per thread in flight: their leaf indices, then the
         // records (apl is a power of two)
-        const int32_t nu = min(__ldg(&a.ucount[blk]), a.ucap);
+        const int32_t nu = min(a.ucount[blk], a.ucap);
         const int32_t m = min(nu * a.apl, a.smrec);
         const int32_t lsh = __ffs(a.apl) - 1, emask = a.apl - 1;
         constexpr int32_t NT = APB * TPA;
@@ -1443,13 +1443,13 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int32_t kk = k + j * NT;
-                lf[j] = kk < m ? __ldg(&U[kk >> lsh]) : 0;
+                lf[j] = kk < m ? U[kk >> lsh] : 0;
             }
             int4 r[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int32_t kk = k + j * NT;
-                if (kk < m) r[j] = __ldg(&a.rec_in[((int64_t)lf[j] << lsh) + (kk & emask)]);
+                if (kk < m) r[j] = a.rec_in[((int64_t)lf[j] << lsh) + (kk & emask)];
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -1486,8 +1486,8 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
     }
     // near entries (words 0, 1, ...) and the others (from the last word down)
     const int32_t nn = list_near(cpk), nf = cpk >> 16;
-    const uint16_t* __restrict__ L = a.llist + (int64_t)blk * list_block(a.lcap);
-    const uint2* __restrict__ LW = reinterpret_cast<const uint2*>(L) + tid;
+    const uint16_t* L = a.llist + (int64_t)blk * list_block(a.lcap);
+    const uint2* LW = reinterpret_cast<const uint2*>(L) + tid;
     auto near_entry = [&](int32_t s) -> int32_t { return L[near_at(s, tid)]; };
     auto far_entry = [&](int32_t s) -> int32_t { return L[far_at(s, tid, a.lcap)]; };
     const int32_t lsh = __ffs(a.apl) - 1, emask = a.apl - 1;
@@ -1505,11 +1505,11 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
         constexpr bool ALL = decltype(staged)::value;
         auto fetch = [&](int32_t li) -> int4 {
             if (ALL || li < a.smrec) return srec[li];
-            return __ldg(&a.rec_in[((int64_t)__ldg(&U[li >> lsh]) << lsh) + (li & emask)]);
+            return a.rec_in[((int64_t)U[li >> lsh] << lsh) + (li & emask)];
         };
         // fine bits of a union entry's record (near pairs only)
         auto fine = [&](int32_t li) -> uint2 {
-            return __ldg(&a.recf_in[((int64_t)__ldg(&U[li >> lsh]) << lsh) + (li & emask)]);
+            return a.recf_in[((int64_t)U[li >> lsh] << lsh) + (li & emask)];
         };
         if constexpr (MEASURE || BATCH) {
             // near entries of this thread's slice, the next index loaded ahead
@@ -1527,9 +1527,9 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             // near entries two at a time (packed), half a word each, the next
             // word loaded ahead; an odd last one alone
             int32_t s = 0, w = 0;
-            uint2 cur = nn > 0 ? __ldg(&LW[0]) : make_uint2(0u, 0u), nxt = cur;
+            uint2 cur = nn > 0 ? LW[0] : make_uint2(0u, 0u), nxt = cur;
             for (; s + 1 < nn; s += 2) {
-                if ((s & 2) == 0 && s + 4 < nn) nxt = __ldg(&LW[++w * kBlock]);
+                if ((s & 2) == 0 && s + 4 < nn) nxt = LW[++w * kBlock];
                 const int32_t la = cur.x & 0xffffu, lb = cur.x >> 16;
                 const int4 ra = fetch(la), rb = fetch(lb);
                 const uint2 fa = fine(la), fb = fine(lb);
@@ -1569,8 +1569,8 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             [[maybe_unused]] uint64_t fx2 = 0, fy2 = 0, fz2 = 0;  // packed (0.0f, 0.0f)
             [[maybe_unused]] float gx = 0.f, gy = 0.f, gz = 0.f;  // measure pass: odd entries
             int32_t s = 0;
-            const uint2* __restrict__ lw = LW + (list_words(a.lcap) - 1) * kBlock;
-            uint2 cur = nf > 0 ? __ldg(lw) : make_uint2(0u, 0u);
+            const uint2* lw = LW + (list_words(a.lcap) - 1) * kBlock;
+            uint2 cur = nf > 0 ? *lw : make_uint2(0u, 0u);
             for (; s + 4 <= nf; s += 4) {
                 int4 rj[4];
                 rj[0] = fetch((int32_t)(cur.x & 0xffffu));
@@ -1578,7 +1578,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
                 rj[2] = fetch((int32_t)(cur.y & 0xffffu));
                 rj[3] = fetch((int32_t)(cur.y >> 16));
                 lw -= kBlock;
-                if (s + 4 < nf) cur = __ldg(lw);
+                if (s + 4 < nf) cur = *lw;
                 if constexpr (MEASURE) {
                     // even entries into (fx, fy, fz), odd ones into (gx, gy, gz),
                     // as the two halves of the packed form
@@ -1681,7 +1681,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             fz = __fadd_rn(nacc.zh, nacc.zl);
         }
     };
-    if (min(__ldg(&a.ucount[blk]), a.ucap) * a.apl <= a.smrec)
+    if (min(a.ucount[blk], a.ucap) * a.apl <= a.smrec)
         pairs(std::true_type{});
     else
         pairs(std::false_type{});
@@ -1735,7 +1735,7 @@ __global__ void __launch_bounds__(kBlock * TPA / SPLIT, TPA == 1 ? 4 : 1) k_md_s
             wv[d] = a.w[d][i];
             xv[d] = a.x[d][i];
         }
-        const int4 rb = __ldg(&a.rec_build[i]);
+        const int4 rb = a.rec_build[i];
         const double imv = MASS ? a.im[i] : 1.0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {

@@ -99,13 +99,13 @@ struct StepArgs {
     int32_t first;     // the first step after an upload (a half kick only)
     int32_t has_mass;  // im holds inverse masses (else all masses are 1)
     int32_t smrec;  // union records staged in shared memory (the rest read from global)
-    const int32_t* __restrict__ ulist;
-    const int32_t* __restrict__ ucount;
-    const uint16_t* __restrict__ llist;
-    const int32_t* __restrict__ ncount;
-    const int4* __restrict__ rec_in;
+    const int32_t* ulist;
+    const int32_t* ucount;
+    const uint16_t* llist;
+    const int32_t* ncount;
+    const int4* rec_in;
     int4* __restrict__ rec_out;
-    const uint2* __restrict__ recf_in;  // fine bits of the records
+    const uint2* recf_in;  // fine bits of the records
     uint2* __restrict__ recf_out;
     double* x[3];
     double* w[3];
@@ -113,7 +113,7 @@ struct StepArgs {
     float4* __restrict__ f_out;
     double* __restrict__ v_out[3];  // measure mode: integer-step velocity
     double* __restrict__ acc;       // measure mode: [0] potential, [1] kinetic
-    const int4* __restrict__ rec_build;     // records at the last rebuild
+    const int4* rec_build;     // records at the last rebuild
     unsigned long long* __restrict__ diag;  // [0] atom-steps moved > skin/2 since the build
     int32_t* err;
     float half_skin2u;  // (skin/2)^2 in fixed-point units
