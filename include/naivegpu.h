@@ -422,7 +422,10 @@ nd_status nd_collect_objects(nd_ctx* ctx, const nd_collector* collector, uint64_
 /*
  * Forces and energy of a configuration with the library's own neighbour search
  * (spatial-order leaf BVH at radius p->cutoff): the fused hot-path force kernel
- * run once.  Same physics and outputs as nd_forces_pairs.
+ * run once.  Same physics and outputs as nd_forces_pairs.  The context keeps up
+ * to 512 MB of the call's device buffers for the next such call; nd_md_destroy
+ * and nd_adj_destroy of any of its engines, an allocation of the library that
+ * fails, and nd_ctx_destroy give them back.
  */
 nd_status nd_forces(nd_ctx* ctx, const nd_md_params* p, int32_t n, const double* x,
                     const double* q, float* force, double* energy);
@@ -442,6 +445,7 @@ nd_status nd_md_create(nd_ctx* ctx, const nd_md_params* p, int32_t n, const doub
 /* Same, from device arrays (x, v: N x 3 FP64; q, m: N FP64 or NULL). */
 nd_status nd_md_create_dev(nd_ctx* ctx, const nd_md_params* p, int32_t n, const double* x,
                            const double* v, const double* q, const double* m, nd_md** out);
+/* Frees the engine's device memory, and what the context kept of nd_forces. */
 nd_status nd_md_destroy(nd_md* md);
 /* Advance `steps` steps; enqueued on the context stream (captured CUDA graphs of
  * one rebuild window).  Does not synchronise. */

@@ -775,11 +775,8 @@ nd_status adj_destroy(AdjEngine* A) {
     DevBuf* bufs[] = {&A->ckpt, &A->perms, &A->codes, &A->statics, &A->traj, &A->trajrec, &A->recK, &A->lam, &A->lam_tmp, &A->g4[0],
                       &A->g4[1], &A->gpart, &A->xK, &A->hatom, &A->hist, &A->target, &A->cb,
                       &A->scal, &A->outs, &A->flags};
-    for (DevBuf* b : bufs) {
-        if (!b->p) continue;
-        if (A->m && A->m->sub.pool) A->m->sub.pool->put(*b);
-        else cudaFree(b->p);
-    }
+    for (DevBuf* b : bufs)
+        if (b->p) cudaFree(b->p);
     if (A->m) md_destroy(A->m);
     delete A;
     return ND_OK;

@@ -831,6 +831,7 @@ nd_status nd_md_destroy(nd_md* md) {
         nd::set_device(&md->ctx->c);
         md->ctx->engines.erase(md);
         nd::md_destroy(md->e);
+        md->ctx->pool.clear();
     }
     delete md;
     return ND_OK;
@@ -989,6 +990,7 @@ nd_status nd_adj_destroy(nd_adj* a) {
         nd::set_device(&a->ctx->c);
         a->ctx->adjoints.erase(a);
         nd::adj_destroy(a->e);
+        a->ctx->pool.clear();
     }
     delete a;
     return ND_OK;

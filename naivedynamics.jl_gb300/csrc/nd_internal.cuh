@@ -140,13 +140,14 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
-// Device buffers of destroyed engines, kept by their context for the next
-// engine: an engine holds about 35 of them, and a call that makes one for
-// itself (forces(), simulate_ with a log) spent a third of its time in
-// cudaMalloc and cudaFree.  At most kMost blocks and kBytes bytes wait; they
-// are freed with the context, or when an allocation fails.  A buffer comes
-// here only after its stream was synchronised, and one context's engines share
-// one stream.
+// Device buffers of the engine that a call made for itself (forces()), kept by
+// the context for the next such call: an engine holds about 35 of them, and the
+// call spent a third of its time in cudaMalloc and cudaFree.  At most kMost
+// blocks and kBytes bytes wait.  They go back to the device when the caller
+// destroys an engine (whose own buffers are freed at once: it may want the
+// room), when an allocation of the library fails, and with the context.  A
+// buffer comes here only after its stream was synchronised, and one context's
+// engines share one stream.
 class BufPool {
 public:
     bool take(DevBuf& b, size_t bytes);
@@ -283,7 +284,8 @@ nd_status md_create(Ctx* parent, const nd_md_params* p, int32_t n, const double*
 // Forces (host, N x 3) and potential energy (may be null) of a configuration.
 nd_status md_forces(Ctx* parent, const nd_md_params* p, int32_t n, const double* x,
                     const double* q, float* force, double* energy);
-nd_status md_destroy(MDEngine* m);
+// keep: its buffers go to the context's idle ones instead of to the device.
+nd_status md_destroy(MDEngine* m, bool keep = false);
 nd_status md_create_batch(Ctx* parent, const nd_md_params* p, int32_t nsys, const nd_system* sys,
                           const double* x, const double* v, const double* q, const double* mass,
                           bool host, MDEngine** out);

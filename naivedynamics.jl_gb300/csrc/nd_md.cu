@@ -2583,7 +2583,6 @@ static nd_status md_size_lists(MDEngine* m) {
     return sync_and_check(c, "md first build");
 }
 
-nd_status md_destroy(MDEngine* m);
 
 // Copy x, v (N x 3), q, m (N) from host or device memory into state set 0 in
 // the caller's order and reset the step bookkeeping.
@@ -2961,7 +2960,7 @@ done:
     return result;
 }
 
-nd_status md_destroy(MDEngine* m) {
+nd_status md_destroy(MDEngine* m, bool keep) {
     if (!m) return ND_OK;
     if (m->graph_main) cudaGraphExecDestroy(m->graph_main);
     if (m->graph_first) cudaGraphExecDestroy(m->graph_first);
@@ -2976,7 +2975,7 @@ nd_status md_destroy(MDEngine* m) {
     if (m->sub.stream) cudaStreamSynchronize(m->sub.stream);
     for (DevBuf* b : bufs) {
         if (!b->p) continue;
-        if (m->sub.pool) m->sub.pool->put(*b);
+        if (keep && m->sub.pool) m->sub.pool->put(*b);
         else cudaFree(b->p);
     }
     if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
@@ -3143,7 +3142,7 @@ nd_status md_forces(Ctx* parent, const nd_md_params* p, int32_t n, const double*
     if (st == ND_OK && energy) *energy = pot;
     if (st) parent->last_error = c->last_error;
     parent->launches += c->launches;
-    md_destroy(m);
+    md_destroy(m, true);
     return st;
 }
 
@@ -3239,32 +3238,34 @@ nd_status md_list_pairs(MDEngine* m, int32_t* pi, int32_t* pj, uint8_t* near, in
     Ctx* c = &m->sub;
     nd_status st = sync_and_check(c, "md list pairs");
     if (st) return st;
-    int32_t *dpi = nullptr, *dpj = nullptr;
-    uint8_t* dn = nullptr;
-    unsigned long long* cur = nullptr;
     const size_t k = (size_t)std::max<int64_t>(cap, 1);
-    cudaError_t e = cudaMalloc(&dpi, k * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&dpj, k * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&dn, k);
-    if (e == cudaSuccess) e = cudaMalloc(&cur, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemsetAsync(cur, 0, sizeof(unsigned long long), c->stream);
+    DevBuf bi, bj, bn, cur;
+    st = ensure(c, bi, k * sizeof(int32_t));
+    if (st == ND_OK) st = ensure(c, bj, k * sizeof(int32_t));
+    if (st == ND_OK) st = ensure(c, bn, k);
+    if (st == ND_OK) st = ensure(c, cur, sizeof(unsigned long long));
     unsigned long long total = 0;
-    if (e == cudaSuccess) {
+    cudaError_t e = cudaSuccess;
+    if (st == ND_OK) {
+        e = cudaMemsetAsync(cur.p, 0, sizeof(unsigned long long), c->stream);
         k_md_list_pairs<<<(unsigned)cdiv(m->n, 256), 256, 0, c->stream>>>(
             (const int32_t*)m->ncount.p, (const uint16_t*)m->llist.p, (const int32_t*)m->ulist.p,
-            m->set[m->cur].orig, m->n, m->apl, m->ucap, m->lcap, dpi, dpj, dn, cap, cur);
+            m->set[m->cur].orig, m->n, m->apl, m->ucap, m->lcap, (int32_t*)bi.p, (int32_t*)bj.p,
+            (uint8_t*)bn.p, cap, (unsigned long long*)cur.p);
         c->launches++;
-        e = cudaMemcpyAsync(&total, cur, sizeof(total), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&total, cur.p, sizeof(total), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+        const int64_t got = std::min<int64_t>((int64_t)total, cap);
+        if (e == cudaSuccess && got > 0 && pi)
+            e = cudaMemcpy(pi, bi.p, got * sizeof(int32_t), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && got > 0 && pj)
+            e = cudaMemcpy(pj, bj.p, got * sizeof(int32_t), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess && got > 0 && near)
+            e = cudaMemcpy(near, bn.p, got, cudaMemcpyDeviceToHost);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    const int64_t got = std::min<int64_t>((int64_t)total, cap);
-    if (e == cudaSuccess && got > 0 && pi) e = cudaMemcpy(pi, dpi, got * sizeof(int32_t), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && got > 0 && pj) e = cudaMemcpy(pj, dpj, got * sizeof(int32_t), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && got > 0 && near) e = cudaMemcpy(near, dn, got, cudaMemcpyDeviceToHost);
-    cudaFree(dpi);
-    cudaFree(dpj);
-    cudaFree(dn);
-    cudaFree(cur);
+    for (DevBuf* b : {&bi, &bj, &bn, &cur}) cudaFree(b->p);
+    if (st) return st;
     if (e != cudaSuccess) return cuda_fail(c, e, "md list pairs");
     m->parent->launches += c->launches;
     c->launches = 0;
