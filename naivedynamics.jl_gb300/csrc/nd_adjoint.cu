@@ -821,11 +821,8 @@ nd_status adj_create(Ctx* parent, const nd_md_params* p, int32_t n, const double
     const int static_sm = (int)(sizeof(float) * 5 * kBlock * (kAdjTPA - 1)) + 2048;
     A->smrec = std::max(0, std::min(m->ucap_sm * m->apl, (maxsm - static_sm) / 32));
     A->rev_smem = 32 * (size_t)A->smrec;
-    cudaError_t e = cudaFuncSetAttribute((const void*)k_adj_reverse<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->rev_smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute((const void*)k_adj_reverse<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A->rev_smem);
+    cudaError_t e = raise_smem_limit((const void*)k_adj_reverse<true>, maxsm);
+    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_adj_reverse<false>, maxsm);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->cap_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { st = cuda_fail(parent, e, "adjoint setup"); adj_destroy(A); return st; }
     if ((st = ensure(c, A->ckpt, A->ckpt_bytes * A->nseg)) ||

@@ -1903,7 +1903,7 @@ static nd_status md_alloc(MDEngine* m) {
     return ND_OK;
 }
 
-static cudaError_t raise_smem_limit(const void* fn, int maxsm) {
+cudaError_t raise_smem_limit(const void* fn, int maxsm) {
     cudaFuncAttributes fa{};
     cudaError_t e = cudaFuncGetAttributes(&fa, fn);
     if (e != cudaSuccess) return e;

@@ -224,6 +224,11 @@ __host__ __device__ inline int64_t list_block(int32_t lcap) {
     return (int64_t)list_words(lcap) * 4 * kBlock;
 }
 
+// Raises kernel fn's dynamic shared memory limit to the device's maximum (maxsm)
+// less its static shared memory: the limit belongs to the process, so it must not
+// follow the size of one engine.
+cudaError_t raise_smem_limit(const void* fn, int maxsm);
+
 // Rebuild of the neighbour lists (re-sort or refit; see nd_md.cu).
 nd_status md_rebuild(MDEngine* m, int kind, int rec = -1, unsigned* counter = nullptr,
                      bool sizing = false, const unsigned* gate = nullptr, bool opens = false);
