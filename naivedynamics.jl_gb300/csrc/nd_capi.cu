@@ -755,7 +755,7 @@ nd_status nd_forces(nd_ctx* h, const nd_md_params* p, int32_t n, const double* x
     nd_status st = nd::set_device(c);
     if (st) return st;
     nd_md_params pp = *p;
-    if (pp.rebuild_every <= 0) pp.rebuild_every = 1;
+    pp.rebuild_every = 1;  // no step is taken
     if (!(pp.dt > 0)) pp.dt = 1.0;
     return nd::md_forces(c, &pp, n, x, q, force, energy);
 }

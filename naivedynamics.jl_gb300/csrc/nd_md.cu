@@ -145,7 +145,7 @@ __global__ void k_md_init_scalars(const double* __restrict__ q_in, const double*
 // kCtlWindow windows begun, kCtlPressure a list near its capacity since the
 // last re-sort, kCtlDecision the last window's choice, kCtlResorts and
 // kCtlRefits rebuilds done at the start of windows; from kCtlVotes on one word
-// per step of a window: the step's vote for an early refit.
+// per checked step of a window: the step's vote for an early refit.
 constexpr int kCtlEarly = 2, kCtlWindow = 3, kCtlPressure = 4, kCtlDecision = 5, kCtlResorts = 6,
               kCtlRefits = 7, kCtlVotes = 8;
 
@@ -1851,10 +1851,13 @@ __global__ void k_pair_forces(const double* __restrict__ x, const double* __rest
 // ------------------------------------------------------------- engine
 
 
-// Steps of a window that vote, and the bytes of the control array.
-static int32_t md_votes(const MDEngine* m) { return m->p.rebuild_every; }
+// Steps of a window that vote (0, M, 2M, ... but not the last, M = check_every),
+// and the bytes of the control array.
+static int32_t md_votes(const MDEngine* m) {
+    return m->p.rebuild_every > 1 ? (m->p.rebuild_every - 2) / m->check_every + 1 : 0;
+}
 static size_t md_ctl_bytes(const MDEngine* m) {
-    return sizeof(unsigned) * (size_t)(kCtlVotes + md_votes(m));
+    return sizeof(unsigned) * ((size_t)kCtlVotes + (size_t)md_votes(m));
 }
 
 static nd_status md_alloc(MDEngine* m) {
@@ -2436,7 +2439,7 @@ static nd_status md_steps(MDEngine* m, int32_t k, int32_t pos0, bool capture = f
         const int32_t p = (pos0 + s) % R;
         const bool check = p != R - 1 && p % m->check_every == 0;
         StepArgs a = md_step_args(m, m->rc);
-        a.vote = check ? ctl_word(m, kCtlVotes + p) : nullptr;
+        a.vote = check ? ctl_word(m, kCtlVotes + p / m->check_every) : nullptr;
         a.unchecked = !check && p != R - 1 ? 1 : 0;
         if (ev) cudaEventRecord(ev[2 * s], c->stream);
         launch_step<0>(m, a, m->first);
