@@ -262,7 +262,8 @@ typedef struct {
 } nd_pair;
 
 /* Receives a list's length and returns host memory for that many entries (NULL:
- * give up, ND_ERR_NOMEM).  Called once, on the calling thread, inside the call. */
+ * give up, ND_ERR_NOMEM, no output of the call written).  Called once, on the
+ * calling thread, inside the call. */
 typedef nd_pair* (*nd_pair_alloc)(int64_t count, void* user);
 
 /*

@@ -637,6 +637,21 @@ nd_status nd_leaf_pair_list(nd_ctx* h, const float* xyz, const nd_bvh_spec* s, i
     if (have > 0 &&
         (st = nd::write_pair_triples(c, t, r, r2, total_dev, have, (int32_t*)c->pairs_i.p)))
         return st;
+    if ((st = nd::sync_and_check(c, "pair list"))) return st;
+    int64_t total = 0;
+    memcpy(&total, c->h_err + 4, sizeof(total));
+    // nothing of the caller's is written before it has given the list's memory
+    nd_pair* out = alloc(total, user);
+    if (!out && total > 0) {
+        c->last_error = "no memory for the pair list";
+        return ND_ERR_NOMEM;
+    }
+    *count = total;
+    if (total > have) {
+        if ((st = nd::ensure(c, c->pairs_i, sizeof(nd_pair) * (size_t)total))) return st;
+        if ((st = nd::write_pair_triples(c, t, r, r2, total_dev, total, (int32_t*)c->pairs_i.p)))
+            return st;
+    }
     cudaError_t e = cudaSuccess;
     if (keys && nkeys > 0) {
         nd::root_overwrite(c, t.keys, nL);
@@ -656,23 +671,9 @@ nd_status nd_leaf_pair_list(nd_ctx* h, const float* xyz, const nd_bvh_spec* s, i
         e = cudaMemcpyAsync(position, c->xyz.p, 3 * nb, cudaMemcpyDeviceToHost, c->stream);
     }
     if (e != cudaSuccess) return nd::cuda_fail(c, e, "pair list download");
-    if ((st = nd::sync_and_check(c, "pair list"))) return st;
-    int64_t total = 0;
-    memcpy(&total, c->h_err + 4, sizeof(total));
-    nd_pair* out = alloc(total, user);
-    if (!out && total > 0) {
-        c->last_error = "no memory for the pair list";
-        return ND_ERR_NOMEM;
-    }
-    *count = total;
-    if (total == 0) return ND_OK;
-    if (total > have) {
-        if ((st = nd::ensure(c, c->pairs_i, sizeof(nd_pair) * (size_t)total))) return st;
-        if ((st = nd::write_pair_triples(c, t, r, r2, total_dev, total, (int32_t*)c->pairs_i.p)))
-            return st;
-    }
-    e = cudaMemcpyAsync(out, c->pairs_i.p, sizeof(nd_pair) * (size_t)total, cudaMemcpyDeviceToHost,
-                        c->stream);
+    if (total > 0)
+        e = cudaMemcpyAsync(out, c->pairs_i.p, sizeof(nd_pair) * (size_t)total,
+                            cudaMemcpyDeviceToHost, c->stream);
     if (e != cudaSuccess) return nd::cuda_fail(c, e, "pair list download");
     return nd::sync_and_check(c, "pair list");
 }

@@ -146,9 +146,9 @@ def _pair_list(ctx, x, spec, order, criterion=ND_CRIT_SQUARED, kept=None, tree=N
             if into is None:
                 out = np.empty(count, PAIR_DTYPE)
             else:
-                into.resize(count, refcheck=False)
                 if not into.flags.writeable:
                     raise ValueError("neighborlist is read-only")
+                into.resize(count, refcheck=False)
                 out = into
         except (MemoryError, ValueError) as e:
             got.append(e)
