@@ -1026,9 +1026,14 @@ __device__ __forceinline__ float leaf_slack(const Node& a) {
 // Whether two leaves whose key boxes (atom boxes -/+ r/2) overlap can hold a
 // pair within r: the per-axis gaps of the atom boxes (key-box gap + r, each
 // lowered by the rounding slack of the -/+ r/2) must have a Euclidean norm
-// below r (r2g = r^2 widened a little: a filter, the distance test decides).
+// below r (r2g = gap_limit: a filter, the distance test decides).
 // Boxes that overlap on every axis only bound each gap by r; this drops the
 // leaf pairs diagonally apart.
+__device__ __forceinline__ float gap_limit(float r, float r2) {
+    // r^2 or the threshold on d^2 (above r^2 where r^2 underflows), widened a
+    // little, at the bottom of the range by a few of its steps
+    return fmaf(fmaxf(r * r, r2), 1.0001f, 1e-44f);
+}
 __device__ __forceinline__ bool leaf_gap_ok(const Node& a, const Node& b, float r, float r2g,
                                             float slack) {
     const float gx = fmaxf(fmaxf(a.mnx - b.mxx, b.mnx - a.mxx) + r - slack, 0.0f);
@@ -1218,7 +1223,7 @@ __global__ void __launch_bounds__(128)
     }
     const unsigned below = (1u << lane) - 1u;
     const Node ql = load_node(keys, q + 1);
-    const float slack = leaf_slack(ql), r2g = r * r * 1.0001f;
+    const float slack = leaf_slack(ql), r2g = gap_limit(r, r2);
     if constexpr (APL > 0) {
         int32_t* queue = squeue[w];
         float4 qa[APL];
@@ -1448,7 +1453,7 @@ __global__ void __launch_bounds__(128, 6)
                  float r, float r2, unsigned long long* cursor, int64_t cap, int32_t* pi,
                  int32_t* pj, float* pd, int32_t* err) {
     constexpr int APL = 4;
-    const float r2g = r * r * 1.0001f;
+    const float r2g = gap_limit(r, r2);
     __shared__ int2 sbij[4][kWarpBuf];
     __shared__ float sbd[4][kWarpBuf];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1660,7 +1665,7 @@ __global__ void __launch_bounds__(128, 6)
     __shared__ PairBuf sbuf[4];
     __shared__ float4 sbox[4][2][64];  // leaf boxes of the task's groups, their slack beside
     __shared__ int2 squeue[4][64];
-    const float r2g = r * r * 1.0001f;  // the gap test is a filter: the distance test decides
+    const float r2g = gap_limit(r, r2);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     const int64_t ntask = (int64_t)*tcount;
