@@ -1956,8 +1956,8 @@ nd_status write_pair_triples(Ctx* c, const TreeBuffers& t, float r, float r2,
 
 __global__ void k_unpack_positions(const float4* __restrict__ pos4, int32_t n,
                                    float* __restrict__ out) {
-    const int32_t m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < 3 * n) out[m] = reinterpret_cast<const float*>(pos4)[4 * (m / 3) + m % 3];
+    const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (m < 3 * (int64_t)n) out[m] = reinterpret_cast<const float*>(pos4)[4 * (m / 3) + m % 3];
 }
 
 void unpack_positions(Ctx* c, const float4* pos4, int32_t n, float* out) {
