@@ -269,7 +269,7 @@ template <int ITEMS>
 __global__ void __launch_bounds__(1024)
     k_small_order(const float* __restrict__ xyz, int32_t n, int32_t order, float binwidth,
                   CodeFrame frame, uint32_t* keys, int32_t* vals, int passes, int32_t* err) {
-    __shared__ uint16_t s_cnt[32][RS_BINS];
+    __shared__ __align__(4) uint16_t s_cnt[32][RS_BINS];
     __shared__ uint32_t s_x[1024 * ITEMS];
     __shared__ uint32_t s_part[4][RS_BINS];
     __shared__ uint32_t s_warp[8];
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256 * GROUPS)
               uint32_t* __restrict__ kout, int32_t* __restrict__ vout, int32_t n, int shift,
               const uint32_t* __restrict__ hist, uint32_t* __restrict__ hist_next, int32_t ntiles) {
     constexpr int ITEMS = 4, THREADS = 256 * GROUPS, W = 8 * GROUPS, TILE = THREADS * ITEMS;
-    __shared__ uint16_t s_cnt[W][RS_BINS];
+    __shared__ __align__(4) uint16_t s_cnt[W][RS_BINS];
     __shared__ uint32_t s_pre[GROUPS][RS_BINS], s_tot[GROUPS][RS_BINS], s_part[GROUPS][RS_BINS];
     __shared__ uint32_t s_base[RS_BINS], s_warp[8];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5, d = t & 255, g = t >> 8;
