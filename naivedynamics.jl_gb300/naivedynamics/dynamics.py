@@ -551,8 +551,9 @@ def autotune_cache_path() -> str:
         os.path.expanduser("~"), ".cache", "naivedynamics", "autotune.json")
 
 
-# the tuner's candidate set: a cached result from another set is not reused
-TUNER_VERSION = 3
+# the tuner's candidate set and the kernels it times: a cached result of another
+# set, or of kernels whose prices have changed, is not reused
+TUNER_VERSION = 4
 
 
 def _tune_key(ctx, params: MDParams, n: int, systems, has_q: bool, has_m: bool) -> str:
