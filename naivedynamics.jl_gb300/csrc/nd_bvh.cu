@@ -1023,17 +1023,19 @@ __device__ __forceinline__ float leaf_slack(const Node& a) {
     return mag * 9.5367431640625e-7f;  // 8 * 2^-23
 }
 
+// The limit r2g of the gap filter below, computed once a launch: r^2 or the
+// threshold on d^2 (above r^2 where r^2 underflows), widened a little, at the
+// bottom of the range by a few of its steps.
+static float gap_limit(float r, float r2) {
+    return std::fma(std::fmax(r * r, r2), 1.0001f, 1e-44f);
+}
+
 // Whether two leaves whose key boxes (atom boxes -/+ r/2) overlap can hold a
 // pair within r: the per-axis gaps of the atom boxes (key-box gap + r, each
 // lowered by the rounding slack of the -/+ r/2) must have a Euclidean norm
 // below r (r2g = gap_limit: a filter, the distance test decides).
 // Boxes that overlap on every axis only bound each gap by r; this drops the
 // leaf pairs diagonally apart.
-__device__ __forceinline__ float gap_limit(float r, float r2) {
-    // r^2 or the threshold on d^2 (above r^2 where r^2 underflows), widened a
-    // little, at the bottom of the range by a few of its steps
-    return fmaf(fmaxf(r * r, r2), 1.0001f, 1e-44f);
-}
 __device__ __forceinline__ bool leaf_gap_ok(const Node& a, const Node& b, float r, float r2g,
                                             float slack) {
     const float gx = fmaxf(fmaxf(a.mnx - b.mxx, b.mnx - a.mxx) + r - slack, 0.0f);
@@ -1206,7 +1208,7 @@ template <int APL, int WRITE>
 __global__ void __launch_bounds__(128)
     k_leaf_wide(const float4* __restrict__ keys, const float4* __restrict__ gbox,
                 const float4* __restrict__ pos, int32_t nL, int32_t apl, float r, float r2,
-                int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
+                float r2g, int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
                 const int64_t* __restrict__ total, int64_t cap, int32_t* __restrict__ pi,
                 int32_t* __restrict__ pj, float* __restrict__ pd) {
     constexpr int BUF = APL > 0 && WRITE != 0 ? 32 * APL * APL : 1;
@@ -1223,7 +1225,7 @@ __global__ void __launch_bounds__(128)
     }
     const unsigned below = (1u << lane) - 1u;
     const Node ql = load_node(keys, q + 1);
-    const float slack = leaf_slack(ql), r2g = gap_limit(r, r2);
+    const float slack = leaf_slack(ql);
     if constexpr (APL > 0) {
         int32_t* queue = squeue[w];
         float4 qa[APL];
@@ -1450,10 +1452,9 @@ __device__ __forceinline__ unsigned leaf_tests16(const float4 (&qa)[4], const fl
 
 __global__ void __launch_bounds__(128, 6)
     k_leaf_warp4(const float4* __restrict__ keys, const float4* __restrict__ pos, int32_t nL,
-                 float r, float r2, unsigned long long* cursor, int64_t cap, int32_t* pi,
-                 int32_t* pj, float* pd, int32_t* err) {
+                 float r, float r2, float r2g, unsigned long long* cursor, int64_t cap,
+                 int32_t* pi, int32_t* pj, float* pd, int32_t* err) {
     constexpr int APL = 4;
-    const float r2g = gap_limit(r, r2);
     __shared__ int2 sbij[4][kWarpBuf];
     __shared__ float sbd[4][kWarpBuf];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1657,7 +1658,7 @@ __device__ __forceinline__ void pair_buf_flush(PairBuf& b, int& nb, unsigned lon
 
 __global__ void __launch_bounds__(128, 6)
     k_group_pairs(const float4* __restrict__ keys, const float4* __restrict__ gbox,
-                  const float4* __restrict__ pos, int32_t nL, float r, float r2,
+                  const float4* __restrict__ pos, int32_t nL, float r, float r2, float r2g,
                   const unsigned long long* __restrict__ tcount, int64_t tcap,
                   const int2* __restrict__ tasks, unsigned long long* ticket,
                   unsigned long long* cursor, int64_t cap, int32_t* __restrict__ pi,
@@ -1665,7 +1666,6 @@ __global__ void __launch_bounds__(128, 6)
     __shared__ PairBuf sbuf[4];
     __shared__ float4 sbox[4][2][64];  // leaf boxes of the task's groups, their slack beside
     __shared__ int2 squeue[4][64];
-    const float r2g = gap_limit(r, r2);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
     const int64_t ntask = (int64_t)*tcount;
@@ -1829,7 +1829,7 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
         // no scratch for candidate pairs: the one-pass walk
         cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), c->stream);
         k_leaf_warp4<<<(unsigned)cdiv(t.nL, 128), 128, 0, c->stream>>>(
-            t.keys, t.pos4, t.nL, r, r2, cursor, capacity, pi, pj, pd, c->d_err);
+            t.keys, t.pos4, t.nL, r, r2, gap_limit(r, r2), cursor, capacity, pi, pj, pd, c->d_err);
         c->launches++;
         if ((st = check_launch(c, "leaf pairs (unordered)"))) return st;
         unsigned long long tot = 0;
@@ -1857,8 +1857,8 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
         k_group_tasks<<<(unsigned)cdiv(ng, 4), 128, 0, c->stream>>>(gbox, t.nL, tcursor, tcap,
                                                                     (int2*)c->tasks.p);
         k_group_pairs<<<(unsigned)(nsm * std::max(occ, 1)), 128, 0, c->stream>>>(
-            t.keys, gbox, t.pos4, t.nL, r, r2, tcursor, tcap, (const int2*)c->tasks.p, ticket,
-            cursor, capacity, pi, pj, pd);
+            t.keys, gbox, t.pos4, t.nL, r, r2, gap_limit(r, r2), tcursor, tcap,
+            (const int2*)c->tasks.p, ticket, cursor, capacity, pi, pj, pd);
         c->launches += 2;
         if ((st = check_launch(c, "leaf pairs (unordered)"))) return st;
         unsigned long long h[2] = {0, 0};
@@ -1896,8 +1896,8 @@ nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
         k_group_boxes<<<(unsigned)ns, 1024, 0, c->stream>>>(t.keys, t.nL, gbox);
         const unsigned grid = (unsigned)cdiv(t.nL, 4);
 #define ND_COUNT(A)                                                                              \
-    k_leaf_wide<A, 0><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, \
-                                                       counts, nullptr, nullptr, 0, nullptr,     \
+    k_leaf_wide<A, 0><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,           \
+                                                   gap_limit(r, r2), counts, nullptr, nullptr, 0, nullptr,     \
                                                        nullptr, nullptr)
         if (t.apl == 4) ND_COUNT(4);
         else if (t.apl == 2) ND_COUNT(2);
@@ -1920,8 +1920,8 @@ nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
         const float4* gbox = (const float4*)c->store.p;
         const unsigned grid = (unsigned)cdiv(t.nL, 4);
 #define ND_WRITE(A)                                                                              \
-    k_leaf_wide<A, 1><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,  \
-                                                      nullptr, offsets, total_dev, cap, pi, pj, pd)
+    k_leaf_wide<A, 1><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,           \
+                                                   gap_limit(r, r2), nullptr, offsets, total_dev, cap, pi, pj, pd)
         if (t.apl == 4) ND_WRITE(4);
         else if (t.apl == 2) ND_WRITE(2);
         else ND_WRITE(0);
@@ -1943,8 +1943,8 @@ nd_status write_pair_triples(Ctx* c, const TreeBuffers& t, float r, float r2,
     const float4* gbox = (const float4*)c->store.p;
     const unsigned grid = (unsigned)cdiv(t.nL, 4);
 #define ND_WRITE(A)                                                                             \
-    k_leaf_wide<A, 2><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,    \
-                                                   nullptr, offsets, total_dev, cap, out, nullptr, \
+    k_leaf_wide<A, 2><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,           \
+                                                   gap_limit(r, r2), nullptr, offsets, total_dev, cap, out, nullptr, \
                                                    nullptr)
     if (t.apl == 4) ND_WRITE(4);
     else if (t.apl == 2) ND_WRITE(2);
