@@ -1111,13 +1111,30 @@ __device__ __forceinline__ void atom_query(int32_t qi, const float4* __restrict_
 // ascending, the overlapping leaves t > q ascending, atoms of q outer, atoms
 // of t inner, and any search that enumerates those leaves in order gives it.
 // Here one warp searches for one query leaf over a 32-wide hierarchy of the
-// sorted leaves (groups of 32 leaves, super-groups of 32 groups): 32 boxes are
+// sorted leaves (groups of 32 leaves, super-groups of 32 groups, and for many
+// leaves two levels more, see kDirectSupers): 32 boxes are
 // tested per step, one a lane, and the hits are taken in index order from the
 // ballot.  A thread per leaf walking the binary tree's ropes, the form before,
 // had 1 node load in flight a thread and wrote each thread's pairs to its own
 // place: 262,144 atoms at density 0.83, r 2.5: count 237 and write 563 us, and
 // 20,000 atoms in reference order (whose boxes overlap almost all others, no
 // tree prunes them): 2.9 and 6.8 ms.
+
+// The levels above nL leaves: groups of 32 leaves, super-groups of 32 groups,
+// and so on.  Their boxes lie one level after the other, stored like leaf keys.
+struct GroupLevels {
+    int32_t ng, ns, n3, n4;
+    __host__ __device__ explicit GroupLevels(int32_t nL)
+        : ng((nL + 31) >> 5), ns((ng + 31) >> 5), n3((ns + 31) >> 5), n4((n3 + 31) >> 5) {}
+    __host__ __device__ int64_t boxes() const { return (int64_t)ng + ns + n3 + n4; }
+};
+
+// Up to this many super-groups (262,144 leaves) they are tested 32 after 32;
+// beyond, the two levels above them say which.  Testing them all grows with the
+// square of the leaves: the ordered list of 4,194,304 points (density 0.83, r
+// 1.3, four atoms a leaf) took 4.3 ms and takes 2.8, of 134,217,728 points (r
+// 1.0) 2.5 s and 95 ms, the unordered one 96 and 39 ms.
+constexpr int32_t kDirectSupers = 256;
 
 // Boxes of the groups of 32 leaves at [0, ngroups) and of the super-groups of
 // 32 groups after them, stored like leaf keys.  One warp per group, one block
@@ -1164,34 +1181,109 @@ __global__ void __launch_bounds__(1024)
     }
 }
 
+// Boxes of the nodes of one level (nout of them at `out`) over 32 nodes each of
+// the level below (nin at `in`).  One warp a node.
+__global__ void __launch_bounds__(256)
+    k_upper_boxes(const float4* __restrict__ in, int32_t nin, float4* __restrict__ out, int32_t nout) {
+    const int lane = threadIdx.x & 31;
+    const int32_t o = (int32_t)blockIdx.x * 8 + (int32_t)(threadIdx.x >> 5);
+    if (o >= nout) return;  // whole warp
+    float v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    const int64_t i = (int64_t)o * 32 + lane;
+    if (i < nin) {
+        const float4 a = __ldg(&in[2 * i]), b = __ldg(&in[2 * i + 1]);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            v[d] = fminf(v[d], __shfl_xor_sync(0xffffffffu, v[d], s));
+            v[3 + d] = fmaxf(v[3 + d], __shfl_xor_sync(0xffffffffu, v[3 + d], s));
+        }
+    if (lane == 0) {
+        out[2 * (int64_t)o] = make_float4(v[0], v[1], v[2], v[3]);
+        out[2 * (int64_t)o + 1] = make_float4(v[4], v[5], 0.f, 0.f);
+    }
+}
+
+// The boxes of every level over the leaves.
+static void group_boxes(Ctx* c, const float4* keys, int32_t nL, float4* gbox) {
+    const GroupLevels v(nL);
+    k_group_boxes<<<(unsigned)v.ns, 1024, 0, c->stream>>>(keys, nL, gbox);
+    c->launches++;
+    if (v.ns <= kDirectSupers) return;
+    float4* sbox = gbox + 2 * (int64_t)v.ng;
+    float4* box3 = sbox + 2 * (int64_t)v.ns;
+    k_upper_boxes<<<(unsigned)cdiv(v.n3, 8), 256, 0, c->stream>>>(sbox, v.ns, box3, v.n3);
+    k_upper_boxes<<<(unsigned)cdiv(v.n4, 8), 256, 0, c->stream>>>(box3, v.n3,
+                                                                  box3 + 2 * (int64_t)v.n3, v.n4);
+    c->launches += 2;
+}
+
+// Every group >= g0 that overlaps box q, in index order: hit(base, m) is called
+// by the whole warp for 32 consecutive groups at a time, bit k of m telling
+// whether group base + k overlaps.  DEEP: more than kDirectSupers super-groups.
+template <bool DEEP, class F>
+__device__ __forceinline__ void wide_groups(const Node& q, int32_t g0,
+                                            const float4* __restrict__ gbox, int32_t nL, F&& hit) {
+    const int lane = threadIdx.x & 31;
+    const int32_t ng = (nL + 31) >> 5, ns = (ng + 31) >> 5;
+    const int32_t s0 = g0 >> 5;
+    // super-groups sb .. sb + 31
+    auto supers = [&](int32_t sb) {
+        const int32_t s = sb + lane;
+        unsigned sm = __ballot_sync(0xffffffffu, s >= s0 && s < ns &&
+                                                     overlap(q, load_node(gbox, ng + min(s, ns - 1) + 1)));
+        while (sm) {
+            const int32_t base = (sb + __ffs(sm) - 1) * 32, g = base + lane;
+            sm &= sm - 1;
+            hit(base, __ballot_sync(0xffffffffu, g >= g0 && g < ng &&
+                                                     overlap(q, load_node(gbox, min(g, ng - 1) + 1))));
+        }
+    };
+    if constexpr (!DEEP) {
+        for (int32_t sb = s0; sb < ns; sb += 32) supers(sb);
+    } else {
+        const GroupLevels v(nL);
+        const int32_t t0 = s0 >> 5, f0 = t0 >> 5;
+        const float4* __restrict__ box3 = gbox + 2 * ((int64_t)ng + ns);
+        const float4* __restrict__ box4 = box3 + 2 * (int64_t)v.n3;
+        for (int32_t b4 = f0; b4 < v.n4; b4 += 32) {
+            const int32_t f = b4 + lane;
+            unsigned m4 = __ballot_sync(
+                0xffffffffu, f < v.n4 && overlap(q, load_node(box4, min(f, v.n4 - 1) + 1)));
+            while (m4) {
+                const int32_t b3 = (b4 + __ffs(m4) - 1) * 32, t = b3 + lane;
+                m4 &= m4 - 1;
+                unsigned m3 = __ballot_sync(0xffffffffu,
+                                            t >= t0 && t < v.n3 &&
+                                                overlap(q, load_node(box3, min(t, v.n3 - 1) + 1)));
+                while (m3) {
+                    supers((b3 + __ffs(m3) - 1) * 32);
+                    m3 &= m3 - 1;
+                }
+            }
+        }
+    }
+}
+
 // Every leaf t >= t0 (0-based) that overlaps box q, in index order: hit(t,
 // box, in) is called by the whole warp for 32 consecutive leaves at a time,
 // `in` telling whether this lane's leaf overlaps.
-template <class F>
+template <bool DEEP, class F>
 __device__ __forceinline__ void wide_search(const Node& q, int32_t t0,
                                             const float4* __restrict__ keys,
                                             const float4* __restrict__ gbox, int32_t nL, F&& hit) {
     const int lane = threadIdx.x & 31;
-    const int32_t ng = (nL + 31) >> 5, ns = (ng + 31) >> 5;
-    const int32_t g0 = t0 >> 5, s0 = g0 >> 5;
-    for (int32_t sb = s0; sb < ns; sb += 32) {
-        const int32_t s = sb + lane;
-        unsigned sm = __ballot_sync(0xffffffffu, s < ns && overlap(q, load_node(gbox, ng + min(s, ns - 1) + 1)));
-        while (sm) {
-            const int32_t sg = sb + __ffs(sm) - 1;
-            sm &= sm - 1;
-            const int32_t g = sg * 32 + lane;
-            unsigned gm = __ballot_sync(
-                0xffffffffu, g >= g0 && g < ng && overlap(q, load_node(gbox, min(g, ng - 1) + 1)));
-            while (gm) {
-                const int32_t gg = sg * 32 + __ffs(gm) - 1;
-                gm &= gm - 1;
-                const int32_t t = gg * 32 + lane;
-                const Node b = load_node(keys, min(t, nL - 1) + 1);
-                hit(t, b, t >= t0 && t < nL && overlap(q, b));
-            }
+    wide_groups<DEEP>(q, t0 >> 5, gbox, nL, [&](int32_t base, unsigned m) {
+        while (m) {
+            const int32_t t = (base + __ffs(m) - 1) * 32 + lane;
+            m &= m - 1;
+            const Node b = load_node(keys, min(t, nL - 1) + 1);
+            hit(t, b, t >= t0 && t < nL && overlap(q, b));
         }
-    }
+    });
 }
 
 // One warp per query leaf.  WRITE 0: counts[q] = its pairs; 1: its pairs at
@@ -1204,7 +1296,7 @@ __device__ __forceinline__ void wide_search(const Node& q, int32_t t0,
 // the hits leave through shared memory as contiguous runs.  APL 0 (any other
 // width): the warp runs the apl^2 tests of one leaf pair together, 32 at a
 // time in list order.
-template <int APL, int WRITE>
+template <int APL, int WRITE, bool DEEP>
 __global__ void __launch_bounds__(128)
     k_leaf_wide(const float4* __restrict__ keys, const float4* __restrict__ gbox,
                 const float4* __restrict__ pos, int32_t nL, int32_t apl, float r, float r2,
@@ -1290,7 +1382,7 @@ __global__ void __launch_bounds__(128)
         };
         if (lane == 0) queue[0] = q;  // the pairs inside the leaf come first
         int32_t qn = 1;
-        wide_search(ql, q + 1, keys, gbox, nL, [&](int32_t t, const Node& b, bool in) {
+        wide_search<DEEP>(ql, q + 1, keys, gbox, nL, [&](int32_t t, const Node& b, bool in) {
             const bool want = in && leaf_gap_ok(ql, b, r, r2g, slack);
             const unsigned m = __ballot_sync(0xffffffffu, want);
             if (want) queue[qn + __popc(m & below)] = t;  // < 64: qn < 32 here
@@ -1347,7 +1439,7 @@ __global__ void __launch_bounds__(128)
             }
         };
         leaf(q);
-        wide_search(ql, q + 1, keys, gbox, nL, [&](int32_t t, const Node& b, bool in) {
+        wide_search<DEEP>(ql, q + 1, keys, gbox, nL, [&](int32_t t, const Node& b, bool in) {
             unsigned m =
                 __ballot_sync(0xffffffffu, in && leaf_gap_ok(ql, b, r, r2g, slack));
             const int32_t base = t - lane;
@@ -1577,14 +1669,14 @@ __global__ void __launch_bounds__(128)
 // ring while its reservation is under way 13900 (more instructions).
 constexpr int kTaskBuf = 128;  // tasks buffered per warp
 
+template <bool DEEP>
 __global__ void __launch_bounds__(128)
     k_group_tasks(const float4* __restrict__ gbox, int32_t nL, unsigned long long* tcursor,
                   int64_t tcap, int2* __restrict__ tasks) {
     __shared__ int32_t sbuf[4][kTaskBuf];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int32_t ng = (nL + 31) >> 5, ns = (ng + 31) >> 5;
     const int32_t g = (int32_t)blockIdx.x * 4 + w;
-    if (g >= ng) return;  // whole warp
+    if (g >= GroupLevels(nL).ng) return;  // whole warp
     int32_t* buf = sbuf[w];
     const Node un = load_node(gbox, g + 1);
     if (lane == 0) buf[0] = g;  // the pairs inside the group, whatever its box
@@ -1599,20 +1691,11 @@ __global__ void __launch_bounds__(128)
         __syncwarp();
         nb = 0;
     };
-    for (int32_t sb = g >> 10; sb < ns; sb += 32) {
-        const int32_t s = sb + lane;
-        unsigned sm = __ballot_sync(
-            0xffffffffu, s < ns && overlap(un, load_node(gbox, ng + min(s, ns - 1) + 1)));
-        while (sm) {
-            const int32_t h = (sb + __ffs(sm) - 1) * 32 + lane;
-            sm &= sm - 1;
-            const bool in = h > g && h < ng && overlap(un, load_node(gbox, min(h, ng - 1) + 1));
-            const unsigned m = __ballot_sync(0xffffffffu, in);
-            if (in) buf[nb + __popc(m & ((1u << lane) - 1u))] = h;
-            nb += __popc(m);
-            if (nb > kTaskBuf - 32) flush();
-        }
-    }
+    wide_groups<DEEP>(un, g + 1, gbox, nL, [&](int32_t base, unsigned m) {
+        if ((m >> lane) & 1u) buf[nb + __popc(m & ((1u << lane) - 1u))] = base + lane;
+        nb += __popc(m);
+        if (nb > kTaskBuf - 32) flush();
+    });
     if (nb) flush();
 }
 
@@ -1845,17 +1928,18 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
     int nsm = 0, occ = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_group_pairs, 128, 0);
-    const int64_t ng = cdiv(t.nL, 32), ns = cdiv(ng, 32);
-    if ((st = ensure(c, c->store, 32 * (size_t)(ng + ns)))) return st;
+    const GroupLevels lev(t.nL);
+    const int64_t ng = lev.ng;
+    if ((st = ensure(c, c->store, 32 * (size_t)lev.boxes()))) return st;
     if ((st = ensure(c, c->tasks, sizeof(int2) * 128 * (size_t)ng))) return st;
     float4* gbox = (float4*)c->store.p;
-    k_group_boxes<<<(unsigned)ns, 1024, 0, c->stream>>>(t.keys, t.nL, gbox);
-    c->launches++;
+    group_boxes(c, t.keys, t.nL, gbox);
     for (int attempt = 0;; ++attempt) {
         const int64_t tcap = (int64_t)(c->tasks.bytes / sizeof(int2));
         cudaMemsetAsync(cursor, 0, 3 * sizeof(unsigned long long), c->stream);
-        k_group_tasks<<<(unsigned)cdiv(ng, 4), 128, 0, c->stream>>>(gbox, t.nL, tcursor, tcap,
-                                                                    (int2*)c->tasks.p);
+        const auto tasks_fn = lev.ns <= kDirectSupers ? k_group_tasks<false> : k_group_tasks<true>;
+        tasks_fn<<<(unsigned)cdiv(ng, 4), 128, 0, c->stream>>>(gbox, t.nL, tcursor, tcap,
+                                                               (int2*)c->tasks.p);
         k_group_pairs<<<(unsigned)(nsm * std::max(occ, 1)), 128, 0, c->stream>>>(
             t.keys, gbox, t.pos4, t.nL, r, r2, gap_limit(r, r2), tcursor, tcap,
             (const int2*)c->tasks.p, ticket, cursor, capacity, pi, pj, pd);
@@ -1875,6 +1959,15 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
     }
 }
 
+// k_leaf_wide for a tree's leaf width and number of super-groups.
+template <int WRITE>
+static auto leaf_wide(const TreeBuffers& t) {
+    const bool deep = GroupLevels(t.nL).ns > kDirectSupers;
+    if (t.apl == 4) return deep ? k_leaf_wide<4, WRITE, true> : k_leaf_wide<4, WRITE, false>;
+    if (t.apl == 2) return deep ? k_leaf_wide<2, WRITE, true> : k_leaf_wide<2, WRITE, false>;
+    return deep ? k_leaf_wide<0, WRITE, true> : k_leaf_wide<0, WRITE, false>;
+}
+
 // Ordered emission: per-query counts, their scan, then the pairs at their
 // places.  total_dev receives the number of pairs (device); the write pass
 // reads it and writes nothing when it exceeds the capacity, so no host round
@@ -1890,20 +1983,13 @@ nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
     if (kind == 0) {
         // the group boxes take the place of the build's CAS slots, which the
         // ordered emission has no more use for
-        const size_t ng = (size_t)cdiv(t.nL, 32), ns = (size_t)cdiv(t.nL, 1024);
-        if ((st = ensure(c, c->store, 32 * (ng + ns)))) return st;
+        if ((st = ensure(c, c->store, 32 * (size_t)GroupLevels(t.nL).boxes()))) return st;
         float4* gbox = (float4*)c->store.p;
-        k_group_boxes<<<(unsigned)ns, 1024, 0, c->stream>>>(t.keys, t.nL, gbox);
-        const unsigned grid = (unsigned)cdiv(t.nL, 4);
-#define ND_COUNT(A)                                                                              \
-    k_leaf_wide<A, 0><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,           \
-                                                   gap_limit(r, r2), counts, nullptr, nullptr, 0, nullptr,     \
-                                                       nullptr, nullptr)
-        if (t.apl == 4) ND_COUNT(4);
-        else if (t.apl == 2) ND_COUNT(2);
-        else ND_COUNT(0);
-#undef ND_COUNT
-        c->launches += 2;
+        group_boxes(c, t.keys, t.nL, gbox);
+        leaf_wide<0>(t)<<<(unsigned)cdiv(t.nL, 4), 128, 0, c->stream>>>(
+            t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), counts, nullptr, nullptr, 0,
+            nullptr, nullptr, nullptr);
+        c->launches++;
     } else {
         k_atom_count<<<(unsigned)cdiv(nq, 128), 128, 0, c->stream>>>(t.keys, t.pos4, t.n, t.apl, r2,
                                                                      counts, c->d_err);
@@ -1918,14 +2004,9 @@ nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
     const int64_t* offsets = (const int64_t*)c->offsets.p;
     if (kind == 0) {
         const float4* gbox = (const float4*)c->store.p;
-        const unsigned grid = (unsigned)cdiv(t.nL, 4);
-#define ND_WRITE(A)                                                                              \
-    k_leaf_wide<A, 1><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,           \
-                                                   gap_limit(r, r2), nullptr, offsets, total_dev, cap, pi, pj, pd)
-        if (t.apl == 4) ND_WRITE(4);
-        else if (t.apl == 2) ND_WRITE(2);
-        else ND_WRITE(0);
-#undef ND_WRITE
+        leaf_wide<1>(t)<<<(unsigned)cdiv(t.nL, 4), 128, 0, c->stream>>>(
+            t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), nullptr, offsets, total_dev,
+            cap, pi, pj, pd);
     } else {
         k_atom_write<<<(unsigned)cdiv(t.n, 128), 128, 0, c->stream>>>(
             t.keys, t.pos4, t.n, t.apl, r2, offsets, total_dev, cap, pi, pj, pd, c->d_err);
@@ -1941,15 +2022,9 @@ nd_status write_pair_triples(Ctx* c, const TreeBuffers& t, float r, float r2,
                              const int64_t* total_dev, int64_t cap, int32_t* out) {
     const int64_t* offsets = (const int64_t*)c->offsets.p;
     const float4* gbox = (const float4*)c->store.p;
-    const unsigned grid = (unsigned)cdiv(t.nL, 4);
-#define ND_WRITE(A)                                                                             \
-    k_leaf_wide<A, 2><<<grid, 128, 0, c->stream>>>(t.keys, gbox, t.pos4, t.nL, t.apl, r, r2,           \
-                                                   gap_limit(r, r2), nullptr, offsets, total_dev, cap, out, nullptr, \
-                                                   nullptr)
-    if (t.apl == 4) ND_WRITE(4);
-    else if (t.apl == 2) ND_WRITE(2);
-    else ND_WRITE(0);
-#undef ND_WRITE
+    leaf_wide<2>(t)<<<(unsigned)cdiv(t.nL, 4), 128, 0, c->stream>>>(
+        t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), nullptr, offsets, total_dev, cap,
+        out, nullptr, nullptr);
     c->launches++;
     return check_launch(c, "pair write");
 }
