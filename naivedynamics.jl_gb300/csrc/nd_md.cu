@@ -799,45 +799,65 @@ __global__ void __launch_bounds__(kBlock)
         w.x = __byte_perm(w.x, w.y, 0x5432);
         w.y = __byte_perm(w.y, li, 0x5432);
     };
+    // branch-free: every step predicated
+    auto test = [&](const float4& q, uint32_t li) {
+        const float d2 = dist2_ref(p.x, p.y, p.z, q.x, q.y, q.z);
+        const bool hit = d2 < rl2 && __float_as_int(q.w) != self;
+        const bool put = hit && cnt < lcap;
+        const bool near = put && d2 < nb2, far = put && !(d2 < nb2);
+        if (far) {
+            push(fw, li);
+            if ((++nf & 3) == 0) { *farp = fw; farp -= kBlock; }
+        }
+        if (near) {
+            push(nw, li);
+            if ((++nn & 3) == 0) { *nearp = nw; nearp += kBlock; }
+        }
+        cnt += hit ? 1 : 0;
+    };
     // compiled twice: for a block whose whole union is staged (block-uniform)
     // the positions come from shared memory with no test
     auto walk = [&](auto staged) {
         constexpr bool ALL = decltype(staged)::value;
-        uint4 nxt = nc > 0 ? C[0] : make_uint4(0u, 0u, 0u, 0u);
-        for (int32_t k0 = 0; k0 < nc; k0 += 8) {
-            const uint4 cur = nxt;
-            if (k0 + 8 < nc) nxt = C[(k0 >> 3) + 1];
-            const uint32_t cw[4] = {cur.x, cur.y, cur.z, cur.w};
+        if constexpr (APL > 8) {
+            // leaves of 16 and 32 atoms eight atoms at a time: unrolled like the
+            // others, their 128 and 256 tests did not fit the instruction cache
+            // (131,072 atoms, leaves of 32: 116 us a step, 68 so)
+            const uint16_t* cand = reinterpret_cast<const uint16_t*>(C);
+            for (int32_t k = 0; k < nc; ++k) {
+                const int32_t u = cand[k];
+                const float4* src = ALL || (u + 1) * APL <= smpos ? spos + u * APL
+                                                                  : pos + (int64_t)U[u] * APL;
+#pragma unroll 1
+                for (int e0 = 0; e0 < APL; e0 += 8) {
+                    float4 q[8];
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                if (k0 + h >= nc) break;
-                const int32_t u = (int32_t)((cw[h >> 1] >> (16 * (h & 1))) & 0xffffu);
-                float4 q[APL];
-                if (ALL || (u + 1) * APL <= smpos) {
+                    for (int e = 0; e < 8; ++e) q[e] = src[e0 + e];
 #pragma unroll
-                    for (int e = 0; e < APL; ++e) q[e] = spos[u * APL + e];
-                } else {
-                    const int64_t base = (int64_t)U[u] * APL;
-#pragma unroll
-                    for (int e = 0; e < APL; ++e) q[e] = pos[base + e];
+                    for (int e = 0; e < 8; ++e) test(q[e], (uint32_t)(u * APL + e0 + e));
                 }
+            }
+        } else {
+            uint4 nxt = nc > 0 ? C[0] : make_uint4(0u, 0u, 0u, 0u);
+            for (int32_t k0 = 0; k0 < nc; k0 += 8) {
+                const uint4 cur = nxt;
+                if (k0 + 8 < nc) nxt = C[(k0 >> 3) + 1];
+                const uint32_t cw[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
-                for (int e = 0; e < APL; ++e) {
-                    // branch-free: every step predicated
-                    const float d2 = dist2_ref(p.x, p.y, p.z, q[e].x, q[e].y, q[e].z);
-                    const bool hit = d2 < rl2 && __float_as_int(q[e].w) != self;
-                    const bool put = hit && cnt < lcap;
-                    const bool near = put && d2 < nb2, far = put && !(d2 < nb2);
-                    const uint32_t li = (uint32_t)(u * APL + e);
-                    if (far) {
-                        push(fw, li);
-                        if ((++nf & 3) == 0) { *farp = fw; farp -= kBlock; }
+                for (int h = 0; h < 8; ++h) {
+                    if (k0 + h >= nc) break;
+                    const int32_t u = (int32_t)((cw[h >> 1] >> (16 * (h & 1))) & 0xffffu);
+                    float4 q[APL];
+                    if (ALL || (u + 1) * APL <= smpos) {
+#pragma unroll
+                        for (int e = 0; e < APL; ++e) q[e] = spos[u * APL + e];
+                    } else {
+                        const int64_t base = (int64_t)U[u] * APL;
+#pragma unroll
+                        for (int e = 0; e < APL; ++e) q[e] = pos[base + e];
                     }
-                    if (near) {
-                        push(nw, li);
-                        if ((++nn & 3) == 0) { *nearp = nw; nearp += kBlock; }
-                    }
-                    cnt += hit ? 1 : 0;
+#pragma unroll
+                    for (int e = 0; e < APL; ++e) test(q[e], (uint32_t)(u * APL + e));
                 }
             }
         }
