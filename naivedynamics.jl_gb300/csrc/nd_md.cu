@@ -1934,14 +1934,19 @@ cudaError_t raise_smem_limit(const void* fn, int maxsm) {
                                 maxsm - (int)fa.sharedSizeBytes);
 }
 
-// Whether the lists are built by a warp per leaf: while there are at most two
-// blocks of kBlock atoms per SM, whose threads (one an atom) would walk their
-// candidates on a part of the chip, and the candidates fit shared memory.  A
-// rebuild with a thread an atom and with a warp a leaf, us: 40,960 atoms 228
-// and 175, 65,536 atoms 251 and 220; but 98,304 atoms 250 and 266, 262,144
-// atoms 536 and 706.
+// Whether the lists are built by a warp per leaf: while the threads of an atom
+// each would walk their candidates on a part of the chip, and the candidates fit
+// shared memory.  Up to two blocks of kBlock atoms per SM with four or more
+// atoms a leaf; leaves of two or one are that many warps more, each with as many
+// boxes to test, so up to one block and half a block per SM; leaves of 32 leave
+// too few warps.  us a step (a rebuild every tenth) with a thread an atom and
+// with a warp a leaf: leaves of 4, 32,768 atoms 32.1 and 29.8, 77,824 49.6 and
+// 43.2, 131,072 63.6 and 66.3; of 2, 32,768 33.2 and 32.9, 49,152 46.0 and 47.7;
+// of 1, 16,384 29.8 and 27.1, 24,576 37.2 and 38.9, 65,536 51.8 and 71.4; of 32,
+// 2,048 20.4 and 24.8, 65,536 53.1 and 70.4.
 static bool md_leaf_warps(const MDEngine* m) {
-    return m->nblocks <= 2 * m->nsm && 8 * sizeof(uint2) * (size_t)m->lcap_leaf <= 200 * 1024;
+    return m->apl < 32 && 2 * m->nblocks <= std::min(m->apl, 4) * m->nsm &&
+           8 * sizeof(uint2) * (size_t)m->lcap_leaf <= 200 * 1024;
 }
 
 // Union and list buffers for capacities (ucap, lcap), and the shared-memory
@@ -2019,7 +2024,6 @@ static nd_status md_alloc_lists(MDEngine* m, int32_t fcap, int32_t ucap, int32_t
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<16>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<16>, maxsm);
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_block_lists<32>, maxsm);
-    if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_leaf_lists<32>, maxsm);
 #define ND_SMEM(C, MODE)                                                                        \
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_step<C, MODE, false>, maxsm);   \
     if (e == cudaSuccess) e = raise_smem_limit((const void*)k_md_step<C, MODE, true>, maxsm);    \
@@ -2208,7 +2212,7 @@ nd_status md_rebuild(MDEngine* m, int kind, int rec, unsigned* counter, bool siz
     do {                                                                                         \
         if (md_leaf_warps(m))                                                                    \
             launch_chained(                                                                      \
-                c, gate != nullptr, k_md_leaf_lists<A>,                                          \
+                c, gate != nullptr, k_md_leaf_lists<(A < 32 ? A : 16)>, /* (never for 32) */     \
                 (unsigned)m->nblocks * (kBlock / A / 8), kBlock,                                 \
                 8 * sizeof(uint2) * (size_t)m->lcap_leaf, keys, (const float4*)m->pos32.p, m->nL, rl, rl * rl, rnb2, sid, sys, m->ucap,    \
                 (const int32_t*)m->ulist.p, (const int32_t*)m->ucount.p, m->lcap_leaf, m->lcap,  \
