@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(288) k_cs_lj(const float* __restrict__ x, int3
 // a row, and down a column) and runs each pair's two updates as written gives
 // every atom the same sequence of roundings as the sequential loop.
 //
-// Bands (up to kBandMaxAtoms atoms): a warp owns 256 consecutive rows, eight a
+// Bands (kLevelAtoms < n <= kBandMaxAtoms): a warp owns 256 consecutive rows, eight a
 // lane, whose running forces stay in registers; the columns flow through its
 // lanes, four at a time.  At step t lane l takes the four columns 256 b + 4 (t -
 // l) .. + 3 from lane l - 1 by shuffles, adds the pair terms to its rows' forces
@@ -543,9 +543,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     cluster.sync();  // the next block's array is written until here
 }
 
-// Beyond kBandMaxAtoms: the pairs with i + j = s form one level whose pairs
-// touch distinct atoms, and level s follows level s - 1; one block runs the
-// levels in order.  The pair terms are stored level by level (level s at
+// Up to kLevelAtoms and beyond kBandMaxAtoms: the pairs with i + j = s form one
+// level whose pairs touch distinct atoms, and level s follows level s - 1; one
+// block runs the levels in order.  The pair terms are stored level by level (level s at
 // level_off(s); its pairs by increasing i).
 
 __host__ __device__ inline int32_t level_lo(int32_t s, int32_t n) { return max(0, s - (n - 1)); }
@@ -574,6 +574,11 @@ __global__ void k_cs_cterms(const float* __restrict__ x, const float* __restrict
                               x[3 * (int64_t)j], x[3 * (int64_t)j + 1], x[3 * (int64_t)j + 2], q[j]);
     }
 }
+
+// The bands take 32 steps and a cluster launch at least, whatever the size.  us a
+// step of simulate!, levels and bands: 1 atom 10.4 and 23.9, 4 atoms 15.1 and
+// 22.1, 16 atoms 21.2 and 23.8, 24 atoms 27.4 and 23.1.
+constexpr int kLevelAtoms = 16;
 
 constexpr int kLevelThreads = 128;  // fewest warps paying the per-level overhead (measured: 128 of 32-1024)
 
@@ -700,7 +705,7 @@ nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x
         poslog ? std::max<int64_t>(1, std::min<int64_t>(spec->duration, chunk_frames)) : 0;
     nd_status st;
     // Coulomb terms: in band order, or by level for the global-memory form
-    const bool bands = !force_global && n <= kBandMaxAtoms;
+    const bool bands = !force_global && n > kLevelAtoms && n <= kBandMaxAtoms;
     const int32_t nband = (int32_t)cdiv(n, kBandRows), P4 = band_steps(n);
     const int32_t nlev = std::max(2 * n - 3, 0);
     const size_t ncterm =
