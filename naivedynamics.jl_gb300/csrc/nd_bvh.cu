@@ -848,6 +848,7 @@ nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t a
     out->idx = (const int32_t*)c->idx.p;
     out->keys = keys;
     out->nkeys = nkeys;
+    out->internal = !leaves_only;
     return check_launch(c, "tree");
 }
 
@@ -896,6 +897,7 @@ nd_status build_tree_kept(Ctx* c, const float* xyz_dev, int32_t n, float r, int3
     out->idx = (const int32_t*)c->idx.p;
     out->keys = keys;
     out->nkeys = nkeys;
+    out->internal = true;
     return check_launch(c, "kept tree");
 }
 
@@ -1044,7 +1046,8 @@ __device__ __forceinline__ bool leaf_gap_ok(const Node& a, const Node& b, float 
     return gx * gx + gy * gy + gz * gz < r2g;
 }
 
-// Emission sinks of the per-atom path: COUNT counts, WRITE writes at a running cursor.
+// Emission sinks of the walks: Count counts, Write and Triples write at a running
+// cursor.
 struct SinkCount {
     int64_t n = 0;
     __device__ __forceinline__ void push(int32_t, int32_t, float) { ++n; }
@@ -1054,6 +1057,15 @@ struct SinkWrite {
     int64_t cur;
     __device__ __forceinline__ void push(int32_t i, int32_t j, float d) {
         pi[cur] = i; pj[cur] = j; pd[cur] = d; ++cur;
+    }
+};
+
+struct SinkTriples {
+    int32_t* out;
+    int64_t cur;
+    __device__ __forceinline__ void push(int32_t i, int32_t j, float d) {
+        int32_t* o = out + 3 * cur++;
+        o[0] = i; o[1] = j; o[2] = __float_as_int(d);
     }
 };
 
@@ -1128,6 +1140,9 @@ struct GroupLevels {
         : ng((nL + 31) >> 5), ns((ng + 31) >> 5), n3((ns + 31) >> 5), n4((n3 + 31) >> 5) {}
     __host__ __device__ int64_t boxes() const { return (int64_t)ng + ns + n3 + n4; }
 };
+
+// Leaves above which an ordered list may come from rope walks (see sparse_leaves).
+constexpr int32_t kWalkLeaves = 131072;
 
 // Up to this many super-groups (262,144 leaves) they are tested 32 after 32;
 // beyond, the two levels above them say which.  Testing them all grows with the
@@ -1207,12 +1222,12 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// The boxes of every level over the leaves.
-static void group_boxes(Ctx* c, const float4* keys, int32_t nL, float4* gbox) {
+// The boxes of the groups and super-groups, and (upper) of the levels above.
+static void group_boxes(Ctx* c, const float4* keys, int32_t nL, float4* gbox, bool upper) {
     const GroupLevels v(nL);
     k_group_boxes<<<(unsigned)v.ns, 1024, 0, c->stream>>>(keys, nL, gbox);
     c->launches++;
-    if (v.ns <= kDirectSupers) return;
+    if (!upper) return;
     float4* sbox = gbox + 2 * (int64_t)v.ng;
     float4* box3 = sbox + 2 * (int64_t)v.ns;
     k_upper_boxes<<<(unsigned)cdiv(v.n3, 8), 256, 0, c->stream>>>(sbox, v.ns, box3, v.n3);
@@ -1286,7 +1301,8 @@ __device__ __forceinline__ void wide_search(const Node& q, int32_t t0,
     });
 }
 
-// One warp per query leaf.  WRITE 0: counts[q] = its pairs; 1: its pairs at
+// One warp per query leaf (DEEP: per leaf of `list`, of nq leaves, if there is
+// one).  WRITE 0: counts[q] = its pairs; 1: its pairs at
 // offsets[q] .. in three arrays (nothing when the total exceeds cap); 2: the
 // same as triples of words in pi.
 // APL 2 or 4: the overlapping leaves go through a queue of candidates so that
@@ -1302,14 +1318,16 @@ __global__ void __launch_bounds__(128)
                 const float4* __restrict__ pos, int32_t nL, int32_t apl, float r, float r2,
                 float r2g, int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
                 const int64_t* __restrict__ total, int64_t cap, int32_t* __restrict__ pi,
-                int32_t* __restrict__ pj, float* __restrict__ pd) {
+                int32_t* __restrict__ pj, float* __restrict__ pd, const int32_t* __restrict__ list,
+                int32_t nq) {
     constexpr int BUF = APL > 0 && WRITE != 0 ? 32 * APL * APL : 1;
     __shared__ int2 sbij[4][BUF];
     __shared__ float sbd[4][BUF];
     __shared__ int32_t squeue[4][64];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int32_t q = (int32_t)blockIdx.x * 4 + w;
-    if (q >= nL) return;  // whole warp
+    int32_t q = (int32_t)blockIdx.x * 4 + w;
+    if (q >= (DEEP ? nq : nL)) return;  // whole warp
+    if (DEEP && list) q = __ldg(&list[q]);
     int64_t cur = 0;
     if (WRITE) {
         if (*total > cap) return;
@@ -1450,6 +1468,136 @@ __global__ void __launch_bounds__(128)
         });
         if (!WRITE && lane == 0) counts[q] = n;
     }
+}
+
+// ------------------------------------------- ordered emission, rope walks
+//
+// leafneighbor_traverse (BVHTraverse.jl:1236-1323) as it is, a thread a leaf: the
+// ropes of the binary tree lead past what does not overlap.  Each thread writes
+// its pairs to its own place, and the walk has one node load in flight; but a
+// walk is short where few leaves overlap, and the search above spends a warp and
+// its chain of loads on every leaf (see sparse_leaves).  Leaves whose atoms extend
+// further than `widest` are left to the search: the walk of one that spans two
+// clusters is as long as hundreds of others'.
+__device__ __forceinline__ float leaf_extent(const Node& b, float r) {
+    return fmaxf(fmaxf(fmaxf(b.mxx - b.mnx, b.mxy - b.mny), b.mxz - b.mnz) - r, 0.0f);
+}
+template <int APL, int WRITE>
+__global__ void __launch_bounds__(128)
+    k_leaf_walk(const float4* __restrict__ keys, const float4* __restrict__ pos, int32_t nL,
+                int32_t apl, float r, float r2, float widest, int64_t* __restrict__ counts,
+                const int64_t* __restrict__ offsets, const int64_t* __restrict__ total, int64_t cap,
+                int32_t* pi, int32_t* pj, float* pd, int32_t* err) {
+    const int32_t q = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x) + 1;
+    if (q > nL || (WRITE && *total > cap)) return;
+    const Node ql = load_node(keys, q);
+    if (leaf_extent(ql, r) > widest) return;
+    const int32_t na = APL > 0 ? APL : apl, nnodes = 2 * nL - 1;
+    const int64_t A = (int64_t)(q - 1) * na;
+    auto run = [&](auto& s) {
+        [[maybe_unused]] float4 qa[APL > 0 ? APL : 1];
+        if constexpr (APL > 0)
+#pragma unroll
+            for (int i = 0; i < APL; ++i) qa[i] = __ldg(&pos[A + i]);
+        // the atoms of leaf t (tri: only those behind the query atom)
+        auto leaf = [&](int32_t t, bool tri) {
+            const int64_t B = (int64_t)(t - 1) * na;
+            if constexpr (APL > 0) {
+                float4 tb[APL];
+#pragma unroll
+                for (int j = 0; j < APL; ++j) tb[j] = __ldg(&pos[B + j]);
+#pragma unroll
+                for (int i = 0; i < APL; ++i)
+#pragma unroll
+                    for (int j = 0; j < APL; ++j) {
+                        const float d2 = dist2_ref(qa[i].x, qa[i].y, qa[i].z, tb[j].x, tb[j].y, tb[j].z);
+                        if (d2 < r2 && (!tri || j > i))
+                            s.push(__float_as_int(qa[i].w), __float_as_int(tb[j].w), __fsqrt_rn(d2));
+                    }
+            } else {
+                for (int32_t i = 0; i < apl; ++i) {
+                    const float4 a = __ldg(&pos[A + i]);
+                    for (int32_t j = tri ? i + 1 : 0; j < apl; ++j) {
+                        const float4 b = __ldg(&pos[B + j]);
+                        const float d2 = dist2_ref(a.x, a.y, a.z, b.x, b.y, b.z);
+                        if (d2 < r2) s.push(__float_as_int(a.w), __float_as_int(b.w), __fsqrt_rn(d2));
+                    }
+                }
+            }
+        };
+        leaf(q, true);
+        int32_t visits = 0;
+        for (int32_t t = ql.skip; t != 0;) {
+            ND_WALK_GUARD(t, nnodes, visits, err, q)
+            const Node nd_ = load_node(keys, t);
+            const bool in = overlap(ql, nd_);
+            if (in && nd_.left == 0) leaf(t, false);
+            t = in && nd_.left != 0 ? nd_.left : nd_.skip;
+        }
+    };
+    if constexpr (WRITE == 0) {
+        SinkCount s;
+        run(s);
+        counts[q - 1] = s.n;
+    } else if constexpr (WRITE == 1) {
+        SinkWrite s{pi, pj, pd, offsets[q - 1]};
+        run(s);
+    } else {
+        SinkTriples s{pi, offsets[q - 1]};
+        run(s);
+    }
+}
+
+// What the choice between search and walk looks at: the leaves behind the query
+// leaf that overlap it, summed over kSampled query leaves spread over all and the
+// most of one, and the largest and the summed extent of the leaves' atoms (their
+// widest axis).
+struct LeafSample {
+    unsigned long long overlaps;
+    unsigned most;
+    float widest;
+    double extents;
+};
+constexpr int kSampled = 512;
+template <bool DEEP>
+__global__ void __launch_bounds__(128)
+    k_overlap_sample(const float4* __restrict__ keys, const float4* __restrict__ gbox, int32_t nL,
+                     LeafSample* out) {
+    const int32_t k = (int32_t)(blockIdx.x * 4 + (threadIdx.x >> 5));
+    const int32_t q = (int32_t)((int64_t)k * nL / kSampled);
+    const Node ql = load_node(keys, q + 1);
+    unsigned n = 0;
+    wide_search<DEEP>(ql, q + 1, keys, gbox, nL, [&](int32_t, const Node&, bool in) { n += in; });
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&out->overlaps, (unsigned long long)n);
+        atomicMax(&out->most, n);
+    }
+}
+__global__ void __launch_bounds__(256)
+    k_leaf_extents(const float4* __restrict__ keys, int32_t nL, float r, LeafSample* out) {
+    float widest = 0.0f, sum = 0.0f;
+    for (int64_t l = blockIdx.x * 256 + threadIdx.x; l < nL; l += (int64_t)gridDim.x * 256) {
+        const float e = leaf_extent(load_node(keys, (int32_t)l + 1), r);
+        widest = fmaxf(widest, e);
+        sum += e;
+    }
+    const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(widest));  // (not negative)
+    double d = sum;
+    for (int s = 16; s > 0; s >>= 1) d += __shfl_xor_sync(0xffffffffu, d, s);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(reinterpret_cast<unsigned*>(&out->widest), w);
+        atomicAdd(&out->extents, d);
+    }
+}
+
+__global__ void __launch_bounds__(256)
+    k_wide_leaves(const float4* __restrict__ keys, int32_t nL, float r, float widest, int32_t cap,
+                  int32_t* __restrict__ list, unsigned long long* count) {
+    const int32_t l = (int32_t)(blockIdx.x * 256 + threadIdx.x);
+    if (l >= nL || !(leaf_extent(load_node(keys, l + 1), r) > widest)) return;
+    const unsigned long long k = atomicAdd(count, 1ull);
+    if (k < (unsigned long long)cap) list[k] = l;
 }
 
 // One-pass emission, warp-cooperative (atomsperleaf 4; the pair multiset of
@@ -1933,7 +2081,7 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
     if ((st = ensure(c, c->store, 32 * (size_t)lev.boxes()))) return st;
     if ((st = ensure(c, c->tasks, sizeof(int2) * 128 * (size_t)ng))) return st;
     float4* gbox = (float4*)c->store.p;
-    group_boxes(c, t.keys, t.nL, gbox);
+    group_boxes(c, t.keys, t.nL, gbox, lev.ns > kDirectSupers);
     for (int attempt = 0;; ++attempt) {
         const int64_t tcap = (int64_t)(c->tasks.bytes / sizeof(int2));
         cudaMemsetAsync(cursor, 0, 3 * sizeof(unsigned long long), c->stream);
@@ -1959,21 +2107,116 @@ nd_status emit_unordered(Ctx* c, const TreeBuffers& t, float r, float r2, int32_
     }
 }
 
-// k_leaf_wide for a tree's leaf width and number of super-groups.
+// k_leaf_wide and k_leaf_walk for a tree's leaf width.
 template <int WRITE>
-static auto leaf_wide(const TreeBuffers& t) {
-    const bool deep = GroupLevels(t.nL).ns > kDirectSupers;
+static auto leaf_wide(const TreeBuffers& t, bool deep) {
     if (t.apl == 4) return deep ? k_leaf_wide<4, WRITE, true> : k_leaf_wide<4, WRITE, false>;
     if (t.apl == 2) return deep ? k_leaf_wide<2, WRITE, true> : k_leaf_wide<2, WRITE, false>;
     return deep ? k_leaf_wide<0, WRITE, true> : k_leaf_wide<0, WRITE, false>;
+}
+template <int WRITE>
+static auto leaf_walk(const TreeBuffers& t) {
+    return t.apl == 4 ? k_leaf_walk<4, WRITE> : t.apl == 2 ? k_leaf_walk<2, WRITE> : k_leaf_walk<0, WRITE>;
+}
+
+// The ordered list's group boxes: in place of the build's CAS slots, which it has
+// no use for, or behind them where it may still build the tree.
+static size_t group_box_at(int32_t nL) {
+    return nL > kWalkLeaves ? (sizeof(int32_t) * (size_t)nL + 255) / 256 * 256 : 0;
+}
+
+// One pass (WRITE as in k_leaf_wide) over all query leaves.
+template <int WRITE>
+static void leaf_pass(Ctx* c, const TreeBuffers& t, float r, float r2, int64_t* counts,
+                      const int64_t* offsets, const int64_t* total, int64_t cap, int32_t* pi,
+                      int32_t* pj, float* pd) {
+    const float4* gbox = (const float4*)((const char*)c->store.p + group_box_at(t.nL));
+    if (t.walk) {
+        leaf_walk<WRITE>(t)<<<(unsigned)cdiv(t.nL, 128), 128, 0, c->stream>>>(
+            t.keys, t.pos4, t.nL, t.apl, r, r2, t.widest, counts, offsets, total, cap, pi, pj, pd,
+            c->d_err);
+        c->launches++;
+        if (t.nwide == 0) return;
+    }
+    const int32_t nq = t.walk ? t.nwide : t.nL;
+    const bool deep = t.walk || GroupLevels(t.nL).ns > kDirectSupers;
+    leaf_wide<WRITE>(t, deep)<<<(unsigned)cdiv(nq, 4), 128, 0, c->stream>>>(
+        t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), counts, offsets, total, cap, pi, pj,
+        pd, t.walk ? (const int32_t*)c->tasks.p : nullptr, nq);
+    c->launches++;
+}
+
+// Above kWalkLeaves leaves, where the search is bound by its warps' chains of
+// loads, a sample of query leaves says how many leaves overlap one (behind it),
+// and the walk is taken when the tests that makes are few: overlaps * width^2
+// below 80 at 262,144 leaves on the mean, in proportion to the leaves up to 160,
+// and below 1024 for every sampled leaf, as the longest walk sets the end (three
+// atoms a leaf fill a third of the search's lanes: two and a half times these).
+// The list of points at density 0.83, us, search and walk (overlaps): leaves of
+// four, 1,048,576 points r 0.4 705 and 542 (2.5), r 0.7 747 and 703 (5.5), r 1.3
+// 807 and 1005 (13); 4,194,304 points r 0.4 2453 and 1424, r 1.0 2749 and 2396 (9),
+// r 1.7 3051 and 3735 (17); leaves of two, 2,097,152 points r 0.4 1690 and 815
+// (1.0), r 1.7 2302 and 1946 (18), r 2.2 2536 and 2584 (32); leaves of eight,
+// 4,194,304 points r 0.05 1296 and 1269 (1.0), r 0.4 2008 and 3212 (4.4).  64
+// clusters of 32,768 points in all 2,097,152, leaves of four, r 0.2: 1471 and 4992
+// (3.1, the most 88).  131,072 leaves: 342 and 296 at r 0.05, about what the sample
+// takes.
+static bool sparse_leaves(const LeafSample& h, const TreeBuffers& t) {
+    const double tests = (double)t.apl * t.apl / (t.apl == 3 ? 2.5 : 1.0);
+    return tests * h.overlaps / kSampled < std::min(160.0, 80.0 * t.nL / 262144) &&
+           tests * h.most < 1024.0;
+}
+
+// Leaves that extend eight times as far as the mean leaf are left to the search
+// (evenly spread points have none: the widest of 16.8 million is 5.5 times the
+// mean), up to one leaf in 32.
+constexpr double kWidest = 8.0;
+
+// Whether the ordered list of t comes from rope walks (t.walk), and their tree.
+static nd_status choose_walk(Ctx* c, TreeBuffers& t, float r, const float4* gbox) {
+    if (t.nL <= kWalkLeaves || c->no_alloc) return ND_OK;
+    nd_status st = ensure(c, c->misc, 64);
+    if (st) return st;
+    LeafSample* ds = (LeafSample*)c->misc.p;
+    LeafSample h{};
+    auto read = [&](void* dst, size_t bytes) {
+        cudaError_t e = cudaMemcpyAsync(dst, c->misc.p, bytes, cudaMemcpyDeviceToHost, c->stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+    };
+    cudaMemsetAsync(ds, 0, sizeof(h), c->stream);
+    const bool deep = GroupLevels(t.nL).ns > kDirectSupers;
+    (deep ? k_overlap_sample<true> : k_overlap_sample<false>)<<<kSampled / 4, 128, 0, c->stream>>>(
+        t.keys, gbox, t.nL, ds);
+    k_leaf_extents<<<152 * 4, 256, 0, c->stream>>>(t.keys, t.nL, r, ds);
+    c->launches += 2;
+    cudaError_t e = read(&h, sizeof(h));
+    if (e != cudaSuccess) return cuda_fail(c, e, "leaf sample");
+    if (!sparse_leaves(h, t)) return ND_OK;
+    t.widest = (float)(kWidest * h.extents / t.nL);
+    t.nwide = 0;
+    if (h.widest > t.widest) {
+        const int32_t cap = t.nL / 32;
+        if ((st = ensure(c, c->tasks, sizeof(int32_t) * (size_t)cap))) return st;
+        unsigned long long n = 0;
+        cudaMemsetAsync(ds, 0, sizeof(n), c->stream);
+        k_wide_leaves<<<(unsigned)cdiv(t.nL, 256), 256, 0, c->stream>>>(
+            t.keys, t.nL, r, t.widest, cap, (int32_t*)c->tasks.p, (unsigned long long*)ds);
+        c->launches++;
+        if ((e = read(&n, sizeof(n))) != cudaSuccess) return cuda_fail(c, e, "wide leaves");
+        if (n > (unsigned long long)cap) return ND_OK;
+        t.nwide = (int32_t)n;
+    }
+    t.walk = true;
+    if (t.internal) return ND_OK;
+    t.internal = true;
+    return build_internal_nodes(c, t.keys, (int32_t*)c->store.p, t.codes, t.nL, t.apl);
 }
 
 // Ordered emission: per-query counts, their scan, then the pairs at their
 // places.  total_dev receives the number of pairs (device); the write pass
 // reads it and writes nothing when it exceeds the capacity, so no host round
 // trip lies between the two passes.
-nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
-                      int64_t* total_dev) {
+nd_status count_pairs(Ctx* c, TreeBuffers& t, float r, float r2, int kind, int64_t* total_dev) {
     nd_status st;
     int64_t nq = (kind == 0) ? t.nL : t.n;
     if ((st = ensure(c, c->counts, sizeof(int64_t) * (size_t)(nq + 1)))) return st;
@@ -1981,15 +2224,12 @@ nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
     int64_t* counts = (int64_t*)c->counts.p;
     int64_t* offsets = (int64_t*)c->offsets.p;
     if (kind == 0) {
-        // the group boxes take the place of the build's CAS slots, which the
-        // ordered emission has no more use for
-        if ((st = ensure(c, c->store, 32 * (size_t)GroupLevels(t.nL).boxes()))) return st;
-        float4* gbox = (float4*)c->store.p;
-        group_boxes(c, t.keys, t.nL, gbox);
-        leaf_wide<0>(t)<<<(unsigned)cdiv(t.nL, 4), 128, 0, c->stream>>>(
-            t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), counts, nullptr, nullptr, 0,
-            nullptr, nullptr, nullptr);
-        c->launches++;
+        const size_t at = group_box_at(t.nL);
+        if ((st = ensure(c, c->store, at + 32 * (size_t)GroupLevels(t.nL).boxes()))) return st;
+        float4* gbox = (float4*)((char*)c->store.p + at);
+        group_boxes(c, t.keys, t.nL, gbox, t.nL > kWalkLeaves);
+        if ((st = choose_walk(c, t, r, gbox))) return st;
+        leaf_pass<0>(c, t, r, r2, counts, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
     } else {
         k_atom_count<<<(unsigned)cdiv(nq, 128), 128, 0, c->stream>>>(t.keys, t.pos4, t.n, t.apl, r2,
                                                                      counts, c->d_err);
@@ -2003,15 +2243,12 @@ nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
                       const int64_t* total_dev, int64_t cap, int32_t* pi, int32_t* pj, float* pd) {
     const int64_t* offsets = (const int64_t*)c->offsets.p;
     if (kind == 0) {
-        const float4* gbox = (const float4*)c->store.p;
-        leaf_wide<1>(t)<<<(unsigned)cdiv(t.nL, 4), 128, 0, c->stream>>>(
-            t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), nullptr, offsets, total_dev,
-            cap, pi, pj, pd);
+        leaf_pass<1>(c, t, r, r2, nullptr, offsets, total_dev, cap, pi, pj, pd);
     } else {
         k_atom_write<<<(unsigned)cdiv(t.n, 128), 128, 0, c->stream>>>(
             t.keys, t.pos4, t.n, t.apl, r2, offsets, total_dev, cap, pi, pj, pd, c->d_err);
+        c->launches++;
     }
-    c->launches++;
     return check_launch(c, "pair write");
 }
 
@@ -2020,12 +2257,8 @@ nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
 // a second tree: 2.36 of 2.99 ms for 20,000 atoms (now 0.63 with the copies).
 nd_status write_pair_triples(Ctx* c, const TreeBuffers& t, float r, float r2,
                              const int64_t* total_dev, int64_t cap, int32_t* out) {
-    const int64_t* offsets = (const int64_t*)c->offsets.p;
-    const float4* gbox = (const float4*)c->store.p;
-    leaf_wide<2>(t)<<<(unsigned)cdiv(t.nL, 4), 128, 0, c->stream>>>(
-        t.keys, gbox, t.pos4, t.nL, t.apl, r, r2, gap_limit(r, r2), nullptr, offsets, total_dev, cap,
-        out, nullptr, nullptr);
-    c->launches++;
+    leaf_pass<2>(c, t, r, r2, nullptr, (const int64_t*)c->offsets.p, total_dev, cap, out, nullptr,
+                 nullptr);
     return check_launch(c, "pair write");
 }
 

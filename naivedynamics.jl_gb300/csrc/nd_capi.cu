@@ -234,7 +234,7 @@ static bool unordered_emission(const nd_bvh_spec* s, int32_t mode) {
     return mode == ND_PAIRS_UNORDERED && s->atomsperleaf == 4;
 }
 
-static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec* s,
+static nd_status pairs_from_tree(Ctx* c, TreeBuffers& t, const nd_bvh_spec* s,
                                  int32_t mode, int kind, bool host, int32_t* pi, int32_t* pj,
                                  float* pd, int64_t capacity, int64_t* count, int32_t criterion);
 
@@ -274,7 +274,7 @@ static int64_t list_capacity(const Ctx* c) {
 }
 
 // Pair emission over a built tree (the second half of pairs_common).
-static nd_status pairs_from_tree(Ctx* c, const TreeBuffers& t, const nd_bvh_spec* s,
+static nd_status pairs_from_tree(Ctx* c, TreeBuffers& t, const nd_bvh_spec* s,
                                  int32_t mode, int kind, bool host, int32_t* pi, int32_t* pj,
                                  float* pd, int64_t capacity, int64_t* count,
                                  int32_t criterion) {

@@ -229,6 +229,12 @@ struct TreeBuffers {
     const int32_t* idx = nullptr;    // sorted 1-based original index (n)
     float4* keys = nullptr;          // 2 float4 per node, nd_gridkey layout (nkeys)
     int64_t nkeys = 0;
+    bool internal = false;  // the internal nodes are built
+    // the ordered leaf list (count_pairs decides): by rope walks, but for nwide leaves
+    // (listed in Ctx::tasks) whose atoms extend further than `widest`
+    bool walk = false;
+    int32_t nwide = 0;
+    float widest = 0.0f;
 };
 
 // Morton codes of n float3 positions (device, AoS) into codes + iota values.
@@ -329,8 +335,7 @@ nd_status collect_objects(Ctx* c, const nd_collector* cl, uint64_t seed, float* 
 // simulate! as written over the all-pairs list (host arrays in and out).
 nd_status compat_simulate(Ctx* c, const nd_compat_sim* spec, int32_t n, float* x, float* v,
                           float* force, const float* mass, const float* q, float* poslog);
-nd_status count_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
-                      int64_t* total_dev);
+nd_status count_pairs(Ctx* c, TreeBuffers& t, float r, float r2, int kind, int64_t* total_dev);
 nd_status write_pairs(Ctx* c, const TreeBuffers& t, float r, float r2, int kind,
                       const int64_t* total_dev, int64_t cap, int32_t* pi, int32_t* pj, float* pd);
 // The leaf path's pairs as (i, j, d) triples of words.

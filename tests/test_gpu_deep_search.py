@@ -10,24 +10,30 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("leaves,apl", [(262144, 2), (262145, 2), (262144 + 33, 4), (266241, 3),
                                         (2**20 + 32 * 32 + 1, 2)])
 def test_order_and_pairs(nd, leaves, apl):
+    check_list(nd, leaves, apl, 1.1)
+
+
+def check_list(nd, leaves, apl, r):
+    """The device list of leaves * apl points at density 0.52; its length."""
     import torch
-    n, r, side = leaves * apl, 1.1, 100.0 * (leaves * apl / 524288) ** (1 / 3)
+    n, side = leaves * apl, 100.0 * (leaves * apl / 524288) ** (1 / 3)
     x = nd.synth.uniform_positions(leaves, n, side)
     spec = nd.SpheresBVHSpecs(r, n, apl)
     ctx = nd.Context()
     dev = torch.device("cuda")
     xd = torch.from_numpy(x).to(dev)
-    cap = 4 * n
+    cap = int((2 * r**3 + 1) * n)
     out = [torch.empty(cap, dtype=t, device=dev) for t in (torch.int32, torch.int32, torch.float32)]
 
     def listed(mode):
         torch.cuda.synchronize()
         st, k = nd.neighbor_pairs_dev(xd, spec, *out, cap, order=nd.ND_ORDER_SPATIAL, mode=mode,
                                       ctx=ctx)
-        assert st == 0 and k > n
+        assert st == 0 and k > 0
         return k, nd.pair_hash_dev(*out, k, ctx=ctx)
 
     k, h = listed(nd.ND_PAIRS_ORDERED)
+    first = {f: o[:k].cpu().numpy() for f, o in zip(("i", "j", "d"), out)}
     # query leaf, target leaf, atom of the one, atom of the other, each outer to
     # the next: increasing from entry to entry
     _, pos, _, _ = nd.leafTreeData(x, spec, order=nd.ND_ORDER_SPATIAL, ctx=ctx)
@@ -47,3 +53,7 @@ def test_order_and_pairs(nd, leaves, apl):
     w = [torch.from_numpy(np.ascontiguousarray(p[f])).to(dev) for f in ("i", "j", "d")]
     torch.cuda.synchronize()
     assert nd.pair_hash_dev(*w, k, ctx=ctx) == h
+    entries = nd.leafbuild_traverse_bvh(x, spec, order=nd.ND_ORDER_SPATIAL, ctx=ctx)
+    for f in first:
+        assert np.array_equal(np.ascontiguousarray(entries[f]), first[f])
+    return k
