@@ -212,7 +212,8 @@ SIGNATURES = {
     "nd_synth_charges": (_i32, [_u64, _i32, _vp]),
 }
 
-_lock = threading.Lock()
+# (re-entrant: the garbage collector may close a Context in the thread that holds it)
+_lock = threading.RLock()
 _lib = None
 
 
@@ -319,5 +320,5 @@ def default_context(device: int = 0) -> Context:
     if c is None:
         c = Context(device)
         with _lock:
-            _default[device] = c
+            c = _default.setdefault(device, c)
     return c
