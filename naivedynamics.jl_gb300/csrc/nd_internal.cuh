@@ -189,8 +189,11 @@ struct Ctx {
 // kernel is resident.  (4,096 atoms, a check after every step:
 // 16.3 -> 15.5 us a step; chaining the steps to each other or a rebuild's own
 // kernels gained nothing, steps lost 0.8 us.)
-__device__ __forceinline__ void chain_wait() {
+__device__ __forceinline__ void chain_open() {  // lets the next kernel's blocks in
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chain_wait() {
+    chain_open();
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... P, class... A>

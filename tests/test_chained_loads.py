@@ -44,6 +44,18 @@ def test_no_read_only_loads_of_what_the_chain_writes(name):
         assert set(const) <= STATIC, set(const) - STATIC
 
 
+def test_steps_read_only_loads_follow_the_chaining():
+    # the step kernel's loads go through step_ld, read-only where the step does not
+    # wait inside the chain; the host chains exactly those that do
+    src = open(os.path.join(PKG, "csrc", "nd_md.cu")).read()
+    head, body = KERNELS["k_md_step"]
+    assert "constexpr bool CHAIN = kStepChained<TPA>;" in body
+    assert "if constexpr (MODE == 0 && CHAIN) chain_wait();" in body
+    assert set(re.findall(r"step_ld<(\w+)>", body)) == {"CHAIN"}
+    assert "constexpr bool kStepChained = TPA > 1;" in src
+    assert "chained = MODE == 0 && m->gated && m->nsys == 0 && m->tpa > 1;" in src
+
+
 def test_step_arguments():
     text = open(os.path.join(PKG, "csrc", "nd_md_engine.cuh")).read()
     args = text[text.index("struct StepArgs"):text.index("struct MDEngine")]
