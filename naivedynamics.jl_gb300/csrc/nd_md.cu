@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstring>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "nd_md_engine.cuh"
@@ -2972,24 +2973,16 @@ nd_status md_autotune(Ctx* parent, const nd_md_params* p, int32_t n, int32_t nsy
         if (nsys == 0) {
             const nd_md_params s6 = win;
             double tbest = -1.0;
-            for (int32_t t : {1, 2, kSmallTPA}) {
+            // with 4 threads per atom also the thread blocks per block of atoms
+            // (each pair for itself: 2 threads can be faster than 4 in one thread
+            // block and slower than 4 in four)
+            for (auto [t, sp] : {std::pair{1, 1}, {2, 1}, {kSmallTPA, 1}, {kSmallTPA, 2}, {kSmallTPA, 4}}) {
                 c = s6;
                 c.threads_per_atom = t;
-                c.cta_split = 1;
+                c.cta_split = sp;
                 double tt = -1.0;
                 if ((result = trial(c, &tt))) goto done;
                 if (tt > 0.0 && (tbest < 0.0 || tt < tbest)) { tbest = tt; win = c; }
-            }
-            // with 4 threads per atom, the thread blocks per block of atoms
-            if (win.threads_per_atom == kSmallTPA) {
-                const nd_md_params s7 = win;
-                for (int32_t sp : {2, 4}) {
-                    c = s7;
-                    c.cta_split = sp;
-                    double tt = -1.0;
-                    if ((result = trial(c, &tt))) goto done;
-                    if (tt > 0.0 && (tbest < 0.0 || tt < tbest)) { tbest = tt; win = c; }
-                }
             }
             if (tbest > 0.0) best_t = tbest;
         }
