@@ -253,7 +253,8 @@ nd_status pairs_common(Ctx* c, const nd_bvh_spec* s, int32_t order, int32_t mode
     const int32_t boxes = (kind == 0) ? ND_BOX_LEAF : ND_BOX_ATOM;
     if (kind == 0 && n - 1 < 2 * nL - 1) return ND_ERR_SPEC;  // leafTreeData needs apl >= 2
     TreeBuffers t;
-    // only the allocation-free unordered walk follows the tree's ropes
+    // only the allocation-free unordered walk follows the tree's ropes (and sparse
+    // ordered lists, for which count_pairs builds it)
     const bool leaves_only = kind == 0 && !(c->no_alloc && unordered_emission(s, mode));
     if (host) {
         st = tree_from_host(c, xyz, s, order, boxes, 2LL * nL - 1, false, &t, leaves_only);

@@ -253,7 +253,7 @@ nd_status order_positions(Ctx* c, const float* xyz, int32_t n, int32_t order, in
                           int32_t* perm, const float* frame = nullptr);
 size_t sort_scratch_bytes(int32_t n);
 // Full tree pipeline: codes -> sort -> gather -> leaf boxes -> Apetrei build
-// (leaves_only: no internal nodes, all the leaf pair lists need).
+// (leaves_only: no internal nodes, which the leaf pair lists mostly do without).
 nd_status build_tree(Ctx* c, const float* xyz_dev, int32_t n, float r, int32_t apl,
                      int32_t order, int32_t boxes, int64_t nkeys, bool overwrite_root,
                      TreeBuffers* out, bool leaves_only = false);
